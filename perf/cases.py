@@ -47,27 +47,27 @@ MORE_TOKENS = {"decode": 4096, "mixed": 4096}  # positions a live request may gr
 def listed() -> list[dict]:
     return [
         # one user's next token on the smallest shape: launches and latency
-        _case("one token, 0.5B", "qwen2-0.5b", "decode", requests=1, context=512),
+        _case("one token 0.5B", "qwen2-0.5b", "decode", requests=1, context=512),
         # a short exact-mode run: the float32 path answers ragged prompts (it is what replays and comparisons use)
-        _case("float32 prompts, 0.5B", "qwen2-0.5b", "prompt", dtype="float32", requests=3, tokens=210),
+        _case("float32 prompts 0.5B", "qwen2-0.5b", "prompt", dtype="float32", requests=3, tokens=210),
         # a small batch job from prompts to sampled ids: the whole loop with its host side
-        _case("generate, 0.5B", "qwen2-0.5b-untied", "generate", requests=8, tokens=48, new=16),
+        _case("generate 0.5B", "qwen2-0.5b-untied", "generate", requests=8, tokens=48, new=16),
         # a server's steady state: eight conversations of the headline shape
-        _case("decode 8, 7B", "qwen2-7b", "decode", requests=8, context=2048),
+        _case("decode 8 7B", "qwen2-7b", "decode", requests=8, context=2048),
         # the same server under load
-        _case("decode 64, 7B", "qwen2-7b", "decode", requests=64, context=512, page_size=64),
+        _case("decode 64 7B", "qwen2-7b", "decode", requests=64, context=512, page_size=64),
         # time to first token of a long prompt on the headline shape: the largest case
-        _case("prompt 2048, 7B", "qwen2-7b", "prompt", requests=1, tokens=2048),
+        _case("prompt 2048 7B", "qwen2-7b", "prompt", requests=1, tokens=2048),
         # prompts of each hybrid design: delta rule and state space; retention, selective scan and experts with two prompts in the
         # step; attention over latents and time mixing at an odd length; lightning, channel decay, gates and experts
-        _case("prompt, Nunivik", "nunivik-2k", "prompt", requests=1, tokens=2048),
-        _case("two prompts, Mirovik", "mirovik-2k", "prompt", requests=2, tokens=1400),
-        _case("odd prompt, Kudazen", "kudazen-2k", "prompt", requests=1, tokens=1531, page_size=32),
-        _case("prompt, Tobadra", "tobadra-2k", "prompt", requests=1, tokens=2048),
+        _case("prompt Nunivik", "nunivik-2k", "prompt", requests=1, tokens=2048),
+        _case("two prompts Mirovik", "mirovik-2k", "prompt", requests=2, tokens=1400),
+        _case("odd prompt Kudazen", "kudazen-2k", "prompt", requests=1, tokens=1531, page_size=32),
+        _case("prompt Tobadra", "tobadra-2k", "prompt", requests=1, tokens=2048),
         # routed experts fetch most of their matrices for a handful of tokens
-        _case("decode 16, Zurevik", "zurevik-2k", "decode", requests=16, context=1500),
+        _case("decode 16 Zurevik", "zurevik-2k", "decode", requests=16, context=1500),
         # a new prompt joins conversations that go on
-        _case("mixed step, Biropel", "biropel-2k", "mixed", requests=7, context=900, tokens=1000),
+        _case("mixed step Biropel", "biropel-2k", "mixed", requests=7, context=900, tokens=1000),
     ]
 
 
