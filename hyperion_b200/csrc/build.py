@@ -130,7 +130,7 @@ def build_many(requests: Iterable[tuple[str, Mapping[str, object]]], workers: in
     for module, defines in requests:
         defines = dict(defines or {})
         tag = _tag(module, defines)
-        if tag in seen:
+        if tag in seen or tag in _loaded:  # a loaded library is what load() gives, whatever has become of its source
             continue
         seen.add(tag)
         target = library_path(module, defines)

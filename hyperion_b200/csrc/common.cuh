@@ -27,6 +27,7 @@ enum : int {
     HB_STATUS_IN_ATTENTION_TMA_TILES = 0x400,
     HB_STATUS_IN_ATTENTION_TMA_TOKENS = 0x800,
     HB_STATUS_IN_ATTENTION_TCGEN05 = 0x1000,
+    HB_STATUS_IN_CHUNKED_WALK = 0x2000,
 };
 
 __device__ __forceinline__ float to_float(float v) { return v; }

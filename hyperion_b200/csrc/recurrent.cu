@@ -151,6 +151,7 @@ struct ScanArgs {
     float q_scale;
     int values;          // value columns of a head (0: e); a column from there on takes the constant 1
     int out_e;           // columns of a head in `out` (0: e)
+    int below;           // rows of this many tokens or more are left alone (0: none is)
 };
 
 template <int NG, int LPC, int CPT, int MODE>  // NG groups of four entries per lane, LPC lanes per column (n <= NG * 4 * LPC), CPT columns per thread
@@ -175,6 +176,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) state_scan_kernel(const ScanArgs
     const int l = lane % LPC, cw = warp * (32 / LPC) + lane / LPC;  // this thread's columns: col0 + cw + GROUPS * c
     const int col0 = blockIdx.x * COLUMNS;
     const int t0 = a.row_start[row], t1 = a.row_start[row + 1];
+    if (a.below && t1 - t0 >= a.below) return;
     const int group = head / (a.heads / a.groups);
     float* const head_state = a.state + (size_t)a.slots[row] * a.slot_stride + a.state_off + (size_t)head * a.e * a.n_padded;
 
@@ -584,15 +586,16 @@ HB_EXPORT int hb_conv_state_update(const float* x, int x_stride, int col0, int c
 // mode 0: gated delta rule (keys and queries made unit vectors, q times q_scale; decay = exp(-exp(a_log) softplus(proj[decay_off] + dt_bias)),
 // step = sigmoid(proj[step_off])).  mode 1: state space (step = softplus(proj[decay_off] + dt_bias), decay = exp(-exp(a_log) step), skip = D).
 // The state of (slot, head) is S^T [e, n_padded] at state + slot * slot_stride + state_off; n_padded, state_off and slot_stride are multiples of 4.
+// below > 0: rows of that many tokens or more are left alone, outputs and all (chunked_float.cu takes them).
 HB_EXPORT int hb_state_scan(int mode, const float* conv, int conv_stride, int k_off, int q_off, int v_off, const float* proj, int proj_stride,
                             int decay_off, int step_off, const float* a_log, const float* dt_bias, const float* skip, float* state,
                             long long slot_stride, int state_off, const int* slots, const int* row_start, float* out, int rows, int heads,
-                            int groups, int n, int n_padded, int e, float q_scale, cudaStream_t stream) {
+                            int groups, int n, int n_padded, int e, float q_scale, int below, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (n <= 0 || n > 256 || e <= 0 || heads <= 0 || groups <= 0 || heads % groups || rows > 65535 || heads > 65535) return HB_UNSUPPORTED_SIZE;
     if (n_padded < n || (n_padded & 3) || (state_off & 3) || (slot_stride & 3) || (((uintptr_t)state) & 15)) return HB_BAD_ARGUMENT;
     ScanArgs a{conv + k_off, conv + q_off, conv + v_off, conv_stride, conv_stride, conv_stride, proj, proj_stride, decay_off, step_off, proj, proj_stride, a_log, dt_bias, skip,
-               state, (size_t)slot_stride, state_off, slots, row_start, out, heads, groups, n, n_padded, e, q_scale};
+               state, (size_t)slot_stride, state_off, slots, row_start, out, heads, groups, n, n_padded, e, q_scale, 0, 0, below};
     if (mode == MODE_DELTA) return launch_scan<MODE_DELTA>(a, rows, stream);
     if (mode == MODE_STATE_SPACE) return launch_scan<MODE_STATE_SPACE>(a, rows, stream);
     if (mode == MODE_RETENTION) return launch_scan<MODE_RETENTION>(a, rows, stream);
@@ -605,12 +608,12 @@ HB_EXPORT int hb_state_scan(int mode, const float* conv, int conv_stride, int k_
 HB_EXPORT int hb_channel_delta_scan(const float* conv, int conv_stride, int k_off, int q_off, int v_off, const float* decay, int decay_stride, int decay_off,
                                     const float* step, int step_stride, int step_off, const float* a_log, const float* dt_bias, float* state,
                                     long long slot_stride, int state_off, const int* slots, const int* row_start, float* out, int rows, int heads,
-                                    int groups, int n, int n_padded, int e, float q_scale, cudaStream_t stream) {
+                                    int groups, int n, int n_padded, int e, float q_scale, int below, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (n <= 0 || n > 256 || e <= 0 || heads <= 0 || groups <= 0 || heads % groups || rows > 65535 || heads > 65535) return HB_UNSUPPORTED_SIZE;
     if (n_padded < n || (n_padded & 3) || (state_off & 3) || (slot_stride & 3) || (((uintptr_t)state) & 15) || !a_log || !dt_bias) return HB_BAD_ARGUMENT;
     ScanArgs a{conv + k_off, conv + q_off, conv + v_off, conv_stride, conv_stride, conv_stride, decay, decay_stride, decay_off, step_off, step, step_stride,
-               a_log, dt_bias, nullptr, state, (size_t)slot_stride, state_off, slots, row_start, out, heads, groups, n, n_padded, e, q_scale};
+               a_log, dt_bias, nullptr, state, (size_t)slot_stride, state_off, slots, row_start, out, heads, groups, n, n_padded, e, q_scale, 0, 0, below};
     return launch_scan<MODE_CHANNEL_DELTA>(a, rows, stream);
 }
 
@@ -618,12 +621,12 @@ HB_EXPORT int hb_channel_delta_scan(const float* conv, int conv_stride, int k_of
 // decays' pre-activations x [tokens, heads * n] (w = exp(-exp(x + w0))), w0 and the bonus u [heads * n].  The state as in hb_state_scan.
 HB_EXPORT int hb_wkv_scan(const float* k, int k_stride, const float* q, int q_stride, const float* v, int v_stride, const float* x, int x_stride, int x_off,
                           const float* w0, const float* bonus, float* state, long long slot_stride, int state_off, const int* slots, const int* row_start,
-                          float* out, int rows, int heads, int n, int n_padded, int e, cudaStream_t stream) {
+                          float* out, int rows, int heads, int n, int n_padded, int e, int below, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (n <= 0 || n > 256 || e <= 0 || heads <= 0 || rows > 65535 || heads > 65535) return HB_UNSUPPORTED_SIZE;
     if (n_padded < n || (n_padded & 3) || (state_off & 3) || (slot_stride & 3) || (((uintptr_t)state) & 15) || !w0 || !bonus) return HB_BAD_ARGUMENT;
     ScanArgs a{k, q, v, k_stride, q_stride, v_stride, x, x_stride, x_off, 0, x, x_stride, w0, bonus, nullptr, state, (size_t)slot_stride, state_off, slots, row_start, out,
-               heads, heads, n, n_padded, e, 1.f};
+               heads, heads, n, n_padded, e, 1.f, 0, 0, below};
     return launch_scan<MODE_WKV>(a, rows, stream);
 }
 

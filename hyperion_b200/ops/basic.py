@@ -11,7 +11,7 @@ _STATUS: dict[int, torch.Tensor] = {}
 STATUS_BITS = {1: "a block-table entry that had to be valid was missing", 2: "a token id outside the vocabulary",
                4: "a position beyond the position table", 8: "a bounded wait inside a kernel ran out",
                0x100: "(in the tile-shaped GEMM)", 0x200: "(in the swapped GEMM)", 0x400: "(in the TMA attention, tile shape)",
-               0x800: "(in the TMA attention, token shape)", 0x1000: "(in the tcgen05 attention)"}
+               0x800: "(in the TMA attention, token shape)", 0x1000: "(in the tcgen05 attention)", 0x2000: "(in the walk through chunks)"}
 
 
 def status_word(device: torch.device) -> torch.Tensor:

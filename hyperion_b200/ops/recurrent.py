@@ -8,7 +8,8 @@ import ctypes
 
 import torch
 
-from .native import KernelError, check, f32, i32, is_bf16, library, ptr, require_cuda, stream_ptr
+from .basic import status_word
+from .native import LAUNCHES, KernelError, check, f32, i32, is_bf16, library, ptr, require_cuda, sm_count, stream_ptr
 
 MODE_DELTA, MODE_STATE_SPACE, MODE_RETENTION = 0, 1, 2
 
@@ -78,19 +79,28 @@ def silu_columns_(x: torch.Tensor, col0: int, columns: int) -> None:
     check(library("recurrent").hb_silu_columns(ptr(x), i32(x.stride(0)), i32(col0), i32(columns), i32(x.shape[0]), stream_ptr()), "silu_columns")
 
 
+def _rows_for(out: torch.Tensor | None, tokens: int, columns: int, device) -> torch.Tensor:
+    if out is None:
+        return torch.empty((tokens, columns), dtype=torch.float32, device=device)
+    if out.dtype != torch.float32 or out.shape != (tokens, columns) or not out.is_contiguous():
+        raise KernelError("a scan's results are a dense float matrix of [tokens, heads * e]")
+    return out
+
+
 def state_scan(mode: int, conv: torch.Tensor, k_off: int, q_off: int, v_off: int, proj: torch.Tensor, decay_off: int, step_off: int,
                a_log: torch.Tensor, dt_bias: torch.Tensor, skip: torch.Tensor | None, state: torch.Tensor, state_off: int, slots: torch.Tensor,
                row_start: torch.Tensor, rows: int, heads: int, groups: int, n: int, n_padded: int, e: int, q_scale: float = 1.0,
-               states_only: bool = False) -> torch.Tensor | None:
+               states_only: bool = False, below: int = 0, out: torch.Tensor | None = None) -> torch.Tensor | None:
     """Walk every row's tokens through the recurrence of ``mode`` from and into its slot of ``state``; returns [tokens, heads * e]
-    (nothing with ``states_only``: the walk then only leaves the rows' states)."""
-    require_cuda(conv, proj, a_log, dt_bias, skip, state, slots, row_start)
+    (nothing with ``states_only``: the walk then only leaves the rows' states).  ``below`` > 0: rows of that many tokens or more are left
+    alone; ``out`` then holds what others have written for them."""
+    require_cuda(conv, proj, a_log, dt_bias, skip, state, slots, row_start, out)
     _floats(conv, proj, a_log, dt_bias, skip, state)
-    out = None if states_only else torch.empty((conv.shape[0], heads * e), dtype=torch.float32, device=conv.device)
+    out = None if states_only else _rows_for(out, conv.shape[0], heads * e, conv.device)
     check(library("recurrent").hb_state_scan(i32(mode), ptr(conv), i32(conv.stride(0)), i32(k_off), i32(q_off), i32(v_off), ptr(proj), i32(proj.stride(0)),
                                              i32(decay_off), i32(step_off), ptr(a_log), ptr(dt_bias), ptr(skip), ptr(state),
                                              ctypes.c_longlong(state.stride(0)), i32(state_off), ptr(slots), ptr(row_start), ptr(out), i32(rows),
-                                             i32(heads), i32(groups), i32(n), i32(n_padded), i32(e), f32(q_scale), stream_ptr()), "state_scan")
+                                             i32(heads), i32(groups), i32(n), i32(n_padded), i32(e), f32(q_scale), i32(below), stream_ptr()), "state_scan")
     return out
 
 
@@ -144,38 +154,40 @@ def matrix_memory_norm(y: torch.Tensor, gates: torch.Tensor, gate: torch.Tensor,
 
 def channel_delta_scan(conv: torch.Tensor, k_off: int, q_off: int, v_off: int, decay: torch.Tensor, step: torch.Tensor, step_off: int, a_log: torch.Tensor,
                        dt_bias: torch.Tensor, state: torch.Tensor, state_off: int, slots: torch.Tensor, row_start: torch.Tensor, rows: int, heads: int, groups: int,
-                       n: int, n_padded: int, e: int, q_scale: float = 1.0) -> torch.Tensor:
+                       n: int, n_padded: int, e: int, q_scale: float = 1.0, below: int = 0, out: torch.Tensor | None = None) -> torch.Tensor:
     """The gated delta rule with a decay per head and key entry, per head:  S <- diag(g) S;  u = b (v - S^T k);  S <- S + k u^T;  o = S^T q  with
     g_i = exp(-exp(a_log) softplus(decay_i + dt_bias_i)), b = sigmoid(step), k and q made unit vectors and q times ``q_scale``.  ``conv``
     [tokens, *] holds keys, queries and values at their offsets, ``decay`` [tokens, heads * n] the decays' pre-activations, ``step`` [tokens, *]
     the steps' at ``step_off``; ``a_log`` has one entry per head, ``dt_bias`` one per head and key entry.  Every row's tokens walk from
-    and into its slot of ``state``.  Returns [tokens, heads * e]."""
-    require_cuda(conv, decay, step, a_log, dt_bias, state, slots, row_start)
+    and into its slot of ``state``.  Returns [tokens, heads * e].  ``below`` and ``out`` as in :func:`state_scan`."""
+    require_cuda(conv, decay, step, a_log, dt_bias, state, slots, row_start, out)
     _floats(conv, decay, step, a_log, dt_bias, state)
     if a_log.numel() != heads or dt_bias.numel() != heads * n or decay.shape[1] != heads * n or not a_log.is_contiguous() or not dt_bias.is_contiguous():
         raise KernelError("channel_delta_scan: a rate per head, a bias and a pre-activation per head and key entry")
-    out = torch.empty((conv.shape[0], heads * e), dtype=torch.float32, device=conv.device)
+    out = _rows_for(out, conv.shape[0], heads * e, conv.device)
     check(library("recurrent").hb_channel_delta_scan(ptr(conv), i32(conv.stride(0)), i32(k_off), i32(q_off), i32(v_off), ptr(decay), i32(decay.stride(0)), i32(0),
                                                      ptr(step), i32(step.stride(0)), i32(step_off), ptr(a_log), ptr(dt_bias), ptr(state),
                                                      ctypes.c_longlong(state.stride(0)), i32(state_off), ptr(slots), ptr(row_start), ptr(out), i32(rows), i32(heads),
-                                                     i32(groups), i32(n), i32(n_padded), i32(e), f32(q_scale), stream_ptr()), "channel_delta_scan")
+                                                     i32(groups), i32(n), i32(n_padded), i32(e), f32(q_scale), i32(below), stream_ptr()), "channel_delta_scan")
     return out
 
 
 def wkv_scan(k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, x: torch.Tensor, x_off: int, w0: torch.Tensor, bonus: torch.Tensor, state: torch.Tensor,
-             state_off: int, slots: torch.Tensor, row_start: torch.Tensor, rows: int, heads: int, n: int, n_padded: int, e: int) -> torch.Tensor:
+             state_off: int, slots: torch.Tensor, row_start: torch.Tensor, rows: int, heads: int, n: int, n_padded: int, e: int, below: int = 0,
+             out: torch.Tensor | None = None) -> torch.Tensor:
     """The recurrence with a decay per key entry computed from the token and a bonus for the current token, per head:
     o = S^T q + (sum_i u_i k_i q_i) v;  S <- diag(w) S + k v^T  with w = exp(-exp(x + w0)).  ``k``, ``q`` [tokens, heads * n] and ``v``
     [tokens, heads * e] are float matrices of their own, ``x`` [tokens, *] holds the decays' pre-activations at column ``x_off``,
-    ``w0`` and ``bonus`` have heads * n entries.  Every row's tokens walk from and into its slot of ``state``.  Returns [tokens, heads * e]."""
-    require_cuda(k, q, v, x, w0, bonus, state, slots, row_start)
+    ``w0`` and ``bonus`` have heads * n entries.  Every row's tokens walk from and into its slot of ``state``.  Returns [tokens, heads * e].
+    ``below`` and ``out`` as in :func:`state_scan`."""
+    require_cuda(k, q, v, x, w0, bonus, state, slots, row_start, out)
     _floats(k, q, v, x, w0, bonus, state)
     if w0.numel() != heads * n or bonus.numel() != heads * n or not w0.is_contiguous() or not bonus.is_contiguous():
         raise KernelError("wkv_scan: the decay offset and the bonus have an entry per head and key entry")
-    out = torch.empty((k.shape[0], heads * e), dtype=torch.float32, device=k.device)
+    out = _rows_for(out, k.shape[0], heads * e, k.device)
     check(library("recurrent").hb_wkv_scan(ptr(k), i32(k.stride(0)), ptr(q), i32(q.stride(0)), ptr(v), i32(v.stride(0)), ptr(x), i32(x.stride(0)), i32(x_off),
                                            ptr(w0), ptr(bonus), ptr(state), ctypes.c_longlong(state.stride(0)), i32(state_off), ptr(slots), ptr(row_start),
-                                           ptr(out), i32(rows), i32(heads), i32(n), i32(n_padded), i32(e), stream_ptr()), "wkv_scan")
+                                           ptr(out), i32(rows), i32(heads), i32(n), i32(n_padded), i32(e), i32(below), stream_ptr()), "wkv_scan")
     return out
 
 
@@ -329,6 +341,79 @@ def chunk_planner(dtype: torch.dtype) -> dict:
             packer.add("scan_chunk_row", cut[1])
 
     return {("scan_chunks", CHUNK): plan}
+
+
+RULE_DELTA, RULE_CHANNEL_DELTA, RULE_RETENTION, RULE_WKV = 0, 1, 2, 3
+SCRATCH_BYTES = 160 << 20  # of chunked_rule: longer steps take it in turns
+# In a step with a long row, rows of fewer tokens go token by token after it: a decoded token in a chunk of its own costs what 64 tokens do (300 tokens and 40
+# decoded ones at 16 heads of 128 x 128: 261 us all in chunks, 200 us all token by token)
+CHUNKED_RULE_ROWS = 16
+
+
+def plan_rule_chunks(counts) -> tuple[list[int], list[int], bool] | None:
+    """What :func:`chunked_rule` takes of a step: (first token and number of tokens of every chunk; the chunks of every row that is walked, from and up to, and the
+    row; whether other rows are left), or None when no row is long enough for the chunked form to pay."""
+    if max(counts) < CHUNKED_FROM:
+        return None
+    chunks, walks, at = [], [], 0
+    for row, count in enumerate(counts):
+        if count >= CHUNKED_RULE_ROWS:
+            begun = len(chunks) // 2
+            for first in range(0, int(count), CHUNK):
+                chunks += [at + first, min(CHUNK, int(count) - first)]
+            walks += [begun, len(chunks) // 2, row]
+        at += int(count)
+    return chunks, walks, len(walks) < 3 * len(counts)
+
+
+def rule_planner(dtype: torch.dtype) -> dict:
+    """The step planner of mixers that walk long rows with :func:`chunked_rule`: in bfloat16, a step with a long row gets ``rule_chunks`` and ``rule_walks`` among its
+    arrays and (chunks, walks, whether other rows are left) in ``step.host["rule_chunks"]`` (None otherwise)."""
+    if dtype != torch.bfloat16:
+        return {}
+
+    def plan(rows, packer, host):
+        if "rule_chunks" in host:
+            return
+        counts = rows.counts if hasattr(rows, "counts") else [row.count for row in rows]
+        cut = plan_rule_chunks([int(c) for c in counts])
+        host["rule_chunks"] = None if cut is None else (len(cut[0]) // 2, len(cut[1]) // 3, cut[2])
+        if cut is not None:
+            packer.add("rule_chunks", cut[0])
+            packer.add("rule_walks", cut[1])
+
+    return {("rule_chunks", CHUNK): plan}
+
+
+def chunked_rule_fits(n: int, e: int) -> bool:
+    """Whether :func:`chunked_rule` takes heads of this size; others walk token by token."""
+    return 0 < n <= 128 and e > 0 and e % 16 == 0
+
+
+def chunked_rule(rule: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, x: torch.Tensor | None, x_off: int, step: torch.Tensor | None, step_off: int, rate: torch.Tensor,
+                 bias: torch.Tensor | None, state: torch.Tensor, state_off: int, slots: torch.Tensor, table: torch.Tensor, chunks: int, walk_table: torch.Tensor, walks: int,
+                 heads: int, groups: int, n: int, n_padded: int, e: int, q_scale: float = 1.0) -> torch.Tensor:
+    """The recurrences of :func:`state_scan` (delta rule, retention), :func:`channel_delta_scan` and :func:`wkv_scan` over the chunks of a step (:func:`plan_rule_chunks`), at float
+    precision; tokens of other rows get nothing.  ``k``, ``q`` (group g at g * n), ``v`` (head h at h * e) are float views [tokens, *]; ``x`` at ``x_off`` holds the decays' pre-activations and ``step`` at
+    ``step_off`` the delta rules' steps'; ``rate`` and ``bias`` are a_log and dt_bias, or the decays and nothing (retention), or w0 and the bonus (wkv).  Returns [tokens, heads * e]."""
+    require_cuda(k, q, v, x, step, rate, bias, state, slots, table, walk_table)
+    _floats(k, q, v, x, step, rate, bias, state)
+    entries = heads * n if rule in (RULE_CHANNEL_DELTA, RULE_WKV) else heads
+    if not rate.is_contiguous() or rate.numel() != (entries if rule == RULE_WKV else heads) or (bias is not None and (not bias.is_contiguous() or bias.numel() != entries)):
+        raise KernelError("chunked_rule: a rate and a bias per head, or per head and key entry")
+    native = library("chunked_float")
+    native.hb_chunked_float_scratch.restype = ctypes.c_longlong
+    piece = native.hb_chunked_float_scratch(i32(rule), i32(n), i32(e)) * heads
+    span = max(1, min(chunks, SCRATCH_BYTES // (4 * piece))) if piece else 1
+    scratch = torch.empty(max(1, span * piece), dtype=torch.float32, device=k.device)
+    out = torch.empty((k.shape[0], heads * e), dtype=torch.float32, device=k.device)
+    stride = lambda t: i32(t.stride(0) if t is not None else 0)  # noqa: E731
+    check(native.hb_chunked_float(i32(rule), ptr(k), stride(k), ptr(q), stride(q), ptr(v), stride(v), ptr(x), stride(x), i32(x_off), ptr(step), stride(step), i32(step_off), ptr(rate),
+                                  ptr(bias), ptr(scratch), ptr(state), ctypes.c_longlong(state.stride(0)), i32(state_off), ptr(slots), ptr(table), i32(chunks), ptr(walk_table),
+                                  i32(walks), i32(span), ptr(out), i32(heads), i32(groups), i32(n), i32(n_padded), i32(e), f32(q_scale), i32(sm_count(k.device)), ptr(status_word(k.device)), stream_ptr()),
+          "chunked_rule")
+    LAUNCHES[0] += 2 * -(-chunks // span) - 1  # two kernels per span
+    return out
 
 
 def chunked_scan(kind: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, decay_off: int, step_off: int, state: torch.Tensor, state_off: int,

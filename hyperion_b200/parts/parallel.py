@@ -46,6 +46,7 @@ from .attention import GroupedQueryAttention
 from .base import MIXERS, POSITIONS, BuildContext, Mixer, PagedTokens, RequestState, WeightSpec, make, register_mixer
 from .branch import Branch, common_dtype
 from .norm import NormedSum
+from .recurrent import ConstantDecay
 from .spec import PartSpec
 
 
@@ -140,7 +141,7 @@ class BiasedAttention(Branch):
                               cache.page_size, self.scale, distance_bias=self.by_distance, gate=proj, gate_off=v_off + self.v_width, out_scale=scale, out=out)
 
 
-class Retention(Branch):
+class Retention(Branch, ConstantDecay):
     in_names = ("q", "k", "v", "g")
     out_name = "o"
 
@@ -174,27 +175,17 @@ class Retention(Branch):
         return RequestState((self.record,), torch.float32)
 
     def kernel_modules(self):
-        return [("heads_prepare", {}), ("recurrent", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})]
+        return [("heads_prepare", {}), ("recurrent", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})] + self._chunked_modules()
 
     def step_plans(self):
-        return recurrent.segment_planner(self.dtype)
+        return self._constant_decay_plans()
 
     def core(self, proj, col0, step, cache, out, scale):
         k_off, v_off = col0 + self.qk_width, col0 + 2 * self.qk_width
         ops.heads_prepare_wide(proj, col0, k_off, v_off, self.heads, self.heads, self.n, self.e, step.positions, q_out=proj[:, col0:k_off],
                                k_out=proj[:, k_off:v_off], inv_freq=self.position.inv_freq if self.position is not None else None,
                                rot_dims=self.position.dims if self.position is not None else 0, rot_half=True, k_scale=self.n ** -0.5)
-        # Segments pay while one pass leaves the GPU mostly idle: a row's walk is a chain of dependent steps (0.23 us a token on a
-        # B200) that few blocks share, and cutting it doubles the arithmetic.  Measured at heads of 128 x 128: 64 blocks 482 -> 290 us for
-        # 2,048 tokens, 128 blocks 487 -> 509 us.
-        blocks = self.heads * -(-self.e // 32)
-        segments = step.host.get("scan_segments", 0) if self.dtype == torch.bfloat16 and blocks <= 100 else 0
-        if segments:
-            o = recurrent.retention_in_segments(proj, k_off, col0, v_off, self.decay, cache.state, cache.slots, step.extra["scan_seg_start"],
-                                                step.extra["scan_seg_row"], segments, self.heads, self.n, self.n_padded, self.e)
-        else:
-            o = recurrent.state_scan(recurrent.MODE_RETENTION, proj, k_off, col0, v_off, proj, 0, 0, self.decay, self.decay, None, cache.state, 0, cache.slots,
-                                     step.row_start, step.n_rows, self.heads, self.heads, self.n, self.n_padded, self.e)
+        o = self._retain(proj, k_off, col0, v_off, cache, step)
         recurrent.gated_group_norm(o, proj, v_off + self.core_width, None, self.e, False, self.eps, self.dtype, scale=scale, out=out)
 
 

@@ -78,8 +78,50 @@ def _round_up(value: int, step: int) -> int:
     return -(-value // step) * step
 
 
-def _chunked_module(dtype: torch.dtype) -> list[tuple[str, dict]]:
-    return [("chunked_scan", {})] if dtype == torch.bfloat16 else []
+def _chunked_module(dtype: torch.dtype, module: str = "chunked_scan") -> list[tuple[str, dict]]:
+    return [(module, {})] if dtype == torch.bfloat16 else []
+
+
+class ChunkedRule:
+    """What the mixers share whose recurrence :func:`hyperion_b200.ops.recurrent.chunked_rule` takes: heads of a size that it fits walk long bfloat16 rows in chunks."""
+
+    def _chunked_modules(self):
+        return _chunked_module(self.dtype, "chunked_float") if recurrent.chunked_rule_fits(self.n, self.e) else []
+
+    def _chunk_plans(self) -> dict:
+        return recurrent.rule_planner(self.dtype) if recurrent.chunked_rule_fits(self.n, self.e) else {}
+
+    def _walk(self, rule, k, q, v, x, x_off, step_in, step_off, rate, bias, cache, step, groups, q_scale, by_token):
+        """Long rows in chunks, the others by ``by_token(below, out)``."""
+        cut = step.host.get("rule_chunks") if recurrent.chunked_rule_fits(self.n, self.e) else None
+        if cut is None:
+            return by_token(0, None)
+        chunks, walks, others = cut
+        out = recurrent.chunked_rule(rule, k, q, v, x, x_off, step_in, step_off, rate, bias, cache.state, 0, cache.slots, step.extra["rule_chunks"], chunks,
+                                     step.extra["rule_walks"], walks, self.heads, groups, self.n, self.n_padded, self.e, q_scale)
+        return by_token(recurrent.CHUNKED_RULE_ROWS, out) if others else out
+
+
+class ConstantDecay(ChunkedRule):
+    """A state that fades by a constant of the head (retention, lightning attention)."""
+
+    def _constant_decay_plans(self) -> dict:
+        return {**recurrent.segment_planner(self.dtype), **self._chunk_plans()}
+
+    def _retain(self, proj, k_off, q_off, v_off, cache, step):
+        def by_token(below, out):
+            # Heads that no chunk fits walk long bfloat16 rows in segments while one pass leaves the GPU mostly idle: a row's walk is a chain of dependent steps
+            # (0.23 us a token on a B200) that few blocks share, and cutting it doubles the arithmetic.  Measured at heads of 128 x 128: 64 blocks
+            # 482 -> 290 us for 2,048 tokens, 128 blocks 487 -> 509 us.
+            blocks = self.heads * -(-self.e // 32)
+            segments = step.host.get("scan_segments", 0) if self.dtype == torch.bfloat16 and blocks <= 100 and not recurrent.chunked_rule_fits(self.n, self.e) else 0
+            if segments:
+                return recurrent.retention_in_segments(proj, k_off, q_off, v_off, self.decay, cache.state, cache.slots, step.extra["scan_seg_start"],
+                                                       step.extra["scan_seg_row"], segments, self.heads, self.n, self.n_padded, self.e)
+            return recurrent.state_scan(recurrent.MODE_RETENTION, proj, k_off, q_off, v_off, proj, 0, 0, self.decay, self.decay, None, cache.state, 0, cache.slots,
+                                        step.row_start, step.n_rows, self.heads, self.heads, self.n, self.n_padded, self.e, below=below, out=out)
+
+        return self._walk(recurrent.RULE_RETENTION, proj[:, k_off:], proj[:, q_off:], proj[:, v_off:], None, 0, None, 0, self.decay, None, cache, step, self.heads, 1.0, by_token)
 
 
 class _ScanMixer(Mixer):
@@ -112,7 +154,7 @@ class _ScanMixer(Mixer):
         return tensor.to(torch.float32).contiguous()
 
 
-class GatedDeltaRule(_ScanMixer):
+class GatedDeltaRule(_ScanMixer, ChunkedRule):
     mode = recurrent.MODE_DELTA
 
     def __init__(self, spec: PartSpec, build: BuildContext):
@@ -145,6 +187,12 @@ class GatedDeltaRule(_ScanMixer):
         self.norm = self._float(tensors["norm"])
         self.w_o = tensors["o"].contiguous()
 
+    def kernel_modules(self):
+        return super().kernel_modules() + self._chunked_modules()
+
+    def step_plans(self):
+        return self._chunk_plans()
+
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("the delta rule keeps a state per request; the schedule gave it none")
@@ -152,9 +200,11 @@ class GatedDeltaRule(_ScanMixer):
         state, slots, rows = cache.state, cache.slots, step.n_rows
         conv = recurrent.causal_conv_silu(proj, 0, self.w_conv, None, state, self.conv_off, slots, step.token_row, step.row_start)
         recurrent.conv_state_update(proj, 0, self.conv_channels, self.taps, state, self.conv_off, slots, step.row_start, rows)
-        o = recurrent.state_scan(self.mode, conv, self.qk_width, 0, 2 * self.qk_width, proj, self.decay_off, self.beta_off, self.a_log, self.dt_bias,
-                                 None, state, 0, slots, step.row_start, rows, self.heads, self.groups, self.n, self.n_padded, self.e,
-                                 q_scale=self.n ** -0.5)
+        o = self._walk(recurrent.RULE_DELTA, conv[:, self.qk_width :], conv, conv[:, 2 * self.qk_width :], proj, self.decay_off, proj, self.beta_off, self.a_log, self.dt_bias,
+                       cache, step, self.groups, self.n ** -0.5,
+                       lambda below, out: recurrent.state_scan(self.mode, conv, self.qk_width, 0, 2 * self.qk_width, proj, self.decay_off, self.beta_off, self.a_log, self.dt_bias,
+                                                               None, state, 0, slots, step.row_start, rows, self.heads, self.groups, self.n, self.n_padded, self.e,
+                                                               q_scale=self.n ** -0.5, below=below, out=out))
         y = recurrent.gated_group_norm(o, proj, self.gate_off, self.norm, self.e, False, self.eps, self.dtype)
         return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
@@ -323,13 +373,14 @@ class SelectiveScanMixer(Mixer):
         return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
-class WkvMixer(Mixer):
+class WkvMixer(Mixer, ChunkedRule):
     MIXES = ("r", "k", "v", "g", "w")
 
     def __init__(self, spec: PartSpec, build: BuildContext):
         super().__init__(spec, build)
         p = spec.params
         self.hidden, self.heads, self.n = int(p["hidden_size"]), int(p["heads"]), int(p["head_dim"])
+        self.e = self.n
         self.decay_rank, self.eps = int(p.get("decay_rank") or 16), float(p["eps"])
         if self.n > 256:
             raise ValueError(f"a state of {self.n} per column is above the scan kernel's limit of 256")
@@ -359,7 +410,10 @@ class WkvMixer(Mixer):
         return RequestState((self.record,), torch.float32)
 
     def kernel_modules(self):
-        return [("recurrent", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})]
+        return [("recurrent", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})] + self._chunked_modules()
+
+    def step_plans(self):
+        return self._chunk_plans()
 
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
@@ -370,12 +424,14 @@ class WkvMixer(Mixer):
         r, k, v, gate = (ops.linear(mixed[i], w, None, torch.float32) for i, w in enumerate(self.w_in))
         inner = recurrent.tanh_rows(ops.linear(mixed[4], self.w_1, None, torch.float32), self.dtype)
         decay_in = ops.linear(inner, self.w_2, None, torch.float32)
-        o = recurrent.wkv_scan(k, r, v, decay_in, 0, self.w0, self.bonus, state, 0, slots, step.row_start, rows, self.heads, self.n, self.n_padded, self.n)
+        o = self._walk(recurrent.RULE_WKV, k, r, v, decay_in, 0, None, 0, self.w0, self.bonus, cache, step, self.heads, 1.0,
+                       lambda below, out: recurrent.wkv_scan(k, r, v, decay_in, 0, self.w0, self.bonus, state, 0, slots, step.row_start, rows, self.heads, self.n, self.n_padded,
+                                                             self.n, below=below, out=out))
         y = recurrent.gated_group_norm(o, gate, 0, self.norm, self.n, False, self.eps, self.dtype)
         return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
-class ChannelDeltaRule(_ScanMixer):
+class ChannelDeltaRule(_ScanMixer, ChunkedRule):
     def __init__(self, spec: PartSpec, build: BuildContext):
         super().__init__(spec, build)
         p = spec.params
@@ -413,6 +469,12 @@ class ChannelDeltaRule(_ScanMixer):
         self.norm = self._float(tensors["norm"])
         self.w_o = tensors["o"].contiguous()
 
+    def kernel_modules(self):
+        return super().kernel_modules() + self._chunked_modules()
+
+    def step_plans(self):
+        return self._chunk_plans()
+
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("the delta rule keeps a state per request; the schedule gave it none")
@@ -422,13 +484,16 @@ class ChannelDeltaRule(_ScanMixer):
         recurrent.conv_state_update(proj, 0, self.conv_channels, self.taps, state, self.conv_off, slots, step.row_start, rows)
         decay = ops.linear(proj[:, self.a1_off : self.a1_off + self.decay_rank], self.w_a2, None, torch.float32)
         gate = ops.linear(proj[:, self.g1_off : self.g1_off + self.gate_rank], self.w_g2, None, torch.float32)
-        o = recurrent.channel_delta_scan(conv, self.qk_width, 0, 2 * self.qk_width, decay, proj, self.beta_off, self.a_log, self.dt_bias, state, 0, slots,
-                                         step.row_start, rows, self.heads, self.groups, self.n, self.n_padded, self.e, q_scale=self.n ** -0.5)
+        o = self._walk(recurrent.RULE_CHANNEL_DELTA, conv[:, self.qk_width :], conv, conv[:, 2 * self.qk_width :], decay, 0, proj, self.beta_off, self.a_log, self.dt_bias, cache,
+                       step, self.groups, self.n ** -0.5,
+                       lambda below, out: recurrent.channel_delta_scan(conv, self.qk_width, 0, 2 * self.qk_width, decay, proj, self.beta_off, self.a_log, self.dt_bias, state, 0, slots,
+                                                                       step.row_start, rows, self.heads, self.groups, self.n, self.n_padded, self.e, q_scale=self.n ** -0.5,
+                                                                       below=below, out=out))
         y = recurrent.gated_group_norm(o, gate, 0, self.norm, self.e, False, self.eps, self.dtype, sigmoid_gate=True)
         return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
-class LightningAttention(Mixer):
+class LightningAttention(Mixer, ConstantDecay):
     def __init__(self, spec: PartSpec, build: BuildContext):
         super().__init__(spec, build)
         p = spec.params
@@ -460,10 +525,10 @@ class LightningAttention(Mixer):
         return RequestState((self.record,), torch.float32)
 
     def kernel_modules(self):
-        return [("recurrent", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})]
+        return [("recurrent", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})] + self._chunked_modules()
 
     def step_plans(self):
-        return recurrent.segment_planner(self.dtype)
+        return self._constant_decay_plans()
 
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
@@ -471,15 +536,7 @@ class LightningAttention(Mixer):
         proj = ops.linear(x, self.w_in, None, torch.float32)
         k_off, v_off = self.qk_width, 2 * self.qk_width
         recurrent.silu_columns_(proj, 0, v_off + self.v_width)
-        # long rows in segments while one pass leaves the GPU mostly idle, as for the package's other constant-decay recurrence
-        blocks = self.heads * -(-self.e // 32)
-        segments = step.host.get("scan_segments", 0) if self.dtype == torch.bfloat16 and blocks <= 100 else 0
-        if segments:
-            o = recurrent.retention_in_segments(proj, k_off, 0, v_off, self.decay, cache.state, cache.slots, step.extra["scan_seg_start"],
-                                                step.extra["scan_seg_row"], segments, self.heads, self.n, self.n_padded, self.e)
-        else:
-            o = recurrent.state_scan(recurrent.MODE_RETENTION, proj, k_off, 0, v_off, proj, 0, 0, self.decay, self.decay, None, cache.state, 0, cache.slots,
-                                     step.row_start, step.n_rows, self.heads, self.heads, self.n, self.n_padded, self.e)
+        o = self._retain(proj, k_off, 0, v_off, cache, step)
         y = recurrent.gated_group_norm(o, proj, v_off + self.v_width, self.norm, self.v_width, False, self.eps, self.dtype, sigmoid_gate=True)
         return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 

@@ -1,0 +1,106 @@
+"""The recurrences that walk long bfloat16 rows in chunks at float precision (csrc/chunked_float.cu): the plan on the CPU, the kernels against 64-bit arithmetic."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from hyperion_b200.ops import recurrent
+
+
+def test_the_plan_covers_every_long_row_once():
+    assert recurrent.plan_rule_chunks([127, 64, 1]) is None
+    for counts in ([128], [1, 300, 15, 16, 64, 65, 2], [2048, 1], [129] * 3):
+        chunks, walks, others = recurrent.plan_rule_chunks(counts)
+        covered = [t for first, count in zip(chunks[::2], chunks[1::2]) for t in range(first, first + count)]
+        starts = [sum(counts[:i]) for i in range(len(counts))]
+        long_rows = [i for i, c in enumerate(counts) if c >= recurrent.CHUNKED_RULE_ROWS]
+        assert covered == [t for i in long_rows for t in range(starts[i], starts[i] + counts[i])]
+        assert all(0 < c <= recurrent.CHUNK for c in chunks[1::2]) and others == (len(long_rows) < len(counts))
+        assert walks[2::3] == long_rows and walks[0::3] == [0, *walks[1::3]][: len(long_rows)] and walks[-2] == len(chunks) // 2
+        for begun, end, row in zip(walks[::3], walks[1::3], walks[2::3]):
+            assert sum(chunks[2 * begun + 1 : 2 * end : 2]) == counts[row]
+
+
+def token_by_token(rule, k, q, v, a, beta, S, bonus):
+    out = torch.empty_like(v)
+    for t in range(k.shape[0]):
+        kv = k[t][:, :, None] * v[t][:, None, :]
+        if rule == recurrent.RULE_WKV:
+            out[t] = torch.einsum("hde,hd->he", S + bonus[:, :, None] * kv, q[t])
+            S = a[t][:, :, None] * S + kv
+            continue
+        S = S * a[t][:, :, None]
+        if beta is not None:
+            kv = k[t][:, :, None] * (beta[t][:, None] * (v[t] - torch.einsum("hde,hd->he", S, k[t])))[:, None, :]
+        S = S + kv
+        out[t] = torch.einsum("hde,hd->he", S, q[t])
+    return out, S
+
+
+# heads, groups, key size, value size: one tile and several, a padded key, a key of one tile row less than the kernel's, strides that allow no 16-byte loads (an odd key size)
+SHAPES = [(2, 1, 128, 128), (3, 3, 64, 16), (2, 2, 100, 48), (2, 1, 21, 32)]
+COUNTS = [128 + 65, 1, 16, 15, 64, 130, 17]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("steep", [False, True])
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("rule", [recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA, recurrent.RULE_RETENTION, recurrent.RULE_WKV])
+def test_rules_in_chunks(rule, shape, steep, monkeypatch):
+    """Rows of 1 to 193 tokens (those below the limit are left alone) from states that are not zero, columns of wider matrices, decays from nearly 1 down to 1e-9 a token
+    (``steep``: the pairs of a sub-block one by one), scratch for three chunks at a time.
+
+    Both this and the token-by-token scan are sums of float terms: a result's error is some 1e-7 of the norm of what it adds up, several times that where decays are near 1 and a
+    state has passed 200 tokens; 3e-6 is ten times the largest seen (5e-7 here)."""
+    heads, groups, n, e = shape
+    if rule in (recurrent.RULE_RETENTION, recurrent.RULE_WKV):
+        groups = heads
+    monkeypatch.setattr(recurrent, "SCRATCH_BYTES", 3 * 4 * heads * (3 * 64 * 136 + 64 * 68 + 64 * e + 256))
+    g = torch.Generator().manual_seed(rule * 10 + n)
+    tokens, width, n_padded = sum(COUNTS), groups * n, -(-n // 4) * 4
+    rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    x = rnd(tokens, 2 * width + heads * e + 3)
+    entries = heads * n if rule in (recurrent.RULE_CHANNEL_DELTA, recurrent.RULE_WKV) else heads
+    pre, step = rnd(tokens, entries + 2), rnd(tokens, heads + 1)
+    if rule == recurrent.RULE_RETENTION:
+        rate, bias = torch.linspace(0.999, 1e-3 if steep else 0.9, heads), None
+        a = rate.double()[None, :, None].expand(tokens, heads, n)
+    elif rule == recurrent.RULE_WKV:
+        rate, bias = torch.rand(entries, generator=g) * (9 if steep else 5) - 6, rnd(entries) * 0.5
+        a = torch.exp(-torch.exp(pre[:, :entries].double() + rate.double())).view(tokens, heads, n)
+    else:
+        rate, bias = torch.linspace(0, 2.7, heads), torch.rand(entries, generator=g) * (4 if steep else 5) - (1 if steep else 7)
+        a = torch.exp(-torch.exp(rate.double())[:, None] * torch.nn.functional.softplus(pre[:, :entries].double() + bias.double()).view(tokens, heads, -1)).expand(tokens, heads, n)
+    delta = rule in (recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA)
+    q_scale = n ** -0.5 if delta else 1.0
+    q, k, v = (t.double().view(tokens, h, w) for t, h, w in ((x[:, :width], groups, n), (x[:, width : 2 * width], groups, n), (x[:, 2 * width : 2 * width + heads * e], heads, e)))
+    if delta:
+        q = q / torch.sqrt(q.pow(2).sum(-1, keepdim=True) + 1e-6) * q_scale
+        k = k / torch.sqrt(k.pow(2).sum(-1, keepdim=True) + 1e-6)
+    q, k = (t.repeat_interleave(heads // groups, 1) for t in (q, k))
+    beta = torch.sigmoid(step[:, :heads].double()) if delta else None
+    record = heads * e * n_padded
+    begin = rnd(len(COUNTS) + 2, record + 5)
+    begin[:, :record].view(-1, heads, e, n_padded)[..., n:] = 0
+    slots = torch.tensor([5, 0, 8, 3, 1, 7, 2], dtype=torch.int32)
+
+    table, walks, others = recurrent.plan_rule_chunks(COUNTS)
+    assert others
+    dev = lambda t: None if t is None else t.cuda()  # noqa: E731
+    state, xd = begin.cuda(), x.cuda()
+    got = recurrent.chunked_rule(rule, xd[:, width:], xd, xd[:, 2 * width :], dev(pre) if rule != recurrent.RULE_RETENTION else None, 0, dev(step) if delta else None, 0, dev(rate), dev(bias), state, 0,
+                                 slots.cuda(), torch.tensor(table, dtype=torch.int32).cuda(), len(table) // 2, torch.tensor(walks, dtype=torch.int32).cuda(), len(walks) // 3, heads, groups, n,
+                                 n_padded, e, q_scale).cpu().view(tokens, heads, e)
+    at = 0
+    for row, count in enumerate(COUNTS):
+        here, slot = slice(at, at + count), int(slots[row])
+        at += count
+        if count < recurrent.CHUNKED_RULE_ROWS:
+            assert torch.equal(state[slot].cpu(), begin[slot])
+            continue
+        S = begin[slot, :record].double().view(heads, e, n_padded)[..., :n].transpose(1, 2)
+        want, S = token_by_token(rule, k[here], q[here], v[here], a[here], None if beta is None else beta[here], S, bias.double().view(heads, n) if rule == recurrent.RULE_WKV else None)
+        kept = state[slot, :record].cpu().double().view(heads, e, n_padded)
+        for name, one, other in (("outputs", got[here].double(), want), ("state", kept[..., :n].transpose(1, 2), S)):
+            assert torch.isfinite(one).all() and (one - other).norm() <= 3e-6 * other.norm(), (name, row, float((one - other).norm() / other.norm()))
+        assert not kept[..., n:].any() and torch.equal(state[slot, record:].cpu(), begin[slot, record:])
