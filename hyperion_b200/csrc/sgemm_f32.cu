@@ -3,60 +3,113 @@
 // is one sequential chain of fused multiply-adds over k = 0..K-1, so its value depends on neither M,
 // nor the tile it falls in, nor what else is in the batch. The reference has no device float path;
 // its float arithmetic is the f64 `linear` of helios/crates/helios-hal/src/reference.rs:24-41.
+//
+// A thread owns TM x TN outputs, BM / TM and BN / TN apart, and reads four k of each of its rows and columns at a time from shared memory in 16-byte pieces; slices of BK k
+// are copied ahead into a ring of STAGES, as they lie in memory. Bound by the FFMA pipes (74 TFLOP/s) where a product has tiles enough, else by the waits of a chain.
+// Two shapes: 64 x 128 with 8 x 8 outputs a thread for products that fill the GPU with such tiles; 32 x 32 with 4 x 4 for the others, which spreads a narrow product over
+// all SMs. Measured on one B200 (before: one shape of 64 x 64 with 4 x 4 outputs a thread, copied when needed): 394 rows, K 896, 9,728 columns 340 -> 246 us, K 4,864, 896 columns
+// 302 -> 166 us; 3 rows, 151,936 columns 625 -> 244 us; 1 row, K 4,864 265 -> 101 us; 2,048 rows, 9,728 columns 1,393 -> 819 us (44 TFLOP/s).
 #include "common.cuh"
 
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+__device__ __forceinline__ void copy16(float* to, const float* from, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(live ? 16 : 0));
+}
+__device__ __forceinline__ void copy4(float* to, const float* from, bool live) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from), "r"(live ? 4 : 0));
+}
 
-__global__ void __launch_bounds__(256) sgemm_kernel(const float* __restrict__ a, const float* __restrict__ w,
-                                                    const float* __restrict__ bias, float* __restrict__ c, int m, int n,
-                                                    int k, int lda, int ldc) {
-    __shared__ float as[BK][BM + 4];
-    __shared__ float ws[BK][BN + 4];
-    const int tid = threadIdx.x;
+template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool WIDE>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) sgemm_kernel(const float* __restrict__ a, const float* __restrict__ w, const float* __restrict__ bias,
+                                                                       float* __restrict__ c, int m, int n, int k, int lda, int ldc) {
+    constexpr int DOWN = BM / TM, ACROSS = BN / TN, THREADS = DOWN * ACROSS, QUADS = BK / 4, LD = BK + 4, STAGE = (BM + BN) * LD;
+    extern __shared__ __align__(16) float ring[];  // STAGES times [BM + BN][LD]: rows of A, then rows of W
+    const int tid = threadIdx.x, ty = tid / ACROSS, tx = tid % ACROSS;
     const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
-    const int ty = tid / 16, tx = tid % 16;
     float acc[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
-    // each thread loads 4 consecutive k of one row of each tile: 64 rows x 16 k = 256 threads x 4
-    const int lrow = tid / 4, lk = (tid % 4) * 4;
-    for (int k0 = 0; k0 < k; k0 += BK) {
+    // a slice's rows as they lie in memory; zeros past the matrix (they add exact zeros to a chain's end)
+    auto fetch = [&](int slice) {
+        float* stage = ring + slice % STAGES * STAGE;
+        const int k0 = slice * BK;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int kk = k0 + lk + e;
-            const int ar = row0 + lrow, wr = col0 + lrow;
-            as[lk + e][lrow] = (ar < m && kk < k) ? a[(size_t)ar * lda + kk] : 0.f;
-            ws[lk + e][lrow] = (wr < n && kk < k) ? w[(size_t)wr * k + kk] : 0.f;
+        for (int unit = tid; unit < (BM + BN) * QUADS; unit += THREADS) {
+            const int r = unit / QUADS, kk = k0 + unit % QUADS * 4;
+            const bool from_a = r < BM;
+            const int at = from_a ? row0 + r : col0 + r - BM;
+            const bool live = at < (from_a ? m : n);
+            const float* p = from_a ? a + (size_t)(live ? at : 0) * lda : w + (size_t)(live ? at : 0) * k;
+            float* to = stage + r * LD + unit % QUADS * 4;
+            if (WIDE) {
+                copy16(to, p + (kk < k ? kk : 0), live && kk < k);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) copy4(to + e, p + (kk + e < k ? kk + e : 0), live && kk + e < k);
+            }
         }
-        __syncthreads();
+    };
+    const int slices = (k + BK - 1) / BK;
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float av[TM], wv[TN];
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < slices) fetch(s);
+        asm volatile("cp.async.commit_group;");
+    }
+    for (int slice = 0; slice < slices; ++slice) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2));
+        __syncthreads();  // this slice is there, and the one before it has been read
+        if (slice + STAGES - 1 < slices) fetch(slice + STAGES - 1);
+        asm volatile("cp.async.commit_group;");
+        const float* as = ring + slice % STAGES * STAGE + ty * LD;
+        const float* ws = ring + slice % STAGES * STAGE + (BM + tx) * LD;
 #pragma unroll
-            for (int i = 0; i < TM; ++i) av[i] = as[kk][ty * TM + i];
+        for (int kk = 0; kk < BK; kk += 4) {
+            float av[TM][4], wv[TN][4];
 #pragma unroll
-            for (int j = 0; j < TN; ++j) wv[j] = ws[kk][tx * TN + j];
+            for (int i = 0; i < TM; ++i) load4(as + i * DOWN * LD + kk, av[i]);
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
+            for (int j = 0; j < TN; ++j) load4(ws + j * ACROSS * LD + kk, wv[j]);
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+            for (int e = 0; e < 4; ++e)
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i][e], wv[j][e], acc[i][j]);
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        const int r = row0 + ty * TM + i;
+        const int r = row0 + ty + i * DOWN;
         if (r >= m) continue;
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-            const int col = col0 + tx * TN + j;
+            const int col = col0 + tx + j * ACROSS;
             if (col < n) c[(size_t)r * ldc + col] = acc[i][j] + (bias ? bias[col] : 0.f);
         }
     }
+}
+
+template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool WIDE>
+int launch_kernel(dim3 grid, const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda, int ldc, cudaStream_t stream) {
+    constexpr int bytes = STAGES * (BM + BN) * (BK + 4) * 4;
+    if (bytes > 48 * 1024) {
+        const int status = (int)cudaFuncSetAttribute(sgemm_kernel<BM, BN, TM, TN, BK, STAGES, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (status) return status;
+    }
+    sgemm_kernel<BM, BN, TM, TN, BK, STAGES, WIDE><<<grid, (BM / TM) * (BN / TN), bytes, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
+    return launch_status();
+}
+
+template <int BM, int BN, int TM, int TN, int BK, int STAGES>
+int launch_tiles(const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda, int ldc, cudaStream_t stream) {
+    const dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
+    if (grid.y > 65535) return HB_UNSUPPORTED_SIZE;
+    const bool wide = ((lda | k) & 3) == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
+    return wide ? launch_kernel<BM, BN, TM, TN, BK, STAGES, true>(grid, a, w, bias, c, m, n, k, lda, ldc, stream)
+                : launch_kernel<BM, BN, TM, TN, BK, STAGES, false>(grid, a, w, bias, c, m, n, k, lda, ldc, stream);
 }
 }  // namespace
 
@@ -66,8 +119,8 @@ HB_EXPORT int hb_sgemm_f32(const float* a, const float* w, const float* bias, fl
                            int ldc, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return HB_BAD_ARGUMENT;
-    dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
-    if (grid.y > 65535) return HB_UNSUPPORTED_SIZE;
-    sgemm_kernel<<<grid, 256, 0, stream>>>(a, w, bias, c, m, n, k, lda, ldc);
-    return launch_status();
+    // large tiles from two to an SM on (394 rows, 9,728 columns: 532 of them 246 us; 896 columns: 49 of them would leave two SMs in three idle) and where rows do not leave half of one empty
+    const long long large = (long long)((m + 63) / 64) * ((n + 127) / 128);
+    if (m > 32 && large >= 296) return launch_tiles<64, 128, 8, 8, 16, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
+    return launch_tiles<32, 32, 4, 4, 32, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
 }
