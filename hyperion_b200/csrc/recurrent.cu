@@ -775,12 +775,12 @@ HB_EXPORT int hb_matrix_memory_gates(const float* x, int x_stride, int i_off, in
 // [values + 1, n_padded], its last row the sum of keys; out [tokens, heads, out_e] with out_e > values, entry `values` being n . q.
 HB_EXPORT int hb_matrix_memory_scan(const float* x, int x_stride, int k_off, int q_off, int v_off, const float* gates, float* state, long long slot_stride, int state_off,
                                     const int* slots, const int* row_start, float* out, int rows, int heads, int n, int n_padded, int values, int out_e, float q_scale,
-                                    cudaStream_t stream) {
+                                    int below, cudaStream_t stream) {
     if (rows <= 0) return 0;
     if (n <= 0 || n > 256 || values <= 0 || heads <= 0 || rows > 65535 || heads > 65535 || out_e <= values) return HB_UNSUPPORTED_SIZE;
     if (n_padded < n || (n_padded & 3) || (state_off & 3) || (slot_stride & 3) || (((uintptr_t)state) & 15)) return HB_BAD_ARGUMENT;
     ScanArgs a{x + k_off, x + q_off, x + v_off, x_stride, x_stride, x_stride, gates, 4 * heads, 0, heads, gates, 4 * heads, nullptr, nullptr, nullptr,
-               state, (size_t)slot_stride, state_off, slots, row_start, out, heads, heads, n, n_padded, values + 1, q_scale, values, out_e};
+               state, (size_t)slot_stride, state_off, slots, row_start, out, heads, heads, n, n_padded, values + 1, q_scale, values, out_e, below};
     return launch_scan<MODE_GIVEN>(a, rows, stream);
 }
 

@@ -124,17 +124,19 @@ def matrix_memory_columns(values: int) -> int:
 
 
 def matrix_memory_scan(x: torch.Tensor, k_off: int, q_off: int, v_off: int, gates: torch.Tensor, state: torch.Tensor, state_off: int, slots: torch.Tensor,
-                       row_start: torch.Tensor, rows: int, heads: int, n: int, n_padded: int, values: int, q_scale: float) -> torch.Tensor:
+                       row_start: torch.Tensor, rows: int, heads: int, n: int, n_padded: int, values: int, q_scale: float, below: int = 0,
+                       out: torch.Tensor | None = None) -> torch.Tensor:
     """S <- a S + b k v^T per head with decay a and step b from ``gates`` (:func:`matrix_memory_gates`), and the same for the sum of keys, a further column of S.
     Keys, queries and values are columns of ``x``; every row's tokens walk from and into its slot of ``state`` ([heads, values + 1, n_padded] floats at
-    ``state_off``).  Returns [tokens, heads, :func:`matrix_memory_columns`]: S^T q and, at entry ``values``, n . q, with q times ``q_scale``."""
-    require_cuda(x, gates, state, slots, row_start)
+    ``state_off``).  Returns [tokens, heads, :func:`matrix_memory_columns`]: S^T q and, at entry ``values``, n . q, with q times ``q_scale``.
+    ``below`` and ``out`` as in :func:`state_scan`."""
+    require_cuda(x, gates, state, slots, row_start, out)
     _floats(x, gates, state)
     columns = matrix_memory_columns(values)
-    out = torch.empty((x.shape[0], heads, columns), dtype=torch.float32, device=x.device)
+    out = _rows_for(None if out is None else out.view(x.shape[0], heads * columns), x.shape[0], heads * columns, x.device).view(x.shape[0], heads, columns)
     check(library("recurrent").hb_matrix_memory_scan(ptr(x), i32(x.stride(0)), i32(k_off), i32(q_off), i32(v_off), ptr(gates), ptr(state), ctypes.c_longlong(state.stride(0)),
                                                      i32(state_off), ptr(slots), ptr(row_start), ptr(out), i32(rows), i32(heads), i32(n), i32(n_padded), i32(values), i32(columns),
-                                                     f32(q_scale), stream_ptr()), "matrix_memory_scan")
+                                                     f32(q_scale), i32(below), stream_ptr()), "matrix_memory_scan")
     return out
 
 
@@ -326,7 +328,8 @@ def plan_chunks(counts) -> tuple[list[int], list[int]] | None:
 
 def chunk_planner(dtype: torch.dtype) -> dict:
     """The step planner of mixers that walk long rows in chunks on the tensor cores (:func:`chunked_scan`): in bfloat16, a step with a long row gets ``scan_chunk_start``
-    and ``scan_chunk_row`` among its arrays and their number in ``step.host["scan_chunks"]`` (0 otherwise)."""
+    and ``scan_chunk_row`` among its arrays and their number in ``step.host["scan_chunks"]`` (0 otherwise); ``step.host["scan_short_rows"]``: whether some rows are short
+    enough to go token by token all the same."""
     if dtype != torch.bfloat16:
         return {}
 
@@ -336,6 +339,7 @@ def chunk_planner(dtype: torch.dtype) -> dict:
         counts = rows.counts if hasattr(rows, "counts") else [row.count for row in rows]
         cut = plan_chunks([int(c) for c in counts])
         host["scan_chunks"] = 0 if cut is None else len(cut[1])
+        host["scan_short_rows"] = cut is not None and int(min(counts)) < CHUNKED_RULE_ROWS
         if cut is not None:
             packer.add("scan_chunk_start", cut[0])
             packer.add("scan_chunk_row", cut[1])
@@ -419,13 +423,13 @@ def chunked_rule(rule: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, x
 def chunked_scan(kind: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, gate: torch.Tensor, decay_off: int, step_off: int, state: torch.Tensor, state_off: int,
                  slots: torch.Tensor, chunk_start: torch.Tensor, chunk_row: torch.Tensor, chunks: int, heads: int, groups: int, n: int, n_padded: int, e: int, *,
                  a_log: torch.Tensor | None = None, dt_bias: torch.Tensor | None = None, skip: torch.Tensor | None = None, sums_keys: bool = False,
-                 q_scale: float = 1.0, columns: int | None = None) -> torch.Tensor:
+                 q_scale: float = 1.0, columns: int | None = None, below: int = 0) -> torch.Tensor:
     """A recurrence whose state fades by one number per token and head, S <- a S + b k v^T, o = S^T q, over the chunks of a step (:func:`plan_chunks`) on the tensor cores.
     ``k``, ``q`` (group g at g * n, the query times ``q_scale``) and ``v`` (head h at h * e) are float views [tokens, *].  ``KIND_STATE_SPACE``: the
     step is softplus(``gate``[decay_off + h] + dt_bias), a = exp(-exp(a_log) step), D = ``skip``; ``KIND_GIVEN``: ln a and b are the columns ``decay_off + h`` and
     ``step_off + h`` of ``gate``.  The rows' states ([heads, e, n_padded], with ``sums_keys`` one more row for the sum of keys) lie at ``state_off`` of ``state``.  Returns
     [tokens, heads, ``columns``] (``e`` unless stated; with ``sums_keys`` entry e of a head is n . q).  Differs from the one-pass scan by bfloat16 roundings of
-    keys, queries and values."""
+    keys, queries and values.  ``below`` > 0: rows of fewer tokens are left alone."""
     require_cuda(k, q, v, gate, state, slots, chunk_start, chunk_row, a_log, dt_bias, skip)
     _floats(k, q, v, gate, state, a_log, dt_bias, skip)
     rows = e + (1 if sums_keys else 0)
@@ -439,7 +443,7 @@ def chunked_scan(kind: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, g
     check(library("chunked_scan").hb_chunked_scan(
         i32(kind), ptr(k), i32(k.stride(0)), ptr(q), i32(q.stride(0)), ptr(v), i32(v.stride(0)), ptr(gate), i32(gate.stride(0)), i32(decay_off), i32(step_off), ptr(a_log), ptr(dt_bias),
         ptr(skip), ptr(ends), ptr(decays), ptr(begins), ptr(state), ctypes.c_longlong(state.stride(0)), i32(state_off), ptr(slots), ptr(chunk_start), ptr(chunk_row), i32(chunks),
-        ptr(out), i32(columns), i32(heads), i32(groups), i32(n), i32(n_padded), i32(e), i32(1 if sums_keys else 0), f32(q_scale), stream_ptr()), "chunked_scan")
+        i32(slots.numel()), i32(below), ptr(out), i32(columns), i32(heads), i32(groups), i32(n), i32(n_padded), i32(e), i32(1 if sums_keys else 0), f32(q_scale), stream_ptr()), "chunked_scan")
     from . import native
 
     native.LAUNCHES[0] += 2  # three kernels: the chunks' sums, the chain through them, the outputs

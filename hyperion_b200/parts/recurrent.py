@@ -253,13 +253,16 @@ class StateSpaceMixer(_ScanMixer, Branch):
         recurrent.conv_state_update(proj, conv_col, self.conv_channels, self.taps, state, self.conv_off, slots, step.row_start, rows)
         bn = self.groups * self.n
         chunks = step.host.get("scan_chunks", 0)
-        if chunks:  # long rows in bfloat16: the tensor cores walk the step in chunks
+        # a step with a long row in bfloat16: the tensor cores walk it in chunks, the shortest rows go token by token all the same
+        short = recurrent.CHUNKED_RULE_ROWS if chunks and step.host["scan_short_rows"] else 0
+        y = None
+        if chunks:
             y = recurrent.chunked_scan(recurrent.KIND_STATE_SPACE, conv[:, self.inner :], conv[:, self.inner + bn :], conv, proj, dt_off, 0, state, 0, slots,
                                        step.extra["scan_chunk_start"], step.extra["scan_chunk_row"], chunks, self.heads, self.groups, self.n, self.n_padded, self.e,
-                                       a_log=self.a_log, dt_bias=self.dt_bias, skip=self.skip).view(proj.shape[0], self.inner)
-        else:
+                                       a_log=self.a_log, dt_bias=self.dt_bias, skip=self.skip, below=short).view(proj.shape[0], self.inner)
+        if not chunks or short:
             y = recurrent.state_scan(self.mode, conv, self.inner, self.inner + bn, 0, proj, dt_off, dt_off, self.a_log, self.dt_bias, self.skip, state, 0, slots, step.row_start,
-                                     rows, self.heads, self.groups, self.n, self.n_padded, self.e)
+                                     rows, self.heads, self.groups, self.n, self.n_padded, self.e, below=short, out=y)
         recurrent.gated_group_norm(y, proj, col0, self.norm, self.inner // self.norm_groups, True, self.eps, self.dtype, scale=scale, out=out)
 
 
@@ -308,13 +311,16 @@ class MatrixMemoryMixer(_ScanMixer, Branch):
         i_off = g_off + self.core_width
         gates = recurrent.matrix_memory_gates(proj, i_off, i_off + self.heads, self.b_i, self.b_f, self.cap, state, self.max_off, slots, step.row_start, step.n_rows, self.heads)
         chunks = step.host.get("scan_chunks", 0)
-        if chunks:  # long rows in bfloat16: the tensor cores walk the step in chunks
+        short = recurrent.CHUNKED_RULE_ROWS if chunks and step.host["scan_short_rows"] else 0  # as for the state space
+        y = None
+        if chunks:
             flat = gates.view(proj.shape[0], 4 * self.heads)
             y = recurrent.chunked_scan(recurrent.KIND_GIVEN, proj[:, k_off:], proj[:, col0:], proj[:, v_off:], flat, 3 * self.heads, self.heads, state, 0, slots,
                                        step.extra["scan_chunk_start"], step.extra["scan_chunk_row"], chunks, self.heads, self.heads, self.n, self.n_padded, self.e,
-                                       sums_keys=True, q_scale=self.n ** -0.5, columns=recurrent.matrix_memory_columns(self.e))
-        else:
-            y = recurrent.matrix_memory_scan(proj, k_off, col0, v_off, gates, state, 0, slots, step.row_start, step.n_rows, self.heads, self.n, self.n_padded, self.e, self.n ** -0.5)
+                                       sums_keys=True, q_scale=self.n ** -0.5, columns=recurrent.matrix_memory_columns(self.e), below=short)
+        if not chunks or short:
+            y = recurrent.matrix_memory_scan(proj, k_off, col0, v_off, gates, state, 0, slots, step.row_start, step.n_rows, self.heads, self.n, self.n_padded, self.e, self.n ** -0.5,
+                                             below=short, out=y)
         recurrent.matrix_memory_norm(y, gates, proj, g_off, self.norm, self.e, self.eps, out)
 
 

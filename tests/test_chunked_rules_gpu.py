@@ -104,3 +104,34 @@ def test_rules_in_chunks(rule, shape, steep, monkeypatch):
         for name, one, other in (("outputs", got[here].double(), want), ("state", kept[..., :n].transpose(1, 2), S)):
             assert torch.isfinite(one).all() and (one - other).norm() <= 3e-6 * other.norm(), (name, row, float((one - other).norm() / other.norm()))
         assert not kept[..., n:].any() and torch.equal(state[slot, record:].cpu(), begin[slot, record:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("counts", [[1, 130, 15, 16, 1, 65], [200], [3, 128, 1]])
+def test_short_rows_beside_chunked_ones(counts):
+    """The state-space recurrence in bfloat16-valued chunks with its rows of fewer than 16 tokens left to the token-by-token scan: the same as all rows in the scan, and the chunks touch
+    neither the short rows' outputs nor their states."""
+    heads, n, e = 3, 24, 40
+    tokens, g = sum(counts), torch.Generator().manual_seed(len(counts))
+    x = torch.randn(tokens, 2 * n + heads * e, generator=g).to(torch.bfloat16).float().cuda()
+    gate = torch.randn(tokens, heads, generator=g).cuda()
+    a_log, dt_bias, skip = torch.linspace(-2, 1, heads).cuda(), torch.linspace(-4, 1, heads).cuda(), torch.randn(heads, generator=g).cuda()
+    starts = [sum(counts[:i]) for i in range(len(counts) + 1)]
+    row_start, slots = (torch.tensor(v, dtype=torch.int32).cuda() for v in (starts, list(range(len(counts)))[::-1]))
+    one, many = (torch.randn(len(counts), heads * e * n, generator=torch.Generator().manual_seed(7)).cuda() for _ in range(2))
+    begin = many.clone()
+    cut = recurrent.plan_chunks(counts)
+    chunk_start, chunk_row = (torch.tensor(v, dtype=torch.int32).cuda() for v in cut)
+    want = recurrent.state_scan(recurrent.MODE_STATE_SPACE, x, 0, n, 2 * n, gate, 0, 0, a_log, dt_bias, skip, one, 0, slots, row_start, len(counts), heads, 1, n, n, e)
+    below = recurrent.CHUNKED_RULE_ROWS
+    got = recurrent.chunked_scan(recurrent.KIND_STATE_SPACE, x, x[:, n:], x[:, 2 * n :], gate, 0, 0, many, 0, slots, chunk_start, chunk_row, len(cut[1]), heads, 1, n, n, e, a_log=a_log,
+                                 dt_bias=dt_bias, skip=skip, below=below).view(tokens, heads * e)
+    for row, count in enumerate(counts):
+        assert torch.equal(many[slots[row].long()], begin[slots[row].long()]) == (count < below)
+    got = recurrent.state_scan(recurrent.MODE_STATE_SPACE, x, 0, n, 2 * n, gate, 0, 0, a_log, dt_bias, skip, many, 0, slots, row_start, len(counts), heads, 1, n, n, e, below=below, out=got)
+    for row, count in enumerate(counts):
+        here, slot = slice(starts[row], starts[row + 1]), slots[row].long()
+        if count < below:
+            assert torch.equal(got[here], want[here]) and torch.equal(many[slot], one[slot])
+        else:  # two float computations of the same sums, states and scores as bfloat16 pairs: 2e-5 of the norm
+            assert (got[here] - want[here]).norm() <= 2e-5 * want[here].norm() and (many[slot] - one[slot]).norm() <= 2e-5 * one[slot].norm()
