@@ -283,6 +283,103 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_grouped_rows_kernel(const b
         else stream_tile<ROWS_AT_ONCE>(we, rows, out, count, n, k, act);
     }
 }
+
+// ---------------------------------------------------------------- some rows per expert: the matrices stream into the tensor cores
+// Steps that bring each expert a few rows read the experts' matrices once for them, so they are bound by how many bytes are on their way; the kernel above also spends its float
+// units on every row.  Here a warp owns 16 columns of the result and walks all of k in pieces of 32: a lane asks for 16 bytes of two matrix rows per piece, eight pieces ahead, and they
+// go straight into the fragments of mma.m16n8k16 (a sum over k may take a piece's k in any order; the rows of `a`, in shared memory, are read in the same order).  Nothing but the rows'
+// staging is shared between warps: eight of them, as every row in shared memory takes its bytes from the L1, which holds the loads in flight.  A row's sum has the same shape whatever
+// other rows there are.  Measured over 16 experts of [7168, 4096], two per token, against the kernel above: 32 tokens 133 us (6.2 TB/s), 249 before; 64 tokens 169 us, 389 before;
+// [4096, 3584] and 16 tokens 71 us (6.2 TB/s), 82 before.  With two warps to 16 columns, each over half of k: 145, 195 and 79 us.
+constexpr int STREAM_WARPS = 8, STREAM_COLUMNS = 16 * STREAM_WARPS, STREAM_THREADS = 32 * STREAM_WARPS, AHEAD = 8, PIECE = 32;
+
+__host__ __device__ constexpr int padded_row(int k) {  // 64 bytes past a multiple of 128, so that two rows' 64-byte pieces fall on different banks
+    const int whole = (k + PIECE - 1) / PIECE * PIECE;
+    return whole % 64 == 0 ? whole + 32 : whole;
+}
+__device__ __forceinline__ void multiply(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Columns col0 .. col0 + 15 of `count` (up to 8 TILES) rows in shared memory.
+template <int TILES>
+__device__ __forceinline__ void stream_columns(const bf16* __restrict__ we, const bf16* rows, bf16* __restrict__ c, int col0, int count, int n, int k, int act) {
+    static_assert(TILES == 1 || TILES == 2, "eight or sixteen rows");
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, pieces = (k + PIECE - 1) / PIECE, ld = padded_row(k);
+    const bf16* w0 = we + (size_t)min(col0 + g, n - 1) * k + t * 8;
+    const bf16* w1 = we + (size_t)min(col0 + g + 8, n - 1) * k + t * 8;
+    const bf16* mine[TILES];  // the row a lane reads (the last one for rows that are not there; their products go nowhere)
+#pragma unroll
+    for (int z = 0; z < TILES; ++z) mine[z] = rows + (size_t)min(z * 8 + g, count - 1) * ld + t * 8;
+    float acc[TILES][4];
+#pragma unroll
+    for (int z = 0; z < TILES; ++z) acc[z][0] = acc[z][1] = acc[z][2] = acc[z][3] = 0.f;
+    uint4 lo[AHEAD], hi[AHEAD];
+    auto fetch = [&](int u, int piece) {
+        const int at = piece * PIECE;
+        lo[u] = hi[u] = make_uint4(0, 0, 0, 0);
+        if (at + t * 8 < k) {
+            asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(lo[u].x), "=r"(lo[u].y), "=r"(lo[u].z), "=r"(lo[u].w) : "l"(w0 + at));
+            asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(hi[u].x), "=r"(hi[u].y), "=r"(hi[u].z), "=r"(hi[u].w) : "l"(w1 + at));
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) fetch(u, u);
+    for (int first = 0; first < pieces; first += AHEAD) {
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u) {
+            if (first + u < pieces) {
+#pragma unroll
+                for (int z = 0; z < TILES; ++z) {
+                    const uint4 b = *reinterpret_cast<const uint4*>(mine[z] + (first + u) * PIECE);
+                    multiply(acc[z], lo[u].x, hi[u].x, lo[u].y, hi[u].y, b.x, b.y);
+                    multiply(acc[z], lo[u].z, hi[u].z, lo[u].w, hi[u].w, b.z, b.w);
+                }
+            }
+            fetch(u, first + AHEAD + u);
+        }
+    }
+#pragma unroll
+    for (int z = 0; z < TILES; ++z)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = z * 8 + 2 * t + (i & 1), column = col0 + g + 8 * (i >> 1);
+            if (row < count && column < n) c[(size_t)row * n + column] = __float2bfloat16_rn(activated(acc[z][i], act));
+        }
+}
+
+// row_token: null, or the row of `a` that stands in a slot (the rows then need not be gathered first).  at_once: rows in shared memory, up to 16.
+__global__ void __launch_bounds__(STREAM_THREADS, 2) gemm_grouped_stream_kernel(const bf16* __restrict__ a, int a_stride, const int* __restrict__ row_token,
+                                                                           const bf16* __restrict__ w, bf16* __restrict__ c, const int* __restrict__ tile_expert,
+                                                                           const int* __restrict__ tile_rows, int pad, int at_once, int n, int k, int act) {
+    extern __shared__ __align__(16) unsigned char rows_raw[];
+    bf16* rows = reinterpret_cast<bf16*>(rows_raw);  // [at_once, padded_row(k)]
+    let_next_kernel_start();
+    wait_for_previous_kernels();  // the tile list and the rows come from the kernels before
+    const int tile = blockIdx.y;
+    const int expert = tile_expert[tile];
+    if (expert < 0) return;
+    const int real = tile_rows[tile], ld = padded_row(k), chunks = (k + PIECE - 1) / PIECE * (PIECE / 8);  // 16-byte pieces of a row
+    const bf16* we = w + (size_t)expert * n * k;
+    const int col0 = (blockIdx.x * STREAM_WARPS + (threadIdx.x >> 5)) * 16;
+    for (int first = 0; first < real; first += at_once) {
+        const int count = min(at_once, real - first);
+        if (first) __syncthreads();
+        for (int e = threadIdx.x; e < count * chunks; e += STREAM_THREADS) {
+            const int r = e / chunks, piece = e - r * chunks, slot = tile * pad + first + r;
+            uint4 value = make_uint4(0, 0, 0, 0);
+            if (piece * 8 < k) value = *reinterpret_cast<const uint4*>(a + (size_t)(row_token ? row_token[slot] : slot) * a_stride + piece * 8);
+            *reinterpret_cast<uint4*>(rows + (size_t)r * ld + piece * 8) = value;
+        }
+        __syncthreads();
+        if (col0 >= n) continue;
+        bf16* out = c + (size_t)(tile * pad + first) * n;
+        if (count <= 8) stream_columns<1>(we, rows, out, col0, count, n, k, act);
+        else stream_columns<2>(we, rows, out, col0, count, n, k, act);
+    }
+}
 }  // namespace
 
 // a [rows, k] and c [rows, n] dense bfloat16 (rows a multiple of 128), w [experts, n, k] dense bfloat16, k a multiple of 8.
@@ -321,4 +418,25 @@ HB_EXPORT int hb_moe_gemm_rows(const void* a, int a_stride, const int* row_token
     const dim3 grid((n + COLUMNS_PER_BLOCK - 1) / COLUMNS_PER_BLOCK, rows / pad);
     return launch_after_previous(gemm_grouped_rows_kernel, grid, dim3(ROWS_THREADS), shared, stream, (const bf16*)a, a_stride, row_token, (const bf16*)w, (bf16*)c, tile_expert,
                                  tile_rows, pad, n, k, act);
+}
+
+// The same with some rows per expert: `most` real rows per tile at the most, any number of rows and columns.  row_token (or null): the row of `a` that stands in
+// a slot, rows a_stride elements apart.
+HB_EXPORT int hb_moe_gemm_stream(const void* a, int a_stride, const int* row_token, const void* w, void* c, const int* tile_expert, const int* tile_rows, int pad, int most, int rows, int n,
+                               int k, int act, cudaStream_t stream) {
+    if (rows <= 0 || n <= 0) return 0;
+    if (k <= 0 || pad <= 0 || most <= 0 || rows % pad || (k % 8) || (a_stride % 8) || !tile_expert || !tile_rows) return HB_BAD_ARGUMENT;
+    if ((((uintptr_t)a | (uintptr_t)w) & 15)) return HB_BAD_ARGUMENT;
+    const size_t per_row = (size_t)padded_row(k) * sizeof(bf16);
+    // shared memory for no more rows than a tile can have: what is left decides how many blocks, and bytes on their way, an SM holds
+    const int limit = most < pad ? most : pad, at_once = limit > 8 && 16 * per_row <= 100 * 1024 ? (limit < 16 ? limit : 16) : (limit < 8 ? limit : 8);
+    const size_t shared = at_once * per_row;
+    if ((size_t)8 * k * sizeof(bf16) > 200 * 1024 || rows / pad > 65535) return HB_UNSUPPORTED_SIZE;
+    if (shared > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const dim3 grid((n + STREAM_COLUMNS - 1) / STREAM_COLUMNS, rows / pad);
+    return launch_after_previous(gemm_grouped_stream_kernel, grid, dim3(STREAM_THREADS), shared, stream, (const bf16*)a, a_stride, row_token, (const bf16*)w, (bf16*)c, tile_expert,
+                                 tile_rows, pad, at_once, n, k, act);
 }

@@ -14,6 +14,7 @@ from .native import KernelError, check, f32, i32, is_bf16, library, ptr, require
 PAD = 128  # an expert's rows are padded to whole tiles of this many rows
 STREAM_ROWS = 8  # rows the streaming kernel takes at once
 FEW_PAIRS = 128  # steps of at most this many (token, choice) pairs stream the matrices of the experts they use instead of taking tensor-core tiles
+SOME_ROWS = 2  # (token, choice) pairs per expert from which on the streamed matrices go through the tensor cores
 
 
 @dataclass
@@ -148,9 +149,15 @@ def grouped_linear(a: torch.Tensor, w: torch.Tensor, where: Plan, activation: st
     if takes_tensor_cores(a, w):
         lib = library("moe_gemm_tcgen05")
         if where.pairs <= FEW_PAIRS:
-            check(lib.hb_moe_gemm_rows(ptr(a), i32(a.shape[1]), ptr(where.slot_token if ungathered else None), ptr(w), ptr(out), ptr(where.tile_expert),
-                                       ptr(where.tile_rows), i32(where.pad), i32(where.capacity), i32(w.shape[1]),
-                                       i32(w.shape[2]), act, stream_ptr()), "moe_gemm_rows")
+            # From two rows per expert on (if the choices spread) the tensor cores' kernel: at one, its blocks of 128 columns leave a short last wave (11 matrices of
+            # [3584, 4096]: 67 us, 54 with the other); at two it takes 71 us where the other takes 82 ([4096, 3584], 14 of them).
+            some = where.pairs >= SOME_ROWS * w.shape[0]
+            operands = (ptr(a), i32(a.shape[1]), ptr(where.slot_token if ungathered else None), ptr(w), ptr(out), ptr(where.tile_expert), ptr(where.tile_rows), i32(where.pad))
+            sizes = (i32(where.capacity), i32(w.shape[1]), i32(w.shape[2]), act, stream_ptr())
+            if some:
+                check(lib.hb_moe_gemm_stream(*operands, i32(-(-where.pairs // where.top)), *sizes), "moe_gemm_stream")
+            else:
+                check(lib.hb_moe_gemm_rows(*operands, *sizes), "moe_gemm_rows")
         else:
             check(lib.hb_moe_gemm_tiles(ptr(a), ptr(w), ptr(out), ptr(where.tile_expert), i32(where.capacity), i32(w.shape[0]), i32(w.shape[1]),
                                         i32(w.shape[2]), act, ptr(status_word(a.device)), stream_ptr()), "moe_gemm_tiles")

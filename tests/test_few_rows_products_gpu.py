@@ -1,0 +1,36 @@
+"""Products of steps that bring every expert a few rows, against 64 bits."""
+import pytest
+import torch
+
+from hyperion_b200.ops import moe
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("activation", [None, "relu_squared"])
+@pytest.mark.parametrize("streams", [True, False])
+@pytest.mark.parametrize("tokens,top,experts,n,k", [
+    (4, 2, 4, 128, 64), (8, 1, 4, 16, 32),          # the least that takes the kernel: two rows per expert; one warp's columns
+    (17, 2, 5, 130, 40), (20, 2, 4, 259, 1000),     # columns and k that end inside a warp's and a piece's
+    (9, 1, 1, 64, 8), (33, 1, 1, 48, 264),          # nine rows of one expert, thirty-three: several passes over a tile
+    (64, 2, 16, 300, 2056),                         # the most pairs
+    (3, 2, 16, 96, 520), (7, 2, 8, 33, 24),         # fewer: the other kernel
+    (16, 1, 1, 24, 6400),                           # rows too long for sixteen in shared memory
+])
+def test_few_rows_per_expert(tokens, top, experts, n, k, streams, activation):
+    g = torch.Generator("cuda").manual_seed(tokens * 1000 + k)
+    x = torch.randn(tokens, k, device="cuda", generator=g).to(torch.bfloat16)
+    w = (torch.randn(experts, n, k, device="cuda", generator=g) / k**0.5).to(torch.bfloat16)
+    chosen = torch.stack([torch.randperm(experts, device="cuda", generator=g)[:top] for _ in range(tokens)]).to(torch.int32)
+    where = moe.plan(chosen, None, experts, streams)
+    assert where.streams == streams
+    rows = x if streams else moe.gather(x, where)
+    slots = where.slot_of.view(tokens, top).long()
+    got = moe.grouped_linear(rows, w, where, activation)[slots].double()
+    per_choice = w.double()[chosen.long()]
+    want = torch.einsum("tk,tjnk->tjn", x.double(), per_choice)
+    # every one of k exact products is added once in float (half a unit per addition, a whole one where the sum is cut off), and the result is rounded to bfloat16
+    room = torch.einsum("tk,tjnk->tjn", x.double().abs(), per_choice.abs()) * k * 2.0**-23
+    if activation:
+        want, room = want.clamp(min=0).square(), 2 * want.abs() * room + room.square()
+    assert ((got - want).abs() <= room + want.abs() * 2.0**-8 + 1e-30).all()
