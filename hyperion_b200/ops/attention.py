@@ -323,13 +323,22 @@ def latent_supported(record: int, value: int) -> bool:
     return record % 16 == 0 and value % 8 == 0 and 0 < value <= record <= LATENT_LARGEST_RECORD
 
 
-def choose_latent_shape(rows: int, longest_count: int, heads: int, longest_context: int, sms: int | None = None) -> tuple[bool, int]:
-    """(blocks of 32 rows instead of 16, splits of the keys): 32 rows as soon as one request brings more than 16 (token, head) pairs;
-    the keys are split only when the blocks would leave most of the device idle, into shares of at least two key tiles."""
-    wide = longest_count * heads > 16
+def latent_two_sets(record: int) -> bool:
+    """Whether two sets of 32 rows and two key tiles fit a block's shared memory (``TWO_SETS`` of the kernel)."""
+    return record % 64 == 0 and record <= 576
+
+
+def choose_latent_shape(rows: int, longest_count: int, heads: int, longest_context: int, sms: int | None = None, record: int = 0) -> tuple[int, int]:
+    """(a block's rows: 0 for 16, 1 for 32, 2 for two sets of 32; splits of the keys): 32 rows as soon as one request brings more than 16
+    (token, head) pairs; the keys are split only when the blocks would leave most of the device idle, into shares of at least two key tiles."""
+    wide = int(longest_count * heads > 16)
+    sms = sms or sm_count()
+    # two sets per block pay from one and a half blocks of 64 rows per SM on: at 250 blocks 99 us (134 with 32 rows each), at 150 they leave half the
+    # schedulers idle at the end (68 us, 64 with 32 rows; 16 heads of 576-entry records, 1,000 and 600 tokens)
+    if record and latent_two_sets(record) and 2 * rows * -(-longest_count * heads // 64) >= 3 * sms:
+        return 2, 1
     blocks = rows * -(-longest_count * heads // (32 if wide else 16))
     key_tiles = -(-longest_context // KEY_TILE)
-    sms = sms or sm_count()
     if 2 * blocks > sms:
         return wide, 1
     return wide, max(1, min(sms // blocks, key_tiles // 2, 64))
@@ -337,7 +346,7 @@ def choose_latent_shape(rows: int, longest_count: int, heads: int, longest_conte
 
 def attention_latent(query: torch.Tensor, heads: int, record: int, value: int, cache: torch.Tensor, block_table: torch.Tensor, row_start: torch.Tensor,
                      positions: torch.Tensor, n_rows: int, longest_count: int, longest_context: int, scale: float, sinks: torch.Tensor | None = None,
-                     out: torch.Tensor | None = None, workspace: torch.Tensor | None = None, shape: tuple[bool, int] | None = None) -> torch.Tensor:
+                     out: torch.Tensor | None = None, workspace: torch.Tensor | None = None, shape: tuple[int, int] | None = None) -> torch.Tensor:
     """Causal attention of ``heads`` query heads over one shared key/value head: ``query`` [tokens, heads * record] bfloat16 meets the
     records of ``cache`` [pages, 1, page_size, record]; a record's first ``value`` entries are its value.  ``row_start`` [rows + 1] int32:
     the tokens of each request row (consecutive positions); ``longest_count`` the most tokens of a row and ``longest_context`` the
@@ -355,7 +364,7 @@ def attention_latent(query: torch.Tensor, heads: int, record: int, value: int, c
         out = torch.empty((tokens, heads * value), dtype=torch.bfloat16, device=query.device)
     elif out.dtype != torch.bfloat16 or out.shape[0] != tokens or out.shape[1] < heads * value or out.stride(1) != 1:
         raise KernelError("attention_latent: the output is a bfloat16 [tokens, >= heads * value] view")
-    wide, splits = shape if shape is not None else choose_latent_shape(n_rows, longest_count, heads, longest_context)
+    wide, splits = shape if shape is not None else choose_latent_shape(n_rows, longest_count, heads, longest_context, record=record)
     if splits > 1:
         need = tokens * heads * splits * (value + 2)
         if workspace is None:
@@ -366,7 +375,7 @@ def attention_latent(query: torch.Tensor, heads: int, record: int, value: int, c
     check(library("attention_latent", HB_RECORD=record, HB_VALUE=value).hb_attention_latent(
         ptr(query), i32(query.stride(0)), ptr(out), i32(out.stride(0)), ptr(workspace if splits > 1 else None), ptr(cache), ptr(block_table),
         i32(block_table.shape[1]), ptr(row_start), ptr(positions), ptr(sinks), i32(tokens), i32(n_rows), i32(longest_count), i32(heads), i32(page_size),
-        i32(pages), i32(splits), i32(1 if wide else 0), f32(scale), ptr(status_word(query.device)), stream_ptr()), "attention_latent")
+        i32(pages), i32(splits), i32(1 << int(wide)), f32(scale), ptr(status_word(query.device)), stream_ptr()), "attention_latent")
     if splits > 1:
         from . import native
 

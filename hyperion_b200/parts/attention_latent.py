@@ -16,7 +16,7 @@ Per step: one product for both down-projections (kept in float); one kernel that
 and writes the record to its page (``csrc/heads_prepare.cu``); the queries' up-projection; the batched product with K_h; one
 kernel that puts the query of every head together (rotating its rotated part); attention; the batched product with V_h; the
 output projection.  In bfloat16, with records of a multiple of 16 entries and latents of a multiple of 8, attention runs on the
-tensor cores (``csrc/attention_latent.cu``: blocks of 16 or 32 (token, head) pairs over key tiles of 64 records, the keys split over
+tensor cores (``csrc/attention_latent.cu``: blocks of 16, 32 or 64 (token, head) pairs over key tiles of 64 records, the keys split over
 several blocks when a step brings few tokens).  Everything else, and float32, runs in ``csrc/attention_generic.cu``.
 
 Parameters: ``hidden_size``, ``heads``, ``head_dim``, ``rot_dim``, ``value_dim``, ``kv_rank``, ``q_rank``, ``scale``, ``position`` (a PartSpec
