@@ -15,7 +15,8 @@
 //      same key tile, transposed by ldmatrix, as B fragments.
 // A tile's score phase alone reads 36 KB of fragments per warp from shared memory and its three phases meet at barriers, so one set of eight warps leaves the SM waiting
 // (16 heads over 1,531 tokens of 576-entry records: 277 us, 146 TFLOP/s).  Where a step has the rows for it, a block holds two sets of 32 rows and eight warps each that
-// share the key tiles and meet only where a tile changes hands: 222 us; 471 -> 353 us at 2,048 tokens, 963 -> 705 us with 32 heads.
+// share the key tiles and meet only where a tile changes hands: 222 us; 471 -> 353 us at 2,048 tokens, 963 -> 705 us with 32 heads; 1,000 tokens beside seven decoded ones
+// behind 1,500: 144 -> 107 us (a decoded token leaves the block's second set without rows: it only copies).
 // With splits > 1 a block walks only its share of the key tiles and leaves an unnormalised result with its maximum and sum in a
 // workspace; a second kernel merges the shares.  A row's result depends on the positions of the key tiles only, never on how the
 // request was cut into steps or on the rest of the batch.
@@ -196,6 +197,7 @@ __global__ void __launch_bounds__(SETS * WARPS * 32, 1) attention_latent_kernel(
         if (tile + 1 < tile_hi) load_tile(next, buf ^ 1);
         copies_commit();
         next = look_up(tile + 2);
+        if (SETS > 1 && set_f >= total) continue;  // a set without a row helps with the copies only
         const __nv_bfloat16* kb = kbuf + (size_t)buf * BN * STRIDE;
 
         // 1. scores of 16 rows against 8 * SN keys: fragments are fetched ahead of the products that use them, and several sets of accumulators

@@ -328,14 +328,16 @@ def latent_two_sets(record: int) -> bool:
     return record % 64 == 0 and record <= 576
 
 
-def choose_latent_shape(rows: int, longest_count: int, heads: int, longest_context: int, sms: int | None = None, record: int = 0) -> tuple[int, int]:
+def choose_latent_shape(rows: int, longest_count: int, heads: int, longest_context: int, sms: int | None = None, record: int = 0,
+                        tokens: int = 0) -> tuple[int, int]:
     """(a block's rows: 0 for 16, 1 for 32, 2 for two sets of 32; splits of the keys): 32 rows as soon as one request brings more than 16
-    (token, head) pairs; the keys are split only when the blocks would leave most of the device idle, into shares of at least two key tiles."""
+    (token, head) pairs; the keys are split only when the blocks would leave most of the device idle, into shares of at least two key tiles.
+    ``record`` and ``tokens`` (the step's, all requests together) are wanted for two sets."""
     wide = int(longest_count * heads > 16)
     sms = sms or sm_count()
     # two sets per block pay from one and a half blocks of 64 rows per SM on: at 250 blocks 99 us (134 with 32 rows each), at 150 they leave half the
-    # schedulers idle at the end (68 us, 64 with 32 rows; 16 heads of 576-entry records, 1,000 and 600 tokens)
-    if record and latent_two_sets(record) and 2 * rows * -(-longest_count * heads // 64) >= 3 * sms:
+    # schedulers idle at the end (68 us, 64 with 32 rows; 16 heads of 576-entry records, 1,000 and 600 tokens).  Requests of fewer than 32 pairs would leave a set's rows empty.
+    if record and latent_two_sets(record) and tokens * heads >= max(96 * sms, 32 * rows):
         return 2, 1
     blocks = rows * -(-longest_count * heads // (32 if wide else 16))
     key_tiles = -(-longest_context // KEY_TILE)
@@ -364,7 +366,7 @@ def attention_latent(query: torch.Tensor, heads: int, record: int, value: int, c
         out = torch.empty((tokens, heads * value), dtype=torch.bfloat16, device=query.device)
     elif out.dtype != torch.bfloat16 or out.shape[0] != tokens or out.shape[1] < heads * value or out.stride(1) != 1:
         raise KernelError("attention_latent: the output is a bfloat16 [tokens, >= heads * value] view")
-    wide, splits = shape if shape is not None else choose_latent_shape(n_rows, longest_count, heads, longest_context, record=record)
+    wide, splits = shape if shape is not None else choose_latent_shape(n_rows, longest_count, heads, longest_context, record=record, tokens=tokens)
     if splits > 1:
         need = tokens * heads * splits * (value + 2)
         if workspace is None:

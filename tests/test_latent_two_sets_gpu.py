@@ -4,9 +4,8 @@ import torch
 
 from hyperion_b200.ops import attention as fast
 
-pytestmark = pytest.mark.gpu
 
-
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads,record,value,page", [(16, 576, 512, 32), (5, 320, 256, 16), (7, 64, 56, 8), (32, 128, 64, 16)])
 @pytest.mark.parametrize("with_sink", [False, True])
 def test_two_sets_equal_one(heads, record, value, page, with_sink):
@@ -32,8 +31,16 @@ def test_two_sets_equal_one(heads, record, value, page, with_sink):
         assert torch.equal(one, two), splits
 
 
-def test_rule():
-    assert fast.choose_latent_shape(1, 2048, 16, 2048, sms=148, record=576) == (2, 1)
-    assert fast.choose_latent_shape(1, 2048, 16, 2048, sms=148, record=592) == (1, 1)  # no room, or no whole 128 bytes
-    assert fast.choose_latent_shape(1, 2048, 16, 2048, sms=148, record=560) == (1, 1)
-    assert fast.choose_latent_shape(8, 1, 16, 2048, sms=148, record=576) == (0, 16)
+@pytest.mark.parametrize("asked,shape", [
+    ((1, 2048, 16, 2048, 576, 2048), (2, 1)),
+    ((1, 2048, 16, 2048, 592, 2048), (1, 1)),  # no room for two sets
+    ((1, 2048, 16, 2048, 560, 2048), (1, 1)),  # records of no whole 128 bytes
+    ((1, 600, 16, 600, 576, 600), (1, 1)),     # too few blocks of 64 rows
+    ((8, 1, 16, 2048, 576, 8), (0, 16)),       # decoded tokens
+    ((1000, 1, 16, 2048, 576, 1000), (0, 1)),  # many of them: sixteen pairs each
+    ((9, 100, 16, 2048, 576, 108), (1, 1)),    # a short prompt beside decoded tokens
+    ((8, 1000, 16, 2048, 576, 1007), (2, 1)),  # a long one
+])
+def test_rule(asked, shape):
+    *sizes, record, tokens = asked
+    assert fast.choose_latent_shape(*sizes, sms=148, record=record, tokens=tokens) == shape
