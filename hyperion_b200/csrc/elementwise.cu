@@ -824,23 +824,53 @@ HB_EXPORT int hb_norm_add_norm(float* h, const void* y, int y_is_bf16, const flo
     return launch_status();
 }
 
-// ---------------------------------------------------------------- GELU in its tanh form
-// out = 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))), in float, rounded once.
-template <typename T>
-__global__ void gelu_tanh_kernel(const T* __restrict__ x, T* __restrict__ out, size_t count) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-        const float z = to_float(x[i]);
-        out[i] = from_float<T>(0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))));
+// ---------------------------------------------------------------- GELU, in its tanh and its exact form
+// out = 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))) or 0.5 z (1 + erf(z / sqrt(2))), in float, rounded once.
+struct GeluTanh {
+    static __device__ __forceinline__ float of(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
+};
+struct GeluErf {
+    static __device__ __forceinline__ float of(float z) { return 0.5f * z * (1.f + erff(z * 0.7071067811865476f)); }
+};
+
+template <typename T, typename GELU>
+__global__ void gelu_kernel(const T* __restrict__ x, T* __restrict__ out, size_t count) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) out[i] = from_float<T>(GELU::of(to_float(x[i])));
+}
+
+// Eight entries per thread and access, for 16-byte aligned tensors of a multiple of eight entries: two bytes per access kept the chip waiting on accesses, not on bytes or on erf
+// (6,144 x 2,048: exact form 31 -> 16 us, tanh 30 -> 14; 16 x 8,192: 1.7 -> 1.5).
+template <typename GELU>
+__global__ void gelu_bf16x8_kernel(const uint4* __restrict__ x, uint4* __restrict__ out, size_t eights) {
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < eights; i += (size_t)gridDim.x * blockDim.x) {
+        uint4 raw = x[i];
+        __nv_bfloat162* pairs = reinterpret_cast<__nv_bfloat162*>(&raw);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 f = __bfloat1622float2(pairs[k]);
+            pairs[k] = __floats2bfloat162_rn(GELU::of(f.x), GELU::of(f.y));
+        }
+        out[i] = raw;
     }
 }
 
-HB_EXPORT int hb_gelu_tanh(const void* x, void* out, int is_bf16, long long count, cudaStream_t stream) {
+template <typename GELU>
+int launch_gelu(const void* x, void* out, int is_bf16, long long count, cudaStream_t stream) {
     if (count <= 0) return 0;
-    const int blocks = (int)((count + 255) / 256 < 8192 ? (count + 255) / 256 : 8192);
-    if (is_bf16) gelu_tanh_kernel<<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, (size_t)count);
-    else gelu_tanh_kernel<<<blocks, 256, 0, stream>>>((const float*)x, (float*)out, (size_t)count);
-    return launch_status();
+    const bool eights = is_bf16 && count % 8 == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0;
+    const long long items = eights ? count / 8 : count, wanted = (items + 255) / 256;
+    const dim3 blocks((unsigned)(wanted < 16384 ? wanted : 16384));
+    if (eights) return launch_after_previous(gelu_bf16x8_kernel<GELU>, blocks, dim3(256), 0, stream, (const uint4*)x, (uint4*)out, (size_t)items);
+    if (is_bf16) return launch_after_previous(gelu_kernel<__nv_bfloat16, GELU>, blocks, dim3(256), 0, stream, (const __nv_bfloat16*)x, (__nv_bfloat16*)out, (size_t)count);
+    return launch_after_previous(gelu_kernel<float, GELU>, blocks, dim3(256), 0, stream, (const float*)x, (float*)out, (size_t)count);
 }
+
+HB_EXPORT int hb_gelu_tanh(const void* x, void* out, int is_bf16, long long count, cudaStream_t stream) { return launch_gelu<GeluTanh>(x, out, is_bf16, count, stream); }
+HB_EXPORT int hb_gelu_erf(const void* x, void* out, int is_bf16, long long count, cudaStream_t stream) { return launch_gelu<GeluErf>(x, out, is_bf16, count, stream); }
 
 // ---------------------------------------------------------------- a sigmoid gate on rows, in place
 // x[t, c] <- x[t, c] * scale * sigmoid(gate[t, gate_off + c]) for c < width; the gate is float, the product is rounded once.
@@ -1080,24 +1110,8 @@ HB_EXPORT int hb_clamped_glu(const void* gate_up, void* out, int is_bf16, int to
     return launch_status();
 }
 
-// ---------------------------------------------------------------- GELU in its exact form, and a scale in place
-// out = 0.5 z (1 + erf(z / sqrt(2))), in float, rounded once.  hb_scale_rows: x <- x * scale over a dense float tensor.
-template <typename T>
-__global__ void gelu_erf_kernel(const T* __restrict__ x, T* __restrict__ out, size_t count) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-        const float z = to_float(x[i]);
-        out[i] = from_float<T>(0.5f * z * (1.f + erff(z * 0.7071067811865476f)));
-    }
-}
-
-HB_EXPORT int hb_gelu_erf(const void* x, void* out, int is_bf16, long long count, cudaStream_t stream) {
-    if (count <= 0) return 0;
-    const int blocks = (int)((count + 255) / 256 < 8192 ? (count + 255) / 256 : 8192);
-    if (is_bf16) gelu_erf_kernel<<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, (size_t)count);
-    else gelu_erf_kernel<<<blocks, 256, 0, stream>>>((const float*)x, (float*)out, (size_t)count);
-    return launch_status();
-}
-
+// ---------------------------------------------------------------- a scale in place
+// hb_scale_rows: x <- x * scale over a dense float tensor.
 __global__ void scale_rows_kernel(float* __restrict__ x, float scale, size_t count) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) x[i] *= scale;
 }
