@@ -386,6 +386,7 @@ __global__ void __launch_bounds__(THREADS) prepare_chunks_kernel(const Args a) {
         // are made in float by substitution, a column per lane; the rest are products, in which a warp keeps to columns of its own.
         constexpr int XLD = 2 * LD, WIDE = XLD - 8, ILD = SUB + 4;
         float* xs = qs;  // [64][WIDE columns at a time], over the queries and the keys that have been written out
+        __syncthreads();  // a diagonal block of L may be another warp's pair
         if (warp < SUBS && lane < SUB) {
             const float* lower = at + warp * SUB * TLD + warp * SUB;
             float column[SUB];

@@ -107,6 +107,29 @@ def test_rules_in_chunks(rule, shape, steep, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("steep", [False, True])
+@pytest.mark.parametrize("rule", [recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA])
+def test_delta_rules_give_the_same_bits_again(rule, steep):
+    """A chunk's triangular system is put together by all warps and solved by others: 976 chunks of many heads, last chunks of 17, 33 and 64 tokens (fewer pairs to make before the
+    solution starts), sub-blocks with and without steep decays, twelve times over; every time the same bits in outputs and states."""
+    heads, n, e, counts = 16, 128, 64, [2048 + 17, 1024 + 33, 640]
+    tokens, g = sum(counts), torch.Generator("cuda").manual_seed(rule)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)  # noqa: E731
+    entries = heads * n if rule == recurrent.RULE_CHANNEL_DELTA else heads
+    x, pre, step, rate = rnd(tokens, heads * (2 * n + e)), rnd(tokens, entries), rnd(tokens, heads), torch.linspace(0, 2.7, heads, device="cuda")
+    bias, begin, slots = rnd(entries) * 0.5 + (2 if steep else -3), rnd(len(counts), heads * e * n), torch.arange(len(counts), dtype=torch.int32, device="cuda")
+    table, walks, _ = recurrent.plan_rule_chunks(counts)
+    table, walks = (torch.tensor(t, dtype=torch.int32, device="cuda") for t in (table, walks))
+    first = None
+    for _ in range(12):
+        state = begin.clone()
+        out = recurrent.chunked_rule(rule, x[:, heads * n :], x, x[:, 2 * heads * n :], pre, 0, step, 0, rate, bias, state, 0, slots, table, table.numel() // 2, walks, len(counts), heads, heads, n, n,
+                                     e, n ** -0.5)
+        first = first or (out, state)
+        assert torch.equal(out, first[0]) and torch.equal(state, first[1]) and torch.isfinite(out).all()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("counts", [[1, 130, 15, 16, 1, 65], [200], [3, 128, 1]])
 def test_short_rows_beside_chunked_ones(counts):
     """The state-space recurrence in bfloat16-valued chunks with its rows of fewer than 16 tokens left to the token-by-token scan: the same as all rows in the scan, and the chunks touch
