@@ -7,7 +7,8 @@
 //     S_end = A(0, end] S0 + sum_j (A(j, end] k_j) u_j^T                              (no rule: u = v; wkv: the query's decay ends a token earlier).
 // prepare_chunks works on all chunks side by side: it makes the small matrices and solves the triangular system for [b K | b V], so that a chunk's
 // u = U0 - W S0.  walk_chunks carries the state through a row's chunks, a block per head and ETILE value columns: two products of 64 x n and n x 64 per
-// chunk instead of 64 dependent tokens.
+// chunk instead of 64 dependent tokens.  What a token holds reaches later tokens only: a value that is not finite leaves the tokens before it as they are (and those behind it,
+// where an infinity counts, NaN; the scan may keep the infinity).
 //
 // Precision.  The scan that takes the tokens one after another (recurrent.cu: decoded tokens, other sizes, the float32 mode) is what these kernels must not fall behind.
 //  * Products run on the tensor cores over floats cut into three bfloat16 values each, which together are the float; of the nine products the three below 2^-27 of a term are
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(Layout<RULE, N>::THREADS, Layout<RULE, N>::BLO
             double product = 1.0;
 #pragma unroll
             for (int i = 0; i < SUB; ++i) product *= as[(sub * SUB + i) * LD + c];
-            if (product < STEEP) steep[sub] = 1;
+            if (!(product >= STEEP)) steep[sub] = 1;  // a NaN too: the pairs below reach forward only, whatever they hold
             whole[sub * N + c] = (float)product;
         }
         __syncthreads();

@@ -173,6 +173,32 @@ def test_chunks_are_as_close_to_64_bits_as_the_scan(rule, decays):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("rule", [recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA, recurrent.RULE_RETENTION, recurrent.RULE_WKV])
+def test_earlier_tokens_do_not_see_what_is_not_finite(rule, value):
+    """One value, query, key, decay or step of a token in the middle of a block of sixteen in the middle of a chunk: outputs before it are those of the clean inputs, and from it on the same
+    ones are finite as in the token-by-token scan, the state's entries too."""
+    heads, n, e, tokens, t = 2, 64, 32, 200, 64 + 37
+    g = torch.Generator("cuda").manual_seed(rule)
+    given, _ = inputs_for_scan(rule, heads, n, e, tokens, 1, g)
+    begin = torch.randn(1, heads * e * n, device="cuda", generator=g)
+    (clean, _), _ = both_ways(rule, heads, n, e, tokens, given, begin)
+    places = [(0, 5), (0, heads * n + 7), (0, 2 * heads * n + e + 3)]  # a query's entry, a key's, a value's
+    if rule != recurrent.RULE_RETENTION:
+        places.append((1, 1))
+    if rule in (recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA):
+        places.append((1, heads + 1) if rule == recurrent.RULE_DELTA else (2, 1))
+    for which, column in places:
+        spoilt = [x.clone() if isinstance(x, torch.Tensor) else x for x in given]
+        spoilt[which][t, column] = value
+        if rule == recurrent.RULE_DELTA:
+            spoilt[2] = spoilt[1][:, heads:].contiguous()
+        (got, state), (scan, kept) = both_ways(rule, heads, n, e, tokens, spoilt, begin)
+        assert torch.isfinite(got[:t]).all() and (got[:t] - clean[:t]).norm() <= 1e-6 * clean[:t].norm(), (which, column)
+        assert torch.equal(torch.isfinite(got), torch.isfinite(scan)) and torch.equal(torch.isfinite(state), torch.isfinite(kept)), (which, column)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("steep", [False, True])
 @pytest.mark.parametrize("rule", [recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA])
 def test_delta_rules_give_the_same_bits_again(rule, steep):
