@@ -289,18 +289,19 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_grouped_rows_kernel(const b
 // units on every row.  Here a warp owns 16 columns of the result and walks all of k in pieces of 32: a lane asks for 16 bytes of two matrix rows per piece, eight pieces ahead, and they
 // go straight into the fragments of mma.m16n8k16 (a sum over k may take a piece's k in any order; the rows of `a`, in shared memory, are read in the same order).  Nothing but the rows'
 // staging is shared between warps: eight of them, as every row in shared memory takes its bytes from the L1, which holds the loads in flight.  A row's sum has the same shape whatever
-// other rows there are.  Measured over 16 experts of [7168, 4096], two per token, against the kernel above: 32 tokens 133 us (6.2 TB/s), 249 before; 64 tokens 169 us, 389 before;
-// [4096, 3584] and 16 tokens 71 us (6.2 TB/s), 82 before.  With two warps to 16 columns, each over half of k: 145, 195 and 79 us.
+// other rows there are.  Measured over 16 experts of [7168, 4096], two per token, against the kernel above: 32 tokens 139 us (5.9 TB/s), 249 before; 64 tokens 180 us, 389 before;
+// [4096, 3584] and 16 tokens 75 us (5.9 TB/s), 82 before.  (In one running sum of the tensor cores, which loses to the kernel above in precision: 133, 169 and 71 us; two warps to 16
+// columns, each over half of k: 145, 195 and 79 us; pieces added up two by two: 143, 190 and 77 us.)
 constexpr int STREAM_WARPS = 8, STREAM_COLUMNS = 16 * STREAM_WARPS, STREAM_THREADS = 32 * STREAM_WARPS, AHEAD = 8, PIECE = 32;
 
 __host__ __device__ constexpr int padded_row(int k) {  // 64 bytes past a multiple of 128, so that two rows' 64-byte pieces fall on different banks
     const int whole = (k + PIECE - 1) / PIECE * PIECE;
     return whole % 64 == 0 ? whole + 32 : whole;
 }
-__device__ __forceinline__ void multiply(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+__device__ __forceinline__ void multiply(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // Columns col0 .. col0 + 15 of `count` (up to 8 TILES) rows in shared memory.
@@ -328,14 +329,23 @@ __device__ __forceinline__ void stream_columns(const bf16* __restrict__ we, cons
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) fetch(u, u);
     for (int first = 0; first < pieces; first += AHEAD) {
+        // The tensor cores cut sums off towards zero, so they add up sixteen products and float the rest, in short sums: of four pieces each, then of these
+        float run[2][TILES][4];
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u) {
-            if (first + u < pieces) {
 #pragma unroll
-                for (int z = 0; z < TILES; ++z) {
+            for (int z = 0; z < TILES; ++z) {
+                float one[4] = {}, other[4] = {};
+                if (first + u < pieces) {
                     const uint4 b = *reinterpret_cast<const uint4*>(mine[z] + (first + u) * PIECE);
-                    multiply(acc[z], lo[u].x, hi[u].x, lo[u].y, hi[u].y, b.x, b.y);
-                    multiply(acc[z], lo[u].z, hi[u].z, lo[u].w, hi[u].w, b.z, b.w);
+                    multiply(one, lo[u].x, hi[u].x, lo[u].y, hi[u].y, b.x, b.y);
+                    multiply(other, lo[u].z, hi[u].z, lo[u].w, hi[u].w, b.z, b.w);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float& sum = run[u & 1][z][i];
+                    sum = u < 2 ? one[i] + other[i] : sum + (one[i] + other[i]);
+                    if (u == AHEAD - 1) acc[z][i] += run[0][z][i] + run[1][z][i];
                 }
             }
             fetch(u, first + AHEAD + u);

@@ -15,6 +15,7 @@ PAD = 128  # an expert's rows are padded to whole tiles of this many rows
 STREAM_ROWS = 8  # rows the streaming kernel takes at once
 FEW_PAIRS = 128  # steps of at most this many (token, choice) pairs stream the matrices of the experts they use instead of taking tensor-core tiles
 SOME_ROWS = 2  # (token, choice) pairs per expert from which on the streamed matrices go through the tensor cores
+SOME_COLUMNS = 1024  # of the matrices: only longer sums go through them
 
 
 @dataclass
@@ -150,8 +151,9 @@ def grouped_linear(a: torch.Tensor, w: torch.Tensor, where: Plan, activation: st
         lib = library("moe_gemm_tcgen05")
         if where.pairs <= FEW_PAIRS:
             # From two rows per expert on (if the choices spread) the tensor cores' kernel: at one, its blocks of 128 columns leave a short last wave (11 matrices of
-            # [3584, 4096]: 67 us, 54 with the other); at two it takes 71 us where the other takes 82 ([4096, 3584], 14 of them).
-            some = where.pairs >= SOME_ROWS * w.shape[0]
+            # [3584, 4096]: 67 us, 54 with the other); at two it takes 75 us where the other takes 82 ([4096, 3584], 14 of them).  Its sums of sixteen are cut off, not rounded,
+            # which shorter sums elsewhere make up for in long rows only: a sum's distance from 64 bits is 1.06 times the other kernel's at 512 columns, 1.01 at 1,024, below it from 1,536 on.
+            some = where.pairs >= SOME_ROWS * w.shape[0] and w.shape[2] > SOME_COLUMNS
             operands = (ptr(a), i32(a.shape[1]), ptr(where.slot_token if ungathered else None), ptr(w), ptr(out), ptr(where.tile_expert), ptr(where.tile_rows), i32(where.pad))
             sizes = (i32(where.capacity), i32(w.shape[1]), i32(w.shape[2]), act, stream_ptr())
             if some:

@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
     (3, 2, 16, 96, 520), (7, 2, 8, 33, 24),         # fewer: the other kernel
     (16, 1, 1, 24, 6400),                           # rows too long for sixteen in shared memory
 ])
-def test_few_rows_per_expert(tokens, top, experts, n, k, streams, activation):
+def test_few_rows_per_expert(tokens, top, experts, n, k, streams, activation, monkeypatch):
+    monkeypatch.setattr(moe, "SOME_COLUMNS", 0)  # the kernel takes any, the dispatch gives it the longer ones
     g = torch.Generator("cuda").manual_seed(tokens * 1000 + k)
     x = torch.randn(tokens, k, device="cuda", generator=g).to(torch.bfloat16)
     w = (torch.randn(experts, n, k, device="cuda", generator=g) / k**0.5).to(torch.bfloat16)
@@ -29,8 +30,28 @@ def test_few_rows_per_expert(tokens, top, experts, n, k, streams, activation):
     got = moe.grouped_linear(rows, w, where, activation)[slots].double()
     per_choice = w.double()[chosen.long()]
     want = torch.einsum("tk,tjnk->tjn", x.double(), per_choice)
-    # every one of k exact products is added once in float (half a unit per addition, a whole one where the sum is cut off), and the result is rounded to bfloat16
+    # every one of k exact products is added once in float (half a unit per addition, a whole one where sixteen are cut off), and the result is rounded to bfloat16
     room = torch.einsum("tk,tjnk->tjn", x.double().abs(), per_choice.abs()) * k * 2.0**-23
     if activation:
         want, room = want.clamp(min=0).square(), 2 * want.abs() * room + room.square()
     assert ((got - want).abs() <= room + want.abs() * 2.0**-8 + 1e-30).all()
+
+
+@pytest.mark.parametrize("tokens,k", [(64, 1536), (64, 2048), (64, 4096), (9, 7176)])
+def test_sums_are_as_close_as_without_tensor_cores(tokens, k, monkeypatch):
+    """Every product stands beside its negative somewhere else in the row, so the sums are exactly zero and the results nothing but the sums' roundings (which the result's own rounding to
+    bfloat16 would hide).  Over a thousand columns and more the tensor cores' are not larger than the float units'."""
+    experts, n, top = 4, 1024, 1
+    g = torch.Generator("cuda").manual_seed(k)
+    half = torch.randn(tokens, k // 2, device="cuda", generator=g).to(torch.bfloat16)
+    weights = (torch.randn(experts, n, k // 2, device="cuda", generator=g) / k**0.5).to(torch.bfloat16)
+    places = torch.randperm(k, device="cuda", generator=g)
+    x, w = torch.cat([half, -half], 1)[:, places].contiguous(), torch.cat([weights, weights], 2)[..., places].contiguous()
+    where = moe.plan((torch.arange(tokens, device="cuda", dtype=torch.int32) % experts).view(tokens, top), None, experts, True)
+    assert k > moe.SOME_COLUMNS
+    far = []
+    for rows_per_expert in (0, 1 << 20):  # all steps through the tensor cores, none
+        monkeypatch.setattr(moe, "SOME_ROWS", rows_per_expert)
+        got = moe.grouped_linear(x, w, where)[where.slot_of.view(tokens, top).long()].double()
+        far.append(float(got.square().mean().sqrt()))
+    assert 0 < far[0] <= far[1], far
