@@ -348,7 +348,7 @@ def chunk_planner(dtype: torch.dtype) -> dict:
 
 
 RULE_DELTA, RULE_CHANNEL_DELTA, RULE_RETENTION, RULE_WKV = 0, 1, 2, 3
-SCRATCH_BYTES = 160 << 20  # of chunked_rule: longer steps take it in turns
+SCRATCH_BYTES = 160 << 20  # of chunked_rule at the most: longer steps take it in turns
 # In a step with a long row, rows of fewer tokens go token by token after it: a decoded token in a chunk of its own costs what 64 tokens do (300 tokens and 40
 # decoded ones at 16 heads of 128 x 128: 261 us all in chunks, 200 us all token by token)
 CHUNKED_RULE_ROWS = 16
@@ -394,6 +394,19 @@ def chunked_rule_fits(n: int, e: int) -> bool:
     return 0 < n <= 128 and e > 0 and e % 16 == 0
 
 
+def _scratch_of_chunks(chunks: int, piece: int, device) -> tuple[int, torch.Tensor]:
+    """(chunks at a time, scratch for them at ``piece`` floats each).  The token-by-token scans take no scratch and a cache may have been given all memory but what they need: where the
+    device has no room for so many chunks, fewer go at a time, down to one (some 3 MB at 16 heads of 128 x 128).  Results do not depend on it."""
+    span = max(1, min(chunks, SCRATCH_BYTES // (4 * piece))) if piece else 1
+    while True:
+        try:
+            return span, torch.empty(max(1, span * piece), dtype=torch.float32, device=device)
+        except torch.cuda.OutOfMemoryError:
+            if span == 1:
+                raise
+            span = -(-span // 2)
+
+
 def chunked_rule(rule: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, x: torch.Tensor | None, x_off: int, step: torch.Tensor | None, step_off: int, rate: torch.Tensor,
                  bias: torch.Tensor | None, state: torch.Tensor, state_off: int, slots: torch.Tensor, table: torch.Tensor, chunks: int, walk_table: torch.Tensor, walks: int,
                  heads: int, groups: int, n: int, n_padded: int, e: int, q_scale: float = 1.0) -> torch.Tensor:
@@ -408,8 +421,7 @@ def chunked_rule(rule: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, x
     native = library("chunked_float")
     native.hb_chunked_float_scratch.restype = ctypes.c_longlong
     piece = native.hb_chunked_float_scratch(i32(rule), i32(n), i32(e)) * heads
-    span = max(1, min(chunks, SCRATCH_BYTES // (4 * piece))) if piece else 1
-    scratch = torch.empty(max(1, span * piece), dtype=torch.float32, device=k.device)
+    span, scratch = _scratch_of_chunks(chunks, piece, k.device)
     out = torch.empty((k.shape[0], heads * e), dtype=torch.float32, device=k.device)
     stride = lambda t: i32(t.stride(0) if t is not None else 0)  # noqa: E731
     check(native.hb_chunked_float(i32(rule), ptr(k), stride(k), ptr(q), stride(q), ptr(v), stride(v), ptr(x), stride(x), i32(x_off), ptr(step), stride(step), i32(step_off), ptr(rate),

@@ -21,6 +21,26 @@ def test_the_plan_covers_every_long_row_once():
             assert sum(chunks[2 * begun + 1 : 2 * end : 2]) == counts[row]
 
 
+def test_chunks_go_fewer_at_a_time_where_memory_is_short(monkeypatch):
+    """A device with room for so many floats and no more: as many chunks as fit after halving, one at the least, and an error only where one does not fit."""
+    piece, empty = 1000, torch.empty
+
+    def short_of(room):
+        def allocate(size, **kwargs):
+            if size > room:
+                raise torch.cuda.OutOfMemoryError(f"{size} of {room}")
+            return empty(size, **kwargs)
+        return allocate
+
+    for room, span in ((40_000, 40), (39_999, 20), (11_000, 10), (4_999, 3), (1_000, 1)):
+        monkeypatch.setattr(torch, "empty", short_of(room))
+        got, scratch = recurrent._scratch_of_chunks(40, piece, "cpu")
+        assert got == span and scratch.numel() == span * piece
+    monkeypatch.setattr(torch, "empty", short_of(999))
+    with pytest.raises(torch.cuda.OutOfMemoryError):
+        recurrent._scratch_of_chunks(40, piece, "cpu")
+
+
 def token_by_token(rule, k, q, v, a, beta, S, bonus):
     out = torch.empty_like(v)
     for t in range(k.shape[0]):
