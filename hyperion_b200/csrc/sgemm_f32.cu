@@ -114,13 +114,14 @@ int launch_tiles(const float* a, const float* w, const float* bias, float* c, in
 }  // namespace
 
 // A rows are `lda` floats apart, C rows `ldc`; W is dense [n, k]. Zero padding of the k tail adds
-// exact zeros to the chain and does not change the result.
+// exact zeros to the chain and does not change the result.  sms: the device's multiprocessors.
 HB_EXPORT int hb_sgemm_f32(const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda,
-                           int ldc, cudaStream_t stream) {
+                           int ldc, int sms, cudaStream_t stream) {
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return HB_BAD_ARGUMENT;
-    // large tiles from two to an SM on (394 rows, 9,728 columns: 532 of them 246 us; 896 columns: 49 of them would leave two SMs in three idle) and where rows do not leave half of one empty
+    // large tiles from two to an SM on (148 SMs, 394 rows, 9,728 columns: 532 of them 246 us; 896 columns: 49 of them would leave two SMs in three idle) and where rows do not leave half
+    // of one empty
     const long long large = (long long)((m + 63) / 64) * ((n + 127) / 128);
-    if (m > 32 && large >= 296) return launch_tiles<64, 128, 8, 8, 16, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
+    if (m > 32 && large >= 2LL * sms) return launch_tiles<64, 128, 8, 8, 16, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
     return launch_tiles<32, 32, 4, 4, 32, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
 }

@@ -5,7 +5,7 @@ import ctypes
 
 import torch
 
-from .native import KernelError, check, f32, i32, is_bf16, library, ptr, require_cuda, stream_ptr
+from .native import KernelError, check, f32, i32, is_bf16, library, ptr, require_cuda, sm_count, stream_ptr
 
 _STATUS: dict[int, torch.Tensor] = {}
 STATUS_BITS = {1: "a block-table entry that had to be valid was missing", 2: "a token id outside the vocabulary",
@@ -481,7 +481,7 @@ def sgemm_f32(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None =
     for start in range(0, m, step):
         count = min(step, m - start)
         check(lib.hb_sgemm_f32(ptr(x[start:]), ptr(weight), ptr(bias), ptr(out[start:]), i32(count), i32(n), i32(k),
-                               i32(x.stride(0)), i32(out.stride(0)), stream_ptr()), "sgemm_f32")
+                               i32(x.stride(0)), i32(out.stride(0)), i32(sm_count(x.device)), stream_ptr()), "sgemm_f32")
     return out
 
 

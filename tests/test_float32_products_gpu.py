@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from hyperion_b200 import ops
+from hyperion_b200.ops import basic
 
 pytestmark = pytest.mark.gpu
 
@@ -24,3 +25,19 @@ def test_tiles(m, n, k, aligned):
     for rows in {1, min(m, 30), min(m, 64)}:  # few rows take the small tiles, whatever the whole took
         assert torch.equal(ops.sgemm_f32(x[:rows], w, b), got[:rows])
     assert torch.equal(ops.sgemm_f32(x, w[: min(n, 40)].contiguous(), b[: min(n, 40)].contiguous()), got[:, : min(n, 40)])
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 300, 36), (33, 256, 17), (200, 20000, 64)])
+def test_the_tile_follows_the_device(m, n, k, monkeypatch):
+    """Two large tiles to an SM decide on the tile: on a device of one SM all of these (two such tiles and more) take large ones, on one of a million none does, and the bits are the same."""
+    g = torch.Generator().manual_seed(k)
+    x, w = torch.randn(m, k, generator=g).cuda(), torch.randn(n, k, generator=g).cuda()
+    results = []
+    for sms in (1, 10**6):
+        monkeypatch.setattr(basic, "sm_count", lambda device, sms=sms: sms)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+            results.append(ops.sgemm_f32(x, w))
+            torch.cuda.synchronize()
+        names = [event.name for event in profile.events() if "sgemm_kernel" in event.name]
+        assert names and all(("64, 128" in name) == (sms == 1) for name in names), names
+    assert torch.equal(*results)
