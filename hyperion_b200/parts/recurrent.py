@@ -106,7 +106,7 @@ class ConstantDecay(ChunkedRule):
     """A state that fades by a constant of the head (retention, lightning attention)."""
 
     def _constant_decay_plans(self) -> dict:
-        return {**recurrent.segment_planner(self.dtype), **self._chunk_plans()}
+        return self._chunk_plans() if recurrent.chunked_rule_fits(self.n, self.e) else recurrent.segment_planner(self.dtype)
 
     def _retain(self, proj, k_off, q_off, v_off, cache, step):
         def by_token(below, out):

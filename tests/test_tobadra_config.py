@@ -126,3 +126,13 @@ def test_the_plain_pieces_on_cases_made_by_hand():
     w["correction"] = torch.tensor([-0.6, -0.6, 0.0, 0.0], dtype=torch.float64)  # negative choice scores: an excluded group is not chosen for being "zero"
     chosen, _ = plain.route(scores.log(), w, "", {"top": 2, "scale": 1.0, "groups": {"count": 2, "keep": 1}})
     assert sorted(chosen.tolist()[0]) == [2, 3]
+
+
+@pytest.mark.parametrize("dim, vdim, plans", [(16, 32, {"rule_chunks"}), (14, 9, {"scan_segments"}), (132, 32, {"scan_segments"})])
+def test_a_constant_decay_plans_what_it_walks(dim, vdim, plans):
+    """In bfloat16, heads that the chunks take (a key size up to 128, a value size of whole sixteens) have their long rows planned in chunks, others in segments; neither plans both."""
+    document = copy.deepcopy(DOCUMENT)
+    document["layers"] = [{"type": "lightning", "mixer": {"heads": 2, "dim": dim, "vdim": vdim, "decay": [0.5, 0.9]}, "mlp": None}]
+    entry = get_architecture("Tobadra")
+    model = DecoderModel(entry.build_spec(entry.read_config(document)), torch.bfloat16, torch.device("meta"))
+    assert {key[0] for key in model.step_planners()} == plans
