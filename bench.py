@@ -381,6 +381,19 @@ def timed(fn, reps: int = 10, warmup: int = 3) -> float:
     return statistics.median(times)
 
 
+def rule_walk(rule: int, counts, k, q, v, x, step, step_off: int, rate, bias, state, slots, heads: int, groups: int, n: int, e: int, q_scale: float = 1.0, x_off: int = 0):
+    """The recurrence as the bfloat16 engine walks a step's long rows (one call of ``recurrent.chunked_rule``), or None for steps and heads that it does not take."""
+    import torch
+
+    from hyperion_b200.ops import recurrent
+
+    cut = recurrent.plan_rule_chunks(counts)
+    if cut is None or not recurrent.chunked_rule_fits(n, e):
+        return None
+    table, walks = (torch.tensor(part, dtype=torch.int32, device=k.device) for part in cut[:2])
+    return lambda: recurrent.chunked_rule(rule, k, q, v, x, x_off, step, step_off, rate, bias, state, 0, slots, table, table.numel() // 2, walks, walks.numel() // 3, heads, groups, n, n, e, q_scale)
+
+
 def nunivik_kernels(size: dict, measured: dict) -> dict:
     """The design's own kernels alone at this size, a prompt of 2,048 tokens in one row and 8 rows of one decoded token: time, the bytes
     each must move and, for the scans, the float32 operations, against the measured copy bandwidth (no float32 peak is measured: the
@@ -444,6 +457,10 @@ def nunivik_kernels(size: dict, measured: dict) -> dict:
                                                 len(counts), heads, groups, n, n, e, q_scale=n ** -0.5)
             moved = 4 * (tokens * (2 * groups * n + 2 * heads * e + 2 * heads) + 2 * len(counts) * heads * e * n)
             report(f"{kind}.scan/{shape}", timed(scan), moved, flops=2.0 * (3 if kind == "delta" else 2) * tokens * heads * n * e)
+            walk = kind == "delta" and rule_walk(recurrent.RULE_DELTA, counts, conv[:, k_off:], conv, conv[:, v_off:], proj, proj, step_off, a_log, dt_bias, state, slots, heads, groups, n, e,
+                                                 n ** -0.5, decay_off)
+            if walk:
+                report(f"{kind}.scan_in_chunks/{shape}", timed(walk), moved, flops=6.0 * tokens * heads * n * e)
             o = scan()
             norm_w = torch.ones(e if kind == "delta" else heads * e, device=dev)
             report(f"{kind}.gated_norm/{shape}", timed(lambda: recurrent.gated_group_norm(o, proj, gate_off, norm_w, group_width, gate_first, 1e-6, torch.bfloat16)),
@@ -564,8 +581,11 @@ def mirovik_kernels(size: dict, measured: dict) -> dict:
                                             len(counts), heads, heads, n, n, e)
         report(f"retention.scan/{shape}", timed(scan), 4 * (tokens * (2 * heads * n + 2 * heads * e) + 2 * len(counts) * heads * e * n), fp32_flops=4.0 * tokens * heads * n * e)
         o = scan()
+        walk = rule_walk(recurrent.RULE_RETENTION, counts, proj[:, k_off:], proj, proj[:, v_off:], None, None, 0, decay, None, state, slots, heads, heads, n, e)
+        if walk:
+            report(f"retention.scan_in_chunks/{shape}", timed(walk), 4 * (tokens * (2 * heads * n + 2 * heads * e) + 2 * len(counts) * heads * e * n), fp32_flops=4.0 * tokens * heads * n * e)
         cut = recurrent.plan_segments(counts)
-        if cut is not None:  # the long row in segments side by side, as the bfloat16 engine walks it
+        if cut is not None:  # the long row in segments side by side, as the bfloat16 engine walks heads that no chunk fits
             seg_start, seg_row = torch.tensor(cut[0], dtype=torch.int32, device=dev), torch.tensor(cut[1], dtype=torch.int32, device=dev)
             report(f"retention.scan_in_segments/{shape}", timed(lambda: recurrent.retention_in_segments(proj, k_off, 0, v_off, decay, state, slots, seg_start, seg_row,
                                                                                                          len(cut[1]), heads, n, n, e)),
@@ -769,7 +789,7 @@ def kudazen_kernels(size: dict, measured: dict) -> dict:
         sinks = torch.zeros(l_heads, device=dev)
         latent_flops = 2.0 * seen_all * l_heads * (record + rank)
         latent_bytes = rows * context * record * 2 + tokens * l_heads * (record + rank) * 2
-        l_shape = fast.choose_latent_shape(rows, max(counts), l_heads, context)
+        l_shape = fast.choose_latent_shape(rows, max(counts), l_heads, context, record=record, tokens=tokens)
         l_out = torch.empty(tokens, l_heads * rank, dtype=torch.bfloat16, device=dev)
         l_space = torch.empty(tokens * l_heads * l_shape[1] * (rank + 2), dtype=torch.float32, device=dev)
         report(f"latent.attention/{shape}", timed(lambda: fast.attention_latent(query, l_heads, record, rank, l_cache, table, row_start, positions, rows, max(counts),
@@ -789,6 +809,9 @@ def kudazen_kernels(size: dict, measured: dict) -> dict:
         scan = lambda: recurrent.wkv_scan(k, r, v, d, 0, w0, bonus, state, 0, slots, row_start, rows, w_heads, n, n, n)
         moved = 4 * (tokens * 5 * w_heads * n + 2 * rows * w_heads * n * n)
         report(f"wkv.scan/{shape}", timed(scan), moved, fp32_flops=5.0 * tokens * w_heads * n * n)
+        walk = rule_walk(recurrent.RULE_WKV, counts, k, r, v, d, None, 0, w0, bonus, state, slots, w_heads, w_heads, n, n)
+        if walk:
+            report(f"wkv.scan_in_chunks/{shape}", timed(walk), moved, fp32_flops=5.0 * tokens * w_heads * n * n)
         o = scan()
         report(f"wkv.gated_norm/{shape}", timed(lambda: recurrent.gated_group_norm(o, d, 0, w0, n, False, 1e-6, torch.bfloat16)), tokens * w_heads * n * (4 + 4 + 2))
         kqv = torch.cat([k, r, v], dim=1).contiguous()
@@ -930,6 +953,10 @@ def tobadra_kernels(size: dict, measured: dict) -> dict:
         report(f"channel_delta.scan/{shape}", timed(lambda: recurrent.channel_delta_scan(conv, d_heads * n, 0, 2 * d_heads * n, decay_in, step_in, 0, a_log, dt_bias, state, 0, slots,
                                                                                       row_start, rows, d_heads, d_heads, n, n, e, q_scale=n ** -0.5)),
                scan_bytes, fp32_flops=7.0 * tokens * d_heads * n * e)
+        walk = rule_walk(recurrent.RULE_CHANNEL_DELTA, counts, conv[:, d_heads * n :], conv, conv[:, 2 * d_heads * n :], decay_in, step_in, 0, a_log, dt_bias, state, slots, d_heads, d_heads, n, e,
+                         n ** -0.5)
+        if walk:
+            report(f"channel_delta.scan_in_chunks/{shape}", timed(walk), scan_bytes, fp32_flops=7.0 * tokens * d_heads * n * e)
         report(f"nunivik.delta_scan/{shape}", timed(lambda: recurrent.state_scan(recurrent.MODE_DELTA, conv, d_heads * n, 0, 2 * d_heads * n, step_in, d_heads, 0, a_log, dt_head, None,
                                                                               state, 0, slots, row_start, rows, d_heads, d_heads, n, n, e, q_scale=n ** -0.5)),
                scan_bytes - 4 * tokens * d_heads * n, fp32_flops=6.0 * tokens * d_heads * n * e)
@@ -946,8 +973,11 @@ def tobadra_kernels(size: dict, measured: dict) -> dict:
         l_bytes = 4 * (tokens * (2 * l_heads * ln + 2 * l_heads * le) + 2 * rows * l_heads * le * ln)
         report(f"lightning.scan/{shape}", timed(lambda: recurrent.state_scan(recurrent.MODE_RETENTION, qkv, l_heads * ln, 0, 2 * l_heads * ln, qkv, 0, 0, l_decay, l_decay, None, l_state, 0,
                                                                           slots, row_start, rows, l_heads, l_heads, ln, ln, le)), l_bytes, fp32_flops=4.0 * tokens * l_heads * ln * le)
+        walk = rule_walk(recurrent.RULE_RETENTION, counts, qkv[:, l_heads * ln :], qkv, qkv[:, 2 * l_heads * ln :], None, None, 0, l_decay, None, l_state, slots, l_heads, l_heads, ln, le)
+        if walk:
+            report(f"lightning.scan_in_chunks/{shape}", timed(walk), l_bytes, fp32_flops=4.0 * tokens * l_heads * ln * le)
         cut = recurrent.plan_segments(counts)
-        if cut is not None:  # the long row in segments side by side, as the bfloat16 engine walks it
+        if cut is not None:  # the long row in segments side by side, as the bfloat16 engine walks heads that no chunk fits
             seg_start, seg_row = torch.tensor(cut[0], dtype=torch.int32, device=dev), torch.tensor(cut[1], dtype=torch.int32, device=dev)
             report(f"lightning.scan_in_segments/{shape}", timed(lambda: recurrent.retention_in_segments(qkv, l_heads * ln, 0, 2 * l_heads * ln, l_decay, l_state, slots, seg_start, seg_row,
                                                                                                          len(cut[1]), l_heads, ln, ln, le)), l_bytes,
@@ -1341,6 +1371,9 @@ def biropel_kernels(size: dict, measured: dict) -> dict:
         retention = lambda: recurrent.state_scan(recurrent.MODE_RETENTION, m_proj, m_heads * n, 0, 2 * m_heads * n, m_proj, 0, 0, decay, decay, None, r_state, 0, slots, row_start, rows,
                                                  m_heads, m_heads, n, n, e)
         report(f"mirovik.retention_scan/{shape}", timed(retention), moved, fp32_flops=4.0 * tokens * m_heads * n * e)
+        walk = rule_walk(recurrent.RULE_RETENTION, counts, m_proj[:, m_heads * n :], m_proj, m_proj[:, 2 * m_heads * n :], None, None, 0, decay, None, r_state, slots, m_heads, m_heads, n, e)
+        if walk:
+            report(f"mirovik.retention_in_chunks/{shape}", timed(walk), moved, fp32_flops=4.0 * tokens * m_heads * n * e)
         segments = recurrent.plan_segments(counts)
         if segments is not None:
             seg_start, seg_row = torch.tensor(segments[0], dtype=torch.int32, device=dev), torch.tensor(segments[1], dtype=torch.int32, device=dev)

@@ -328,16 +328,15 @@ def latent_two_sets(record: int) -> bool:
     return record % 64 == 0 and record <= 576
 
 
-def choose_latent_shape(rows: int, longest_count: int, heads: int, longest_context: int, sms: int | None = None, record: int = 0,
-                        tokens: int = 0) -> tuple[int, int]:
+def choose_latent_shape(rows: int, longest_count: int, heads: int, longest_context: int, *, record: int, tokens: int, sms: int | None = None) -> tuple[int, int]:
     """(a block's rows: 0 for 16, 1 for 32, 2 for two sets of 32; splits of the keys): 32 rows as soon as one request brings more than 16
     (token, head) pairs; the keys are split only when the blocks would leave most of the device idle, into shares of at least two key tiles.
-    ``record`` and ``tokens`` (the step's, all requests together) are wanted for two sets."""
+    ``record`` (whether two sets fit) and ``tokens`` (the step's, all requests together) decide on two sets."""
     wide = int(longest_count * heads > 16)
     sms = sms or sm_count()
     # two sets per block pay from one and a half blocks of 64 rows per SM on: at 250 blocks 99 us (134 with 32 rows each), at 150 they leave half the
     # schedulers idle at the end (68 us, 64 with 32 rows; 16 heads of 576-entry records, 1,000 and 600 tokens).  Requests of fewer than 32 pairs would leave a set's rows empty.
-    if record and latent_two_sets(record) and tokens * heads >= max(96 * sms, 32 * rows):
+    if latent_two_sets(record) and tokens * heads >= max(96 * sms, 32 * rows):
         return 2, 1
     blocks = rows * -(-longest_count * heads // (32 if wide else 16))
     key_tiles = -(-longest_context // KEY_TILE)

@@ -7,6 +7,8 @@ import json
 import subprocess
 import sys
 
+import pytest
+
 from helpers import ROOT
 
 
@@ -72,3 +74,12 @@ def test_peaks_come_from_the_measured_file_when_it_is_there(tmp_path, monkeypatc
     (tmp_path / "MEASURED_PEAKS.json").write_text(json.dumps({"hbm_gbs": 6000.0, "bf16_tflops": 1500.0, "bf16_tflops_sustained": 1300.0}))
     peaks, source = bench.peaks()
     assert source == "measured" and peaks["hbm_gbs"] == 6000.0
+
+
+def test_a_latent_shape_is_asked_for_with_everything_it_follows():
+    """The shape of attention over latents follows the record's size and the step's tokens; a caller that leaves them out (the benchmark did) would time another kernel than the engine runs."""
+    from hyperion_b200.ops import attention
+
+    with pytest.raises(TypeError):
+        attention.choose_latent_shape(1, 2048, 16, 2048, sms=148)
+    assert attention.choose_latent_shape(1, 2048, 16, 2048, record=576, tokens=2048, sms=148) == (2, 1)
