@@ -298,6 +298,8 @@ __host__ __device__ constexpr int padded_row(int k) {  // 64 bytes past a multip
     const int whole = (k + PIECE - 1) / PIECE * PIECE;
     return whole % 64 == 0 ? whole + 32 : whole;
 }
+constexpr int STREAM_MOST_K = 200 * 1024 / 16, STREAM_MOST_SHARED = 8 * padded_row(STREAM_MOST_K) * 2;  // eight rows of the longest; sixteen are taken up to 100 KB
+static_assert(STREAM_MOST_SHARED <= 227 * 1024, "an SM's shared memory");
 __device__ __forceinline__ void multiply(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
@@ -441,9 +443,9 @@ HB_EXPORT int hb_moe_gemm_stream(const void* a, int a_stride, const int* row_tok
     // shared memory for no more rows than a tile can have: what is left decides how many blocks, and bytes on their way, an SM holds
     const int limit = most < pad ? most : pad, at_once = limit > 8 && 16 * per_row <= 100 * 1024 ? (limit < 16 ? limit : 16) : (limit < 8 ? limit : 8);
     const size_t shared = at_once * per_row;
-    if ((size_t)8 * k * sizeof(bf16) > 200 * 1024 || rows / pad > 65535) return HB_UNSUPPORTED_SIZE;
-    if (shared > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    if (k > STREAM_MOST_K || rows / pad > 65535) return HB_UNSUPPORTED_SIZE;
+    if (shared > 48 * 1024) {  // always the most that any call takes: another thread's call may come between this and the launch
+        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STREAM_MOST_SHARED);
         if (e != cudaSuccess) return (int)e;
     }
     const dim3 grid((n + STREAM_COLUMNS - 1) / STREAM_COLUMNS, rows / pad);

@@ -1,4 +1,6 @@
 """Products of steps that bring every expert a few rows, against 64 bits."""
+from concurrent.futures import ThreadPoolExecutor
+
 import pytest
 import torch
 
@@ -55,3 +57,17 @@ def test_sums_are_as_close_as_without_tensor_cores(tokens, k, monkeypatch):
         got = moe.grouped_linear(x, w, where)[where.slot_of.view(tokens, top).long()].double()
         far.append(float(got.square().mean().sqrt()))
     assert 0 < far[0] <= far[1], far
+
+
+def test_threads_with_rows_of_different_lengths():
+    """Rows of 4,096 and of 6,400 entries take different amounts of shared memory; two threads that launch both kinds at once must not take each other's allowance away."""
+    def products(k, seed):
+        g = torch.Generator("cuda").manual_seed(seed)
+        x, w = torch.randn(16, k, device="cuda", generator=g).to(torch.bfloat16), (torch.randn(2, 64, k, device="cuda", generator=g) / k**0.5).to(torch.bfloat16)
+        where = moe.plan((torch.arange(16, device="cuda", dtype=torch.int32) % 2).view(16, 1), None, 2, True)
+        want = moe.grouped_linear(x, w, where)[where.slot_of.long()]
+        torch.cuda.synchronize()
+        return all(torch.equal(moe.grouped_linear(x, w, where)[where.slot_of.long()], want) for _ in range(150))
+
+    with ThreadPoolExecutor(2) as pool:
+        assert all(pool.map(products, (4096, 6400), (1, 2)))
