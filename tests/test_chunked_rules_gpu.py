@@ -193,6 +193,24 @@ def test_chunks_are_as_close_to_64_bits_as_the_scan(rule, decays):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n, e", [(128, 128), (64, 32), (100, 96)])
+@pytest.mark.parametrize("rule", [recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA, recurrent.RULE_RETENTION, recurrent.RULE_WKV])
+def test_narrow_and_wide_tiles_of_value_columns_give_the_same_bits(rule, n, e, monkeypatch):
+    """Sixteen value columns to a block while such blocks fit the multiprocessors side by side, else thirty-two: a device of one and one of a million multiprocessors."""
+    heads, tokens = 3, 150
+    g = torch.Generator("cuda").manual_seed(n)
+    given, _ = inputs_for_scan(rule, heads, n, e, tokens, 1, g)
+    begin = torch.randn(1, heads * e * n, device="cuda", generator=g)
+    results = []
+    for sms in (1, 10**6):
+        monkeypatch.setattr(recurrent, "sm_count", lambda device, sms=sms: sms)
+        (out, state), (scan, kept) = both_ways(rule, heads, n, e, tokens, given, begin)
+        assert (out - scan).norm() <= 2e-6 * scan.norm() and (state - kept).norm() <= 2e-6 * kept.norm()  # two float computations, 3e-6 from 64 bits at the most together
+        results.append((out, state))
+    assert all(torch.equal(one, other) for one, other in zip(*results))
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 @pytest.mark.parametrize("rule", [recurrent.RULE_DELTA, recurrent.RULE_CHANNEL_DELTA, recurrent.RULE_RETENTION, recurrent.RULE_WKV])
 def test_earlier_tokens_do_not_see_what_is_not_finite(rule, value):
