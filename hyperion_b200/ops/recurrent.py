@@ -326,6 +326,11 @@ def plan_chunks(counts) -> tuple[list[int], list[int]] | None:
     return starts + [at], rows
 
 
+def _counts_of(rows) -> list[int]:
+    """The tokens of a step's rows as a list: a decode step is planned while the GPU waits for it, and a list's largest is found in a third of the time an array's takes."""
+    return rows.counts.tolist() if hasattr(rows, "counts") else [row.count for row in rows]
+
+
 def chunk_planner(dtype: torch.dtype) -> dict:
     """The step planner of mixers that walk long rows in chunks on the tensor cores (:func:`chunked_scan`): in bfloat16, a step with a long row gets ``scan_chunk_start``
     and ``scan_chunk_row`` among its arrays and their number in ``step.host["scan_chunks"]`` (0 otherwise); ``step.host["scan_short_rows"]``: whether some rows are short
@@ -336,10 +341,10 @@ def chunk_planner(dtype: torch.dtype) -> dict:
     def plan(rows, packer, host):
         if "scan_chunks" in host:
             return
-        counts = rows.counts if hasattr(rows, "counts") else [row.count for row in rows]
-        cut = plan_chunks([int(c) for c in counts])
+        counts = _counts_of(rows)
+        cut = plan_chunks(counts)
         host["scan_chunks"] = 0 if cut is None else len(cut[1])
-        host["scan_short_rows"] = cut is not None and int(min(counts)) < CHUNKED_RULE_ROWS
+        host["scan_short_rows"] = cut is not None and min(counts) < CHUNKED_RULE_ROWS
         if cut is not None:
             packer.add("scan_chunk_start", cut[0])
             packer.add("scan_chunk_row", cut[1])
@@ -379,8 +384,8 @@ def rule_planner(dtype: torch.dtype) -> dict:
     def plan(rows, packer, host):
         if "rule_chunks" in host:
             return
-        counts = rows.counts if hasattr(rows, "counts") else [row.count for row in rows]
-        cut = plan_rule_chunks([int(c) for c in counts])
+        counts = _counts_of(rows)
+        cut = plan_rule_chunks(counts)
         host["rule_chunks"] = None if cut is None else (len(cut[0]) // 2, len(cut[1]) // 3, cut[2])
         if cut is not None:
             packer.add("rule_chunks", cut[0])
@@ -488,8 +493,8 @@ def segment_planner(dtype: torch.dtype) -> dict:
     def plan(rows, packer, host):
         if "scan_segments" in host:
             return
-        counts = rows.counts if hasattr(rows, "counts") else [row.count for row in rows]
-        cut = plan_segments([int(c) for c in counts])
+        counts = _counts_of(rows)
+        cut = plan_segments(counts)
         host["scan_segments"] = 0 if cut is None else len(cut[1])
         if cut is not None:
             packer.add("scan_seg_start", cut[0])

@@ -1,6 +1,9 @@
 """The recurrences that walk long bfloat16 rows in chunks at float precision (csrc/chunked_float.cu): the plan on the CPU, the kernels against 64-bit arithmetic."""
 from __future__ import annotations
 
+from types import SimpleNamespace
+
+import numpy as np
 import pytest
 import torch
 
@@ -39,6 +42,23 @@ def test_chunks_go_fewer_at_a_time_where_memory_is_short(monkeypatch):
     monkeypatch.setattr(torch, "empty", short_of(999))
     with pytest.raises(torch.cuda.OutOfMemoryError):
         recurrent._scratch_of_chunks(40, piece, "cpu")
+
+
+@pytest.mark.parametrize("counts", [[1] * 7, [300, 1, 15, 16], [128], [127, 2], [700, 1, 512]])
+def test_the_planners_read_rows_as_arrays_and_as_objects(counts):
+    """A step's rows come as arrays (the runner's) or as a list of rows: the same plans, of plain integers, and none in a step without a long row."""
+    class Packer(dict):
+        add = dict.__setitem__
+
+    arrays, objects = SimpleNamespace(counts=np.array(counts, dtype=np.int32)), [SimpleNamespace(count=c) for c in counts]
+    for planner in (recurrent.rule_planner, recurrent.chunk_planner, recurrent.segment_planner):
+        plan, seen = next(iter(planner(torch.bfloat16).values())), []
+        for rows in (arrays, objects):
+            packer, host = Packer(), {}
+            plan(rows, packer, host)
+            seen.append((dict(packer), host))
+        assert seen[0] == seen[1] and bool(seen[0][0]) == (max(counts) >= (512 if planner is recurrent.segment_planner else 128))
+        assert all(type(value) is int for values in seen[0][0].values() for value in values)
 
 
 def token_by_token(rule, k, q, v, a, beta, S, bonus):
