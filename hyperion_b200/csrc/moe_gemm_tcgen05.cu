@@ -183,7 +183,7 @@ int launch_grouped(const CUtensorMap& map_x, const CUtensorMap& map_w, const Gro
 }
 
 // ---------------------------------------------------------------- a few rows per expert: the matrices stream once
-constexpr int ROWS_AT_ONCE = 8, COLUMNS_PER_BLOCK = 32, COLUMNS_AT_ONCE = 2, ROWS_THREADS = 256;
+constexpr int ROWS_AT_ONCE = 8, COLUMNS_PER_BLOCK = 32, COLUMNS_AT_ONCE = 2, ROWS_THREADS = 256, ROWS_MOST_SHARED = 200 * 1024;
 
 // Columns `col` and `col + 1` of ROWS rows in shared memory: a lane takes every 32nd 16-byte piece of the matrix rows, several of them asked for
 // before the first is used (the step is bound by how many bytes are on their way), the lanes meet in a butterfly.  Every sum has the same
@@ -420,12 +420,10 @@ HB_EXPORT int hb_moe_gemm_rows(const void* a, int a_stride, const int* row_token
     if (k <= 0 || pad <= 0 || rows % pad || (k % 8) || (a_stride % 8) || !tile_expert || !tile_rows) return HB_BAD_ARGUMENT;
     if ((((uintptr_t)a | (uintptr_t)w) & 15)) return HB_BAD_ARGUMENT;
     const size_t shared = (size_t)ROWS_AT_ONCE * k * sizeof(bf16);
-    if (shared > 200 * 1024 || rows / pad > 65535) return HB_UNSUPPORTED_SIZE;
-    static size_t configured = 48 * 1024;
-    if (shared > configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    if (shared > ROWS_MOST_SHARED || rows / pad > 65535) return HB_UNSUPPORTED_SIZE;
+    if (shared > 48 * 1024) {  // always the most that any call takes: another thread's call may come between this and the launch
+        cudaError_t e = cudaFuncSetAttribute(gemm_grouped_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_MOST_SHARED);
         if (e != cudaSuccess) return (int)e;
-        configured = shared;
     }
     const dim3 grid((n + COLUMNS_PER_BLOCK - 1) / COLUMNS_PER_BLOCK, rows / pad);
     return launch_after_previous(gemm_grouped_rows_kernel, grid, dim3(ROWS_THREADS), shared, stream, (const bf16*)a, a_stride, row_token, (const bf16*)w, (bf16*)c, tile_expert,

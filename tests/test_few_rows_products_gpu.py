@@ -59,8 +59,11 @@ def test_sums_are_as_close_as_without_tensor_cores(tokens, k, monkeypatch):
     assert 0 < far[0] <= far[1], far
 
 
-def test_threads_with_rows_of_different_lengths():
+@pytest.mark.parametrize("rows_per_expert", [0, 1 << 20])  # all steps through the tensor cores, none
+def test_threads_with_rows_of_different_lengths(rows_per_expert, monkeypatch):
     """Rows of 4,096 and of 6,400 entries take different amounts of shared memory; two threads that launch both kinds at once must not take each other's allowance away."""
+    monkeypatch.setattr(moe, "SOME_ROWS", rows_per_expert)
+
     def products(k, seed):
         g = torch.Generator("cuda").manual_seed(seed)
         x, w = torch.randn(16, k, device="cuda", generator=g).to(torch.bfloat16), (torch.randn(2, 64, k, device="cuda", generator=g) / k**0.5).to(torch.bfloat16)
