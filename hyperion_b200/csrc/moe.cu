@@ -26,7 +26,7 @@
 #include "common.cuh"
 
 namespace {
-constexpr int ROUTE_THREADS = 256;
+constexpr int ROUTE_THREADS = 256, ROUTE_MOST_SHARED = 200 * 1024;  // always allowed in full: another thread's call may come between a call's allowance and its launch
 
 // One block per token: the row in shared memory as floats, a warp per expert at a time.  A lane adds up every 32nd group of four
 // columns in four chains of its own (columns beyond a multiple of four go to the first chain), the chains are added in a fixed
@@ -487,13 +487,13 @@ HB_EXPORT int hb_moe_route_scored(const void* x, int is_bf16, int x_stride, cons
     if (group_count > 1 && (outputs % group_count || group_keep <= 0 || group_keep > group_count || top > group_keep * (outputs / group_count)))
         return HB_BAD_ARGUMENT;
     const size_t shared = (size_t)(((hidden + 3) & ~3) + 4 * outputs + 2 * (group_count > 0 ? group_count : 1)) * sizeof(float);
-    if (shared > 200 * 1024) return HB_UNSUPPORTED_SIZE;
+    if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
     if (is_bf16) {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_scored_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_scored_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
         moe_route_scored_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const __nv_bfloat16*)x, x_stride, router, correction, hidden, outputs, top,
                                                                           group_count, group_keep, scale, chosen, weights);
     } else {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_scored_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_scored_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
         moe_route_scored_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const float*)x, x_stride, router, correction, hidden, outputs, top, group_count,
                                                                           group_keep, scale, chosen, weights);
     }
@@ -526,12 +526,12 @@ HB_EXPORT int hb_moe_route(const void* x, int is_bf16, int x_stride, const float
     if (tokens <= 0) return 0;
     if (experts <= 0 || experts > 1024 || top <= 0 || top > experts || hidden <= 0) return HB_UNSUPPORTED_SIZE;
     const size_t shared = (size_t)(((hidden + 3) & ~3) + experts) * sizeof(float);
-    if (shared > 200 * 1024) return HB_UNSUPPORTED_SIZE;
+    if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
     if (is_bf16) {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
         moe_route_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const __nv_bfloat16*)x, x_stride, router, hidden, experts, top, weighted, chosen, weights);
     } else {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
         moe_route_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const float*)x, x_stride, router, hidden, experts, top, weighted, chosen, weights);
     }
     return launch_status();
@@ -544,10 +544,10 @@ HB_EXPORT int hb_moe_route_softmax(const void* x, int is_bf16, int x_stride, con
     auto bytes = [&](int at_once) { return (size_t)at_once * (((hidden + 3) & ~3) + experts + top) * sizeof(float); };
     const int at_once = tokens >= 512 && bytes(4) <= 100 * 1024 ? 4 : 1;  // a step of few tokens fills more of the device with a token per block
     const size_t shared = bytes(at_once);
-    if (shared > 200 * 1024) return HB_UNSUPPORTED_SIZE;
+    if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
 #define HB_ROUTE(T, N)                                                                                                                                  \
     {                                                                                                                                                   \
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_softmax_kernel<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);          \
+        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_softmax_kernel<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);          \
         return launch_after_previous(moe_route_softmax_kernel<T, N>, dim3((tokens + N - 1) / N), dim3(ROUTE_THREADS), shared, stream, (const T*)x, x_stride, \
                                      router, bias, tokens, hidden, experts, top, chosen, weights);                                                      \
     }

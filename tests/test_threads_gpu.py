@@ -1,0 +1,42 @@
+"""Kernels whose shared memory follows a width, launched by two threads at widths of their own: neither takes the other's allowance away."""
+from concurrent.futures import ThreadPoolExecutor
+
+import pytest
+import torch
+
+from hyperion_b200 import ops
+from hyperion_b200.ops import moe
+
+pytestmark = pytest.mark.gpu
+
+
+def routes(call, tokens):
+    def prepared(hidden, g, dtype):
+        x, router = torch.randn(tokens, hidden, device="cuda", generator=g).to(dtype), torch.randn(16, hidden, device="cuda", generator=g)
+        return lambda: call(x, router)
+    return prepared
+
+
+# widths of which both take more than a block's ordinary 48 KB; four tokens to a block from 512 on
+CALLS = {
+    "route": (routes(lambda x, r: moe.route(x, r, 2), 3), (13000, 20000)),
+    "route_scored": (routes(lambda x, r: moe.route_scored(x, r, None, 2, 1, 1, 1.0), 3), (13000, 20000)),
+    "route_softmax": (routes(lambda x, r: moe.route_softmax(x, r, None, 2), 3), (13000, 20000)),
+    "route_softmax_by_four": (routes(lambda x, r: moe.route_softmax(x, r, None, 2), 512), (3584, 5120)),
+}
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("name", CALLS)
+def test_threads_at_widths_of_their_own(name, dtype):
+    prepared, widths = CALLS[name]
+
+    def repeated(hidden):
+        g = torch.Generator("cuda").manual_seed(hidden)
+        call = prepared(hidden, g, dtype)
+        want = call()
+        torch.cuda.synchronize()
+        return all(torch.equal(one, other) for _ in range(150) for one, other in zip(call(), want))
+
+    with ThreadPoolExecutor(2) as pool:
+        assert all(pool.map(repeated, widths))
