@@ -793,11 +793,13 @@ __global__ void norm_add_norm_bf16x8_kernel(float* __restrict__ h, const __nv_bf
     *reinterpret_cast<uint4*>(out + (size_t)i * hidden + j) = packed;
 }
 
+constexpr int NORM_MOST_HIDDEN = 49152;  // its shared memory is always allowed in full: another thread's call may come between a call's allowance and its launch
+
 HB_EXPORT int hb_norm_add_norm(float* h, const void* y, int y_is_bf16, const float* w_post, const float* offset, const float* w_next, void* out,
                                int out_is_bf16, const int* rows, int n_rows, int hidden, float eps_post, float eps_next, const float* gate,
                                int gate_stride, int gate_splits, long long gate_split_stride, const float* gate_bias, cudaStream_t stream) {
     if (n_rows <= 0) return 0;
-    if (hidden <= 0 || hidden > 49152 || (y && !w_post) || (w_next && !out) || (gate && gate_splits < 1)) return HB_BAD_ARGUMENT;
+    if (hidden <= 0 || hidden > NORM_MOST_HIDDEN || (y && !w_post) || (w_next && !out) || (gate && gate_splits < 1)) return HB_BAD_ARGUMENT;
     const bool halves = (!y || y_is_bf16) && (!w_next || out_is_bf16);
     if (halves && hidden % 8 == 0 && hidden <= 8192 && (!gate || (gate_stride % 4 == 0 && gate_split_stride % 4 == 0)) &&
         (((uintptr_t)h | (uintptr_t)y | (uintptr_t)w_post | (uintptr_t)offset | (uintptr_t)w_next | (uintptr_t)out | (uintptr_t)gate | (uintptr_t)gate_bias) & 15) == 0) {
@@ -810,7 +812,7 @@ HB_EXPORT int hb_norm_add_norm(float* h, const void* y, int y_is_bf16, const flo
     const size_t shared = (size_t)hidden * sizeof(float);
 #define HB_NORM_ADD_NORM(TY, TO)                                                                                                          \
     do {                                                                                                                                  \
-        if (shared > 48 * 1024) cudaFuncSetAttribute(norm_add_norm_kernel<TY, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared); \
+        if (shared > 48 * 1024) cudaFuncSetAttribute(norm_add_norm_kernel<TY, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, NORM_MOST_HIDDEN * 4); \
         norm_add_norm_kernel<TY, TO><<<n_rows, threads, shared, stream>>>(h, (const TY*)y, w_post, offset, w_next, (TO*)out, rows, hidden,   \
                                                                          eps_post, eps_next, gate, gate_stride, gate_splits,            \
                                                                          (size_t)gate_split_stride, gate_bias);                          \

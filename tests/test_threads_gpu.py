@@ -17,12 +17,23 @@ def routes(call, tokens):
     return prepared
 
 
+def two_norms(hidden, g, dtype):
+    h, y, w = (torch.randn(*shape, device="cuda", generator=g) for shape in ((3, hidden), (3, hidden), (hidden,)))
+    y = y.to(dtype)
+
+    def call():
+        stream = h.clone()
+        return stream, ops.norm_add_norm(stream, y, w, 1e-6, None, w, 1e-6, dtype)
+    return call
+
+
 # widths of which both take more than a block's ordinary 48 KB; four tokens to a block from 512 on
 CALLS = {
     "route": (routes(lambda x, r: moe.route(x, r, 2), 3), (13000, 20000)),
     "route_scored": (routes(lambda x, r: moe.route_scored(x, r, None, 2, 1, 1, 1.0), 3), (13000, 20000)),
     "route_softmax": (routes(lambda x, r: moe.route_softmax(x, r, None, 2), 3), (13000, 20000)),
     "route_softmax_by_four": (routes(lambda x, r: moe.route_softmax(x, r, None, 2), 512), (3584, 5120)),
+    "norm_add_norm": (two_norms, (13000, 20000)),
 }
 
 
