@@ -491,18 +491,24 @@ __global__ void __launch_bounds__(2 * ETILE, 256 / ETILE) chunk_outputs_kernel(c
     }
 }
 
+// Always the most that any call of the kernel takes: another thread's call may come between this and the launch.
 template <typename Kernel>
-int allow_shared(Kernel kernel, int bytes) {
-    return bytes > 48 * 1024 ? (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) : 0;
+int allow_shared(Kernel kernel, int bytes, int most) {
+    return bytes > 48 * 1024 ? (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) : 0;
+}
+__host__ __device__ constexpr int states_bytes(int n16, int etile) { return CHUNK * (n16 + 8) * 2 + 2 * CHUNK * (etile + 8) * 2; }
+__host__ __device__ constexpr int outputs_bytes(int n16, int etile) {
+    const int state = 2 * etile * (n16 + 8) * 2, tiles = CHUNK * (n16 + 8) * 2 + CHUNK * (etile + 8) * 2;
+    return CHUNK * (n16 + 8) * 2 + (state > tiles ? state : tiles);
 }
 
 template <int KIND, int ETILE>
 int launch_states(const ChunkArgs& a, int chunks, cudaStream_t stream) {
-    const int n16 = (a.n + 15) & ~15, bytes = CHUNK * (n16 + 8) * 2 + 2 * CHUNK * (ETILE + 8) * 2;
+    const int n16 = (a.n + 15) & ~15, bytes = states_bytes(n16, ETILE);
     const dim3 grid(chunks, a.heads, (a.e + ETILE - 1) / ETILE);
 #define HB_CHUNK_STATES(NMAX)                                                                        \
     do {                                                                                             \
-        const int status = allow_shared(chunk_states_kernel<KIND, NMAX, ETILE>, bytes);              \
+        const int status = allow_shared(chunk_states_kernel<KIND, NMAX, ETILE>, bytes, states_bytes(NMAX, ETILE)); \
         if (status) return status;                                                                   \
         chunk_states_kernel<KIND, NMAX, ETILE><<<grid, 2 * ETILE, bytes, stream>>>(a);               \
     } while (0)
@@ -515,8 +521,9 @@ int launch_states(const ChunkArgs& a, int chunks, cudaStream_t stream) {
 
 template <int KIND, int ETILE>
 int launch_outputs(const ChunkArgs& a, int chunks, cudaStream_t stream) {
-    const int n16 = (a.n + 15) & ~15, state = 2 * ETILE * (n16 + 8) * 2, tiles = CHUNK * (n16 + 8) * 2 + CHUNK * (ETILE + 8) * 2, bytes = CHUNK * (n16 + 8) * 2 + (state > tiles ? state : tiles);
-    const int status = allow_shared(chunk_outputs_kernel<KIND, ETILE>, bytes);
+    constexpr int MOST_N16 = ETILE == 64 ? 256 : 128;  // the wide tile is for keys of up to 128 entries
+    const int n16 = (a.n + 15) & ~15, bytes = outputs_bytes(n16, ETILE);
+    const int status = allow_shared(chunk_outputs_kernel<KIND, ETILE>, bytes, outputs_bytes(MOST_N16, ETILE));
     if (status) return status;
     chunk_outputs_kernel<KIND, ETILE><<<dim3(chunks, a.heads, (a.e + ETILE - 1) / ETILE), 2 * ETILE, bytes, stream>>>(a);
     return launch_status();

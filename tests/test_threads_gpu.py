@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from hyperion_b200 import ops
-from hyperion_b200.ops import moe
+from hyperion_b200.ops import moe, recurrent
 
 pytestmark = pytest.mark.gpu
 
@@ -27,6 +27,18 @@ def two_norms(hidden, g, dtype):
     return call
 
 
+def chunks(n, g, dtype):
+    heads, e, tokens = 2, 64, 150
+    x, gate = torch.randn(tokens, heads * (2 * n + e), device="cuda", generator=g), -torch.rand(tokens, 2 * heads, device="cuda", generator=g)
+    begin, slots = torch.randn(1, heads * e * n, device="cuda", generator=g), torch.zeros(1, dtype=torch.int32, device="cuda")
+    starts, rows = (torch.tensor(t, dtype=torch.int32, device="cuda") for t in recurrent.plan_chunks([tokens]))
+
+    def call():
+        state = begin.clone()
+        return state, recurrent.chunked_scan(recurrent.KIND_GIVEN, x, x[:, heads * n :], x[:, 2 * heads * n :], gate, 0, heads, state, 0, slots, starts, rows, len(rows), heads, heads, n, n, e)
+    return call
+
+
 # widths of which both take more than a block's ordinary 48 KB; four tokens to a block from 512 on
 CALLS = {
     "route": (routes(lambda x, r: moe.route(x, r, 2), 3), (13000, 20000)),
@@ -34,6 +46,7 @@ CALLS = {
     "route_softmax": (routes(lambda x, r: moe.route_softmax(x, r, None, 2), 3), (13000, 20000)),
     "route_softmax_by_four": (routes(lambda x, r: moe.route_softmax(x, r, None, 2), 512), (3584, 5120)),
     "norm_add_norm": (two_norms, (13000, 20000)),
+    "chunked_scan": (chunks, (128, 256)),
 }
 
 
