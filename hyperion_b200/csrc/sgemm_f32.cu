@@ -5,10 +5,11 @@
 // its float arithmetic is the f64 `linear` of helios/crates/helios-hal/src/reference.rs:24-41.
 //
 // A thread owns TM x TN outputs, BM / TM and BN / TN apart, and reads four k of each of its rows and columns at a time from shared memory in 16-byte pieces; slices of BK k
-// are copied ahead into a ring of STAGES, as they lie in memory. Bound by the FFMA pipes (74 TFLOP/s) where a product has tiles enough, else by the waits of a chain.
+// are copied ahead into a ring of STAGES, as they lie in memory. Bound by issue slots (70 % of an active SM's cycles issue, 60 % of them FFMA) and the last wave where a product has tiles enough,
+// else by the waits of a chain; the FFMA pipes would allow 74 TFLOP/s.
 // Two shapes: 64 x 128 with 8 x 8 outputs a thread for products that fill the GPU with such tiles; 32 x 32 with 4 x 4 for the others, which spreads a narrow product over
-// all SMs. Measured on one B200 (before: one shape of 64 x 64 with 4 x 4 outputs a thread, copied when needed): 394 rows, K 896, 9,728 columns 340 -> 246 us, K 4,864, 896 columns
-// 302 -> 166 us; 3 rows, 151,936 columns 625 -> 244 us; 1 row, K 4,864 265 -> 101 us; 2,048 rows, 9,728 columns 1,393 -> 819 us (44 TFLOP/s).
+// all SMs. Measured on one B200 (before: one shape of 64 x 64 with 4 x 4 outputs a thread, copied when needed): 394 rows, K 896, 9,728 columns 340 -> 229 to 246 us, K 4,864, 896 columns
+// 302 -> 161 to 166 us; 3 rows, 151,936 columns 625 -> 244 us; 1 row, K 4,864 265 -> 101 us; 2,048 rows, 9,728 columns 1,393 -> 819 us (44 TFLOP/s).
 #include "common.cuh"
 
 namespace {
