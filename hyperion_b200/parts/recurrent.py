@@ -53,7 +53,8 @@ Matrix memory with exponential gates (``matrix_memory``; the mLSTM of Beck et al
 The running maximum m starts at 0.  The record holds the heads' matrices with n as one more column each, then the heads' m.
 Parameters: ``hidden_size``, ``heads``, ``head_dim``, ``value_dim``, ``gate_cap``, ``eps``.  Tensors: q, k, v, g, i, i.b, f, f.b, norm, o.
 ``mamba2`` and ``matrix_memory`` are branches (``parts/branch.py``): they also run beside another mixer on the same input.  Both walk a bfloat16 step with a long row
-in chunks on the tensor cores (``csrc/chunked_scan.cu``: the state, its decays and steps stay float).
+in chunks on the tensor cores (``csrc/chunked_scan.cu``: the state, its decays and steps stay float).  The other mixers with a matrix state per head do so at float precision
+(``csrc/chunked_float.cu``) where a head has keys of up to 128 entries and values of whole sixteens.
 
 Lightning attention (``lightning``): a matrix state per head that fades by a constant of the head, with nothing between the projections and
 the recurrence but an activation:
