@@ -825,7 +825,7 @@ int launch_walk(const Args& a, int walks, cudaStream_t stream) {
 }
 
 template <int RULE, int N>
-int launch_rule(const Args& given, int walks, int chunks, int span, int sms, cudaStream_t stream) {
+int launch_rule(const Args& given, int walks, int beside, int chunks, int span, int sms, cudaStream_t stream) {
     constexpr int bytes = Layout<RULE, N>::FLOATS * 4;
     int status = allow_shared(prepare_chunks_kernel<RULE, N>, bytes);
     if (status) return status;
@@ -836,8 +836,9 @@ int launch_rule(const Args& given, int walks, int chunks, int span, int sms, cud
         prepare_chunks_kernel<RULE, N><<<dim3(a.chunk1 - a.chunk0, a.heads), Layout<RULE, N>::THREADS, bytes, stream>>>(a);
         status = launch_status();
         if (status) return status;
-        // 16 value columns to a block while those blocks fit the SMs side by side, else 32, which read the chunk's pieces half as often
-        const bool narrow = a.e % 32 != 0 || a.heads * (a.e / 16) <= sms;
+        // 16 value columns to a block while those blocks, of all rows side by side, fit the SMs, else 32, which read the chunk's pieces half as often (16 heads of 128 x 128, four
+        // rows of 2,048: delta rule 753 us, 882 with 16 columns; retention 473 and 559)
+        const bool narrow = a.e % 32 != 0 || (long long)beside * a.heads * (a.e / 16) <= sms;
         status = narrow ? launch_walk<RULE, N, 16>(a, walks, stream) : launch_walk<RULE, N, 32>(a, walks, stream);
         if (status) return status;
     }
@@ -863,10 +864,10 @@ HB_EXPORT long long hb_chunked_float_scratch(int rule, int n, int e) {
 }
 
 // Rows through their chunks of at most 64 consecutive tokens (tables as in Args; a row's chunks follow one another), `span` chunks at a time: scratch holds span * heads times
-// what hb_chunked_float_scratch says, on a 16-byte boundary.  out [tokens, heads * e] on an 8-byte boundary; tokens of no chunk keep theirs.
+// what hb_chunked_float_scratch says, on a 16-byte boundary.  beside: how many rows of the longest one's length the walks amount to.  out [tokens, heads * e] on an 8-byte boundary; tokens of no chunk keep theirs.
 HB_EXPORT int hb_chunked_float(int rule, const float* k, int k_stride, const float* q, int q_stride, const float* v, int v_stride, const float* x, int x_stride, int x_off,
                                const float* step, int step_stride, int step_off, const float* rate, const float* bias, float* scratch, float* state, long long slot_stride,
-                               int state_off, const int* slots, const int* table, int chunks, const int* walk_table, int walks, int span, float* out, int heads, int groups, int n,
+                               int state_off, const int* slots, const int* table, int chunks, const int* walk_table, int walks, int beside, int span, float* out, int heads, int groups, int n,
                                int n_padded, int e, float q_scale, int sms, int* status, cudaStream_t stream) {
     if (chunks <= 0 || walks <= 0) return 0;
     if (n <= 0 || n > 128 || e <= 0 || e % 16 || heads <= 0 || heads > 65535 || walks > 65535 || groups <= 0 || heads % groups) return HB_UNSUPPORTED_SIZE;
@@ -880,11 +881,11 @@ HB_EXPORT int hb_chunked_float(int rule, const float* k, int k_stride, const flo
                  walk_table, 0, 0, out, heads, groups, n, n_padded, e, q_scale, by_four, (v_stride & 3) == 0 && ((uintptr_t)v & 15) == 0, status};
     const bool small = n <= 64;
     switch (rule) {
-        case RULE_DELTA: return small ? launch_rule<RULE_DELTA, 64>(a, walks, chunks, span, sms, stream) : launch_rule<RULE_DELTA, 128>(a, walks, chunks, span, sms, stream);
+        case RULE_DELTA: return small ? launch_rule<RULE_DELTA, 64>(a, walks, beside, chunks, span, sms, stream) : launch_rule<RULE_DELTA, 128>(a, walks, beside, chunks, span, sms, stream);
         case RULE_CHANNEL_DELTA:
-            return small ? launch_rule<RULE_CHANNEL_DELTA, 64>(a, walks, chunks, span, sms, stream) : launch_rule<RULE_CHANNEL_DELTA, 128>(a, walks, chunks, span, sms, stream);
-        case RULE_RETENTION: return small ? launch_rule<RULE_RETENTION, 64>(a, walks, chunks, span, sms, stream) : launch_rule<RULE_RETENTION, 128>(a, walks, chunks, span, sms, stream);
-        case RULE_WKV: return small ? launch_rule<RULE_WKV, 64>(a, walks, chunks, span, sms, stream) : launch_rule<RULE_WKV, 128>(a, walks, chunks, span, sms, stream);
+            return small ? launch_rule<RULE_CHANNEL_DELTA, 64>(a, walks, beside, chunks, span, sms, stream) : launch_rule<RULE_CHANNEL_DELTA, 128>(a, walks, beside, chunks, span, sms, stream);
+        case RULE_RETENTION: return small ? launch_rule<RULE_RETENTION, 64>(a, walks, beside, chunks, span, sms, stream) : launch_rule<RULE_RETENTION, 128>(a, walks, beside, chunks, span, sms, stream);
+        case RULE_WKV: return small ? launch_rule<RULE_WKV, 64>(a, walks, beside, chunks, span, sms, stream) : launch_rule<RULE_WKV, 128>(a, walks, beside, chunks, span, sms, stream);
     }
     return HB_BAD_ARGUMENT;
 }

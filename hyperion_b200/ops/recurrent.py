@@ -377,7 +377,7 @@ def plan_rule_chunks(counts) -> tuple[list[int], list[int], bool] | None:
 
 def rule_planner(dtype: torch.dtype) -> dict:
     """The step planner of mixers that walk long rows with :func:`chunked_rule`: in bfloat16, a step with a long row gets ``rule_chunks`` and ``rule_walks`` among its
-    arrays and (chunks, walks, whether other rows are left) in ``step.host["rule_chunks"]`` (None otherwise)."""
+    arrays and (chunks, walks, whether other rows are left, the longest row's chunks, tokens in chunks) in ``step.host["rule_chunks"]`` (None otherwise)."""
     if dtype != torch.bfloat16:
         return {}
 
@@ -386,7 +386,7 @@ def rule_planner(dtype: torch.dtype) -> dict:
             return
         counts = _counts_of(rows)
         cut = plan_rule_chunks(counts)
-        host["rule_chunks"] = None if cut is None else (len(cut[0]) // 2, len(cut[1]) // 3, cut[2])
+        host["rule_chunks"] = None if cut is None else (len(cut[0]) // 2, len(cut[1]) // 3, cut[2], -(-max(counts) // CHUNK), sum(cut[0][1::2]))
         if cut is not None:
             packer.add("rule_chunks", cut[0])
             packer.add("rule_walks", cut[1])
@@ -397,6 +397,22 @@ def rule_planner(dtype: torch.dtype) -> dict:
 def chunked_rule_fits(n: int, e: int) -> bool:
     """Whether :func:`chunked_rule` takes heads of this size; others walk token by token."""
     return 0 < n <= 128 and e > 0 and e % 16 == 0
+
+
+def chunks_pay(rule: int, chunks: int, longest: int, tokens: int, heads: int, e: int, sms: int) -> bool:
+    """Whether a step's rows (``tokens`` in ``chunks``, ``longest`` of them in the longest row) are walked faster in chunks than token by token.  A scan of one row is a chain that leaves most of the
+    device idle; many rows fill it, and then a chunk has to beat the scan's arithmetic, which the delta rules' do unless chunks are mostly padding, and retention's in long rows.  The line is where
+    blocks of 32 value columns, as many rows side by side as the chunks amount to, fill the multiprocessors twice.  us on one B200 (148 of them), chunks / scan, 16 heads of 128 x 128 (time mixing 32
+    of 64), in blocks per multiprocessor:
+    0.4: one row of 128 tokens: delta 47 / 54, retention 23 / 27, time mixing 20 / 27;  1.7: four of 128: 68 / 84, 39 / 39, 35 / 35, four of 512: 201 / 319, 117 / 139, 111 / 129;
+    3.5: eight of 128: 111 / 151, 66 / 64, 60 / 54, of 512: 375 / 587, 224 / 241, 213 / 205;  6.9: sixteen of 128: 203 / 295, 119 / 107, 113 / 93.
+    A row of 128 beside seven of 16: 66 / 68, 36 / 31, 32 / 31, with twice the heads 103 / 78, 60 / 43, 54 / 39.  Four rows of 1,024 with twice the heads: retention 442 / 476, time mixing 426 / 404."""
+    padded, fills = 2 * tokens < CHUNK * chunks, chunks * heads * -(-e // 32) > 2 * sms * longest
+    if rule in (RULE_DELTA, RULE_CHANNEL_DELTA):
+        return not (padded and fills and longest <= 4)
+    if padded and longest < 4:
+        return False
+    return not fills or (rule == RULE_RETENTION and longest >= 16)
 
 
 def _scratch_of_chunks(chunks: int, piece: int, device) -> tuple[int, torch.Tensor]:
@@ -414,10 +430,11 @@ def _scratch_of_chunks(chunks: int, piece: int, device) -> tuple[int, torch.Tens
 
 def chunked_rule(rule: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, x: torch.Tensor | None, x_off: int, step: torch.Tensor | None, step_off: int, rate: torch.Tensor,
                  bias: torch.Tensor | None, state: torch.Tensor, state_off: int, slots: torch.Tensor, table: torch.Tensor, chunks: int, walk_table: torch.Tensor, walks: int,
-                 heads: int, groups: int, n: int, n_padded: int, e: int, q_scale: float = 1.0) -> torch.Tensor:
+                 heads: int, groups: int, n: int, n_padded: int, e: int, q_scale: float = 1.0, longest: int = 0) -> torch.Tensor:
     """The recurrences of :func:`state_scan` (delta rule, retention), :func:`channel_delta_scan` and :func:`wkv_scan` over the chunks of a step (:func:`plan_rule_chunks`), at float
     precision; tokens of other rows get nothing.  ``k``, ``q`` (group g at g * n), ``v`` (head h at h * e) are float views [tokens, *]; ``x`` at ``x_off`` holds the decays' pre-activations and ``step`` at
-    ``step_off`` the delta rules' steps'; ``rate`` and ``bias`` are a_log and dt_bias, or the decays and nothing (retention), or w0 and the bonus (wkv).  Returns [tokens, heads * e]."""
+    ``step_off`` the delta rules' steps'; ``rate`` and ``bias`` are a_log and dt_bias, or the decays and nothing (retention), or w0 and the bonus (wkv).  ``longest``: the chunks of the longest row (0: rows of about one length).  Returns
+    [tokens, heads * e]."""
     require_cuda(k, q, v, x, step, rate, bias, state, slots, table, walk_table)
     _floats(k, q, v, x, step, rate, bias, state)
     entries = heads * n if rule in (RULE_CHANNEL_DELTA, RULE_WKV) else heads
@@ -431,7 +448,7 @@ def chunked_rule(rule: int, k: torch.Tensor, q: torch.Tensor, v: torch.Tensor, x
     stride = lambda t: i32(t.stride(0) if t is not None else 0)  # noqa: E731
     check(native.hb_chunked_float(i32(rule), ptr(k), stride(k), ptr(q), stride(q), ptr(v), stride(v), ptr(x), stride(x), i32(x_off), ptr(step), stride(step), i32(step_off), ptr(rate),
                                   ptr(bias), ptr(scratch), ptr(state), ctypes.c_longlong(state.stride(0)), i32(state_off), ptr(slots), ptr(table), i32(chunks), ptr(walk_table),
-                                  i32(walks), i32(span), ptr(out), i32(heads), i32(groups), i32(n), i32(n_padded), i32(e), f32(q_scale), i32(sm_count(k.device)), ptr(status_word(k.device)), stream_ptr()),
+                                  i32(walks), i32(-(-chunks // longest) if longest else walks), i32(span), ptr(out), i32(heads), i32(groups), i32(n), i32(n_padded), i32(e), f32(q_scale), i32(sm_count(k.device)), ptr(status_word(k.device)), stream_ptr()),
           "chunked_rule")
     LAUNCHES[0] += 2 * -(-chunks // span) - 1  # two kernels per span
     return out

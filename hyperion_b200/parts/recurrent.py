@@ -70,6 +70,7 @@ import torch
 
 from .. import ops
 from ..ops import recurrent
+from ..ops.native import sm_count
 from .base import BuildContext, Mixer, RequestState, WeightSpec, register_mixer
 from .branch import Branch
 from .spec import PartSpec
@@ -93,13 +94,15 @@ class ChunkedRule:
         return recurrent.rule_planner(self.dtype) if recurrent.chunked_rule_fits(self.n, self.e) else {}
 
     def _walk(self, rule, k, q, v, x, x_off, step_in, step_off, rate, bias, cache, step, groups, q_scale, by_token):
-        """Long rows in chunks, the others by ``by_token(below, out)``."""
+        """Long rows in chunks where that pays, the others by ``by_token(below, out)``."""
         cut = step.host.get("rule_chunks") if recurrent.chunked_rule_fits(self.n, self.e) else None
         if cut is None:
             return by_token(0, None)
-        chunks, walks, others = cut
+        chunks, walks, others, longest, tokens = cut
+        if not recurrent.chunks_pay(rule, chunks, longest, tokens, self.heads, self.e, sm_count(k.device)):
+            return by_token(0, None)
         out = recurrent.chunked_rule(rule, k, q, v, x, x_off, step_in, step_off, rate, bias, cache.state, 0, cache.slots, step.extra["rule_chunks"], chunks,
-                                     step.extra["rule_walks"], walks, self.heads, groups, self.n, self.n_padded, self.e, q_scale)
+                                     step.extra["rule_walks"], walks, self.heads, groups, self.n, self.n_padded, self.e, q_scale, longest)
         return by_token(recurrent.CHUNKED_RULE_ROWS, out) if others else out
 
 
