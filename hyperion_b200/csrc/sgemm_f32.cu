@@ -104,12 +104,13 @@ int launch_kernel(dim3 grid, const float* a, const float* w, const float* bias, 
     return launch_status();
 }
 
+bool aligned(const float* a, const float* w, int k, int lda) { return ((lda | k) & 3) == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0; }
+
 template <int BM, int BN, int TM, int TN, int BK, int STAGES>
 int launch_tiles(const float* a, const float* w, const float* bias, float* c, int m, int n, int k, int lda, int ldc, cudaStream_t stream) {
     const dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
     if (grid.y > 65535) return HB_UNSUPPORTED_SIZE;
-    const bool wide = ((lda | k) & 3) == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
-    return wide ? launch_kernel<BM, BN, TM, TN, BK, STAGES, true>(grid, a, w, bias, c, m, n, k, lda, ldc, stream)
+    return aligned(a, w, k, lda) ? launch_kernel<BM, BN, TM, TN, BK, STAGES, true>(grid, a, w, bias, c, m, n, k, lda, ldc, stream)
                 : launch_kernel<BM, BN, TM, TN, BK, STAGES, false>(grid, a, w, bias, c, m, n, k, lda, ldc, stream);
 }
 }  // namespace
@@ -121,8 +122,9 @@ HB_EXPORT int hb_sgemm_f32(const float* a, const float* w, const float* bias, fl
     if (m <= 0 || n <= 0) return 0;
     if (k <= 0) return HB_BAD_ARGUMENT;
     // large tiles from two to an SM on (148 SMs, 394 rows, 9,728 columns: 532 of them 246 us; 896 columns: 49 of them would leave two SMs in three idle) and where rows do not leave half
-    // of one empty
+    // of one empty.  Rows that are not on 16-byte boundaries are copied four bytes at a time, twice as many copies an output in small tiles: large ones from three to four SMs on (1,003 columns, K
+    // 1,001: 88 large tiles 90 us, small ones 82; 128: 92 and 124; 288: 155 and 236)
     const long long large = (long long)((m + 63) / 64) * ((n + 127) / 128);
-    if (m > 32 && large >= 2LL * sms) return launch_tiles<64, 128, 8, 8, 16, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
+    if (m > 32 && large >= (aligned(a, w, k, lda) ? 2LL * sms : 3LL * sms / 4)) return launch_tiles<64, 128, 8, 8, 16, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
     return launch_tiles<32, 32, 4, 4, 32, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
 }

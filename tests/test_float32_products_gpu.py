@@ -41,3 +41,15 @@ def test_the_tile_follows_the_device(m, n, k, monkeypatch):
         names = [event.name for event in profile.events() if "sgemm_kernel" in event.name]
         assert names and all(("64, 128" in name) == (sms == 1) for name in names), names
     assert torch.equal(*results)
+
+
+@pytest.mark.parametrize("k,large", [(1000, False), (1001, True)])
+def test_rows_off_16_bytes_take_large_tiles_earlier(k, large, monkeypatch):
+    """128 large tiles on 148 multiprocessors: too few for rows that are copied 16 bytes at a time, enough for rows that go four bytes at a time."""
+    x, w = torch.randn(1000, k, device="cuda"), torch.randn(1003, k, device="cuda")
+    monkeypatch.setattr(basic, "sm_count", lambda device: 148)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as profile:
+        ops.sgemm_f32(x, w)
+        torch.cuda.synchronize()
+    names = [event.name for event in profile.events() if "sgemm_kernel" in event.name]
+    assert names and all(("64, 128" in name) == large for name in names), names
