@@ -54,17 +54,21 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
-// Sum over a block (blockDim.x a multiple of 32, at most 1024). `scratch` holds 32 floats. The
+// Sum over a block (blockDim.x a multiple of 32, at most 1024). `scratch` holds 32 floats on a 16-byte boundary. The
 // partial sums of the warps are added in warp order by every thread, so the result is the same in
-// every thread and for every launch shape.
+// every thread and for every launch shape. They are read four at a time (zeros past the last warp add nothing).
 __device__ __forceinline__ float block_sum(float v, float* scratch) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     v = warp_sum(v);
     __syncthreads();
     if (lane == 0) scratch[warp] = v;
+    if (warp == 0 && lane >= warps) scratch[lane] = 0.f;
     __syncthreads();
     float total = 0.f;
-    for (int w = 0; w < warps; ++w) total += scratch[w];
+    for (int w = 0; w < warps; w += 4) {
+        const float4 part = *reinterpret_cast<const float4*>(scratch + w);
+        total = (((total + part.x) + part.y) + part.z) + part.w;
+    }
     return total;
 }
 
@@ -89,13 +93,23 @@ __device__ __forceinline__ float capped_score_log2(float raw, float pre, float p
     return fmaf(-2.f * post, r, post);
 }
 
-// The activations a product's epilogue can apply to what it stores.
-enum : int { HB_ACT_NONE = 0, HB_ACT_RELU_SQUARED = 1 };
+// 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))) and 0.5 z (1 + erf(z / sqrt(2)))
+struct GeluTanh {
+    static __device__ __forceinline__ float of(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
+};
+struct GeluErf {
+    static __device__ __forceinline__ float of(float z) { return 0.5f * z * (1.f + erff(z * 0.7071067811865476f)); }
+};
+
+// The activations a product's epilogue can apply to what it stores.  (HB_ACT_SWIGLU: only epilogues that hold both halves of a tile, and not here.)
+enum : int { HB_ACT_NONE = 0, HB_ACT_RELU_SQUARED = 1, HB_ACT_GELU_ERF = 2, HB_ACT_GELU_TANH = 3, HB_ACT_SWIGLU = 4 };
 __device__ __forceinline__ float activated(float v, int act) {
     if (act == HB_ACT_RELU_SQUARED) {
         v = fmaxf(v, 0.f);
         return v * v;
     }
+    if (act == HB_ACT_GELU_ERF) return GeluErf::of(v);
+    if (act == HB_ACT_GELU_TANH) return GeluTanh::of(v);
     return v;
 }
 
@@ -176,4 +190,30 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&v)[4]) {
     uint2 x;
     x.x = *reinterpret_cast<const uint32_t*>(&lo), x.y = *reinterpret_cast<const uint32_t*>(&hi);
     *reinterpret_cast<uint2*>(p) = x;
+}
+
+// Eight consecutive elements as floats; p is 16-byte aligned.
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16* p, float (&v)[8]) {
+    const uint4 x = *reinterpret_cast<const uint4*>(p);
+    const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&x);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 f = __bfloat1622float2(pairs[k]);
+        v[2 * k] = f.x, v[2 * k + 1] = f.y;
+    }
+}
+__device__ __forceinline__ void store8(float* p, const float (&v)[8]) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const float (&v)[8]) {
+    uint4 x;
+    __nv_bfloat162* pairs = reinterpret_cast<__nv_bfloat162*>(&x);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) pairs[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+    *reinterpret_cast<uint4*>(p) = x;
 }

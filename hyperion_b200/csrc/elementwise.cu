@@ -80,7 +80,7 @@ HB_EXPORT int hb_place_tokens(int* ids, const int* source, const int* pairs, int
 template <typename TD, typename TO>
 __global__ void add_rmsnorm_kernel(float* __restrict__ h, const TD* __restrict__ delta, const float* __restrict__ weight,
                                    TO* __restrict__ out, const int* __restrict__ rows, int hidden, float eps, int write_h) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int r = blockIdx.x;
     const int s = rows ? rows[r] : r;
     float* hrow = h + (size_t)s * hidden;
@@ -111,7 +111,7 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const TD* __restrict__
 template <typename TD, typename TO>
 __global__ void add_rmsnorm_cached_kernel(float* __restrict__ h, const TD* __restrict__ delta, const float* __restrict__ weight,
                                           TO* __restrict__ out, const int* __restrict__ rows, int hidden, float eps, int write_h) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int r = blockIdx.x;
     const int s = rows ? rows[r] : r;
     float* hrow = h + (size_t)s * hidden;
@@ -155,7 +155,9 @@ __global__ void add_rmsnorm_cached_kernel(float* __restrict__ h, const TD* __res
 // The serving path's shape of it (bfloat16 delta and output, rows of a multiple of 8 values): 8 values per thread and
 // group with 16- and 32-byte accesses, each row read once. G groups per thread cover rows of up to 8 * G * 512 values.
 // With `partials` ([splits, tokens, hidden] floats: the split-K sums of the product that made the delta) the delta is
-// their sum in split order plus the bias, rounded to bfloat16 as the product's own reduction would store it.
+// their sum in split order plus the bias, rounded to bfloat16 as the product's own reduction would store it.  Pieces are a
+// matter of their own instance (PIECES): with the room for them a thread holds 128 registers and an SM one block, and a prompt's
+// rows, which are bound by the bytes in flight, then take 2.4 times as long (2,048 rows of 3,584: 33.7 -> 14.9 us).
 // split-K pieces a thread asks for at once (products of a decode step are split 5 to 10 times); fewer where a thread holds
 // several groups of a wide row
 __host__ __device__ constexpr int pieces_ahead(int groups_per_thread) { return groups_per_thread == 1 ? 12 : (groups_per_thread == 2 ? 8 : 4); }
@@ -167,11 +169,11 @@ struct SplitDelta {
     const __nv_bfloat16* bias_h;
 };
 
-template <int G>
+template <int G, bool PIECES>
 __global__ void __launch_bounds__(512) add_rmsnorm_bf16x8_kernel(float* __restrict__ h, const __nv_bfloat16* __restrict__ delta, const SplitDelta split,
                                           const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, const int* __restrict__ rows,
                                           int hidden, float eps, int write_h) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int r = blockIdx.x;
     const int s = rows ? rows[r] : r;
     float* hrow = h + (size_t)s * hidden;
@@ -194,7 +196,7 @@ __global__ void __launch_bounds__(512) add_rmsnorm_bf16x8_kernel(float* __restri
         if (i < hidden) {
             const float4 a = *reinterpret_cast<const float4*>(hrow + i), b = *reinterpret_cast<const float4*>(hrow + i + 4);
             uint4 d4;
-            if (split.partials) {
+            if (PIECES) {
                 float d[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
                 const float* first = split.partials + (size_t)s * hidden + i;
                 // Every piece is asked for before the first is added: a thread that loads four pieces, adds them and only
@@ -268,11 +270,13 @@ static int launch_bf16x8_norm(float* h, const __nv_bfloat16* delta, const SplitD
     const int groups = hidden / 8;
     const int per_thread = groups > 1024 ? 4 : (groups > 512 ? 2 : 1);  // blocks of at most 512 threads: the kernel holds a row's pieces in registers
     const int width = ((groups + per_thread - 1) / per_thread + 31) / 32 * 32;
-    if (per_thread == 1)
-        return launch_after_previous(add_rmsnorm_bf16x8_kernel<1>, n_rows, width, 0, stream, h, delta, split, weight, out, rows, hidden, eps, write_h);
-    if (per_thread == 2)
-        return launch_after_previous(add_rmsnorm_bf16x8_kernel<2>, n_rows, width, 0, stream, h, delta, split, weight, out, rows, hidden, eps, write_h);
-    return launch_after_previous(add_rmsnorm_bf16x8_kernel<4>, n_rows, width, 0, stream, h, delta, split, weight, out, rows, hidden, eps, write_h);
+#define HB_NORM8(G)                                                                                                                                                     \
+    (split.partials ? launch_after_previous(add_rmsnorm_bf16x8_kernel<G, true>, n_rows, width, 0, stream, h, delta, split, weight, out, rows, hidden, eps, write_h) \
+                    : launch_after_previous(add_rmsnorm_bf16x8_kernel<G, false>, n_rows, width, 0, stream, h, delta, split, weight, out, rows, hidden, eps, write_h))
+    if (per_thread == 1) return HB_NORM8(1);
+    if (per_thread == 2) return HB_NORM8(2);
+    return HB_NORM8(4);
+#undef HB_NORM8
 }
 
 // The same with the delta still in pieces: partials [splits, tokens, hidden] floats (+ a bias) are added up in split order
@@ -479,61 +483,80 @@ __global__ void rope_kv_store_kernel(T* __restrict__ x, int stride, int q_heads,
 }
 
 // bfloat16 with head sizes that are multiples of 16: every thread rotates 8 consecutive pairs (two 16-byte loads, two
-// 16-byte stores) or copies 8 values; same arithmetic per element as the scalar kernel.
-__global__ void rope_kv_store_bf16x8_kernel(__nv_bfloat16* __restrict__ x, int stride, int q_heads, int kv_heads, int head_dim,
+// 16-byte stores) or copies 8 values; same arithmetic per element as the scalar kernel.  A thread takes its piece of a head through TOKENS
+// tokens, whose pieces are all asked for before the first is used: with one token a block, a prompt's step was bound by its
+// blocks coming and going (2,048 tokens of 28 + 4 + 4 heads of 128: 15.5 -> 14.1 us).
+template <int TOKENS>
+__global__ void __launch_bounds__(256) rope_kv_store_bf16x8_kernel(__nv_bfloat16* __restrict__ x, int tokens, int stride, int q_heads, int kv_heads, int head_dim,
                                             const int* __restrict__ positions, const float2* __restrict__ table, int max_positions,
                                             __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, int table_width,
                                             const int* __restrict__ token_row, int page_size, int pages, int* status) {
-    const int t = blockIdx.x;
+    const int t0 = blockIdx.x * TOKENS;
     const int half = head_dim >> 1, chunks = half >> 3;  // 8-pair chunks per head
-    let_next_kernel_start();
-    const int pos = positions[t];  // positions and tables come with the step's one copy from the host, not from a kernel
-    const bool pos_ok = pos >= 0 && pos < max_positions;
-    const int block = pos_ok ? pos / page_size : 0;
-    const int page = pos_ok && block < table_width ? block_table[(size_t)token_row[t] * table_width + block] : -1;
-    wait_for_previous_kernels();
-    if (!pos_ok) {
-        if (threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_POSITION);
-        return;
-    }
-    const bool page_ok = page >= 0 && page < pages;
-    if (!page_ok && threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_PAGE);
-    const int slot = pos - block * page_size;
-    __nv_bfloat16* row = x + (size_t)t * stride;
-    const float2* cs = table + (size_t)pos * half;
-    const size_t page_base = (size_t)(page_ok ? page : 0) * 2 * kv_heads * page_size * head_dim;
     const int rotated = (q_heads + kv_heads) * chunks;
     const int total = rotated + kv_heads * 2 * chunks;  // values: head_dim / 8 chunks per head
-    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < total; e += gridDim.y * blockDim.x) {
-        if (e < rotated) {
-            const int head = e / chunks, i = (e - head * chunks) * 8;
-            __nv_bfloat16* p = row + head * head_dim + i;
-            const uint4 lo4 = *reinterpret_cast<const uint4*>(p), hi4 = *reinterpret_cast<const uint4*>(p + half);
-            const __nv_bfloat16* lo = reinterpret_cast<const __nv_bfloat16*>(&lo4);
-            const __nv_bfloat16* hi = reinterpret_cast<const __nv_bfloat16*>(&hi4);
-            uint4 out_lo, out_hi;
-            __nv_bfloat16* y1 = reinterpret_cast<__nv_bfloat16*>(&out_lo);
-            __nv_bfloat16* y2 = reinterpret_cast<__nv_bfloat16*>(&out_hi);
+    const int e = blockIdx.y * blockDim.x + threadIdx.x;
+    const bool turns = e < rotated;
+    const int head = turns ? e / chunks : (e - rotated) / (2 * chunks);
+    const int i = (turns ? e - head * chunks : e - rotated - head * 2 * chunks) * 8;
+    const int at = (turns ? head : q_heads + kv_heads + head) * head_dim + i;
+    const bool stored = !turns || head >= q_heads;  // goes to the token's page
+    // where the page has this piece's place: keys first, then values
+    const size_t in_page = (size_t)(turns ? head - q_heads : kv_heads + head) * page_size * head_dim + i;
+    let_next_kernel_start();
+    int pos[TOKENS], page[TOKENS];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const float2 c = cs[i + j];
-                const float x1 = __bfloat162float(lo[j]), x2 = __bfloat162float(hi[j]);
-                y1[j] = __float2bfloat16_rn(x1 * c.x - x2 * c.y);
-                y2[j] = __float2bfloat16_rn(x2 * c.x + x1 * c.y);
-            }
-            if (head < q_heads) {
-                *reinterpret_cast<uint4*>(p) = out_lo;
-                *reinterpret_cast<uint4*>(p + half) = out_hi;
-            } else if (page_ok) {
-                __nv_bfloat16* dst = cache + page_base + (((size_t)(head - q_heads)) * page_size + slot) * head_dim + i;
-                *reinterpret_cast<uint4*>(dst) = out_lo;
-                *reinterpret_cast<uint4*>(dst + half) = out_hi;
-            }
-        } else if (page_ok) {
-            const int f = e - rotated, head = f / (2 * chunks), i = (f - head * 2 * chunks) * 8;
-            const uint4 v = *reinterpret_cast<const uint4*>(row + (q_heads + kv_heads + head) * head_dim + i);
-            *reinterpret_cast<uint4*>(cache + page_base + (((size_t)(kv_heads + head)) * page_size + slot) * head_dim + i) = v;
+    for (int u = 0; u < TOKENS; ++u) {  // positions and tables come with the step's one copy from the host, not from a kernel
+        pos[u] = t0 + u < tokens ? positions[t0 + u] : 0;
+        const bool pos_ok = pos[u] >= 0 && pos[u] < max_positions;
+        const int block = pos_ok ? pos[u] / page_size : 0;
+        page[u] = t0 + u < tokens && pos_ok && block < table_width ? block_table[(size_t)token_row[t0 + u] * table_width + block] : -1;
+    }
+    wait_for_previous_kernels();
+    uint4 lo4[TOKENS], hi4[TOKENS];
+#pragma unroll
+    for (int u = 0; u < TOKENS; ++u) {
+        if (e < total && t0 + u < tokens) {
+            const __nv_bfloat16* p = x + (size_t)(t0 + u) * stride + at;
+            lo4[u] = *reinterpret_cast<const uint4*>(p);
+            if (turns) hi4[u] = *reinterpret_cast<const uint4*>(p + half);
         }
+    }
+#pragma unroll
+    for (int u = 0; u < TOKENS; ++u) {
+        const int t = t0 + u;
+        if (t >= tokens) break;
+        if (pos[u] < 0 || pos[u] >= max_positions) {
+            if (threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_POSITION);
+            continue;
+        }
+        const bool page_ok = page[u] >= 0 && page[u] < pages;
+        if (!page_ok && threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_PAGE);
+        if (e >= total || (stored && !page_ok)) continue;
+        __nv_bfloat16* dst = stored ? cache + (size_t)page[u] * 2 * kv_heads * page_size * head_dim + in_page + (size_t)(pos[u] % page_size) * head_dim : x + (size_t)t * stride + at;
+        if (!turns) {
+            *reinterpret_cast<uint4*>(dst) = lo4[u];
+            continue;
+        }
+        const __nv_bfloat16* lo = reinterpret_cast<const __nv_bfloat16*>(&lo4[u]);
+        const __nv_bfloat16* hi = reinterpret_cast<const __nv_bfloat16*>(&hi4[u]);
+        uint4 out_lo, out_hi;
+        __nv_bfloat16* y1 = reinterpret_cast<__nv_bfloat16*>(&out_lo);
+        __nv_bfloat16* y2 = reinterpret_cast<__nv_bfloat16*>(&out_hi);
+        const float* cs = reinterpret_cast<const float*>(table + (size_t)pos[u] * half + i);  // cosine and sine in turn
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+            float c[4];
+            load4(cs + 2 * j, c);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const float x1 = __bfloat162float(lo[j + k]), x2 = __bfloat162float(hi[j + k]);
+                y1[j + k] = __float2bfloat16_rn(x1 * c[2 * k] - x2 * c[2 * k + 1]);
+                y2[j + k] = __float2bfloat16_rn(x2 * c[2 * k] + x1 * c[2 * k + 1]);
+            }
+        }
+        *reinterpret_cast<uint4*>(dst) = out_lo;
+        *reinterpret_cast<uint4*>(dst + half) = out_hi;
     }
 }
 
@@ -542,13 +565,17 @@ HB_EXPORT int hb_rope_kv_store(void* x, int is_bf16, int tokens, int stride, int
                                int table_width, const int* token_row, int page_size, int pages, int* status, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (head_dim & 1) return HB_UNSUPPORTED_SIZE;
-    if (is_bf16 && head_dim % 16 == 0 && stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)cache) & 15) == 0) {
-        const int items = (q_heads + 2 * kv_heads) * (head_dim / 16);
-        const int threads = items >= 256 ? 256 : 128;
-        const dim3 grid8(tokens, tokens >= 512 ? 1 : min(8, (items + threads - 1) / threads));
-        return launch_after_previous(rope_kv_store_bf16x8_kernel, grid8, threads, 0, stream, (__nv_bfloat16*)x, stride, q_heads, kv_heads, head_dim,
-                                     positions, (const float2*)table, max_positions, (__nv_bfloat16*)cache, block_table, table_width, token_row,
-                                     page_size, pages, status);
+    if (is_bf16 && head_dim % 16 == 0 && stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)cache | (uintptr_t)table) & 15) == 0) {
+        const int items = (q_heads + 3 * kv_heads) * (head_dim / 16);  // pairs of eight entries, and the values' eights
+        const int across = (items + 255) / 256, threads = ((items + across - 1) / across + 31) / 32 * 32;
+        if (across > 65535) return HB_UNSUPPORTED_SIZE;
+#define HB_ROPE8(TOKENS)                                                                                                                                                 \
+    return launch_after_previous(rope_kv_store_bf16x8_kernel<TOKENS>, dim3((tokens + TOKENS - 1) / TOKENS, across), threads, 0, stream, (__nv_bfloat16*)x, tokens, stride, \
+                                 q_heads, kv_heads, head_dim, positions, (const float2*)table, max_positions, (__nv_bfloat16*)cache, block_table, table_width, token_row,  \
+                                 page_size, pages, status)
+        if (tokens >= 1024) HB_ROPE8(4);  // enough tokens for two blocks an SM all the same
+        HB_ROPE8(1);
+#undef HB_ROPE8
     }
     const int pairs = (q_heads + 2 * kv_heads) * (head_dim / 2);
     const int slices = tokens >= 512 ? 1 : min(16, (pairs + 255) / 256);
@@ -582,7 +609,7 @@ HB_EXPORT int hb_kv_store(const void* src, int is_bf16, int tokens, int stride, 
 template <typename TY, typename TC>
 __global__ void rmsnorm_add_kernel(float* __restrict__ h, const TY* __restrict__ y, const float* __restrict__ weight,
                                    TC* __restrict__ copy, int hidden, float eps) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int t = blockIdx.x;
     float* hrow = h + (size_t)t * hidden;
     const TY* yrow = y + (size_t)t * hidden;
@@ -602,40 +629,29 @@ __global__ void rmsnorm_add_kernel(float* __restrict__ h, const TY* __restrict__
 
 // bfloat16 sublayer outputs in rows of up to 8,192 values, a multiple of 8: a thread keeps its 8 values in registers between the
 // sum of squares and the add (one trip to memory), with 16-byte accesses.
-__global__ void rmsnorm_add_bf16x8_kernel(float* __restrict__ h, const __nv_bfloat16* __restrict__ y, const float* __restrict__ weight,
+__global__ void __launch_bounds__(1024) rmsnorm_add_bf16x8_kernel(float* __restrict__ h, const __nv_bfloat16* __restrict__ y, const float* __restrict__ weight,
                                           __nv_bfloat16* __restrict__ copy, int hidden, float eps) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int t = blockIdx.x, i = threadIdx.x * 8;
     const bool active = i < hidden;
-    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (active) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(y + (size_t)t * hidden + i);
-        const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&raw);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float2 f = __bfloat1622float2(pairs[k]);
-            v[2 * k] = f.x; v[2 * k + 1] = f.y;
-        }
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, x[8], w[8];
+    float* hrow = h + (size_t)t * hidden + i;
+    let_next_kernel_start();
+    if (active) load8(weight + i, w);
+    wait_for_previous_kernels();
+    if (active) {  // both rows are asked for before the sum
+        load8(y + (size_t)t * hidden + i, v);
+        load8(hrow, x);
     }
     float sum = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) sum = fmaf(v[k], v[k], sum);
     const float inv = 1.0f / sqrtf(block_sum(sum, scratch) / (float)hidden + eps);
     if (!active) return;
-    float* hrow = h + (size_t)t * hidden + i;
-    float4 h0 = *reinterpret_cast<const float4*>(hrow), h1 = *reinterpret_cast<const float4*>(hrow + 4);
-    const float4 w0 = *reinterpret_cast<const float4*>(weight + i), w1 = *reinterpret_cast<const float4*>(weight + i + 4);
-    h0.x += v[0] * inv * w0.x; h0.y += v[1] * inv * w0.y; h0.z += v[2] * inv * w0.z; h0.w += v[3] * inv * w0.w;
-    h1.x += v[4] * inv * w1.x; h1.y += v[5] * inv * w1.y; h1.z += v[6] * inv * w1.z; h1.w += v[7] * inv * w1.w;
-    *reinterpret_cast<float4*>(hrow) = h0;
-    *reinterpret_cast<float4*>(hrow + 4) = h1;
-    if (copy) {
-        uint4 packed;
-        __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(&packed);
-        out[0] = __floats2bfloat162_rn(h0.x, h0.y); out[1] = __floats2bfloat162_rn(h0.z, h0.w);
-        out[2] = __floats2bfloat162_rn(h1.x, h1.y); out[3] = __floats2bfloat162_rn(h1.z, h1.w);
-        *reinterpret_cast<uint4*>(copy + (size_t)t * hidden + i) = packed;
-    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] += v[k] * inv * w[k];
+    store8(hrow, x);
+    if (copy) store8(copy + (size_t)t * hidden + i, x);
 }
 
 HB_EXPORT int hb_rmsnorm_add(float* h, const void* y, int y_is_bf16, const float* weight, void* copy, int tokens, int hidden,
@@ -643,8 +659,7 @@ HB_EXPORT int hb_rmsnorm_add(float* h, const void* y, int y_is_bf16, const float
     if (tokens <= 0) return 0;
     if (y_is_bf16 && hidden % 8 == 0 && hidden <= 8192 && (((uintptr_t)h | (uintptr_t)y | (uintptr_t)weight | (uintptr_t)copy) & 15) == 0) {
         const int lanes = ((hidden / 8 + 31) / 32) * 32;  // which kernel runs follows from the width alone
-        rmsnorm_add_bf16x8_kernel<<<tokens, lanes, 0, stream>>>(h, (const __nv_bfloat16*)y, weight, (__nv_bfloat16*)copy, hidden, eps);
-        return launch_status();
+        return launch_after_previous(rmsnorm_add_bf16x8_kernel, tokens, lanes, 0, stream, h, (const __nv_bfloat16*)y, weight, (__nv_bfloat16*)copy, hidden, eps);
     }
     const int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
     if (y_is_bf16)
@@ -682,7 +697,7 @@ __global__ void norm_add_norm_kernel(float* __restrict__ h, const TY* __restrict
                                      const int* __restrict__ rows, int hidden, float eps_post, float eps_next, const float* __restrict__ gate,
                                      int gate_stride, int gate_splits, size_t gate_split_stride, const float* __restrict__ gate_bias) {
     extern __shared__ float row_values[];
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int i = blockIdx.x, t = rows ? rows[i] : i;
     float* hrow = h + (size_t)t * hidden;
     const TY* yrow = y ? y + (size_t)t * hidden : nullptr;
@@ -723,9 +738,11 @@ __global__ void norm_add_norm_bf16x8_kernel(float* __restrict__ h, const __nv_bf
                                             const float* __restrict__ offset, const float* __restrict__ w_next, __nv_bfloat16* __restrict__ out,
                                             const int* __restrict__ rows, int hidden, float eps_post, float eps_next, const float* __restrict__ gate,
                                             int gate_stride, int gate_splits, size_t gate_split_stride, const float* __restrict__ gate_bias) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int i = blockIdx.x, t = rows ? rows[i] : i, j = threadIdx.x * 8;
     const bool active = j < hidden;
+    let_next_kernel_start();
+    wait_for_previous_kernels();
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float inv_y = 0.f;
     if (y) {
@@ -804,9 +821,8 @@ HB_EXPORT int hb_norm_add_norm(float* h, const void* y, int y_is_bf16, const flo
     if (halves && hidden % 8 == 0 && hidden <= 8192 && (!gate || (gate_stride % 4 == 0 && gate_split_stride % 4 == 0)) &&
         (((uintptr_t)h | (uintptr_t)y | (uintptr_t)w_post | (uintptr_t)offset | (uintptr_t)w_next | (uintptr_t)out | (uintptr_t)gate | (uintptr_t)gate_bias) & 15) == 0) {
         const int lanes = ((hidden / 8 + 31) / 32) * 32;  // which kernel runs follows from the width and the types alone
-        norm_add_norm_bf16x8_kernel<<<n_rows, lanes, 0, stream>>>(h, (const __nv_bfloat16*)y, w_post, offset, w_next, (__nv_bfloat16*)out, rows, hidden,
-                                                                  eps_post, eps_next, gate, gate_stride, gate_splits, (size_t)gate_split_stride, gate_bias);
-        return launch_status();
+        return launch_after_previous(norm_add_norm_bf16x8_kernel, n_rows, lanes, 0, stream, h, (const __nv_bfloat16*)y, w_post, offset, w_next, (__nv_bfloat16*)out,
+                                     rows, hidden, eps_post, eps_next, gate, gate_stride, gate_splits, (size_t)gate_split_stride, gate_bias);
     }
     const int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
     const size_t shared = (size_t)hidden * sizeof(float);
@@ -828,13 +844,6 @@ HB_EXPORT int hb_norm_add_norm(float* h, const void* y, int y_is_bf16, const flo
 
 // ---------------------------------------------------------------- GELU, in its tanh and its exact form
 // out = 0.5 z (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))) or 0.5 z (1 + erf(z / sqrt(2))), in float, rounded once.
-struct GeluTanh {
-    static __device__ __forceinline__ float of(float z) { return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
-};
-struct GeluErf {
-    static __device__ __forceinline__ float of(float z) { return 0.5f * z * (1.f + erff(z * 0.7071067811865476f)); }
-};
-
 template <typename T, typename GELU>
 __global__ void gelu_kernel(const T* __restrict__ x, T* __restrict__ out, size_t count) {
     let_next_kernel_start();
@@ -1151,7 +1160,7 @@ template <typename TD, typename TO, int VEC, int CHUNKS>
 __global__ void __launch_bounds__(512) add_pair_norms_kernel(float* __restrict__ h, const PairInputs in, const float* __restrict__ w1, const float* __restrict__ w2,
                                                              TO* __restrict__ out1, TO* __restrict__ out2, const int* __restrict__ rows, int hidden, float eps,
                                                              int write_h) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int r = blockIdx.x, step = blockDim.x * VEC;
     float weight1[CHUNKS][VEC];
     let_next_kernel_start();

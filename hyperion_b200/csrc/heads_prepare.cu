@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(THREADS) heads_prepare_kernel(
     const T* __restrict__ v_first, int v_first_stride, const float* __restrict__ lambda, T* __restrict__ k_cache, T* __restrict__ v_cache,
     size_t page_stride, size_t head_stride, int token_stride, const int* __restrict__ block_table, int table_width,
     const int* __restrict__ token_row, int page_size, int pages, int* status) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int t = blockIdx.x, head = blockIdx.y;  // heads in the row's order: q heads, k heads, v heads
     const int pos = positions[t];
     T* row = x + (size_t)t * stride;
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(THREADS) heads_prepare_wide_kernel(
     TO* __restrict__ k_cache, TO* __restrict__ v_cache, size_t page_stride, size_t head_stride, int token_stride,
     const int* __restrict__ block_table, int table_width, const int* __restrict__ token_row, int page_size, int pages, float v_unit_eps,
     const float* __restrict__ q_head_scale, const float* __restrict__ v_inv_freq, int v_rot_dims, int v_rot_half, int* status) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int t = blockIdx.x, head = blockIdx.y;  // q heads, then k heads, then v heads
     const int pos = positions[t];
     const float* row = x + (size_t)t * stride;
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(TOKEN_THREADS) heads_prepare_token_kernel(
     TO* __restrict__ v_cache, size_t page_stride, size_t head_stride, int token_stride, const int* __restrict__ block_table, int table_width,
     const int* __restrict__ token_row, int page_size, int pages, float v_unit_eps, const float* __restrict__ q_head_scale,
     const float* __restrict__ v_inv_freq, int v_rot_dims, int v_rot_half, int* status) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     __shared__ float cs[MAX_PAIRS], sn[MAX_PAIRS], vcs[MAX_PAIRS], vsn[MAX_PAIRS];
     const int t = blockIdx.x;
     const int pos = positions[t];
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(TOKEN_THREADS) latent_prepare_kernel(
     const float* __restrict__ q_norm, const float* __restrict__ kv_norm, float eps, const float* __restrict__ inv_freq,
     const int* __restrict__ positions, TO* __restrict__ cq_out, int cq_stride, TO* __restrict__ cache, size_t page_stride, int token_stride,
     const int* __restrict__ block_table, int table_width, const int* __restrict__ token_row, int page_size, int pages, int* status) {
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int t = blockIdx.x;
     const int pos = positions[t];
     const float* row = x + (size_t)t * stride;

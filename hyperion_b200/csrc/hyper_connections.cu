@@ -69,7 +69,7 @@ __device__ __forceinline__ void take_result(const HyperArgs& a, int which, size_
 template <typename TD, typename TO, int VEC, int CHUNKS, int SMAX>
 __global__ void __launch_bounds__(512, CHUNKS <= 2 && SMAX <= 4 ? 2 : 1) hyper_connect_kernel(const HyperArgs a) {
     constexpr bool EXACT = HB_STREAMS > 0, AHEAD = EXACT && CHUNKS == 1;  // a row's streams are asked for before the sums of squares (more of them cost a block of occupancy)
-    __shared__ float scratch[32];
+    __shared__ __align__(16) float scratch[32];
     const int r = blockIdx.x, step = blockDim.x * VEC, hidden = a.hidden;
     const int streams = EXACT ? SMAX : a.streams;
     __shared__ __align__(16) float mix[EXACT ? SMAX : 1][EXACT ? SMAX : 1], share[EXACT ? SMAX : 1], read[EXACT ? SMAX : 1];  // mix[t][s]: from s to t
