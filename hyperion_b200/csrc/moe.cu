@@ -26,62 +26,93 @@
 #include "common.cuh"
 
 namespace {
-constexpr int ROUTE_THREADS = 256, ROUTE_MOST_SHARED = 200 * 1024;  // always allowed in full: another thread's call may come between a call's allowance and its launch
+constexpr int ROUTE_MOST_SHARED = 200 * 1024;  // always allowed in full: another thread's call may come between a call's allowance and its launch
+// a block has a warp for every AT_ONCE experts, as far as that goes; eight tokens' sums leave two blocks of nine warps to an SM
+__host__ __device__ constexpr int route_most_threads(int tokens_of_block) { return tokens_of_block == 8 ? 288 : 512; }
+__host__ __device__ constexpr int route_at_once(int tokens_of_block) { return tokens_of_block == 1 ? 1 : 2; }
 
-// One block per token: the row in shared memory as floats, a warp per expert at a time.  A lane adds up every 32nd group of four
-// columns in four chains of its own (columns beyond a multiple of four go to the first chain), the chains are added in a fixed
-// order and the lanes meet in a butterfly: a logit depends on nothing but the row and the expert's weights.
-template <typename T>
-__device__ __forceinline__ void router_logits(const T* __restrict__ x, int x_stride, const float* __restrict__ router, int hidden, int experts, float* row,
-                                              float* logit) {
-    const int padded = (hidden + 3) & ~3;
-    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < padded; i += ROUTE_THREADS) row[i] = i < hidden ? to_float(x[(size_t)t * x_stride + i]) : 0.f;
+// A block serves TOKENS tokens, their rows in shared memory as floats; a warp takes several experts at a time, so that what it reads of the rows serves
+// them all and what it reads of the router's matrix serves all the block's tokens.  A lane adds up every 32nd group of four columns in four chains of its
+// own (columns beyond a multiple of four go to the first chain), the chains are added in a fixed order and the lanes meet in a butterfly: a logit depends
+// on nothing but the row and the expert's weights, whatever TOKENS is.
+// With a token a block, a prompt is bound by the matrix coming from L2 once per token; with eight, two experts a warp, by what it reads of the rows in
+// shared memory and by too few warps (2,048 tokens of 2,048 columns, 18 outputs: 43.0 -> 20.8 us).  Steps of few tokens, which are one block's latency, take a token a
+// block and a warp per expert, all of a row's pieces asked for at once.
+template <typename T, int TOKENS>
+__device__ __forceinline__ void router_logits(const T* __restrict__ x, int x_stride, const float* __restrict__ router, const float* __restrict__ bias, int first, int count,
+                                              int hidden, int experts, float* rows, float* logits) {
+    constexpr int AT_ONCE = route_at_once(TOKENS), UNROLL = TOKENS == 1 ? 8 : 2;
+    const int threads = blockDim.x;
+    const int padded = (hidden + 3) & ~3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool rows_by_four = (hidden & 3) == 0 && (x_stride & 3) == 0 && (((uintptr_t)x) & (4 * sizeof(T) - 1)) == 0;
+    if (rows_by_four) {
+        const int quads = hidden >> 2, all = TOKENS * quads;
+        for (int base = threadIdx.x; base < all; base += 4 * threads) {  // four pieces are asked for before the first is used
+            float v[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int piece = base + u * threads;
+                if (piece < all) load4(x + (size_t)(first + min(TOKENS == 1 ? 0 : piece / quads, count - 1)) * x_stride + (TOKENS == 1 ? piece : piece % quads) * 4, v[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int piece = base + u * threads;
+                if (piece < all) store4(rows + (size_t)piece * 4, v[u]);  // padded is hidden here
+            }
+        }
+    } else {
+        for (int j = 0; j < TOKENS; ++j)
+            for (int i = threadIdx.x; i < padded; i += threads) rows[(size_t)j * padded + i] = i < hidden ? to_float(x[(size_t)(first + min(j, count - 1)) * x_stride + i]) : 0.f;
+    }
     __syncthreads();
     const bool by_four = (hidden & 3) == 0 && (((uintptr_t)router) & 15) == 0;
-    for (int e = warp; e < experts; e += ROUTE_THREADS / 32) {
-        const float* w = router + (size_t)e * hidden;
-        float part[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int e = AT_ONCE * warp; e < experts; e += AT_ONCE * threads / 32) {
+        const int there = min(AT_ONCE, experts - e);
+        const float* w[AT_ONCE];
+        float part[AT_ONCE][TOKENS][4];
+#pragma unroll
+        for (int s = 0; s < AT_ONCE; ++s) {
+            w[s] = router + (size_t)(e + min(s, there - 1)) * hidden;
+#pragma unroll
+            for (int j = 0; j < TOKENS; ++j) part[s][j][0] = part[s][j][1] = part[s][j][2] = part[s][j][3] = 0.f;
+        }
         if (by_four) {
-#pragma unroll 4
+#pragma unroll UNROLL
             for (int i = lane * 4; i < hidden; i += 128) {
-                const float4 wv = *reinterpret_cast<const float4*>(w + i), rv = *reinterpret_cast<const float4*>(row + i);
-                part[0] = fmaf(rv.x, wv.x, part[0]); part[1] = fmaf(rv.y, wv.y, part[1]);
-                part[2] = fmaf(rv.z, wv.z, part[2]); part[3] = fmaf(rv.w, wv.w, part[3]);
+                float4 wv[AT_ONCE];
+#pragma unroll
+                for (int s = 0; s < AT_ONCE; ++s) wv[s] = *reinterpret_cast<const float4*>(w[s] + i);
+#pragma unroll
+                for (int j = 0; j < TOKENS; ++j) {
+                    const float4 rv = *reinterpret_cast<const float4*>(rows + (size_t)j * padded + i);
+#pragma unroll
+                    for (int s = 0; s < AT_ONCE; ++s) {
+                        part[s][j][0] = fmaf(rv.x, wv[s].x, part[s][j][0]); part[s][j][1] = fmaf(rv.y, wv[s].y, part[s][j][1]);
+                        part[s][j][2] = fmaf(rv.z, wv[s].z, part[s][j][2]); part[s][j][3] = fmaf(rv.w, wv[s].w, part[s][j][3]);
+                    }
+                }
             }
         } else {
             for (int i = lane * 4; i < hidden; i += 128)
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (i + j < hidden) part[j] = fmaf(row[i + j], w[i + j], part[j]);
+                for (int c = 0; c < 4; ++c)
+                    if (i + c < hidden)
+#pragma unroll
+                        for (int s = 0; s < AT_ONCE; ++s)
+#pragma unroll
+                            for (int j = 0; j < TOKENS; ++j) part[s][j][c] = fmaf(rows[(size_t)j * padded + i + c], w[s][i + c], part[s][j][c]);
         }
-        const float sum = warp_sum((part[0] + part[1]) + (part[2] + part[3]));
-        if (lane == 0) logit[e] = sum;
+#pragma unroll
+        for (int s = 0; s < AT_ONCE; ++s) {
+            const float b = bias && s < there ? bias[e + s] : 0.f;
+#pragma unroll
+            for (int j = 0; j < TOKENS; ++j) {
+                const float sum = warp_sum((part[s][j][0] + part[s][j][1]) + (part[s][j][2] + part[s][j][3]));
+                if (lane == 0 && s < there) logits[j * experts + e + s] = sum + b;
+            }
+        }
     }
     __syncthreads();
-}
-
-template <typename T>
-__global__ void __launch_bounds__(ROUTE_THREADS) moe_route_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router, int hidden,
-                                                                  int experts, int top, int weighted, int* __restrict__ chosen,
-                                                                  float* __restrict__ weights) {
-    extern __shared__ __align__(16) float shared[];  // the token's row (padded to a multiple of four), then one logit per expert
-    float* row = shared;
-    float* logit = shared + ((hidden + 3) & ~3);
-    const int t = blockIdx.x;
-    router_logits(x, x_stride, router, hidden, experts, row, logit);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < top; ++k) {
-            int best = -1;
-            float value = -INFINITY;
-            for (int e = 0; e < experts; ++e)
-                if (logit[e] > value || (best < 0 && logit[e] == value)) { best = e; value = logit[e]; }
-            if (best < 0) best = 0;  // only when every logit left is not a number
-            chosen[(size_t)t * top + k] = best;
-            weights[(size_t)t * top + k] = weighted ? 1.0f / (1.0f + expf(-value)) : 1.f;
-            logit[best] = -INFINITY;
-        }
-    }
 }
 
 // The largest value among the lanes, the lowest index among equals; a lane without a candidate brings index INT_MAX.
@@ -94,25 +125,61 @@ __device__ __forceinline__ void warp_best(float& value, int& index) {
     }
 }
 
+// After the logits, warp j searches and weighs token j.
+template <typename T, int TOKENS>
+__global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 1) moe_route_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router, int tokens, int hidden,
+                                                                          int experts, int top, int weighted, int* __restrict__ chosen, float* __restrict__ weights) {
+    extern __shared__ __align__(16) float shared[];  // TOKENS rows (padded to a multiple of four), then a logit per token and expert
+    float* logits = shared + (size_t)TOKENS * ((hidden + 3) & ~3);
+    const int first = blockIdx.x * TOKENS, count = min(TOKENS, tokens - first), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    router_logits<T, TOKENS>(x, x_stride, router, nullptr, first, count, hidden, experts, shared, logits);
+    if (warp >= count) return;
+    float* z = logits + warp * experts;
+    const size_t t = first + warp;
+    for (int k = 0; k < top; ++k) {
+        float value = -INFINITY;
+        int index = 0x7fffffff;
+        for (int e = lane; e < experts; e += 32)
+            if (z[e] > value || (index == 0x7fffffff && z[e] == value)) { value = z[e]; index = e; }
+        warp_best(value, index);
+        if (index == 0x7fffffff) {  // only when every logit left is not a number
+            index = 0;
+            value = -INFINITY;
+        }
+        __syncwarp();
+        if (lane == 0) {
+            chosen[t * top + k] = index;
+            weights[t * top + k] = weighted ? 1.0f / (1.0f + expf(-value)) : 1.f;
+            z[index] = -INFINITY;
+        }
+        __syncwarp();
+    }
+}
+
 // Softmax scores over all `outputs` of the router, choice by score + correction inside the best `group_keep` of `group_count` groups of
 // neighbours (a group's rank is its largest choice score; group_count <= 1: no groups), weights = plain score * scale.  The logits are
-// taken as in the kernel above; everything after them is the first warp's work, sums and searches in a fixed order.
-template <typename T>
-__global__ void __launch_bounds__(ROUTE_THREADS) moe_route_scored_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
-                                                                         const float* __restrict__ correction, int hidden, int outputs, int top,
+// taken as in the kernel above; everything after them is warp j's work for token j, sums and searches in a fixed order.
+template <typename T, int TOKENS>
+__global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 1) moe_route_scored_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
+                                                                         const float* __restrict__ correction, int tokens, int hidden, int outputs, int top,
                                                                          int group_count, int group_keep, float scale, int* __restrict__ chosen,
                                                                          float* __restrict__ weights) {
-    extern __shared__ __align__(16) float shared[];  // the row, then per output: logit, score, choice score, a flag; then per group: best, a flag
-    float* row = shared;
-    float* logit = shared + ((hidden + 3) & ~3);
-    float* score = logit + outputs;
+    extern __shared__ __align__(16) float shared[];  // TOKENS rows; a logit per token and output; then per token: score, choice score and a flag per output, best and a flag per group
+    const int groups = group_count > 0 ? group_count : 1, first = blockIdx.x * TOKENS, count = min(TOKENS, tokens - first), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* logits = shared + (size_t)TOKENS * ((hidden + 3) & ~3);
+    let_next_kernel_start();
+    wait_for_previous_kernels();
+    router_logits<T, TOKENS>(x, x_stride, router, nullptr, first, count, hidden, outputs, shared, logits);
+    if (warp >= count) return;
+    const float* logit = logits + warp * outputs;
+    float* score = logits + TOKENS * outputs + warp * (3 * outputs + 2 * groups);
     float* choice = score + outputs;
     int* dead = reinterpret_cast<int*>(choice + outputs);
     float* group_best = reinterpret_cast<float*>(dead + outputs);
-    int* group_kept = reinterpret_cast<int*>(group_best + (group_count > 0 ? group_count : 1));
-    const int t = blockIdx.x, lane = threadIdx.x & 31;
-    router_logits(x, x_stride, router, hidden, outputs, row, logit);
-    if (threadIdx.x >= 32) return;
+    int* group_kept = reinterpret_cast<int*>(group_best + groups);
+    const size_t t = first + warp;
     float most = -INFINITY;
     for (int e = lane; e < outputs; e += 32) most = fmaxf(most, logit[e]);
 #pragma unroll
@@ -159,21 +226,19 @@ __global__ void __launch_bounds__(ROUTE_THREADS) moe_route_scored_kernel(const T
         warp_best(value, index);
         if (index == 0x7fffffff) index = 0;  // only when fewer outputs can be chosen than are asked for
         if (lane == 0) {
-            chosen[(size_t)t * top + k] = index;
-            weights[(size_t)t * top + k] = score[index] * scale;
+            chosen[t * top + k] = index;
+            weights[t * top + k] = score[index] * scale;
             dead[index] = 1;
         }
         __syncwarp();
     }
 }
 
-// Softmax over the chosen logits alone.  A block serves TOKENS tokens, so that a prompt-sized step reads the router's matrix once per TOKENS
-// tokens; a logit is summed in the same order whatever TOKENS is.  Warp j then searches and weighs token j.
+// Softmax over the chosen logits alone.
 template <typename T, int TOKENS>
-__global__ void __launch_bounds__(ROUTE_THREADS) moe_route_softmax_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
+__global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 1) moe_route_softmax_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
                                                                           const float* __restrict__ bias, int tokens, int hidden, int experts, int top,
                                                                           int* __restrict__ chosen, float* __restrict__ weights) {
-    static_assert(TOKENS <= ROUTE_THREADS / 32, "a warp per token");
     extern __shared__ __align__(16) float shared[];  // TOKENS rows, then per token: a logit per expert, the chosen logits
     const int padded = (hidden + 3) & ~3;
     float* logits = shared + (size_t)TOKENS * padded;
@@ -181,66 +246,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) moe_route_softmax_kernel(const 
     const int first = blockIdx.x * TOKENS, count = min(TOKENS, tokens - first), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     let_next_kernel_start();
     wait_for_previous_kernels();
-    const bool rows_by_four = (hidden & 3) == 0 && (x_stride & 3) == 0 && (((uintptr_t)x) & (4 * sizeof(T) - 1)) == 0;
-    for (int j = 0; j < TOKENS; ++j) {
-        float* row = shared + (size_t)j * padded;
-        const T* from = x + (size_t)(first + min(j, count - 1)) * x_stride;
-        if (rows_by_four) {
-            for (int i = threadIdx.x * 4; i < hidden; i += ROUTE_THREADS * 4) {
-                float v[4];
-                load4(from + i, v);
-                store4(row + i, v);
-            }
-        } else {
-            for (int i = threadIdx.x; i < padded; i += ROUTE_THREADS) row[i] = i < hidden ? to_float(from[i]) : 0.f;
-        }
-    }
-    __syncthreads();
-    const bool by_four = (hidden & 3) == 0 && (((uintptr_t)router) & 15) == 0;
-    // a warp takes two experts at a time, so that what it reads of the rows serves both
-    for (int e = 2 * warp; e < experts; e += ROUTE_THREADS / 16) {
-        const int there = min(2, experts - e);
-        const float* w[2] = {router + (size_t)e * hidden, router + (size_t)(e + there - 1) * hidden};
-        float part[2][TOKENS][4];
-#pragma unroll
-        for (int s = 0; s < 2; ++s)
-#pragma unroll
-            for (int j = 0; j < TOKENS; ++j) part[s][j][0] = part[s][j][1] = part[s][j][2] = part[s][j][3] = 0.f;
-        if (by_four) {
-#pragma unroll 4
-            for (int i = lane * 4; i < hidden; i += 128) {
-                const float4 wv[2] = {*reinterpret_cast<const float4*>(w[0] + i), *reinterpret_cast<const float4*>(w[1] + i)};
-#pragma unroll
-                for (int j = 0; j < TOKENS; ++j) {
-                    const float4 rv = *reinterpret_cast<const float4*>(shared + (size_t)j * padded + i);
-#pragma unroll
-                    for (int s = 0; s < 2; ++s) {
-                        part[s][j][0] = fmaf(rv.x, wv[s].x, part[s][j][0]); part[s][j][1] = fmaf(rv.y, wv[s].y, part[s][j][1]);
-                        part[s][j][2] = fmaf(rv.z, wv[s].z, part[s][j][2]); part[s][j][3] = fmaf(rv.w, wv[s].w, part[s][j][3]);
-                    }
-                }
-            }
-        } else {
-            for (int i = lane * 4; i < hidden; i += 128)
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    if (i + c < hidden)
-#pragma unroll
-                        for (int s = 0; s < 2; ++s)
-#pragma unroll
-                            for (int j = 0; j < TOKENS; ++j) part[s][j][c] = fmaf(shared[(size_t)j * padded + i + c], w[s][i + c], part[s][j][c]);
-        }
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const float b = bias && s < there ? bias[e + s] : 0.f;
-#pragma unroll
-            for (int j = 0; j < TOKENS; ++j) {
-                const float sum = warp_sum((part[s][j][0] + part[s][j][1]) + (part[s][j][2] + part[s][j][3]));
-                if (lane == 0 && s < there) logits[j * experts + e + s] = sum + b;
-            }
-        }
-    }
-    __syncthreads();
+    router_logits<T, TOKENS>(x, x_stride, router, bias, first, count, hidden, experts, shared, logits);
     if (warp >= count) return;
     float* z = logits + warp * experts;
     float* mine = picked + warp * top;
@@ -272,42 +278,89 @@ __global__ void __launch_bounds__(ROUTE_THREADS) moe_route_softmax_kernel(const 
 
 constexpr int PLAN_THREADS = 1024;
 
-// One block.  counts and cursors live in shared memory (experts <= 1024).
+// One block.  counts live in shared memory (experts <= 1024).  A thread keeps its first PLAN_KEPT pairs and their places in their experts' runs in
+// registers between the counting and the writing: one read of the choices and one round of atomics
+// (4,096 pairs of 16 experts: 10.0 -> 7.5 us; it is one block's latency).
+constexpr int PLAN_KEPT = 8;
 __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int* __restrict__ chosen, const float* __restrict__ weights, int pairs, int top,
                                                                 int experts, int pad, int capacity, int* __restrict__ slot_of,
                                                                 int* __restrict__ slot_token, float* __restrict__ slot_weight,
                                                                 int* __restrict__ tile_expert, int* __restrict__ tile_rows) {
-    __shared__ int count[1024], start[1024];
-    const int tid = threadIdx.x;
+    __shared__ int count[1024], start[1025];
+    const int tid = threadIdx.x, lane = tid & 31;
+    // the next kernel is not let in early: while the kernels before still hold some SMs, the streamed product's blocks would crowd onto the free ones and read
+    // the matrices from there alone (14 matrices of [2,048, 2,048]: 47 us instead of 24)
     for (int e = tid; e < experts; e += PLAN_THREADS) count[e] = 0;
-    for (int s = tid; s < capacity; s += PLAN_THREADS) { slot_token[s] = -1; slot_weight[s] = 0.f; }
-    for (int i = tid; i < capacity / pad; i += PLAN_THREADS) { tile_expert[i] = -1; tile_rows[i] = 0; }
-    __syncthreads();
-    for (int i = tid; i < pairs; i += PLAN_THREADS)
-        if (chosen[i] < experts) atomicAdd(&count[chosen[i]], 1);  // a choice beyond the experts with matrices takes no row
-    __syncthreads();
-    if (tid == 0) {
-        int at = 0;
-        for (int e = 0; e < experts; ++e) {
-            start[e] = at;
-            const int tiles = (count[e] + pad - 1) / pad;
-            for (int i = 0; i < tiles; ++i) {
-                tile_expert[at / pad + i] = e;
-                tile_rows[at / pad + i] = min(pad, count[e] - i * pad);
-            }
-            at += tiles * pad;
-            count[e] = 0;  // from here on: the cursor inside the expert's run
-        }
+    wait_for_previous_kernels();
+    int kept[PLAN_KEPT], place[PLAN_KEPT];
+#pragma unroll
+    for (int u = 0; u < PLAN_KEPT; ++u) {
+        const int i = tid + u * PLAN_THREADS;
+        kept[u] = i < pairs ? chosen[i] : experts;
     }
     __syncthreads();
+#pragma unroll
+    for (int u = 0; u < PLAN_KEPT; ++u)  // a choice beyond the experts with matrices takes no row
+        place[u] = kept[u] < experts ? atomicAdd(&count[kept[u]], 1) : 0;
+    if (pairs > PLAN_KEPT * PLAN_THREADS) __syncthreads();  // the places above are the first of every run
+    for (int i = tid + PLAN_KEPT * PLAN_THREADS; i < pairs; i += PLAN_THREADS)
+        if (chosen[i] < experts) atomicAdd(&count[chosen[i]], 1);
+    __syncthreads();
+    if (tid < 32) {  // where every expert's run of whole tiles begins: a scan by the first warp
+        int before = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int e = e0 + lane, tiles = e < experts ? (count[e] + pad - 1) / pad : 0;
+            int upto = tiles;
+#pragma unroll
+            for (int offset = 1; offset < 32; offset <<= 1) {
+                const int other = __shfl_up_sync(0xffffffffu, upto, offset);
+                if (lane >= offset) upto += other;
+            }
+            if (e < experts) start[e] = (before + upto - tiles) * pad;
+            before += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (lane == 0) start[experts] = before * pad;
+    }
+    __syncthreads();
+    for (int i = tid; i < capacity / pad; i += PLAN_THREADS) {
+        const int at = i * pad;
+        int low = 0, high = experts;  // the last expert whose run does not begin after this tile
+        while (high - low > 1) {
+            const int middle = (low + high) / 2;
+            if (start[middle] <= at) low = middle; else high = middle;
+        }
+        const bool used = at < start[experts];
+        tile_expert[i] = used ? low : -1;
+        tile_rows[i] = used ? min(pad, count[low] - (at - start[low])) : 0;
+    }
+    for (int s = tid; s < capacity; s += PLAN_THREADS) {  // what no pair takes
+        const int at = s;
+        int low = 0, high = experts;
+        while (high - low > 1) {
+            const int middle = (low + high) / 2;
+            if (start[middle] <= at) low = middle; else high = middle;
+        }
+        if (at >= start[experts] || at - start[low] >= count[low]) { slot_token[s] = -1; slot_weight[s] = 0.f; }
+    }
     // which slot of its expert's run a pair takes depends on the order of the atomics; a row's result does not depend on its slot
-    for (int i = tid; i < pairs; i += PLAN_THREADS) {
-        const int e = chosen[i];
-        if (e >= experts) { slot_of[i] = -1; continue; }
-        const int slot = start[e] + atomicAdd(&count[e], 1);
+    auto put = [&](int i, int e, int at) {
+        if (e >= experts) { slot_of[i] = -1; return; }
+        const int slot = start[e] + at;
         slot_of[i] = slot;
         slot_token[slot] = i / top;
         slot_weight[slot] = weights ? weights[i] : 1.f;
+    };
+#pragma unroll
+    for (int u = 0; u < PLAN_KEPT; ++u) {
+        const int i = tid + u * PLAN_THREADS;
+        if (i < pairs) put(i, kept[u], place[u]);
+    }
+    if (pairs <= PLAN_KEPT * PLAN_THREADS) return;
+    // longer lists: their ends take their places in a second round, from the ends of the runs down
+    __syncthreads();
+    for (int i = tid + PLAN_KEPT * PLAN_THREADS; i < pairs; i += PLAN_THREADS) {
+        const int e = chosen[i];
+        put(i, e, e < experts ? atomicSub(&count[e], 1) - 1 : 0);
     }
 }
 
@@ -478,7 +531,33 @@ __global__ void moe_combine_weighted_bf16x8_kernel(const __nv_bfloat16* __restri
         *reinterpret_cast<uint4*>(out + (size_t)t * hidden + i) = packed;
     }
 }
+
+// How many tokens a router's block takes: eight where that leaves about a block to an SM, fewer where the step or the shared memory of two blocks on an SM is
+// smaller, one where few tokens would leave the device empty (16 tokens, 16 experts: a token a block 5.6 us, as before).
+template <typename Bytes>
+int tokens_of_block(int tokens, Bytes bytes) {
+    if (tokens >= 1024 && bytes(8) <= 100 * 1024) return 8;
+    return tokens >= 512 && bytes(4) <= 100 * 1024 ? 4 : 1;
+}
+
+template <typename... Params, typename... Args>
+int launch_router(void (*kernel)(Params...), int at_once, int tokens, int outputs, size_t shared, cudaStream_t stream, Args... args) {
+    if (shared > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
+    const int each = route_at_once(at_once), wanted = (outputs + each - 1) / each, least = at_once > 4 ? at_once : 4;  // at least a warp per token
+    const int warps = wanted < least ? least : (wanted > route_most_threads(at_once) / 32 ? route_most_threads(at_once) / 32 : wanted);
+    return launch_after_previous(kernel, dim3((tokens + at_once - 1) / at_once), dim3(32 * warps), shared, stream, args...);
+}
 }  // namespace
+
+#define HB_ROUTE_TOKENS()                        \
+    if (is_bf16) {                               \
+        if (at_once == 8) HB_ROUTE(__nv_bfloat16, 8); \
+        if (at_once == 4) HB_ROUTE(__nv_bfloat16, 4); \
+        HB_ROUTE(__nv_bfloat16, 1);              \
+    }                                            \
+    if (at_once == 8) HB_ROUTE(float, 8);        \
+    if (at_once == 4) HB_ROUTE(float, 4);        \
+    HB_ROUTE(float, 1)
 
 HB_EXPORT int hb_moe_route_scored(const void* x, int is_bf16, int x_stride, const float* router, const float* correction, int tokens, int hidden,
                                   int outputs, int top, int group_count, int group_keep, float scale, int* chosen, float* weights, cudaStream_t stream) {
@@ -486,18 +565,16 @@ HB_EXPORT int hb_moe_route_scored(const void* x, int is_bf16, int x_stride, cons
     if (outputs <= 0 || outputs > 1024 || top <= 0 || top > outputs || hidden <= 0) return HB_UNSUPPORTED_SIZE;
     if (group_count > 1 && (outputs % group_count || group_keep <= 0 || group_keep > group_count || top > group_keep * (outputs / group_count)))
         return HB_BAD_ARGUMENT;
-    const size_t shared = (size_t)(((hidden + 3) & ~3) + 4 * outputs + 2 * (group_count > 0 ? group_count : 1)) * sizeof(float);
+    const int groups = group_count > 0 ? group_count : 1;
+    auto bytes = [&](int at_once) { return (size_t)at_once * (((hidden + 3) & ~3) + 4 * outputs + 2 * groups) * sizeof(float); };
+    const int at_once = tokens_of_block(tokens, bytes);
+    const size_t shared = bytes(at_once);
     if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
-    if (is_bf16) {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_scored_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
-        moe_route_scored_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const __nv_bfloat16*)x, x_stride, router, correction, hidden, outputs, top,
-                                                                          group_count, group_keep, scale, chosen, weights);
-    } else {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_scored_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
-        moe_route_scored_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const float*)x, x_stride, router, correction, hidden, outputs, top, group_count,
-                                                                          group_keep, scale, chosen, weights);
-    }
-    return launch_status();
+#define HB_ROUTE(T, N)                                                                                                                                         \
+    return launch_router(moe_route_scored_kernel<T, N>, N, tokens, outputs, shared, stream, (const T*)x, x_stride, router, correction, tokens, hidden, outputs, top, group_count, \
+                         group_keep, scale, chosen, weights)
+    HB_ROUTE_TOKENS();
+#undef HB_ROUTE
 }
 
 // y [capacity, hidden], x [tokens, x_stride] (what the feed-forward read), base [tokens, hidden] (optional, with an optional gate per token)
@@ -525,16 +602,13 @@ HB_EXPORT int hb_moe_route(const void* x, int is_bf16, int x_stride, const float
                            int* chosen, float* weights, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (experts <= 0 || experts > 1024 || top <= 0 || top > experts || hidden <= 0) return HB_UNSUPPORTED_SIZE;
-    const size_t shared = (size_t)(((hidden + 3) & ~3) + experts) * sizeof(float);
+    auto bytes = [&](int at_once) { return (size_t)at_once * (((hidden + 3) & ~3) + experts) * sizeof(float); };
+    const int at_once = tokens_of_block(tokens, bytes);
+    const size_t shared = bytes(at_once);
     if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
-    if (is_bf16) {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
-        moe_route_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const __nv_bfloat16*)x, x_stride, router, hidden, experts, top, weighted, chosen, weights);
-    } else {
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
-        moe_route_kernel<<<tokens, ROUTE_THREADS, shared, stream>>>((const float*)x, x_stride, router, hidden, experts, top, weighted, chosen, weights);
-    }
-    return launch_status();
+#define HB_ROUTE(T, N) return launch_router(moe_route_kernel<T, N>, N, tokens, experts, shared, stream, (const T*)x, x_stride, router, tokens, hidden, experts, top, weighted, chosen, weights)
+    HB_ROUTE_TOKENS();
+#undef HB_ROUTE
 }
 
 HB_EXPORT int hb_moe_route_softmax(const void* x, int is_bf16, int x_stride, const float* router, const float* bias, int tokens, int hidden, int experts,
@@ -542,22 +616,13 @@ HB_EXPORT int hb_moe_route_softmax(const void* x, int is_bf16, int x_stride, con
     if (tokens <= 0) return 0;
     if (experts <= 0 || experts > 1024 || top <= 0 || top > experts || hidden <= 0) return HB_UNSUPPORTED_SIZE;
     auto bytes = [&](int at_once) { return (size_t)at_once * (((hidden + 3) & ~3) + experts + top) * sizeof(float); };
-    const int at_once = tokens >= 512 && bytes(4) <= 100 * 1024 ? 4 : 1;  // a step of few tokens fills more of the device with a token per block
+    const int at_once = tokens_of_block(tokens, bytes);
     const size_t shared = bytes(at_once);
     if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
-#define HB_ROUTE(T, N)                                                                                                                                  \
-    {                                                                                                                                                   \
-        if (shared > 48 * 1024) cudaFuncSetAttribute(moe_route_softmax_kernel<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);          \
-        return launch_after_previous(moe_route_softmax_kernel<T, N>, dim3((tokens + N - 1) / N), dim3(ROUTE_THREADS), shared, stream, (const T*)x, x_stride, \
-                                     router, bias, tokens, hidden, experts, top, chosen, weights);                                                      \
-    }
-    if (is_bf16) {
-        if (at_once == 4) HB_ROUTE(__nv_bfloat16, 4);
-        HB_ROUTE(__nv_bfloat16, 1);
-    }
-    if (at_once == 4) HB_ROUTE(float, 4);
-    HB_ROUTE(float, 1);
+#define HB_ROUTE(T, N) return launch_router(moe_route_softmax_kernel<T, N>, N, tokens, experts, shared, stream, (const T*)x, x_stride, router, bias, tokens, hidden, experts, top, chosen, weights)
+    HB_ROUTE_TOKENS();
 #undef HB_ROUTE
+#undef HB_ROUTE_TOKENS
 }
 
 // capacity: a multiple of pad, at least pairs + experts * (pad - 1) rounded up to it.  tile_expert and tile_rows (the real rows at the start
@@ -567,8 +632,8 @@ HB_EXPORT int hb_moe_plan(const int* chosen, const float* weights, int pairs, in
     if (pairs <= 0) return 0;
     if (experts <= 0 || experts > 1024 || pad <= 0 || capacity % pad || top <= 0) return HB_UNSUPPORTED_SIZE;
     if ((long long)capacity < (long long)pairs + (long long)experts * (pad - 1)) return HB_BAD_ARGUMENT;
-    moe_plan_kernel<<<1, PLAN_THREADS, 0, stream>>>(chosen, weights, pairs, top, experts, pad, capacity, slot_of, slot_token, slot_weight, tile_expert, tile_rows);
-    return launch_status();
+    return launch_after_previous(moe_plan_kernel, dim3(1), dim3(PLAN_THREADS), 0, stream, chosen, weights, pairs, top, experts, pad, capacity, slot_of, slot_token, slot_weight,
+                                 tile_expert, tile_rows);
 }
 
 HB_EXPORT int hb_moe_gather(const void* x, int is_bf16, int x_stride, const int* slot_token, const float* slot_weight, void* out, int capacity,
