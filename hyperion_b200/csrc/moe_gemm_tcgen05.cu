@@ -11,10 +11,14 @@
 //   warps 2-5 drain a finished accumulator while the next tile's products run.  All three roles read the tile list (written by
 //   the plan kernel just before) and skip the same tiles, so their counters stay in step.  Every wait is bounded; when one runs
 //   out the status word says so, all roles leave their loops, tensor memory is freed and the block returns.
+// * The pair kernel (steps that bring an expert more than a tile of rows on average) is the shape of csrc/gemm_pair_tcgen05.cu: two SMs on two neighbouring
+//   row tiles of one expert, each keeping its own rows and half of the weight tile, so that a weight tile is fetched once for 256 rows and a block moves 32 KB
+//   per 64-deep step where the tile kernel moves 48.  Every block lists the pairs of tiles from the plan's tile list; a run's odd last tile has a pair of its own, whose
+//   second half is not stored.
 // * The rows kernel (steps of a few tokens) streams each used expert's matrix once: a block takes the real rows of one
 //   tile (tile_rows[i] of them, eight at a time) into shared memory and its warps walk output columns two at a time, every lane reading
 //   16 bytes of both matrix rows per step.  Such a step is bound by the bytes of the matrices it touches, not by arithmetic.
-#include "gemm_tcgen05.cuh"
+#include "gemm_pair_tcgen05.cuh"
 
 namespace {
 template <int BN>
@@ -180,6 +184,210 @@ int launch_grouped(const CUtensorMap& map_x, const CUtensorMap& map_w, const Gro
         configured = true;
     }
     return launch_after_previous(gemm_grouped_kernel<BN>, dim3(blocks), THREADS, GroupedLayout<BN>::SMEM, stream, map_x, map_w, p, tiles_m, tiles_n);
+}
+
+// ---------------------------------------------------------------- two row tiles of an expert on two SMs
+constexpr int GP_STAGES = 6, GP_MOST_TILES = 4096;
+constexpr unsigned GP_STAGE_BYTES = 32 * 1024;
+__host__ __device__ constexpr size_t grouped_pair_smem(int tiles_m) { return 1024 + (size_t)GP_STAGES * GP_STAGE_BYTES + 256 + ((size_t)tiles_m * 2 + 15) / 16 * 16; }
+
+// The first tiles of the pairs, in ascending order: bit 15 says that the next tile belongs to the pair too.  One warp; returns how many.
+__device__ __forceinline__ int list_pairs(const int* __restrict__ tile_expert, int tiles_m, unsigned short* list) {
+    const int lane = threadIdx.x & 31;
+    int count = 0, run_start = 0, before = -1;
+    for (int base = 0; base < tiles_m; base += 32) {
+        const int i = base + lane, e = i < tiles_m ? tile_expert[i] : -1, next = i + 1 < tiles_m ? tile_expert[i + 1] : -1;
+        int previous = __shfl_up_sync(0xffffffffu, e, 1);
+        if (lane == 0) previous = before;
+        const unsigned starts = __ballot_sync(0xffffffffu, e >= 0 && e != previous), upto = starts & (0xffffffffu >> (31 - lane));
+        const int start = upto ? base + 31 - __clz(upto) : run_start;
+        const bool begins = e >= 0 && ((i - start) & 1) == 0;
+        const unsigned all = __ballot_sync(0xffffffffu, begins);
+        if (begins) list[count + __popc(all & ((1u << lane) - 1))] = (unsigned short)(i | (next == e ? 0x8000 : 0));
+        count += __popc(all);
+        if (starts) run_start = base + 31 - __clz(starts);
+        before = __shfl_sync(0xffffffffu, e, 31);
+    }
+    return count;
+}
+
+// 32 columns of one row from column c of the tile on; SwiGLU: columns c of the tile's first half (gate) and of its second (up).
+__device__ __forceinline__ void store_grouped_pair_row(const GroupedParams& p, unsigned lane_addr, int r, int tile_n, int begin, int end) {
+    const bool glu = p.act == HB_ACT_SWIGLU;
+    const int width = glu ? p.n / 2 : p.n, out0 = tile_n * (glu ? 128 : 256);
+#pragma unroll 1
+    for (int c = begin; c < end; c += 32) {
+        const int col = out0 + c;
+        if (col >= width) break;
+        float v[32];
+        tmem_ld32(lane_addr + c, v);
+        if (glu) {
+            float u[32];
+            tmem_ld32(lane_addr + 128 + c, u);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = v[j] / (1.0f + expf(-v[j])) * u[j];
+        } else if (p.act != HB_ACT_NONE) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = activated(v[j], p.act);
+        }
+        bf16* dst = p.c + (size_t)r * p.ldc + col;
+        if (col + 32 <= width && (p.ldc & 7) == 0) {
+            uint4 w[4];
+            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(w);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) reinterpret_cast<uint4*>(dst)[j] = w[j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                if (col + j < width) dst[j] = __float2bfloat16_rn(v[j]);
+        }
+    }
+}
+
+// Bound by the matrices where an expert has about a pair of tiles (16 of [2,048, 2,048], 3,640 rows: 58.7 us on single SMs, 39.1 on pairs; their bytes
+// alone take 21), by the products beyond.  The activation is the epilogue's, under the next tile's products.
+__global__ void __launch_bounds__(PAIR_THREADS) gemm_grouped_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                                                                         const GroupedParams p, int tiles_m, int tiles_n) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(tiles + (size_t)GP_STAGES * GP_STAGE_BYTES);  // used in the leader only
+    unsigned long long* empty = full + GP_STAGES;
+    unsigned long long* acc_full = empty + GP_STAGES;  // [2]
+    unsigned long long* acc_empty = acc_full + 2;      // [2], used in the leader only: 16 warps arrive, 8 of each block
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(acc_empty + 2);
+    volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* listed = reinterpret_cast<int*>(tmem_slot + 2);
+    unsigned short* list = reinterpret_cast<unsigned short*>(tiles + (size_t)GP_STAGES * GP_STAGE_BYTES + 256);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned rank = cluster_rank();
+    const bool leader = rank == 0;
+    const int me = blockIdx.x >> 1, all = gridDim.x >> 1;
+    const int k_blocks = (p.k + BK - 1) / BK;
+    let_next_kernel_start();
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < GP_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
+        *failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    wait_for_previous_kernels();  // the tile list and the rows come from the kernels before
+    if (warp == 0) {
+        const int count = list_pairs(p.tile_expert, tiles_m, list);
+        if (lane == 0) *listed = count;
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();  // both blocks' barriers exist before either signals the other's
+    tc_fence_after();
+    const unsigned tmem = *tmem_slot;
+    const int n_pairs = *listed, total = n_pairs * tiles_n;
+
+    if (warp == 0) {
+        if (lane == 0) {  // producer
+            const unsigned full0 = in_leader(&full[0]);
+            int s = 0;
+            unsigned turn = 0;
+            bool ok = true;
+            for (int t = me; t < total && ok; t += all) {
+                const int first = list[t % n_pairs] & 0x7fff, row0 = (first + (int)rank) * BM;
+                const int w_row0 = p.tile_expert[first] * p.n + (t / n_pairs) * 256 + (int)rank * 128;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_ready(smem_u32(&empty[s]), turn ^ 1u) && !mbar_wait(&empty[s], turn ^ 1u, failed)) { *failed = 1; ok = false; break; }
+                    unsigned char* a_tile = tiles + (size_t)s * GP_STAGE_BYTES;
+                    const unsigned bar = full0 + 8u * (unsigned)s;
+                    if (leader) mbar_expect_tx(&full[s], 2u * GP_STAGE_BYTES);
+                    tma_load_2d_pair(a_tile, &map_x, bar, kb * BK, row0);
+                    tma_load_2d_pair(a_tile + A_BYTES, &map_w, bar, kb * BK, w_row0);
+                    if (++s == GP_STAGES) { s = 0; turn ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && leader) {  // tensor-core issuer of the pair
+            const unsigned idesc = pair_idesc(256);
+            const unsigned a_low0 = desc_low(tiles), b_low0 = desc_low(tiles + A_BYTES), step = GP_STAGE_BYTES >> 4;
+            const unsigned full0 = smem_u32(&full[0]), empty0 = smem_u32(&empty[0]);
+            int s = 0;
+            unsigned turn = 0, a_low = a_low0, b_low = b_low0;
+            bool ok = true;
+            for (int t = me, i = 0; t < total && ok; t += all, ++i) {
+                const int buf = i & 1;
+                if (!mbar_wait(&acc_empty[buf], ((i >> 1) & 1) ^ 1, failed)) { *failed = 1; ok = false; break; }  // both epilogues have drained it
+                tc_fence_after();
+                const unsigned acc = tmem + buf * ACC_STRIDE;
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_ready(full0 + 8u * (unsigned)s, turn) && !mbar_wait(&full[s], turn, failed)) { *failed = 1; ok = false; break; }
+                    umma_pair_stage(acc, a_low, b_low, idesc, kb > 0 ? 1u : 0u);
+                    umma_commit_both_at(empty0 + 8u * (unsigned)s);  // the stage is free in both blocks once these products have read it
+                    a_low += step;
+                    b_low += step;
+                    if (++s == GP_STAGES) { s = 0; turn ^= 1u; a_low = a_low0; b_low = b_low0; }
+                }
+                if (ok) umma_commit_both(&acc_full[buf]);
+            }
+        }
+    } else {  // epilogue: warps 2..9; warp w reads lane quarter w % 4 and the half (w - 2) / 4 of this block's columns
+        const int quarter = warp & 3, half = (warp - 2) >> 2, cols = p.act == HB_ACT_SWIGLU ? 128 : 256;
+        bool ok = true;
+        for (int t = me, i = 0; t < total && ok; t += all, ++i) {
+            const int buf = i & 1;
+            if (!mbar_wait(&acc_full[buf], (i >> 1) & 1, failed)) { *failed = 1; ok = false; break; }
+            tc_fence_after();
+            const int entry = list[t % n_pairs];
+            if (leader || (entry & 0x8000))  // a lone tile has no second half
+                store_grouped_pair_row(p, tmem + buf * ACC_STRIDE + ((unsigned)(quarter * 32) << 16), ((entry & 0x7fff) + (int)rank) * BM + quarter * 32 + lane, t / n_pairs,
+                                       half * cols / 2, (half + 1) * cols / 2);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_in_leader(in_leader(&acc_empty[buf]));  // this warp's share of the accumulator may be written again
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x == 0 && *failed) atomicOr(p.status, HB_STATUS_WAIT_EXPIRED | HB_STATUS_IN_GEMM_TILES);
+    cluster_sync();  // neither block leaves while the other may still read its shared memory or signal its barriers
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+cudaLaunchConfig_t grouped_pair_config(int pairs, int tiles_m, cudaStream_t stream, cudaLaunchAttribute (&attributes)[2]) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(2 * pairs);
+    config.blockDim = dim3(PAIR_THREADS);
+    config.dynamicSmemBytes = grouped_pair_smem(tiles_m);
+    config.stream = stream;
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = 2;
+    attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
+    config.attrs = attributes;
+    config.numAttrs = 2;
+    return config;
+}
+
+// How many pairs of blocks the device runs at a time (a pair needs two SMs of one processing cluster); the kernel is allowed its most shared memory once.
+int resident_grouped_pairs() {
+    static const int pairs = [] {
+        if (cudaFuncSetAttribute(gemm_grouped_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)grouped_pair_smem(GP_MOST_TILES)) != cudaSuccess) return -1;
+        cudaLaunchAttribute attributes[2];
+        cudaLaunchConfig_t config = grouped_pair_config(sm_count(), GP_MOST_TILES, nullptr, attributes);
+        config.numAttrs = 1;
+        int clusters = 0;
+        return cudaOccupancyMaxActiveClusters(&clusters, gemm_grouped_pair_kernel, &config) == cudaSuccess && clusters > 0 ? clusters : sm_count() / 2;
+    }();
+    return pairs;
 }
 
 // ---------------------------------------------------------------- a few rows per expert: the matrices stream once
@@ -410,6 +618,26 @@ HB_EXPORT int hb_moe_gemm_tiles(const void* a, const void* w, void* c, const int
     const GroupedParams p{(bf16*)c, tile_expert, rows, n, k, n, act, status};
     return bn == 256 ? launch_grouped<256>(map_x, map_w, p, tiles_m, tiles_n, blocks, stream)
                      : launch_grouped<128>(map_x, map_w, p, tiles_m, tiles_n, blocks, stream);
+}
+
+// The same product on pairs of SMs; act HB_ACT_SWIGLU: every 256 rows of an expert's matrix are 128 gate rows followed by their 128 up rows (n a multiple of 256),
+// c [rows, n / 2].
+HB_EXPORT int hb_moe_gemm_pairs(const void* a, const void* w, void* c, const int* tile_expert, int rows, int experts, int n, int k, int act, int* status,
+                                cudaStream_t stream) {
+    if (rows <= 0 || n <= 0) return 0;
+    if (k <= 0 || rows % BM || experts <= 0 || (k % 8) || !tile_expert || act < HB_ACT_NONE || act > HB_ACT_SWIGLU) return HB_BAD_ARGUMENT;
+    if ((long long)experts * n > 0x7fffffffLL || rows / BM > GP_MOST_TILES || (act == HB_ACT_SWIGLU && n % 256)) return HB_UNSUPPORTED_SIZE;
+    CUtensorMap map_x, map_w;
+    if (int code = make_map(&map_x, a, rows, k, k, BM)) return code;
+    if (int code = make_map(&map_w, w, experts * n, k, k, 128)) return code;
+    const int tiles_m = rows / BM, tiles_n = (n + 255) / 256, resident = resident_grouped_pairs();
+    if (resident < 1) return HB_UNSUPPORTED_SIZE;
+    if ((long long)tiles_m * tiles_n > 0x7fffffffLL) return HB_UNSUPPORTED_SIZE;
+    const GroupedParams p{(bf16*)c, tile_expert, rows, n, k, act == HB_ACT_SWIGLU ? n / 2 : n, act, status};
+    cudaLaunchAttribute attributes[2];
+    const int pairs = tiles_m * tiles_n < resident ? tiles_m * tiles_n : resident;
+    const cudaLaunchConfig_t config = grouped_pair_config(pairs, tiles_m, stream, attributes);
+    return (int)cudaLaunchKernelEx(&config, gemm_grouped_pair_kernel, map_x, map_w, p, tiles_m, tiles_n);
 }
 
 // The same product for steps of a few rows; tile_rows[i]: the real rows at the start of tile i.  row_token (or null): the row of `a` that stands in

@@ -8,7 +8,8 @@ from dataclasses import dataclass
 
 import torch
 
-from .basic import status_word
+from . import gemm
+from .basic import status_word, swiglu
 from .native import KernelError, check, f32, i32, is_bf16, library, ptr, require_cuda, stream_ptr
 
 PAD = 128  # an expert's rows are padded to whole tiles of this many rows
@@ -133,6 +134,10 @@ def takes_tensor_cores(a: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 ACTIVATIONS = {None: 0, "relu_squared": 1}  # what a grouped product can apply to its result before the one rounding
+GELUS = {"gelu_erf": 2, "gelu_tanh": 3}  # the same, by way of :func:`grouped_gelu`
+SWIGLU = 4  # by way of :func:`grouped_swiglu`
+PAIR_ROWS = 128  # (token, choice) pairs per expert from which on two SMs share two row tiles of an expert
+PAIR_MOST_TILES = 4096  # of rows: what the kernel lists in shared memory
 
 
 def grouped_linear(a: torch.Tensor, w: torch.Tensor, where: Plan, activation: str | None = None) -> torch.Tensor:
@@ -141,14 +146,22 @@ def grouped_linear(a: torch.Tensor, w: torch.Tensor, where: Plan, activation: st
     of which every slot takes its token's."""
     if activation not in ACTIVATIONS:
         raise KernelError(f"moe.grouped_linear: no activation {activation!r} (known: {sorted(k for k in ACTIVATIONS if k)})")
-    act = i32(ACTIVATIONS[activation])
+    return _grouped(a, w, where, ACTIVATIONS[activation])
+
+
+def _grouped(a: torch.Tensor, w: torch.Tensor, where: Plan, code: int) -> torch.Tensor:
+    act = i32(code)
     require_cuda(a, w)
     ungathered = where.streams and a.shape[0] != where.capacity
     if a.dtype != w.dtype or not a.is_contiguous() or not w.is_contiguous() or w.dim() != 3 or w.shape[2] != a.shape[1] or (a.shape[0] != where.capacity and not ungathered):
         raise KernelError("moe.grouped_linear: dense operands of one element type, rows [capacity, k] and matrices [experts, n, k]")
-    out = torch.empty((where.capacity, w.shape[1]), dtype=a.dtype, device=a.device)
+    out = torch.empty((where.capacity, w.shape[1] // 2 if code == SWIGLU else w.shape[1]), dtype=a.dtype, device=a.device)
     if takes_tensor_cores(a, w):
         lib = library("moe_gemm_tcgen05")
+        if takes_pairs(w, where):
+            check(lib.hb_moe_gemm_pairs(ptr(a), ptr(w), ptr(out), ptr(where.tile_expert), i32(where.capacity), i32(w.shape[0]), i32(w.shape[1]), i32(w.shape[2]), act,
+                                        ptr(status_word(a.device)), stream_ptr()), "moe_gemm_pairs")
+            return out
         if where.pairs <= FEW_PAIRS:
             # From two rows per expert on (if the choices spread) the tensor cores' kernel: at one, its blocks of 128 columns leave a short last wave (11 matrices of
             # [3584, 4096]: 67 us, 54 with the other); at two it takes 75 us where the other takes 82 ([4096, 3584], 14 of them).  Its sums of sixteen are cut off, not rounded,
@@ -167,6 +180,26 @@ def grouped_linear(a: torch.Tensor, w: torch.Tensor, where: Plan, activation: st
     check(library("moe").hb_moe_gemm(ptr(a), ptr(w), ptr(out), i32(is_bf16(a)), ptr(where.tile_expert), i32(where.pad), i32(where.capacity), i32(w.shape[1]),
                                      i32(w.shape[2]), act, stream_ptr()), "moe_gemm")
     return out
+
+
+def takes_pairs(w: torch.Tensor, where: Plan) -> bool:
+    """Whether a product that takes the tensor cores goes to pairs of SMs: from a row tile per expert on (if the choices spread; 228
+    rows an expert: 39 us on pairs, 59 on single SMs).  Below that the second half of most pairs would be empty, and a pair's ring shares one weight tile between two SMs."""
+    return (where.pairs > FEW_PAIRS and where.pairs >= PAIR_ROWS * w.shape[0] and where.capacity <= PAIR_MOST_TILES * PAD
+            and (w.shape[1] % 256 == 0 or w.shape[1] >= 1024))
+
+
+def grouped_gelu(a: torch.Tensor, w: torch.Tensor, where: Plan, activation: str) -> torch.Tensor:
+    """``activation`` (a key of ``GELUS``) of :func:`grouped_linear`, applied to the product's float result: one rounding, and no pass over the padding."""
+    return _grouped(a, w, where, GELUS[activation])
+
+
+def grouped_swiglu(a: torch.Tensor, w: torch.Tensor, where: Plan, block: int | None) -> torch.Tensor:
+    """silu(gate) * up of a grouped product with matrices [experts, 2I, k] whose rows alternate in runs of ``block`` gate rows and their up rows (None: all gate rows
+    first): in the epilogue where pairs of SMs take the product and ``block`` is 128, else by a kernel behind it."""
+    if block == gemm.SWIGLU_BLOCK and takes_tensor_cores(a, w) and takes_pairs(w, where):
+        return _grouped(a, w, where, SWIGLU)
+    return swiglu(grouped_linear(a, w, where), block=block)
 
 
 def combine(y: torch.Tensor, where: Plan, base: torch.Tensor | None, tokens: int) -> torch.Tensor:

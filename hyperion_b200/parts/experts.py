@@ -35,7 +35,7 @@ from typing import Mapping
 import torch
 
 from .. import ops
-from ..ops import moe
+from ..ops import gemm, moe
 from .base import FEED_FORWARDS, BuildContext, FeedForward, WeightSpec, make, register_feed_forward
 from .spec import PartSpec
 
@@ -67,8 +67,11 @@ class RoutedExperts(FeedForward):
 
     def load(self, tensors: Mapping[str, torch.Tensor]) -> None:
         self.router = tensors["router"].to(torch.float32).contiguous()
-        # per expert [gate rows | up rows], all experts stacked: [experts, 2 * inter, hidden]; down: [experts, hidden, inter]
-        self.w_gate_up = torch.stack([torch.cat([tensors[f"e{e}.gate"], tensors[f"e{e}.up"]], dim=0) for e in range(self.experts)]).contiguous()
+        # per expert gate and up rows, in runs of 128 in turn where a product can apply SwiGLU to them (else the gate rows first), all experts stacked:
+        # [experts, 2 * inter, hidden]; down: [experts, hidden, inter]
+        pairs = [(tensors[f"e{e}.gate"], tensors[f"e{e}.up"]) for e in range(self.experts)]
+        self.block = gemm.SWIGLU_BLOCK if pairs[0][0].dtype == torch.bfloat16 and self.inter % gemm.SWIGLU_BLOCK == 0 else None
+        self.w_gate_up = torch.stack([torch.cat(pair, dim=0) if self.block is None else gemm.interleave_gate_up(*pair) for pair in pairs]).contiguous()
         self.w_down = torch.stack([tensors[f"e{e}.down"] for e in range(self.experts)]).contiguous()
         if self.shared is not None:
             self.shared.load({name: tensors["shared." + name] for name in self.shared.weights()})
@@ -83,7 +86,7 @@ class RoutedExperts(FeedForward):
         chosen, weights = moe.route(x, self.router, self.top)
         where = moe.plan(chosen, weights, self.experts)
         rows = moe.gather(x, where)
-        act = ops.swiglu(moe.grouped_linear(rows, self.w_gate_up, where))
+        act = moe.grouped_swiglu(rows, self.w_gate_up, where, self.block)
         y = moe.grouped_linear(act, self.w_down, where)
         base = None
         if self.shared is not None:
@@ -145,7 +148,7 @@ class ScoredExperts(FeedForward):
         chosen, weights = moe.route_scored(x, self.router, self.correction, self.top, self.group_count, self.group_keep, self.scale)
         where = moe.plan(chosen, None, self.experts)  # the weights multiply what an expert returns, so the rows are gathered as they are
         rows = moe.gather(x, where)
-        act = getattr(ops, self.activation)(moe.grouped_linear(rows, self.w_up, where))
+        act = moe.grouped_gelu(rows, self.w_up, where, self.activation)
         y = moe.grouped_linear(act, self.w_down, where)
         base = gate = None
         if self.shared is not None:
