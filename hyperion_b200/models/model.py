@@ -98,6 +98,8 @@ class DecoderModel:
         modules: list[tuple[str, dict]] = []
         for _, part in self._named_parts():
             modules += part.kernel_modules()
+        if ("gemm_tcgen05", {}) in modules:  # products of a few rows with small matrices
+            modules.append(("few_rows", {}))
         return modules
 
     def step_planners(self) -> dict:

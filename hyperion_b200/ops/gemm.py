@@ -54,6 +54,51 @@ def choose_splits(n: int, k: int, m: int = 64, sms: Optional[int] = None) -> int
     return max(1, min(target // tiles if tiles < target else 1, k_blocks // 4, 16))
 
 
+FEW_ROWS = 16  # rows up to which csrc/few_rows.cu takes a product
+FEW_BF16, FEW_F32, FEW_SWIGLU, FEW_PIECES = 0, 1, 2, 3
+
+
+def takes_few_rows(x: torch.Tensor, w: torch.Tensor, gated_block: Optional[int] = None) -> bool:
+    """Whether a product of a few rows goes to ``csrc/few_rows.cu``: whole tiles of 16 rows of the matrix and of 64 of k, and a matrix small enough that the step is its waits, not
+    its bytes.  Measured in chains of such products, one to eight rows: [896, 896] 4.1 -> 2.2 us, [2,048, 2,048] 3.7 -> 2.8, [4,096, 2,048] 5.9 -> 4.8, [9,728, 896] with SwiGLU
+    8.1 -> 5.0, [16,384, 2,048] with SwiGLU 15.7 -> 14.3; beyond 20 MB only where k is short (a tile's sum over long k keeps few blocks busy: [4,096, 4,096] 6.9 -> 8.0),
+    and not from some 70 MB on ([32,000, 2,048] 21.5 -> 24.6).  Nine to sixteen rows ask for twice the rows per unit: [2,048, 2,048] 3.9 -> 3.4, [4,096, 2,048] 6.1 -> 6.4,
+    [9,728, 896] 8.9 -> 7.0.  ``gated_block``: with SwiGLU in the epilogue, over runs of that many gate rows."""
+    m, (n, k) = x.shape[0], w.shape
+    if m > FEW_ROWS or not supported(x, w) or not w.is_contiguous() or k % 64 or n % 16:
+        return False
+    if gated_block is not None and (n % 32 or gated_block < 8 or (n // 2) % gated_block or (gated_block != n // 2 and gated_block & (gated_block - 1))):
+        return False
+    megabytes = n * k / 2**19
+    if m <= 8:
+        return megabytes <= 20 or (k <= 2048 and megabytes <= 68)
+    return megabytes <= 13 or (k < 2048 and megabytes <= 20)
+
+
+def few_rows(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, epilogue: int = FEW_BF16, block: int = 0):
+    """``x w^T`` (+ bias) for up to 16 rows (``csrc/few_rows.cu``); :data:`FEW_SWIGLU` over gate and up rows in turn in runs of ``block``; :data:`FEW_PIECES`: a
+    :class:`SplitSum`, its bias still to be added, or the whole sum where one block per tile is enough."""
+    require_cuda(x, w, bias)
+    m, k = x.shape
+    n = w.shape[0]
+    sms = sm_count(x.device)
+    parts = 1
+    if epilogue == FEW_PIECES:  # as many parts of k as there is room for two blocks to an SM, four units to a warp at the least
+        parts = max(1, min(2 * sms // (n // 16), k // (64 * 8 * 2), 4))
+        if parts == 1:
+            epilogue = FEW_BF16
+    if epilogue == FEW_PIECES:
+        out = torch.empty((parts, m, n), dtype=torch.float32, device=x.device)
+    else:
+        out = torch.empty((m, n // 2 if epilogue == FEW_SWIGLU else n), dtype=torch.float32 if epilogue == FEW_F32 else torch.bfloat16, device=x.device)
+    given = None if epilogue == FEW_PIECES else bias
+    bias_f = given if given is not None and given.dtype == torch.float32 else None
+    bias_h = given if given is not None and given.dtype == torch.bfloat16 else None
+    check(library("few_rows").hb_few_rows(ptr(x), i32(x.stride(0)), ptr(w), ptr(bias_h), ptr(bias_f), ptr(out), i32(out.stride(-2)), i32(m), i32(n), i32(k), i32(epilogue),
+                                          i32(block), i32(parts), i32(2 * sms), stream_ptr()), "few_rows")
+    return SplitSum(out, bias, torch.bfloat16) if epilogue == FEW_PIECES else out
+
+
 @dataclass
 class SplitSum:
     """A product whose split-K partial sums have not been added up yet: ``partials`` [splits, M, N] float32, to be

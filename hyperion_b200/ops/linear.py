@@ -57,6 +57,12 @@ def _takes_own_kernel(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) ->
     return k >= 2048 and m <= 64
 
 
+def _takes_few_rows(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) -> bool:
+    """Whether a bfloat16 product goes to the kernel for a few rows and a small matrix (``HYPERION_B200_GEMM`` = ``auto`` only)."""
+    return (x.shape[0] <= gemm.FEW_ROWS and gemm_policy() == "auto" and out_dtype in (torch.bfloat16, torch.float32)
+            and (bias is None or (bias.dtype in (torch.bfloat16, torch.float32) and bias.is_contiguous())) and gemm.takes_few_rows(x, weight))
+
+
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
            out_dtype: Optional[torch.dtype] = None, may_leave_partials: bool = False):
     """``may_leave_partials``: the caller's result has one reader that can add up split-K pieces itself (a residual delta, a gate that
@@ -71,6 +77,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if weight.dtype != torch.bfloat16:
         raise KernelError(f"linear: weights are float32 or bfloat16, got {weight.dtype}")
     xin = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
+    if _takes_few_rows(xin, weight, bias, out_dtype):
+        return gemm.few_rows(xin, weight, bias, gemm.FEW_F32 if out_dtype == torch.float32 else gemm.FEW_PIECES if may_leave_partials else gemm.FEW_BF16)
     if _takes_own_kernel(xin, weight, bias, out_dtype):
         epilogue = gemm.EPI_F32 if out_dtype == torch.float32 else gemm.EPI_BF16
         if xin.shape[0] > gemm.PAIR_MIN_ROWS:  # only under HYPERION_B200_GEMM=own: prompt-sized products on pairs of SMs
@@ -109,6 +117,9 @@ def gated_linear(x: torch.Tensor, weight: torch.Tensor, block: Optional[int], ou
     if (block == gemm.SWIGLU_BLOCK and weight.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and x.dtype == torch.bfloat16
             and gemm.supported(x, weight) and fuses_swiglu(x.shape[0], x.shape[1])):
         return gemm.gemm_pair_bf16(x, weight, None, gemm.EPI_SWIGLU)
+    if (x.shape[0] <= gemm.FEW_ROWS and weight.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and x.dtype == torch.bfloat16 and gemm_policy() == "auto"
+            and gemm.takes_few_rows(x, weight, block or weight.shape[0] // 2)):
+        return gemm.few_rows(x, weight, None, gemm.FEW_SWIGLU, block or weight.shape[0] // 2)
     return swiglu(linear(x, weight, None, out_dtype), block=block)
 
 
