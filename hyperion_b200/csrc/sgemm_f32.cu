@@ -7,8 +7,8 @@
 // A thread owns TM x TN outputs, BM / TM and BN / TN apart, and reads four k of each of its rows and columns at a time from shared memory in 16-byte pieces; slices of BK k
 // are copied ahead into a ring of STAGES, as they lie in memory. Bound by issue slots (70 % of an active SM's cycles issue, 60 % of them FFMA) and the last wave where a product has tiles enough,
 // else by the waits of a chain; the FFMA pipes would allow 74 TFLOP/s.
-// Two shapes: 64 x 128 with 8 x 8 outputs a thread for products that fill the GPU with such tiles; 32 x 32 with 4 x 4 for the others, which spreads a narrow product over
-// all SMs. Measured on one B200 (before: one shape of 64 x 64 with 4 x 4 outputs a thread, copied when needed): 394 rows, K 896, 9,728 columns 340 -> 229 to 246 us, K 4,864, 896 columns
+// Two shapes: 64 x 128 with 8 x 8 outputs a thread for products that fill the GPU with such tiles; 32 x 32 with 4 x 4 (4 x 2 where the tiles are few) for the others, which spreads a narrow
+// product over all SMs.  (Two multiply-adds to an instruction, fma.rn.f32x2, take as long as two: 58 TFLOP/s from registers against 64.) Measured on one B200 (before: one shape of 64 x 64 with 4 x 4 outputs a thread, copied when needed): 394 rows, K 896, 9,728 columns 340 -> 229 to 246 us, K 4,864, 896 columns
 // 302 -> 161 to 166 us; 3 rows, 151,936 columns 625 -> 244 us; 1 row, K 4,864 265 -> 101 us; 2,048 rows, 9,728 columns 1,393 -> 819 us (44 TFLOP/s).
 #include "common.cuh"
 
@@ -126,5 +126,9 @@ HB_EXPORT int hb_sgemm_f32(const float* a, const float* w, const float* bias, fl
     // 1,001: 88 large tiles 90 us, small ones 82; 128: 92 and 124; 288: 155 and 236)
     const long long large = (long long)((m + 63) / 64) * ((n + 127) / 128);
     if (m > 32 && large >= (aligned(a, w, k, lda) ? 2LL * sms : 3LL * sms / 4)) return launch_tiles<64, 128, 8, 8, 16, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
+    // Up to three small tiles to an SM a product is the chains of a few warps: twice as many warps, half as many outputs each, and slices of 64 k between barriers (394 rows, K 4,864, 896
+    // columns: 163 -> 138 us; K 896: 35 -> 30; 1 row, K 4,864: 100 -> 63).  With more tiles the loads per output count (3 rows, 151,936 columns: 244 and 278).
+    const long long small = (long long)((m + 31) / 32) * ((n + 31) / 32);
+    if (small <= 3LL * sms) return launch_tiles<32, 32, 4, 2, 64, 3>(a, w, bias, c, m, n, k, lda, ldc, stream);
     return launch_tiles<32, 32, 4, 4, 32, 4>(a, w, bias, c, m, n, k, lda, ldc, stream);
 }

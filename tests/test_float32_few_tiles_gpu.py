@@ -1,0 +1,23 @@
+"""The float32 product where small tiles are few and where they are many: the same bits, and against 64 bits at the edges of a slice of 64 k."""
+import pytest
+import torch
+
+from hyperion_b200 import ops
+from hyperion_b200.ops import basic
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 40, 63), (33, 64, 64), (31, 97, 65), (64, 200, 191), (5, 896, 4864)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_few_tiles(m, n, k, aligned, monkeypatch):
+    """A sum of k products in float, one after another: k rounding errors of at most 2^-24 of the largest partial sum."""
+    g = torch.Generator().manual_seed(m + n + k)
+    pad = 4 - k % 4 if aligned else 1
+    x, w = torch.randn(m, k + pad, generator=g).cuda()[:, :k], torch.randn(n, k, generator=g).cuda()
+    results = []
+    for sms in (148, 1):  # few tiles to an SM, and more than three
+        monkeypatch.setattr(basic, "sm_count", lambda device, sms=sms: sms)
+        results.append(ops.sgemm_f32(x, w))
+    assert torch.equal(*results)
+    assert ((results[0].double() - x.double() @ w.double().t()).abs() <= (k + 1) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().t())).all()
