@@ -26,6 +26,9 @@
 // columns of a key tile and S_L the last, and at an item's end the two softmax threads of a row, whose tensor-memory lanes are the same, take
 // half of the row's columns each:  o = a1 - lambda a2, o / sqrt(mean(o^2) + eps) * post * sigmoid(gate), exchanging what they need of one
 // another (1 / sum, the sum of squares) through shared memory.
+// Queries and keys may be wider than values (HB_KEY_DIM 192 over values of 128: attention over latents whose prompts' keys and values have been made per head); the
+// cache's rows are then as wide as a key and a value is its row's first entries.  1,531 tokens of 16 such heads: 51 us, 165 on mma.sync (attention_tma.cu), 225 over
+// the latents themselves (attention_latent.cu), which takes 3.4 times the operations.
 // Every mbarrier wait is bounded; a wait that runs out sets HB_STATUS_WAIT_EXPIRED, all roles leave their loops, the block
 // takes no further item, tensor memory is freed and the block returns.
 //
@@ -38,19 +41,24 @@
 #ifndef HB_HEAD_DIM
 #define HB_HEAD_DIM 128
 #endif
+#ifndef HB_KEY_DIM
+#define HB_KEY_DIM HB_HEAD_DIM
+#endif
 
 namespace {
 typedef __nv_bfloat16 bf16;
-constexpr int D = HB_HEAD_DIM;
+constexpr int D = HB_HEAD_DIM, DK = HB_KEY_DIM;  // entries of a value and of a result; of a query, of a key, and of a row of the cache (a value is its first D entries)
 static_assert(D == 64 || D == 128, "the tcgen05 attention takes head sizes 64 and 128");
+static_assert(DK == D || DK == 192, "queries and keys as wide as values, or 192 entries");
 constexpr int BM = 128;                       // rows of one half = tensor-memory lanes
 constexpr int ROWS = 2 * BM;                  // virtual rows of a tile
 constexpr int BN = 128;                       // keys per tile
-constexpr int PANELS = D / 64;
+constexpr int PANELS = D / 64, KEY_PANELS = DK / 64;
 constexpr int KV_PANEL = BN * 64;             // elements of a 128-key x 64-column panel (16 KB)
 constexpr int Q_PANEL = ROWS * 64;            // elements of a 256-row x 64-column panel of Q (32 KB)
-constexpr int TILE_BYTES = PANELS * KV_PANEL * 2;  // one K or one V tile
+constexpr int TILE_BYTES = PANELS * KV_PANEL * 2, KEY_TILE_BYTES = KEY_PANELS * KV_PANEL * 2;  // one V tile, one K tile
 constexpr int STAGES = 2;                     // K tiles and V tiles have rings of their own: a K slot is free as soon as both S are done
+constexpr int V_STAGES = DK > 128 ? 1 : STAGES;  // queries and keys of 192 entries leave room for one V tile: the next one comes under the next softmax
 constexpr int THREADS = 320;
 constexpr int TMEM_COLS = 512;                // S_H [0,128) S_L [128,256) O_H [256,256+D) O_L [384,384+D); P_x over S_x's first 64 columns
 constexpr int O_COL = 256;
@@ -253,9 +261,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     let_next_kernel_start();
     unsigned char* k_ring = base;                                                   // STAGES K tiles
-    unsigned char* v_ring = base + (size_t)STAGES * TILE_BYTES;                     // STAGES V tiles
-    bf16* qs = reinterpret_cast<bf16*>(base + (size_t)2 * STAGES * TILE_BYTES);     // PANELS panels of 256 rows x 64
-    unsigned long long* k_full = reinterpret_cast<unsigned long long*>(qs + PANELS * Q_PANEL);
+    unsigned char* v_ring = base + (size_t)STAGES * KEY_TILE_BYTES;                 // V_STAGES V tiles
+    bf16* qs = reinterpret_cast<bf16*>(v_ring + (size_t)V_STAGES * TILE_BYTES);     // KEY_PANELS panels of 256 rows x 64
+    unsigned long long* k_full = reinterpret_cast<unsigned long long*>(qs + KEY_PANELS * Q_PANEL);
     unsigned long long* k_empty = k_full + STAGES;
     unsigned long long* v_full = k_empty + STAGES;
     unsigned long long* v_empty = v_full + STAGES;
@@ -309,7 +317,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
     // the stage held before: earlier keys and values, which are finite. The rings start as zeros so that this holds for
     // the first tiles too. The rows of Q that no copy writes (beyond tokens x heads of a tile) are never stored; they start
     // as zeros all the same.
-    for (int e = tid; e < (2 * STAGES * TILE_BYTES + PANELS * Q_PANEL * 2) / 16; e += THREADS) reinterpret_cast<uint4*>(base)[e] = make_uint4(0, 0, 0, 0);
+    for (int e = tid; e < (STAGES * KEY_TILE_BYTES + V_STAGES * TILE_BYTES + KEY_PANELS * Q_PANEL * 2) / 16; e += THREADS) reinterpret_cast<uint4*>(base)[e] = make_uint4(0, 0, 0, 0);
     // what the first item is needs nothing of the kernel before: the tiles and positions were copied in at the step's start
     if (tid == 0) note_item(0, (int)blockIdx.x);
     wait_for_previous_kernels();  // the queries and the newest keys and values come from the kernel before; so does the counter's reset
@@ -364,8 +372,6 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
     if (warp == 0) {
         // ------------------------------------------------------------------ producer (whole warp)
         const int pages_per_tile = BN >> shift;
-        const int ops = pages_per_tile * PANELS;
-        const unsigned page_bytes = (unsigned)a.page_size * D * 2u;  // of one page of K, or of V
         bool alive = true;
         int g0 = 0;
         for (int round = 0; alive; ++round) {
@@ -389,14 +395,14 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
             if (lane == 0) {
                 if (!mbar_wait(q_empty, (round & 1) ^ 1, failed) || !mbar_wait(q_seen, (round & 1) ^ 1, failed)) { *failed = 1; alive = false; }
                 if (alive) {
-                    mbar_expect_tx(q_full, (unsigned)(PANELS * 128 * gc * tokens_per_tile));
+                    mbar_expect_tx(q_full, (unsigned)(KEY_PANELS * 128 * gc * tokens_per_tile));
                     // (MAPS: the first map's 128 rows and below them the second's, in one panel)
-                    for (int h = 0; h < PANELS; ++h) tma_load_3d(qs + h * (MAPS ? BM * 64 : Q_PANEL), &q_map, q_full, h * 64, it.first_head, it.tok0);
+                    for (int h = 0; h < KEY_PANELS; ++h) tma_load_3d(qs + h * (MAPS ? BM * 64 : Q_PANEL), &q_map, q_full, h * 64, it.first_head, it.tok0);
                 }
             }
             alive = __shfl_sync(0xffffffffu, alive ? 1 : 0, 0) != 0;
             for (int t = 0; t < it.n_tiles && alive; ++t) {
-                const int g = g0 + t, s = g % STAGES, turn = g / STAGES;
+                const int g = g0 + t;
                 const int tile_base = key_tile_base(t, it.n_kept, it.start, BN);
                 int my_page = -1;
                 const int k0 = tile_base + lane * a.page_size;
@@ -408,6 +414,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
                 }
                 const unsigned valid = __popc(__ballot_sync(0xffffffffu, my_page >= 0));
                 for (int which = 0; which < 2 && alive; ++which) {  // the K tile, then the V tile
+                    const int stages = which ? V_STAGES : STAGES, s = g % stages, turn = g / stages, panels = which ? PANELS : KEY_PANELS, ops = pages_per_tile * panels;
+                    const unsigned page_bytes = (unsigned)a.page_size * (which ? D : DK) * 2u;
                     unsigned long long* full = which ? &v_full[s] : &k_full[s];
                     int ok = 1;
                     if (lane == 0) ok = mbar_wait(which ? &v_empty[s] : &k_empty[s], (turn & 1) ^ 1, failed) ? 1 : 0;
@@ -417,10 +425,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
                         if (valid) mbar_expect_tx(full, valid * page_bytes); else mbar_arrive(full);
                     }
                     __syncwarp();
-                    bf16* stage = reinterpret_cast<bf16*>((which ? v_ring : k_ring) + (size_t)s * TILE_BYTES);
+                    bf16* stage = reinterpret_cast<bf16*>(which ? v_ring + (size_t)s * TILE_BYTES : k_ring + (size_t)s * KEY_TILE_BYTES);
                     for (int op0 = 0; op0 < ops; op0 += 32) {
                         const int op = op0 + lane;
-                        const int p = min(op, ops - 1) / PANELS, h = op % PANELS;
+                        const int p = min(op, ops - 1) / panels, h = op % panels;
                         const int page = __shfl_sync(0xffffffffu, my_page, p);
                         if (op < ops && page >= 0)
                             tma_load_2d(stage + h * KV_PANEL + p * a.page_size * 64, &kv_map, full, h * 64,
@@ -440,13 +448,15 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
             const unsigned k_empty0 = smem_u32(&k_empty[0]), v_empty0 = smem_u32(&v_empty[0]), s_full0 = smem_u32(&s_full[0]), o_done0 = smem_u32(&o_done[0]);
             const unsigned q_empty_at = smem_u32(q_empty);
             auto issue_s = [&](int x, int g) {  // S_x = Q_x K(g)^T
-                const unsigned k_low = k_low0 + (unsigned)(g % STAGES) * (TILE_BYTES >> 4), q_low = q_low0 + (unsigned)x * (BM * 128 >> 4);
+                const unsigned k_low = k_low0 + (unsigned)(g % STAGES) * (KEY_TILE_BYTES >> 4), q_low = q_low0 + (unsigned)x * (BM * 128 >> 4);
                 umma_s_panel(tmem + x * BN, q_low, MAPS ? k_low + (unsigned)x * (KV_PANEL * 2 >> 4) : k_low, idesc_s, 0u);
-                if (PANELS == 2 && !MAPS) umma_s_panel(tmem + x * BN, q_low + (Q_PANEL * 2 >> 4), k_low + (KV_PANEL * 2 >> 4), idesc_s, 1u);
+                if (!MAPS)
+#pragma unroll
+                    for (int h = 1; h < KEY_PANELS; ++h) umma_s_panel(tmem + x * BN, q_low + h * (Q_PANEL * 2 >> 4), k_low + h * (KV_PANEL * 2 >> 4), idesc_s, 1u);
                 umma_commit_at(s_full0 + 8u * (unsigned)x);
             };
             auto issue_pv = [&](int x, int g, unsigned accumulate) {  // O_x (+)= P_x V(g); P_x lies over the first 64 columns of S_x
-                const unsigned v_low = v_low0 + (unsigned)(g % STAGES) * (TILE_BYTES >> 4);
+                const unsigned v_low = v_low0 + (unsigned)(g % V_STAGES) * (TILE_BYTES >> 4);
                 umma_pv_64(tmem + O_COL + x * BM, tmem + x * BN, v_low, idesc_o, accumulate);
                 umma_pv_64(tmem + O_COL + x * BM, tmem + x * BN + 32, v_low + 512, idesc_o, 1u);
                 umma_commit_at(o_done0 + 8u * (unsigned)x);
@@ -469,10 +479,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_tc_kernel(const __grid_c
                     const bool more = j + 1 < n_tiles;
                     for (int x = 0; x < halves && ok; ++x) {
                         if (!mbar_wait(&p_full[x], (h0[x] + j) & 1, failed)) { *failed = 1; ok = false; break; }
-                        if (x == 0 && !mbar_wait(&v_full[g % STAGES], (g / STAGES) & 1, failed)) { *failed = 1; ok = false; break; }
+                        if (x == 0 && !mbar_wait(&v_full[g % V_STAGES], (g / V_STAGES) & 1, failed)) { *failed = 1; ok = false; break; }
                         tc_fence_after();
                         issue_pv(x, g, j > 0 ? 1u : 0u);
-                        if (x == halves - 1) umma_commit_at(v_empty0 + 8u * (unsigned)(g % STAGES));
+                        if (x == halves - 1) umma_commit_at(v_empty0 + 8u * (unsigned)(g % V_STAGES));
                         if (more) {
                             if (x == 0) {
                                 if (!mbar_wait(&k_full[(g + 1) % STAGES], ((g + 1) / STAGES) & 1, failed)) { *failed = 1; ok = false; break; }
@@ -745,7 +755,9 @@ EncodeTiled encode_tiled() {
 }
 
 // More than half of an SM's shared memory, so that one block is all an SM takes: the block holds all of its tensor memory.
-constexpr size_t SMEM_USED = 1024 + (size_t)2 * STAGES * TILE_BYTES + (size_t)PANELS * Q_PANEL * sizeof(bf16) + (4 * STAGES + 12) * 8 + 96 + 4 * BM * sizeof(float);
+constexpr size_t SMEM_USED = 1024 + (size_t)STAGES * KEY_TILE_BYTES + (size_t)V_STAGES * TILE_BYTES + (size_t)KEY_PANELS * Q_PANEL * sizeof(bf16) + (4 * STAGES + 12) * 8 + 96 +
+                             (DK == D ? 4 * BM * sizeof(float) : 0);  // the last for two maps per head only
+static_assert(SMEM_USED <= 227 * 1024, "an SM's shared memory");
 constexpr size_t SMEM_BYTES = SMEM_USED > 120 * 1024 ? SMEM_USED : 120 * 1024;
 }  // namespace
 
@@ -764,7 +776,7 @@ HB_EXPORT int hb_attention_tc_tiles_extended(const void* q, int q_stride, void* 
     (void)token_row;
     if (!work) return HB_BAD_ARGUMENT;
     if (keep_first < 0 || maps < 1 || maps > 2) return HB_BAD_ARGUMENT;
-    if (maps == 2 && (D != 128 || bias || sinks || softcap > 0.f || !gate || gate_stride % 4 || ((uintptr_t)gate & 15))) return HB_BAD_ARGUMENT;
+    if (maps == 2 && (D != 128 || DK != D || bias || sinks || softcap > 0.f || !gate || gate_stride % 4 || ((uintptr_t)gate & 15))) return HB_BAD_ARGUMENT;
     if (!window) keep_first = 0;
     if ((keep_first || sinks || gate) && bias) return HB_BAD_ARGUMENT;
     if (bias && (bias_span == 0 || softcap > 0.f)) return HB_BAD_ARGUMENT;
@@ -778,8 +790,8 @@ HB_EXPORT int hb_attention_tc_tiles_extended(const void* q, int q_stride, void* 
     EncodeTiled encode = encode_tiled();
     if (!encode) return HB_BAD_ARGUMENT;
     CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)pages * 2 * kv_heads * page_size};
-    const cuuint64_t strides[1] = {(cuuint64_t)D * 2};
+    const cuuint64_t dims[2] = {(cuuint64_t)DK, (cuuint64_t)pages * 2 * kv_heads * page_size};
+    const cuuint64_t strides[1] = {(cuuint64_t)DK * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)page_size};
     const cuuint32_t elem[2] = {1, 1};
     if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(cache), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -789,8 +801,8 @@ HB_EXPORT int hb_attention_tc_tiles_extended(const void* q, int q_stride, void* 
     const int rows = maps == 2 ? BM : ROWS;  // (token, head) rows of a tile
     const int group = heads / kv_heads, gc = group < rows ? group : rows, head_chunks = (group + gc - 1) / gc;
     CUtensorMap q_map;
-    const cuuint64_t q_dims[3] = {(cuuint64_t)D, (cuuint64_t)heads, (cuuint64_t)n_tokens};
-    const cuuint64_t q_strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)q_stride * 2};
+    const cuuint64_t q_dims[3] = {(cuuint64_t)DK, (cuuint64_t)heads, (cuuint64_t)n_tokens};
+    const cuuint64_t q_strides[2] = {(cuuint64_t)DK * 2, (cuuint64_t)q_stride * 2};
     const cuuint32_t q_box[3] = {64, (cuuint32_t)gc, (cuuint32_t)(rows / gc)};
     const cuuint32_t q_elem[3] = {1, 1, 1};
     if (encode(&q_map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), q_dims, q_strides, q_box, q_elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -807,7 +819,7 @@ HB_EXPORT int hb_attention_tc_tiles_extended(const void* q, int q_stride, void* 
         if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tc_kernel<1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tc_kernel<2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tc_kernel<0, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-#if HB_HEAD_DIM == 128
+#if HB_HEAD_DIM == 128 && HB_KEY_DIM == 128
         if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_tc_kernel<0, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
 #endif
         if (e != cudaSuccess) return (int)e;
@@ -823,7 +835,7 @@ HB_EXPORT int hb_attention_tc_tiles_extended(const void* q, int q_stride, void* 
 #define HB_TC_LAUNCH(BIASED, MAPS, EXTRAS)                                                                                                              \
     return launch_after_previous(attention_tc_kernel<BIASED, MAPS, EXTRAS>, dim3(blocks), THREADS, SMEM_BYTES, stream, map, q_map, a, tiles, n_tiles,   \
                                  kv_heads * head_chunks, gc, head_chunks, work)
-#if HB_HEAD_DIM == 128
+#if HB_HEAD_DIM == 128 && HB_KEY_DIM == 128
     if (maps == 2) HB_TC_LAUNCH(0, true, true);
 #endif
     if (bias && bias_span < 0) HB_TC_LAUNCH(2, false, false);

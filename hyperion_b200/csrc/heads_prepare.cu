@@ -635,7 +635,8 @@ __global__ void __launch_bounds__(TOKEN_THREADS) latent_prepare_kernel(
     const float* __restrict__ x, int stride, int q_off, int q_rank, int kv_off, int kv_rank, int rot_dim, int rot_dims,
     const float* __restrict__ q_norm, const float* __restrict__ kv_norm, float eps, const float* __restrict__ inv_freq,
     const int* __restrict__ positions, TO* __restrict__ cq_out, int cq_stride, TO* __restrict__ cache, size_t page_stride, int token_stride,
-    const int* __restrict__ block_table, int table_width, const int* __restrict__ token_row, int page_size, int pages, int* status) {
+    const int* __restrict__ block_table, int table_width, const int* __restrict__ token_row, int page_size, int pages, TO* __restrict__ latent_out,
+    TO* __restrict__ part_out, int* status) {
     __shared__ __align__(16) float scratch[32];
     const int t = blockIdx.x;
     const int pos = positions[t];
@@ -654,16 +655,73 @@ __global__ void __launch_bounds__(TOKEN_THREADS) latent_prepare_kernel(
         return;
     }
     TO* dst = cache + (size_t)page * page_stride + (size_t)(pos - block * page_size) * token_stride;
-    for (int i = threadIdx.x; i < kv_rank; i += TOKEN_THREADS) dst[i] = from_float<TO>(row[kv_off + i] * inv_c * kv_norm[i]);
+    for (int i = threadIdx.x; i < kv_rank; i += TOKEN_THREADS) {
+        const TO v = from_float<TO>(row[kv_off + i] * inv_c * kv_norm[i]);
+        dst[i] = v;
+        if (latent_out) latent_out[(size_t)t * kv_rank + i] = v;
+    }
     const float* part = row + kv_off + kv_rank;
+    auto put = [&](int i, float value) {
+        const TO v = from_float<TO>(value);
+        dst[kv_rank + i] = v;
+        if (part_out) part_out[(size_t)t * rot_dim + i] = v;
+    };
     for (int i = threadIdx.x; i < rot_dims / 2; i += TOKEN_THREADS) {
         float s, c;
         sincosf((float)pos * inv_freq[i], &s, &c);
         const float u = part[2 * i], v = part[2 * i + 1];
-        dst[kv_rank + 2 * i] = from_float<TO>(u * c - v * s);
-        dst[kv_rank + 2 * i + 1] = from_float<TO>(v * c + u * s);
+        put(2 * i, u * c - v * s);
+        put(2 * i + 1, v * c + u * s);
     }
-    for (int i = rot_dims + threadIdx.x; i < rot_dim; i += TOKEN_THREADS) dst[kv_rank + i] = from_float<TO>(part[i]);
+    for (int i = rot_dims + threadIdx.x; i < rot_dim; i += TOKEN_THREADS) put(i, part[i]);
+}
+
+// For prompts that begin at position 0, whose keys and values per head a product has made from the latents: kv [token, 2 x heads x dim-wide rows, keys then values], the shared key
+// part [token, rot_dim] and the queries q [token, head, dim + rot_dim] become what attention over ordinary heads of dim + rot_dim reads.  Keys [plain | shared part] and values
+// [value | zeros] go to pages [page, 2, head, page_size, dim + rot_dim] of this step's own (table: a request's pages); the queries' rotated part is rotated in place.
+// One block per token, eight entries per access.
+__global__ void __launch_bounds__(TOKEN_THREADS) latent_expand_kernel(__nv_bfloat16* __restrict__ q, int q_stride, int heads, int dim, int value_dim, int rot_dim, int rot_dims,
+                                                                      const __nv_bfloat16* __restrict__ kv, const __nv_bfloat16* __restrict__ part,
+                                                                      const float* __restrict__ inv_freq, const int* __restrict__ positions, const int* __restrict__ token_row,
+                                                                      const int* __restrict__ table, int table_width, int page_size, int pages, __nv_bfloat16* __restrict__ out,
+                                                                      int* status) {
+    __shared__ float cs[MAX_PAIRS], sn[MAX_PAIRS];
+    const int t = blockIdx.x, pos = positions[t], wide = dim + rot_dim;
+    let_next_kernel_start();
+    for (int i = threadIdx.x; i < rot_dims / 2; i += TOKEN_THREADS) sincosf((float)pos * inv_freq[i], &sn[i], &cs[i]);
+    wait_for_previous_kernels();
+    const int block = pos / page_size, page = pos >= 0 && block < table_width ? table[(size_t)token_row[t] * table_width + block] : -1;
+    __syncthreads();
+    if (page < 0 || page >= pages) {
+        if (threadIdx.x == 0) atomicOr(status, HB_STATUS_BAD_PAGE);
+        return;
+    }
+    for (int e = threadIdx.x; e < heads * (rot_dims / 8); e += TOKEN_THREADS) {
+        const int head = e / (rot_dims / 8), u = e % (rot_dims / 8);
+        __nv_bfloat16* p = q + (size_t)t * q_stride + (size_t)head * wide + dim + u * 8;
+        float v[8];
+        load8(p, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float a = v[2 * i], b = v[2 * i + 1], c = cs[u * 4 + i], s = sn[u * 4 + i];
+            v[2 * i] = a * c - b * s;
+            v[2 * i + 1] = b * c + a * s;
+        }
+        store8(p, v);
+    }
+    const int eights = wide / 8;
+    const bool last = t + 1 == (int)gridDim.x || token_row[t + 1] != token_row[t];
+    const __nv_bfloat16* row = kv + (size_t)t * heads * (dim + value_dim);
+    for (int e = threadIdx.x; e < 2 * heads * eights; e += TOKEN_THREADS) {
+        const int which = e / (heads * eights), rest = e - which * heads * eights, head = rest / eights, c = (rest - head * eights) * 8;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (which == 0) v = *reinterpret_cast<const uint4*>(c < dim ? row + (size_t)head * dim + c : part + (size_t)t * rot_dim + c - dim);
+        else if (c < value_dim) v = *reinterpret_cast<const uint4*>(row + (size_t)heads * dim + (size_t)head * value_dim + c);
+        __nv_bfloat16* to = out + ((((size_t)page * 2 + which) * heads + head) * page_size + pos % page_size) * wide + c;
+        *reinterpret_cast<uint4*>(to) = v;
+        if (last)  // what follows in a request's last page is read with it: weights of zero meet zeros there
+            for (int slot = pos % page_size + 1; slot < page_size; ++slot) *reinterpret_cast<uint4*>(to += wide) = make_uint4(0, 0, 0, 0);
+    }
 }
 
 // The query that meets the cached records: per head, the query's unrotated part already carried into the latent's space
@@ -694,19 +752,33 @@ __global__ void __launch_bounds__(THREADS) latent_query_kernel(const T* __restri
 HB_EXPORT int hb_latent_prepare(const float* x, int tokens, int stride, int q_off, int q_rank, int kv_off, int kv_rank, int rot_dim, int rot_dims,
                                 const float* q_norm, const float* kv_norm, float eps, const float* inv_freq, const int* positions, void* cq_out,
                                 int cq_stride, int out_is_bf16, void* cache, long long page_stride, int token_stride, const int* block_table,
-                                int table_width, const int* token_row, int page_size, int pages, int* status, cudaStream_t stream) {
+                                int table_width, const int* token_row, int page_size, int pages, void* latent_out, void* part_out, int* status, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (q_rank <= 0 || kv_rank <= 0 || rot_dim < 0 || rot_dims < 0 || rot_dims > rot_dim || (rot_dims & 1) || page_size <= 0) return HB_UNSUPPORTED_SIZE;
     if (!q_norm || !kv_norm || !cq_out || !cache || (rot_dims && !inv_freq)) return HB_BAD_ARGUMENT;
     if (out_is_bf16)
         latent_prepare_kernel<<<tokens, TOKEN_THREADS, 0, stream>>>(x, stride, q_off, q_rank, kv_off, kv_rank, rot_dim, rot_dims, q_norm, kv_norm, eps, inv_freq,
                                                                     positions, (__nv_bfloat16*)cq_out, cq_stride, (__nv_bfloat16*)cache, (size_t)page_stride,
-                                                                    token_stride, block_table, table_width, token_row, page_size, pages, status);
+                                                                    token_stride, block_table, table_width, token_row, page_size, pages, (__nv_bfloat16*)latent_out,
+                                                                    (__nv_bfloat16*)part_out, status);
     else
         latent_prepare_kernel<<<tokens, TOKEN_THREADS, 0, stream>>>(x, stride, q_off, q_rank, kv_off, kv_rank, rot_dim, rot_dims, q_norm, kv_norm, eps, inv_freq,
                                                                     positions, (float*)cq_out, cq_stride, (float*)cache, (size_t)page_stride, token_stride,
-                                                                    block_table, table_width, token_row, page_size, pages, status);
+                                                                    block_table, table_width, token_row, page_size, pages, (float*)latent_out, (float*)part_out, status);
     return launch_status();
+}
+
+// All bfloat16 and dense but for q_stride; dim, value_dim, rot_dim and rot_dims multiples of 8, value_dim <= dim + rot_dim.
+HB_EXPORT int hb_latent_expand(void* q, int q_stride, int tokens, int heads, int dim, int value_dim, int rot_dim, int rot_dims, const void* kv, const void* part, const float* inv_freq,
+                               const int* positions, const int* token_row, const int* table, int table_width, int page_size, int pages, void* out, int* status, cudaStream_t stream) {
+    if (tokens <= 0) return 0;
+    if (heads <= 0 || dim <= 0 || ((dim | value_dim | rot_dim | rot_dims | q_stride) & 7) || rot_dims > rot_dim || rot_dims / 2 > MAX_PAIRS || value_dim <= 0 || value_dim > dim + rot_dim ||
+        page_size <= 0)
+        return HB_UNSUPPORTED_SIZE;
+    if ((rot_dims && !inv_freq) || ((((uintptr_t)q) | ((uintptr_t)kv) | ((uintptr_t)part) | ((uintptr_t)out)) & 15)) return HB_BAD_ARGUMENT;
+    return launch_after_previous(latent_expand_kernel, dim3(tokens), dim3(TOKEN_THREADS), 0, stream, (__nv_bfloat16*)q, q_stride, heads, dim, value_dim, rot_dim, rot_dims,
+                                 (const __nv_bfloat16*)kv, (const __nv_bfloat16*)part, inv_freq, positions, token_row, table, table_width, page_size, pages, (__nv_bfloat16*)out,
+                                 status);
 }
 
 HB_EXPORT int hb_latent_query(const void* q, int is_bf16, int tokens, int q_stride, int heads, int dim, int rot_dim, int rot_dims, const float* q_lat,

@@ -38,6 +38,8 @@ class ModelRunner:
         self.packer = MetadataPacker(self.device, capacity=1 << 20)  # never reallocated below this: graphs keep its address
         self._packer_generation = self.packer.generation
         self.planners = model.step_planners()
+        # some mixers take prompts that begin at position 0 another way: such steps and others of the same shape are not the same graph
+        self.tells_fresh_prompts = any(getattr(layer.mixer, "expands_fresh_prompts", False) for layer in model.layers)
         build.build_many(model.kernel_modules())
         self.steps_run = 0
         self.use_graphs = use_graphs
@@ -206,6 +208,11 @@ class ModelRunner:
                                                                         host_runtime.address(widths)))
         extras = tuple((name, len(values)) for name, (values, _) in (extra_arrays or {}).items())
         shape = len(keys) if decode else tuple(counts.tolist())
+        if self.tells_fresh_prompts and not decode:
+            lengths, slots = np.empty(len(keys), np.int32), np.empty(len(keys), np.int32)
+            host_runtime.check(host_runtime.library().hb_cache_lengths(self.cache.native, len(keys), host_runtime.address(keys), host_runtime.address(lengths),
+                                                                       host_runtime.address(slots)))
+            shape = (*shape, bool(lengths.any()))
         return (shape, len(want), tuple(widths[: len(self.cache.paged)].tolist()), extras)
 
     def _replay(self, key, context: StepContext):

@@ -104,6 +104,24 @@ def choose_splits(n_items: int, heads: int, kv_heads: int, longest_context: int,
     return max(1, min(target // max(1, blocks), key_tiles // 3, 64))
 
 
+WIDE_KEYS = 192  # entries of a query and of a key over values of 128, the tcgen05 kernel's other shape
+
+
+def attention_wide_keys(q, heads, cache, block_table, token_row, positions, tiles, n_tiles, scale, out, sinks=None):
+    """Prompt portions over keys of 192 entries and values of 128: ``q`` [tokens, heads * 192], ``cache`` [pages, 2, heads, page, 192], a value being its row's first 128 entries, tiles
+    planned for :data:`TC_TILE_ROWS`, ``out`` [tokens, heads * 128]; a key/value head per query head; ``sinks`` as for :func:`attention_tiles`."""
+    _common(q, out, cache, block_table, token_row, positions)
+    require_cuda(sinks)
+    _plain_vector(sinks, heads, "sinks")
+    pages, _, kv_heads, page_size, wide = cache.shape
+    if wide != WIDE_KEYS or kv_heads != heads or q.shape[1] != heads * wide or out.shape[1] != heads * 128:
+        raise KernelError("attention_wide_keys: keys of 192 entries over values of 128, a key/value head per query head")
+    check(library("attention_tcgen05", HB_HEAD_DIM=128, HB_KEY_DIM=WIDE_KEYS).hb_attention_tc_tiles_extended(
+        ptr(q), i32(q.stride(0)), ptr(out), i32(out.stride(0)), ptr(cache), ptr(block_table), i32(block_table.shape[1]), ptr(token_row), ptr(positions), ptr(tiles), i32(n_tiles),
+        i32(q.shape[0]), i32(heads), i32(kv_heads), i32(128), i32(page_size), i32(pages), f32(scale), f32(0.0), i32(0), ptr(None), i32(0), i32(0), ptr(sinks), ptr(None), i32(0),
+        i32(1), f32(0.0), f32(0.0), f32(0.0), ptr(status_word(q.device)), ptr(work_counters(q.device)), stream_ptr()), "attention_wide_keys")
+
+
 _WORK: dict[int, torch.Tensor] = {}
 
 

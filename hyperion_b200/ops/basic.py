@@ -333,12 +333,16 @@ def heads_prepare_wide(x: torch.Tensor, q_off: int, k_off: int, v_off: int, q_he
 
 def latent_prepare(x: torch.Tensor, q_off: int, q_rank: int, kv_off: int, kv_rank: int, rot_dim: int, q_norm: torch.Tensor, kv_norm: torch.Tensor, eps: float,
                    inv_freq: torch.Tensor | None, rot_dims: int, positions: torch.Tensor, out_dtype: torch.dtype, cache: torch.Tensor, block_table: torch.Tensor,
-                   token_row: torch.Tensor, page_size: int) -> torch.Tensor:
+                   token_row: torch.Tensor, page_size: int, latent_out: torch.Tensor | None = None, part_out: torch.Tensor | None = None) -> torch.Tensor:
     """Float down-projections ``x`` [tokens, *]: the query latent (``q_rank`` columns at ``q_off``) and the key/value latent (``kv_rank``
     columns at ``kv_off``) followed by the shared key part of ``rot_dim`` columns.  Both latents pass an RMS norm with a weight per
     entry; the key part's first ``rot_dims`` entries are rotated in adjacent pairs.  Returns the normed query latent [tokens, q_rank]
-    in ``out_dtype``; latent and key part go to ``cache`` [pages, 1, page, kv_rank + rot_dim]."""
-    require_cuda(x, q_norm, kv_norm, inv_freq, positions, cache, block_table, token_row)
+    in ``out_dtype``; latent and key part go to ``cache`` [pages, 1, page, kv_rank + rot_dim], and to ``latent_out`` [tokens, kv_rank] and ``part_out``
+    [tokens, rot_dim] where these are given."""
+    require_cuda(x, q_norm, kv_norm, inv_freq, positions, cache, block_table, token_row, latent_out, part_out)
+    for dense, width in ((latent_out, kv_rank), (part_out, rot_dim)):
+        if dense is not None and (dense.dtype != out_dtype or dense.shape != (x.shape[0], width) or not dense.is_contiguous()):
+            raise KernelError("latent_prepare: dense copies of the latents and of the key parts in the output's element type")
     if x.dtype != torch.float32 or x.stride(-1) != 1 or q_norm.dtype != torch.float32 or kv_norm.dtype != torch.float32:
         raise KernelError("latent_prepare: float32 projections and norm weights")
     if q_norm.numel() != q_rank or kv_norm.numel() != kv_rank or (rot_dims and (inv_freq is None or inv_freq.numel() < rot_dims // 2)):
@@ -350,9 +354,28 @@ def latent_prepare(x: torch.Tensor, q_off: int, q_rank: int, kv_off: int, kv_ran
     check(library("heads_prepare").hb_latent_prepare(
         ptr(x), i32(x.shape[0]), i32(x.stride(0)), i32(q_off), i32(q_rank), i32(kv_off), i32(kv_rank), i32(rot_dim), i32(rot_dims), ptr(q_norm), ptr(kv_norm),
         f32(eps), ptr(inv_freq), ptr(positions), ptr(cq), i32(cq.stride(0)), i32(is_bf16(cq)), ptr(cache), ctypes.c_longlong(cache.shape[2] * record),
-        i32(record), ptr(block_table), i32(block_table.shape[1]), ptr(token_row), i32(page_size), i32(cache.shape[0]), ptr(status_word(x.device)),
-        stream_ptr()), "latent_prepare")
+        i32(record), ptr(block_table), i32(block_table.shape[1]), ptr(token_row), i32(page_size), i32(cache.shape[0]), ptr(latent_out), ptr(part_out),
+        ptr(status_word(x.device)), stream_ptr()), "latent_prepare")
     return cq
+
+
+def latent_expand_(q: torch.Tensor, kv: torch.Tensor, part: torch.Tensor, heads: int, dim: int, value_dim: int, inv_freq: torch.Tensor | None, rot_dims: int, positions: torch.Tensor,
+                   token_row: torch.Tensor, table: torch.Tensor, pages: torch.Tensor) -> None:
+    """``kv`` [tokens, heads * (dim + value_dim)] (every head's unrotated key, then every head's value) and ``part`` [tokens, rot_dim] (the shared, rotated key part) go to ``pages``
+    [pages, 2, heads, page_size, dim + rot_dim] as keys [plain | shared] and values [value | zeros], a request's pages in its row of ``table``; the rotated parts of ``q``
+    [tokens, heads * (dim + rot_dim)] are rotated in place.  All bfloat16."""
+    require_cuda(q, kv, part, inv_freq, positions, token_row, table, pages)
+    tokens, rot_dim = part.shape
+    wide = dim + rot_dim
+    if any(t.dtype != torch.bfloat16 for t in (q, kv, part, pages)) or not kv.is_contiguous() or not part.is_contiguous() or not pages.is_contiguous() or q.stride(1) != 1:
+        raise KernelError("latent_expand: dense bfloat16 operands")
+    if q.shape != (tokens, heads * wide) or kv.shape != (tokens, heads * (dim + value_dim)) or pages.dim() != 5 or pages.shape[1:3] != (2, heads) or pages.shape[4] != wide:
+        raise KernelError("latent_expand: queries, keys and values of one set of heads")
+    if table.dtype != torch.int32 or table.dim() != 2 or not table.is_contiguous():
+        raise KernelError("latent_expand: a dense int32 table of pages, a row per request")
+    check(library("heads_prepare").hb_latent_expand(ptr(q), i32(q.stride(0)), i32(tokens), i32(heads), i32(dim), i32(value_dim), i32(rot_dim), i32(rot_dims), ptr(kv), ptr(part),
+                                                    ptr(inv_freq), ptr(positions), ptr(token_row), ptr(table), i32(table.shape[1]), i32(pages.shape[3]), i32(pages.shape[0]), ptr(pages),
+                                                    ptr(status_word(q.device)), stream_ptr()), "latent_expand")
 
 
 def latent_query(q: torch.Tensor, q_lat: torch.Tensor, heads: int, dim: int, rot_dim: int, inv_freq: torch.Tensor | None, rot_dims: int,

@@ -19,6 +19,10 @@ output projection.  In bfloat16, with records of a multiple of 16 entries and la
 tensor cores (``csrc/attention_latent.cu``: blocks of 16, 32 or 64 (token, head) pairs over key tiles of 64 records, the keys split over
 several blocks when a step brings few tokens).  Everything else, and float32, runs in ``csrc/attention_generic.cu``.
 
+A step of nothing but prompts from position 0 on, long enough, takes the other way round (``_attend_expanded``): every key and value a query sees is a token of the step, so
+the keys and values of all heads are made from the latents by one product, and attention runs over ordinary heads of ``head_dim`` + ``rot_dim`` entries: some third
+of the operations per pair of a query and a key (1,531 tokens of 16 heads: 51 us a layer in csrc/attention_tcgen05.cu beside 225).  The records go to the cache all the same.
+
 Parameters: ``hidden_size``, ``heads``, ``head_dim``, ``rot_dim``, ``value_dim``, ``kv_rank``, ``q_rank``, ``scale``, ``position`` (a PartSpec
 of kind ``rope_interleaved``, or None), ``sink`` (bool), ``eps``.  Tensors: dq, dq.norm, uq, dkv, dkv.norm, uk, uv, sink, o.
 """
@@ -26,6 +30,7 @@ from __future__ import annotations
 
 from typing import Mapping
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -37,6 +42,13 @@ from .spec import PartSpec
 
 def _common_dtype(tensors) -> torch.dtype:
     return torch.float32 if any(t.dtype == torch.float32 for t in tensors) else tensors[0].dtype
+
+
+EXPANDED_TOKENS = 300  # of a step, per prompt.  What the other way saves grows with the square of a prompt, what it adds (one product more, its keys and values written out) with
+# the step's tokens.  A step of 8 layers, 4 of them over latents of 16 heads, expanded and through the latent, in us: one prompt of 200 tokens 872 and 844, two of 256 1,074 and
+# 1,060, five of 300 1,342 and 1,421, three of 400 1,355 and 1,475, one of 1,024 1,622 and 1,906, one of 1,531 2,238 and 2,919; four of 128 999 and 927.
+EXPANDED_BYTES = 256 << 20  # of a step's keys and values per layer; longer prompts keep to the latent
+EXPANDED_PAGE = 64
 
 
 class LatentAttention(Mixer):
@@ -59,6 +71,9 @@ class LatentAttention(Mixer):
             raise ValueError(f"a record of {self.record} entries per token is above the kernel's limit of {LARGEST_HEAD}")
         self.q_head = self.head_dim + self.rot_dim
         self.fast = self.dtype == torch.bfloat16 and fast_attention.latent_supported(self.record, self.kv_rank)
+        # heads that the tcgen05 attention takes
+        self.expands_fresh_prompts = (self.fast and self.q_head == fast_attention.WIDE_KEYS and self.value_dim == 128 and self.kv_rank % 8 == 0
+                                      and not any(n % 8 for n in (self.head_dim, self.rot_dim, self.rot_dims)))
 
     def weights(self) -> dict[str, WeightSpec]:
         wanted = {"dq": WeightSpec((self.q_rank, self.hidden)), "dq.norm": WeightSpec((self.q_rank,), init="one_plus_normal"),
@@ -79,6 +94,7 @@ class LatentAttention(Mixer):
         self.k_heads = tensors["uk"].reshape(self.heads, self.head_dim, self.kv_rank).contiguous()  # q_plain [H, T, d] x this = the query in the latent's space
         self.v_heads = tensors["uv"].reshape(self.heads, self.value_dim, self.kv_rank).transpose(1, 2).contiguous()  # [H, R, e]
         self.sink = tensors["sink"].to(torch.float32).contiguous() if self.has_sink else None
+        self.w_kv = torch.cat([tensors["uk"], tensors["uv"]], dim=0).contiguous() if self.expands_fresh_prompts else None  # every head's keys, then every head's values
 
     def cache_request(self):
         return PagedTokens((1,), (self.record,), 0)
@@ -87,7 +103,49 @@ class LatentAttention(Mixer):
         modules = [("heads_prepare", {}), ("attention_generic", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})]
         if self.fast:
             modules.append(("attention_latent", {"HB_RECORD": self.record, "HB_VALUE": self.kv_rank}))
+        if self.expands_fresh_prompts:
+            modules.append(("attention_tcgen05", {"HB_HEAD_DIM": 128, "HB_KEY_DIM": fast_attention.WIDE_KEYS}))
         return modules
+
+    def step_plans(self):
+        """Pages of the step's own for the keys and values of its prompts, and the prompts cut into tiles, where the step takes :meth:`_attend_expanded`."""
+        if not self.expands_fresh_prompts:
+            return {}
+
+        def plan(rows, packer, host):
+            counts = rows.counts
+            pages = -(-counts // EXPANDED_PAGE)
+            total = int(pages.sum())
+            if (rows.positions.any() or int(counts.min()) <= fast_attention.TOKEN_SHAPE_MAX or int(counts.sum()) < EXPANDED_TOKENS * len(counts)
+                    or total * EXPANDED_PAGE * 2 * self.heads * self.q_head * 2 > EXPANDED_BYTES):
+                return
+            table = np.full((len(counts), int(pages.max())), -1, dtype=np.int32)
+            ends = np.cumsum(pages)
+            for row, (end, n) in enumerate(zip(ends.tolist(), pages.tolist())):
+                table[row, :n] = np.arange(end - n, end)
+            tiles, _ = fast_attention.plan(rows, fast_attention.TC_TILE_ROWS)
+            host[self._expanded_key()] = (total, len(tiles) // 3)
+            packer.add(f"{self._expanded_key()}_table", table.reshape(-1), table.shape)
+            packer.add(f"{self._expanded_key()}_tiles", tiles)
+
+        return {("latent_plan", self._expanded_key()): plan}
+
+    def _expanded_key(self) -> str:
+        return f"latent_{self.heads}_{self.q_head}"
+
+    def _attend_expanded(self, cq, latent, part, step, inv_freq):
+        """[tokens, heads * value_dim]: attention of the step's prompts over their own keys and values."""
+        key = self._expanded_key()
+        pages, n_tiles = step.host[key]
+        tokens = cq.shape[0]
+        q = ops.linear(cq, self.w_uq, None, self.dtype)
+        kv = ops.linear(latent, self.w_kv, None, self.dtype)
+        storage = torch.empty((pages, 2, self.heads, EXPANDED_PAGE, self.q_head), dtype=self.dtype, device=cq.device)
+        table = step.extra[f"{key}_table"]
+        ops.latent_expand_(q, kv, part, self.heads, self.head_dim, self.value_dim, inv_freq, self.rot_dims, step.positions, step.token_row, table, storage)
+        out = torch.empty((tokens, self.heads * self.value_dim), dtype=self.dtype, device=cq.device)
+        fast_attention.attention_wide_keys(q, self.heads, storage, table, step.token_row, step.positions, step.extra[f"{key}_tiles"], n_tiles, self.scale, out, sinks=self.sink)
+        return out
 
     @staticmethod
     def _batched(a: torch.Tensor, b: torch.Tensor, out_dtype: torch.dtype) -> torch.Tensor:
@@ -101,8 +159,13 @@ class LatentAttention(Mixer):
         tokens = x.shape[0]
         inv_freq = self.position.inv_freq if self.position is not None else None
         proj = ops.linear(x, self.w_down, None, torch.float32)
+        expands = self.expands_fresh_prompts and self._expanded_key() in step.host
+        latent = torch.empty((tokens, self.kv_rank), dtype=self.dtype, device=x.device) if expands else None
+        part = torch.empty((tokens, self.rot_dim), dtype=self.dtype, device=x.device) if expands else None
         cq = ops.latent_prepare(proj, 0, self.q_rank, self.q_rank, self.kv_rank, self.rot_dim, self.q_norm, self.kv_norm, self.eps, inv_freq, self.rot_dims,
-                                step.positions, self.dtype, cache.kv, cache.block_table, step.token_row, cache.page_size)
+                                step.positions, self.dtype, cache.kv, cache.block_table, step.token_row, cache.page_size, latent, part)
+        if expands:
+            return ops.linear(self._attend_expanded(cq, latent, part, step, inv_freq), self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
         q = ops.linear(cq, self.w_uq, None, self.dtype)
         plain = q.view(tokens, self.heads, self.q_head)[:, :, : self.head_dim].transpose(0, 1)
         q_lat = self._batched(plain, self.k_heads.to(q.dtype) if self.k_heads.dtype != q.dtype else self.k_heads, torch.float32)
