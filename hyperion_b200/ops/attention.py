@@ -94,6 +94,19 @@ def plan(rows, tokens_per_tile: int) -> tuple[np.ndarray, np.ndarray]:
     return tiles[: 3 * n_tiles.value], items[: n_items.value]
 
 
+def plan_prompts(rows, tokens_per_tile: int, blocks: int, most: float = 0.5) -> tuple[np.ndarray, np.ndarray]:
+    """:func:`plan` for the tcgen05 kernel: tiles of half the rows where tiles times the ``blocks`` (key/value heads and head chunks) of a tile are at most ``most`` of the SMs.
+
+    A block that works on one half's 128 rows alone takes about 0.77 of the time per key tile.  With twice as many blocks and an SM for each that is the step's gain (1,000 tokens of 4
+    key/value heads, 64 blocks: 49 -> 38 us, with a window 29 -> 25); where the tiles come back in a second turn it is lost, unless they differ in length as a whole prompt's do
+    (96 blocks of a 1,531-token prompt: 53 -> 40 us; 128 blocks of a 2,048-token one: 52 -> 60).  How far a tile's keys reach is not among what the captured steps are told apart by,
+    so the general rule asks for one turn."""
+    tiles, items = plan(rows, tokens_per_tile)
+    if tokens_per_tile >= 2 and len(tiles) and len(tiles) // 3 * blocks <= most * sm_count():
+        return plan(rows, tokens_per_tile // 2)
+    return tiles, items
+
+
 def choose_splits(n_items: int, heads: int, kv_heads: int, longest_context: int, sms: int | None = None) -> int:
     """Splits of the keys for the token shape: about two blocks per SM of the device (``sms``, asked from the current
     device when absent) in all, at least 3 key tiles each."""

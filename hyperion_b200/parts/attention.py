@@ -117,6 +117,7 @@ class GroupedQueryAttention(Mixer):
     @staticmethod
     def plans_for(heads: int, kv_heads: int, head_dim: int, rows_of=None) -> dict:
         """``rows_of(page_size)``: the virtual rows per tile, where another kernel than the usual one for this head size will run."""
+        halves = rows_of is None
         rows_of = rows_of or (lambda page_size: fast_attention.tile_rows(head_dim, page_size))
 
         def plan(rows, packer, host):
@@ -125,7 +126,10 @@ class GroupedQueryAttention(Mixer):
             key = f"attn_tiles_{tokens_per_tile}"
             if key in host:
                 return
-            tiles, items = fast_attention.plan(rows, tokens_per_tile)
+            if halves and size == fast_attention.TC_TILE_ROWS:
+                tiles, items = fast_attention.plan_prompts(rows, tokens_per_tile, kv_heads * -(-heads // kv_heads // size))
+            else:
+                tiles, items = fast_attention.plan(rows, tokens_per_tile)
             host[key] = len(tiles) // 3
             host["attn_items"] = len(items)
             if len(tiles):

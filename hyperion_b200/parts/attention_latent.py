@@ -123,7 +123,7 @@ class LatentAttention(Mixer):
             ends = np.cumsum(pages)
             for row, (end, n) in enumerate(zip(ends.tolist(), pages.tolist())):
                 table[row, :n] = np.arange(end - n, end)
-            tiles, _ = fast_attention.plan(rows, fast_attention.TC_TILE_ROWS)
+            tiles, _ = fast_attention.plan_prompts(rows, fast_attention.TC_TILE_ROWS, self.heads, 2 / 3)  # whole prompts: their tiles differ in length
             host[self._expanded_key()] = (total, len(tiles) // 3)
             packer.add(f"{self._expanded_key()}_table", table.reshape(-1), table.shape)
             packer.add(f"{self._expanded_key()}_tiles", tiles)
