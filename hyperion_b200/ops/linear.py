@@ -1,8 +1,8 @@
 """Dense projections y = x W^T (+ b) with W stored [out, in].
 
 float32 weights go through the package's own FFMA kernel (the true 32-bit path: no tensor cores,
-no reduced-precision matrix mode).  bfloat16 weights go either to the package's tcgen05 kernel
-(``ops/gemm.py``; see ``_takes_own_kernel`` for which products) or to the library matrix product, as the
+no reduced-precision matrix mode).  bfloat16 weights go to the package's kernel for a few rows and a
+small matrix (``_takes_few_rows``), to its tcgen05 kernel (``ops/gemm.py``; see ``_takes_own_kernel`` for which products) or to the library matrix product, as the
 reference's engine does for every projection (``cublasGemmEx`` and ``cublasLtMatmul`` with a bias
 epilogue: helios/crates/helios-hal/src/cuda/cublas.rs:158-188, cuda/cublaslt.rs:203-212,302);
 accumulation is float, the bias is added before the one rounding to bfloat16, and the output head
