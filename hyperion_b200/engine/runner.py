@@ -38,8 +38,8 @@ class ModelRunner:
         self.packer = MetadataPacker(self.device, capacity=1 << 20)  # never reallocated below this: graphs keep its address
         self._packer_generation = self.packer.generation
         self.planners = model.step_planners()
-        # some mixers take prompts that begin at position 0 another way: such steps and others of the same shape are not the same graph
-        self.tells_fresh_prompts = any(getattr(layer.mixer, "expands_fresh_prompts", False) for layer in model.layers)
+        # some parts, however deep inside others, plan steps whose rows all begin at position 0 another way: such steps and others of the same shape are not the same graph
+        self.tells_fresh_prompts = any(getattr(plan, "tells_fresh_prompts", False) for plan in self.planners.values())
         build.build_many(model.kernel_modules())
         self.steps_run = 0
         self.use_graphs = use_graphs

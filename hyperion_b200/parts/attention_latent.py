@@ -128,6 +128,7 @@ class LatentAttention(Mixer):
             packer.add(f"{self._expanded_key()}_table", table.reshape(-1), table.shape)
             packer.add(f"{self._expanded_key()}_tiles", tiles)
 
+        plan.tells_fresh_prompts = True  # the runner keeps graphs of such steps apart
         return {("latent_plan", self._expanded_key()): plan}
 
     def _expanded_key(self) -> str:
