@@ -35,6 +35,11 @@ def gemm_policy() -> str:
     return _policy[0]
 
 
+def _is_one_per_column(bias: Optional[torch.Tensor], weight: torch.Tensor) -> bool:
+    """Whether a bias, if there is one, is what the kernels read: a dense number per column in a type they know.  The library broadcasts what is not, or refuses it."""
+    return bias is None or (bias.dtype in (torch.bfloat16, torch.float32) and bias.shape == weight.shape[:1] and bias.is_contiguous())
+
+
 def _takes_own_kernel(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) -> bool:
     """Which bfloat16 products go to the package's tcgen05 kernels.  ``auto``: every product of up to 64 rows with a
     reduction of at least 2,048 (the swapped kernel streams the weights as fast as or faster than the library at every
@@ -47,7 +52,7 @@ def _takes_own_kernel(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) ->
     policy = gemm_policy()
     if policy == "library" or out_dtype not in (torch.bfloat16, torch.float32) or not gemm.supported(x, weight):
         return False
-    if bias is not None and bias.dtype not in (torch.bfloat16, torch.float32):
+    if not _is_one_per_column(bias, weight):
         return False
     if policy == "own":
         return True
@@ -58,9 +63,12 @@ def _takes_own_kernel(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) ->
 
 
 def _takes_few_rows(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) -> bool:
-    """Whether a bfloat16 product goes to the kernel for a few rows and a small matrix (``HYPERION_B200_GEMM`` = ``auto`` only)."""
-    return (x.shape[0] <= gemm.FEW_ROWS and gemm_policy() == "auto" and out_dtype in (torch.bfloat16, torch.float32)
-            and (bias is None or (bias.dtype in (torch.bfloat16, torch.float32) and bias.is_contiguous())) and gemm.takes_few_rows(x, weight))
+    """Whether a bfloat16 product goes to the kernel for a few rows and a small matrix (``HYPERION_B200_GEMM`` = ``auto`` only).  The library keeps what the kernel has no form
+    for: a bias that is not one dense number per column, a matrix of one row without its dimension, nothing to add up, and operands that ask for a gradient."""
+    if x.dim() != 2 or weight.dim() != 2 or not 0 < x.shape[0] <= gemm.FEW_ROWS or 0 in weight.shape or gemm_policy() != "auto" or out_dtype not in (torch.bfloat16, torch.float32):
+        return False
+    asks_for_gradient = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, weight, bias))
+    return _is_one_per_column(bias, weight) and not asks_for_gradient and gemm.takes_few_rows(x, weight)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
