@@ -120,7 +120,7 @@ static inline int launch_status() { return (int)cudaGetLastError(); }
 // stream is still running. It must call wait_for_previous_kernels() before it reads anything an
 // earlier kernel wrote and before it writes global memory at all; what stands before that call
 // (barrier set-up, tensor-memory allocation, loads of weights, which no kernel writes) overlaps
-// the earlier kernel's tail. let_next_kernel_start() allows the kernel after this one to be
+// the earlier kernel's tail.  A kernel whose caller cannot promise that is launched the ordinary way (launch_in_turn with `overlaps` 0). let_next_kernel_start() allows the kernel after this one to be
 // scheduled as soon as every block of this one has called it; that kernel still waits in its own
 // wait_for_previous_kernels() until this one has finished and its writes are visible. Both calls
 // do nothing in a kernel that was launched the ordinary way. HYPERION_B200_PDL=0 turns the
@@ -137,8 +137,7 @@ static inline bool overlap_launches() {
 }
 
 template <typename... Params, typename... Args>
-static inline int launch_after_previous(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
-                                        Args&&... args) {
+static inline int launch_in_turn(bool overlaps, void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream, Args&&... args) {
     cudaLaunchConfig_t config = {};
     config.gridDim = grid;
     config.blockDim = block;
@@ -146,10 +145,16 @@ static inline int launch_after_previous(void (*kernel)(Params...), dim3 grid, di
     config.stream = stream;
     cudaLaunchAttribute attribute[1];
     attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attribute[0].val.programmaticStreamSerializationAllowed = overlap_launches() ? 1 : 0;
+    attribute[0].val.programmaticStreamSerializationAllowed = overlaps && overlap_launches() ? 1 : 0;
     config.attrs = attribute;
     config.numAttrs = 1;
     return (int)cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
+template <typename... Params, typename... Args>
+static inline int launch_after_previous(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
+                                        Args&&... args) {
+    return launch_in_turn(true, kernel, grid, block, shared_bytes, stream, args...);
 }
 
 // The first position that a query at position `pos` sees.  window > 0: the last `window` positions (pos - window + 1 at the least);

@@ -637,9 +637,9 @@ __global__ void __launch_bounds__(1024) rmsnorm_add_bf16x8_kernel(float* __restr
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, x[8], w[8];
     float* hrow = h + (size_t)t * hidden + i;
     let_next_kernel_start();
-    if (active) load8(weight + i, w);
     wait_for_previous_kernels();
-    if (active) {  // both rows are asked for before the sum
+    if (active) {  // both rows and the weights are asked for before the sum
+        load8(weight + i, w);
         load8(y + (size_t)t * hidden + i, v);
         load8(hrow, x);
     }
@@ -739,10 +739,11 @@ __global__ void norm_add_norm_bf16x8_kernel(float* __restrict__ h, const __nv_bf
                                             const int* __restrict__ rows, int hidden, float eps_post, float eps_next, const float* __restrict__ gate,
                                             int gate_stride, int gate_splits, size_t gate_split_stride, const float* __restrict__ gate_bias) {
     __shared__ __align__(16) float scratch[32];
-    const int i = blockIdx.x, t = rows ? rows[i] : i, j = threadIdx.x * 8;
+    const int i = blockIdx.x, j = threadIdx.x * 8;
     const bool active = j < hidden;
     let_next_kernel_start();
     wait_for_previous_kernels();
+    const int t = rows ? rows[i] : i;
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     float inv_y = 0.f;
     if (y) {

@@ -1,8 +1,9 @@
 // Products of a few rows with a matrix of a few megabytes, C[M, N] = A[M, K] W[N, K]^T, M up to 16, bfloat16: what a decoded token asks of a small model.
 //
 // Such a product is a chain of waits: the launch, the weights, the rows, the sums.  Here the weights do not wait for the kernel before: every warp has its first units
-// of the matrix on their way into registers before it waits for that kernel (nobody writes weights), so that afterwards only the rows, which are in L2, and the
-// sums remain (one row, in chains of such products: [896, 896] 4.2 us in the library, 2.2 here; [9,728, 896] with SwiGLU 8.1 in two launches, 5.0 here, 2.7 of them for
+// of the matrix on their way into registers before it waits for that kernel, so that afterwards only the rows, which are in L2, and the
+// sums remain.  That asks for a matrix that no kernel still in flight writes, a model's weights: where the caller does not say so (`settled`), the launch is an ordinary one,
+// behind the kernel before (one row, in chains of such products: [896, 896] 4.2 us in the library, 2.2 here; [9,728, 896] with SwiGLU 8.1 in two launches, 5.0 here, 2.7 of them for
 // the bytes).
 //
 // A unit is 16 rows of W by 64 of k.  A block takes whole tiles of 16 rows (or, for sums that are left in pieces, a part of k of one tile), its warps an even share of their
@@ -177,16 +178,16 @@ __global__ void __launch_bounds__(THREADS, 2) few_rows_kernel(const FewArgs a) {
 }
 
 template <int EPI>
-int launch_few(const FewArgs& a, int blocks, cudaStream_t stream) {
-    if (a.rows <= 8) return launch_after_previous(few_rows_kernel<1, 4, EPI>, dim3(blocks), dim3(THREADS), 0, stream, a);
-    return launch_after_previous(few_rows_kernel<2, 3, EPI>, dim3(blocks), dim3(THREADS), 0, stream, a);
+int launch_few(const FewArgs& a, int blocks, bool settled, cudaStream_t stream) {
+    if (a.rows <= 8) return launch_in_turn(settled, few_rows_kernel<1, 4, EPI>, dim3(blocks), dim3(THREADS), 0, stream, a);
+    return launch_in_turn(settled, few_rows_kernel<2, 3, EPI>, dim3(blocks), dim3(THREADS), 0, stream, a);
 }
 }  // namespace
 
 // x [rows, k] (row stride x_stride), w [n, k] dense, bfloat16; k a multiple of 64, n of 16.  epilogue as above; parts: of epilogue 3 (1 otherwise);
-// blocks: how many the device should hold at a time.
+// blocks: how many the device should hold at a time; settled: no kernel still in flight writes w.
 HB_EXPORT int hb_few_rows(const void* x, int x_stride, const void* w, const void* bias_h, const float* bias_f, void* c, int c_stride, int rows, int n, int k, int epilogue,
-                          int gu_block, int parts, int blocks, cudaStream_t stream) {
+                          int gu_block, int parts, int blocks, int settled, cudaStream_t stream) {
     if (rows <= 0 || n <= 0) return 0;
     if (rows > 16 || k <= 0 || k % UNIT_K || n % 16 || (x_stride & 7) || ((((uintptr_t)x) | ((uintptr_t)w)) & 15)) return HB_UNSUPPORTED_SIZE;
     if (blocks < 1 || parts < 1 || parts > k / UNIT_K || epilogue < FEW_BF16 || epilogue > FEW_PIECES) return HB_BAD_ARGUMENT;
@@ -199,12 +200,12 @@ HB_EXPORT int hb_few_rows(const void* x, int x_stride, const void* w, const void
         if (bias_h || bias_f || n % 32 || gu_block < 8 || inter % gu_block || (gu_block != inter && (gu_block & (gu_block - 1)))) return HB_UNSUPPORTED_SIZE;
         a.gu_block = gu_block;
         a.gu_shift = gu_block == inter ? 31 : __builtin_ctz((unsigned)gu_block);
-        return launch_few<FEW_SWIGLU>(a, grid, stream);
+        return launch_few<FEW_SWIGLU>(a, grid, settled != 0, stream);
     }
     if (epilogue == FEW_PIECES) {
         if (bias_h || bias_f) return HB_BAD_ARGUMENT;
         a.parts = parts;
-        return launch_few<FEW_PIECES>(a, tiles * parts, stream);
+        return launch_few<FEW_PIECES>(a, tiles * parts, settled != 0, stream);
     }
-    return epilogue == FEW_F32 ? launch_few<FEW_F32>(a, grid, stream) : launch_few<FEW_BF16>(a, grid, stream);
+    return epilogue == FEW_F32 ? launch_few<FEW_F32>(a, grid, settled != 0, stream) : launch_few<FEW_BF16>(a, grid, settled != 0, stream);
 }

@@ -9,6 +9,9 @@
 // The row is [q heads x head_dim | k heads x head_dim | v heads x v_dim].  The cache is addressed
 // by two base pointers and the strides of a page, a head and a token (in elements), so keys and
 // values may share a page in any arrangement.
+// The kernels that work in units take a token's sines and cosines while the kernel before still runs, so they want positions and frequencies that no kernel in
+// flight writes.  `settled` says so (a step's positions come with its one copy from the host: 2.0 and 2.2 us for one token of 16 + 4 heads of 128, 5 to 10 % up to
+// 64 tokens); without it they are launched the ordinary way, behind the kernel before.
 #include "common.cuh"
 
 namespace {
@@ -157,7 +160,7 @@ __global__ void __launch_bounds__(UNIT_THREADS) heads_prepare_units_kernel(
     const int t = blockIdx.x, pos = positions[t], units = head_dim >> 3, shift = __ffs(units) - 1, heads = q_heads + kv_heads + (with_values ? kv_heads : 0);
     if (!inv_freq) rot_dims = 0;
     let_next_kernel_start();
-    for (int i = threadIdx.x; i < rot_dims / 2; i += UNIT_THREADS) sincosf((float)pos * inv_freq[i], &sn[i], &cs[i]);  // from what the host sent: no kernel's work
+    for (int i = threadIdx.x; i < rot_dims / 2; i += UNIT_THREADS) sincosf((float)pos * inv_freq[i], &sn[i], &cs[i]);  // settled, or behind the kernel before
     wait_for_previous_kernels();
     __nv_bfloat16* row = x + (size_t)t * stride;
     const int per_part = ((heads + gridDim.y - 1) / gridDim.y) * units, begin = blockIdx.y * per_part, end = min(heads * units, begin + per_part);
@@ -217,7 +220,7 @@ HB_EXPORT int hb_heads_prepare(void* x, int is_bf16, int tokens, int stride, int
                                const float* q_norm, const float* k_norm, float eps, const float* inv_freq, int rot_dims,
                                const int* positions, const void* v_first, int v_first_stride, const float* lambda, void* k_cache,
                                void* v_cache, long long page_stride, long long head_stride, int token_stride, const int* block_table,
-                               int table_width, const int* token_row, int page_size, int pages, int with_values, int* status,
+                               int table_width, const int* token_row, int page_size, int pages, int with_values, int settled, int* status,
                                cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (head_dim <= 0 || v_dim <= 0 || rot_dims < 0 || rot_dims > head_dim || (rot_dims & 1)) return HB_UNSUPPORTED_SIZE;
@@ -229,7 +232,7 @@ HB_EXPORT int hb_heads_prepare(void* x, int is_bf16, int tokens, int stride, int
         (((uintptr_t)q_norm | (uintptr_t)k_norm) & 15) == 0) {  // from sizes and addresses alone: a token's result does not depend on the step
         const int units = heads * (head_dim / 8), most = (units + UNIT_THREADS - 1) / UNIT_THREADS;
         const int parts = tokens >= 256 ? 1 : (most > 256 / tokens ? 256 / tokens : most);
-        return launch_after_previous(heads_prepare_units_kernel, dim3(tokens, parts), dim3(UNIT_THREADS), 0, stream, (__nv_bfloat16*)x, stride, q_heads, kv_heads, head_dim,
+        return launch_in_turn(settled != 0, heads_prepare_units_kernel, dim3(tokens, parts), dim3(UNIT_THREADS), 0, stream, (__nv_bfloat16*)x, stride, q_heads, kv_heads, head_dim,
                                      with_values, q_norm, k_norm, eps, inv_freq, rot_dims, positions, (const __nv_bfloat16*)v_first, v_first_stride, lambda,
                                      (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, (size_t)page_stride, (size_t)head_stride, token_stride, block_table, table_width, token_row,
                                      page_size, pages, status);
@@ -566,7 +569,7 @@ HB_EXPORT int hb_heads_prepare_wide(const float* x, int tokens, int stride, int 
                                     int rot_half, const int* positions, float k_scale, void* q_out, int q_out_stride, void* k_out, int k_out_stride,
                                     int out_is_bf16, void* k_cache, void* v_cache, long long page_stride, long long head_stride, int token_stride,
                                     const int* block_table, int table_width, const int* token_row, int page_size, int pages, float v_unit_eps,
-                                    const float* q_head_scale, const float* v_inv_freq, int v_rot_dims, int v_rot_half, int* status, cudaStream_t stream) {
+                                    const float* q_head_scale, const float* v_inv_freq, int v_rot_dims, int v_rot_half, int settled, int* status, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (head_dim <= 0 || v_dim <= 0 || rot_dims < 0 || rot_dims > head_dim || (rot_dims & 1) || !q_out || (!k_cache && !k_out)) return HB_UNSUPPORTED_SIZE;
     if (!v_inv_freq) v_rot_dims = 0;
@@ -585,7 +588,7 @@ HB_EXPORT int hb_heads_prepare_wide(const float* x, int tokens, int stride, int 
             (((uintptr_t)x | (uintptr_t)q_norm | (uintptr_t)k_norm) & 15) == 0 &&
             (((uintptr_t)q_out | (uintptr_t)k_out | (uintptr_t)k_cache | (uintptr_t)v_cache) & out_mask) == 0) {
 #define HB_UNITS(TO)                                                                                                                                                       \
-    return launch_after_previous(heads_prepare_token_units_kernel<TO>, token_grid, dim3(UNIT_THREADS), 0, stream, x, stride, q_off, k_off, v_off, q_heads, kv_heads, head_dim, \
+    return launch_in_turn(settled != 0, heads_prepare_token_units_kernel<TO>, token_grid, dim3(UNIT_THREADS), 0, stream, x, stride, q_off, k_off, v_off, q_heads, kv_heads, head_dim, \
                                  v_dim, q_norm, k_norm, eps, inv_freq, rot_dims, rot_half, positions, k_scale, (TO*)q_out, q_out_stride, (TO*)k_out, k_out_stride, (TO*)k_cache, \
                                  (TO*)v_cache, (size_t)page_stride, (size_t)head_stride, token_stride, block_table, table_width, token_row, page_size, pages, v_unit_eps,         \
                                  q_head_scale, v_inv_freq, v_rot_dims, v_rot_half, status)
@@ -770,13 +773,13 @@ HB_EXPORT int hb_latent_prepare(const float* x, int tokens, int stride, int q_of
 
 // All bfloat16 and dense but for q_stride; dim, value_dim, rot_dim and rot_dims multiples of 8, value_dim <= dim + rot_dim.
 HB_EXPORT int hb_latent_expand(void* q, int q_stride, int tokens, int heads, int dim, int value_dim, int rot_dim, int rot_dims, const void* kv, const void* part, const float* inv_freq,
-                               const int* positions, const int* token_row, const int* table, int table_width, int page_size, int pages, void* out, int* status, cudaStream_t stream) {
+                               const int* positions, const int* token_row, const int* table, int table_width, int page_size, int pages, void* out, int settled, int* status, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (heads <= 0 || dim <= 0 || ((dim | value_dim | rot_dim | rot_dims | q_stride) & 7) || rot_dims > rot_dim || rot_dims / 2 > MAX_PAIRS || value_dim <= 0 || value_dim > dim + rot_dim ||
         page_size <= 0)
         return HB_UNSUPPORTED_SIZE;
     if ((rot_dims && !inv_freq) || ((((uintptr_t)q) | ((uintptr_t)kv) | ((uintptr_t)part) | ((uintptr_t)out)) & 15)) return HB_BAD_ARGUMENT;
-    return launch_after_previous(latent_expand_kernel, dim3(tokens), dim3(TOKEN_THREADS), 0, stream, (__nv_bfloat16*)q, q_stride, heads, dim, value_dim, rot_dim, rot_dims,
+    return launch_in_turn(settled != 0, latent_expand_kernel, dim3(tokens), dim3(TOKEN_THREADS), 0, stream, (__nv_bfloat16*)q, q_stride, heads, dim, value_dim, rot_dim, rot_dims,
                                  (const __nv_bfloat16*)kv, (const __nv_bfloat16*)part, inv_freq, positions, token_row, table, table_width, page_size, pages, (__nv_bfloat16*)out,
                                  status);
 }

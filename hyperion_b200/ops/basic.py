@@ -207,10 +207,11 @@ def heads_prepare_(x: torch.Tensor, q_heads: int, kv_heads: int, head_dim: int, 
                    q_norm: torch.Tensor | None = None, k_norm: torch.Tensor | None = None, eps: float = 0.0,
                    inv_freq: torch.Tensor | None = None, rot_dims: int = 0, v_first: torch.Tensor | None = None,
                    mix: torch.Tensor | None = None, cache: torch.Tensor | None = None, block_table: torch.Tensor | None = None,
-                   token_row: torch.Tensor | None = None, page_size: int = 0) -> None:
+                   token_row: torch.Tensor | None = None, page_size: int = 0, settled: bool = False) -> None:
     """Rows ``x`` = [q | k | v]: query/key norm per head, rotation of interleaved pairs, value mixing with ``v_first``
     (a view of another layer's value columns) by the scalar ``mix``, queries back in place, keys and values into
-    ``cache`` (either arrangement of :func:`paged_strides`); every step is optional."""
+    ``cache`` (either arrangement of :func:`paged_strides`); every step is optional.  ``settled``: the caller's word that no kernel still in flight writes ``positions``
+    or ``inv_freq``; they are then read while the kernel before still runs."""
     require_cuda(x, positions, q_norm, k_norm, inv_freq, v_first, mix, cache, block_table, token_row)
     if x.stride(-1) != 1 or (v_first is not None and (v_first.stride(-1) != 1 or v_first.dtype != x.dtype)):
         raise KernelError("heads_prepare: rows with unit inner stride")
@@ -230,7 +231,7 @@ def heads_prepare_(x: torch.Tensor, q_heads: int, kv_heads: int, head_dim: int, 
         f32(eps), ptr(inv_freq), i32(rot_dims if inv_freq is not None else 0), ptr(positions), ptr(v_first), i32(v_first.stride(0) if v_first is not None else 0),
         ptr(mix), ptr(cache), v_cache, ctypes.c_longlong(page_stride), ctypes.c_longlong(head_stride), i32(token_stride), ptr(block_table),
         i32(block_table.shape[1] if block_table is not None else 0), ptr(token_row), i32(page_size), i32(pages),
-        i32(1 if (cache is not None or v_first is not None) else 0), ptr(status_word(x.device)), stream_ptr()), "heads_prepare")
+        i32(1 if (cache is not None or v_first is not None) else 0), i32(1 if settled else 0), ptr(status_word(x.device)), stream_ptr()), "heads_prepare")
 
 
 def attention_general(q: torch.Tensor, heads: int, kv_heads: int, head_dim: int, v_dim: int, cache: torch.Tensor, block_table: torch.Tensor,
@@ -292,7 +293,7 @@ def heads_prepare_wide(x: torch.Tensor, q_off: int, k_off: int, v_off: int, q_he
                        rot_dims: int = 0, rot_half: bool = False, k_scale: float = 1.0, cache: torch.Tensor | None = None,
                        block_table: torch.Tensor | None = None, token_row: torch.Tensor | None = None, page_size: int = 0,
                        v_unit_eps: float | None = None, q_head_scale: torch.Tensor | None = None, v_inv_freq: torch.Tensor | None = None,
-                       v_rot_dims: int = 0, v_rot_half: bool = False) -> None:
+                       v_rot_dims: int = 0, v_rot_half: bool = False, settled: bool = False) -> None:
     """Float projections ``x`` [tokens, *] with queries at column ``q_off``, keys at ``k_off``, values at ``v_off``: query/key
     norm (per head with one weight, or over the whole projection with a weight per column), rotation (adjacent pairs, or
     dimension i with i + rot_dims / 2), keys times ``k_scale``; queries to ``q_out`` [tokens, >= q_heads * head_dim], keys and
@@ -300,7 +301,7 @@ def heads_prepare_wide(x: torch.Tensor, q_off: int, k_off: int, v_off: int, q_he
     ``q_out`` and ``k_out`` may be float views of ``x`` itself.  ``v_unit_eps`` (with a cache): every value head is divided by
     sqrt(mean(v^2) + v_unit_eps) before it is stored.  ``q_head_scale`` [q_heads] float: a factor on every query head, after norm and rotation.
     ``v_inv_freq`` (with a cache): every value head is stored turned by its token's position over its first ``v_rot_dims`` entries (pairs as
-    ``v_rot_half`` says, pair i by position * v_inv_freq[i])."""
+    ``v_rot_half`` says, pair i by position * v_inv_freq[i]).  ``settled`` as for :func:`heads_prepare_`, of both sets of frequencies."""
     require_cuda(x, positions, q_out, k_out, q_norm, k_norm, inv_freq, cache, block_table, token_row, q_head_scale, v_inv_freq)
     if v_inv_freq is not None and (v_inv_freq.dtype != torch.float32 or not v_inv_freq.is_contiguous() or v_inv_freq.numel() < v_rot_dims // 2 or cache is None):
         raise KernelError("heads_prepare_wide: the values' frequencies are dense float32, one per rotated pair, and go with a cache")
@@ -327,7 +328,7 @@ def heads_prepare_wide(x: torch.Tensor, q_off: int, k_off: int, v_off: int, q_he
         i32(k_out.stride(0) if k_out is not None else 0), i32(is_bf16(q_out)), ptr(cache), v_cache, ctypes.c_longlong(page_stride),
         ctypes.c_longlong(head_stride), i32(token_stride), ptr(block_table), i32(block_table.shape[1] if block_table is not None else 0),
         ptr(token_row), i32(page_size), i32(pages), f32(-1.0 if v_unit_eps is None else v_unit_eps), ptr(q_head_scale), ptr(v_inv_freq),
-        i32(v_rot_dims if v_inv_freq is not None else 0), i32(1 if v_rot_half else 0), ptr(status_word(x.device)), stream_ptr()),
+        i32(v_rot_dims if v_inv_freq is not None else 0), i32(1 if v_rot_half else 0), i32(1 if settled else 0), ptr(status_word(x.device)), stream_ptr()),
         "heads_prepare_wide")
 
 
@@ -360,10 +361,10 @@ def latent_prepare(x: torch.Tensor, q_off: int, q_rank: int, kv_off: int, kv_ran
 
 
 def latent_expand_(q: torch.Tensor, kv: torch.Tensor, part: torch.Tensor, heads: int, dim: int, value_dim: int, inv_freq: torch.Tensor | None, rot_dims: int, positions: torch.Tensor,
-                   token_row: torch.Tensor, table: torch.Tensor, pages: torch.Tensor) -> None:
+                   token_row: torch.Tensor, table: torch.Tensor, pages: torch.Tensor, settled: bool = False) -> None:
     """``kv`` [tokens, heads * (dim + value_dim)] (every head's unrotated key, then every head's value) and ``part`` [tokens, rot_dim] (the shared, rotated key part) go to ``pages``
     [pages, 2, heads, page_size, dim + rot_dim] as keys [plain | shared] and values [value | zeros], a request's pages in its row of ``table``; the rotated parts of ``q``
-    [tokens, heads * (dim + rot_dim)] are rotated in place.  All bfloat16."""
+    [tokens, heads * (dim + rot_dim)] are rotated in place.  All bfloat16.  ``settled`` as for :func:`heads_prepare_`."""
     require_cuda(q, kv, part, inv_freq, positions, token_row, table, pages)
     tokens, rot_dim = part.shape
     wide = dim + rot_dim
@@ -375,7 +376,7 @@ def latent_expand_(q: torch.Tensor, kv: torch.Tensor, part: torch.Tensor, heads:
         raise KernelError("latent_expand: a dense int32 table of pages, a row per request")
     check(library("heads_prepare").hb_latent_expand(ptr(q), i32(q.stride(0)), i32(tokens), i32(heads), i32(dim), i32(value_dim), i32(rot_dim), i32(rot_dims), ptr(kv), ptr(part),
                                                     ptr(inv_freq), ptr(positions), ptr(token_row), ptr(table), i32(table.shape[1]), i32(pages.shape[3]), i32(pages.shape[0]), ptr(pages),
-                                                    ptr(status_word(q.device)), stream_ptr()), "latent_expand")
+                                                    i32(1 if settled else 0), ptr(status_word(q.device)), stream_ptr()), "latent_expand")
 
 
 def latent_query(q: torch.Tensor, q_lat: torch.Tensor, heads: int, dim: int, rot_dim: int, inv_freq: torch.Tensor | None, rot_dims: int,

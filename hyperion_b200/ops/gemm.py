@@ -75,9 +75,10 @@ def takes_few_rows(x: torch.Tensor, w: torch.Tensor, gated_block: Optional[int] 
     return megabytes <= 13 or (k < 2048 and megabytes <= 20)
 
 
-def few_rows(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, epilogue: int = FEW_BF16, block: int = 0):
+def few_rows(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, epilogue: int = FEW_BF16, block: int = 0, settled: bool = False):
     """``x w^T`` (+ bias) for up to 16 rows (``csrc/few_rows.cu``); :data:`FEW_SWIGLU` over gate and up rows in turn in runs of ``block``; :data:`FEW_PIECES`: a
-    :class:`SplitSum`, its bias still to be added, or the whole sum where one block per tile is enough."""
+    :class:`SplitSum`, its bias still to be added, or the whole sum where one block per tile is enough.
+    ``settled``: the caller's word that no kernel still in flight writes ``w``; the product then fetches it while the kernel before still runs."""
     require_cuda(x, w, bias)
     m, k = x.shape
     n = w.shape[0]
@@ -95,7 +96,7 @@ def few_rows(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = No
     bias_f = given if given is not None and given.dtype == torch.float32 else None
     bias_h = given if given is not None and given.dtype == torch.bfloat16 else None
     check(library("few_rows").hb_few_rows(ptr(x), i32(x.stride(0)), ptr(w), ptr(bias_h), ptr(bias_f), ptr(out), i32(out.stride(-2)), i32(m), i32(n), i32(k), i32(epilogue),
-                                          i32(block), i32(parts), i32(2 * sms), stream_ptr()), "few_rows")
+                                          i32(block), i32(parts), i32(2 * sms), i32(1 if settled else 0), stream_ptr()), "few_rows")
     return SplitSum(out, bias, torch.bfloat16) if epilogue == FEW_PIECES else out
 
 

@@ -10,6 +10,7 @@ keeps float logits (backends/hopper_sm90/session.rs:844-848).
 """
 from __future__ import annotations
 
+import functools
 import os
 from typing import Optional
 
@@ -72,9 +73,12 @@ def _takes_few_rows(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) -> b
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
-           out_dtype: Optional[torch.dtype] = None, may_leave_partials: bool = False):
+           out_dtype: Optional[torch.dtype] = None, may_leave_partials: bool = False, settled: bool = False):
     """``may_leave_partials``: the caller's result has one reader that can add up split-K pieces itself (a residual delta, a gate that
-    the next norm applies), so a product that was split over K may come back as a :class:`hyperion_b200.ops.gemm.SplitSum`."""
+    the next norm applies), so a product that was split over K may come back as a :class:`hyperion_b200.ops.gemm.SplitSum`.
+    ``settled``: the caller's word that no kernel still in flight writes ``weight`` (a model's own matrices, once loaded: :func:`project`); a small product then fetches it while
+    the kernel before still runs.  The tcgen05 kernels of ``ops/gemm.py`` do so in any case: a matrix that a kernel of this package has just written goes to them behind
+    a synchronisation, or behind any launch that waits for the kernel before."""
     require_cuda(x, weight, bias)
     out_dtype = out_dtype or x.dtype
     if weight.dtype == torch.float32:
@@ -86,7 +90,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         raise KernelError(f"linear: weights are float32 or bfloat16, got {weight.dtype}")
     xin = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
     if _takes_few_rows(xin, weight, bias, out_dtype):
-        return gemm.few_rows(xin, weight, bias, gemm.FEW_F32 if out_dtype == torch.float32 else gemm.FEW_PIECES if may_leave_partials else gemm.FEW_BF16)
+        return gemm.few_rows(xin, weight, bias, gemm.FEW_F32 if out_dtype == torch.float32 else gemm.FEW_PIECES if may_leave_partials else gemm.FEW_BF16, settled=settled)
     if _takes_own_kernel(xin, weight, bias, out_dtype):
         epilogue = gemm.EPI_F32 if out_dtype == torch.float32 else gemm.EPI_BF16
         if xin.shape[0] > gemm.PAIR_MIN_ROWS:  # only under HYPERION_B200_GEMM=own: prompt-sized products on pairs of SMs
@@ -103,6 +107,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return y if out_dtype == torch.float32 else y.to(out_dtype)
 
 
+# linear() with a model's own matrix: what the parts call.
+project = functools.partial(linear, settled=True)
+
+
 def fuses_swiglu(m: int, k: int) -> bool:
     """Whether gate+up of ``m`` rows goes to the pair kernel with SwiGLU in its epilogue: from 512 rows on, when the rows
     fill their 256-row tiles to 85 % (measured at the 1.5B, 7B and 32B widths: 1.04 to 1.19 times the library's product
@@ -114,11 +122,11 @@ def fuses_swiglu(m: int, k: int) -> bool:
     return m >= 512 and m >= 0.85 * tiles * 256
 
 
-def gated_linear(x: torch.Tensor, weight: torch.Tensor, block: Optional[int], out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+def gated_linear(x: torch.Tensor, weight: torch.Tensor, block: Optional[int], out_dtype: Optional[torch.dtype] = None, settled: bool = False) -> torch.Tensor:
     """silu(x Wg^T) * (x Wu^T) for a fused gate/up matrix ``weight`` [2I, H].  ``block`` None: the gate rows come first, then
     the up rows.  ``block`` = 128: rows alternate in runs of 128 gate rows and their 128 up rows
     (``ops.gemm.interleave_gate_up``), which lets a prompt-sized product apply SwiGLU in the epilogue of the pair kernel, so
-    that the [tokens, 2I] projections never travel to memory and back."""
+    that the [tokens, 2I] projections never travel to memory and back.  ``settled`` as for :func:`linear`."""
     from .basic import swiglu
 
     out_dtype = out_dtype or x.dtype
@@ -127,8 +135,8 @@ def gated_linear(x: torch.Tensor, weight: torch.Tensor, block: Optional[int], ou
         return gemm.gemm_pair_bf16(x, weight, None, gemm.EPI_SWIGLU)
     if (x.shape[0] <= gemm.FEW_ROWS and weight.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and x.dtype == torch.bfloat16 and gemm_policy() == "auto"
             and gemm.takes_few_rows(x, weight, block or weight.shape[0] // 2)):
-        return gemm.few_rows(x, weight, None, gemm.FEW_SWIGLU, block or weight.shape[0] // 2)
-    return swiglu(linear(x, weight, None, out_dtype), block=block)
+        return gemm.few_rows(x, weight, None, gemm.FEW_SWIGLU, block or weight.shape[0] // 2, settled)
+    return swiglu(linear(x, weight, None, out_dtype, settled=settled), block=block)
 
 
 def fuses_relu_squared(m: int) -> bool:
@@ -138,11 +146,11 @@ def fuses_relu_squared(m: int) -> bool:
     return gemm_policy() != "library" and m >= 2048 and m >= 0.85 * 256 * -(-m // 256)
 
 
-def relu_squared_linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """max(x W^T, 0)^2: in the product's epilogue at prompt sizes, else by a kernel behind it that also adds up split-K pieces."""
+def relu_squared_linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None, settled: bool = False) -> torch.Tensor:
+    """max(x W^T, 0)^2: in the product's epilogue at prompt sizes, else by a kernel behind it that also adds up split-K pieces.  ``settled`` as for :func:`linear`."""
     from .basic import relu_squared
 
     out_dtype = out_dtype or x.dtype
     if weight.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and x.dtype == torch.bfloat16 and gemm.supported(x, weight) and fuses_relu_squared(x.shape[0]):
         return gemm.gemm_pair_bf16(x, weight, None, gemm.EPI_RELU_SQUARED)
-    return relu_squared(linear(x, weight, None, out_dtype, may_leave_partials=True))
+    return relu_squared(linear(x, weight, None, out_dtype, may_leave_partials=True, settled=settled))

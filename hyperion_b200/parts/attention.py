@@ -92,7 +92,7 @@ class GroupedQueryAttention(Mixer):
     def forward(self, x, step, cache, own_cache):
         if cache is None:
             raise ValueError("attention needs a paged cache; the schedule gave it none")
-        qkv = ops.linear(x, self.w_qkv, self.b_qkv, self.dtype)
+        qkv = ops.project(x, self.w_qkv, self.b_qkv, self.dtype)
         stores = own_cache and not self.shares_kv
         if self.position is not None and stores:
             self.position.apply_and_store_(qkv, self.heads, self.kv_heads, self.head_dim, step.positions, cache, step.token_row)
@@ -105,7 +105,7 @@ class GroupedQueryAttention(Mixer):
             attn = self._attend_fast(qkv, step, cache)
         else:
             attn = ops.attention_generic(qkv, self.heads, cache.kv, cache.block_table, step.token_row, step.positions, self.scale, self.window)
-        return ops.linear(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
     # ------------------------------------------------------------------ the tensor-core path
     def step_plans(self):

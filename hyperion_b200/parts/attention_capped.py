@@ -114,7 +114,7 @@ class CappedAttention(GroupedQueryAttention):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("this attention writes a paged cache of its own; the schedule gave it none")
-        qkv = ops.linear(x, self.w_qkv, None, self.dtype)
+        qkv = ops.project(x, self.w_qkv, None, self.dtype)
         v_first = None
         if self.v_mix is not None:
             key = ("v_mix", self.v_mix)
@@ -127,13 +127,13 @@ class CappedAttention(GroupedQueryAttention):
                            eps=self.eps, inv_freq=self.position.inv_freq if self.position is not None else None,
                            rot_dims=self.position.dims if self.position is not None else 0, v_first=v_first,
                            mix=self.mix if v_first is not None else None, cache=cache.kv, block_table=cache.block_table,
-                           token_row=step.token_row, page_size=cache.page_size)
+                           token_row=step.token_row, page_size=cache.page_size, settled=True)
         if self.fast:
             attn = self._attend_fast(qkv, step, cache)
         else:
             attn = ops.attention_general(qkv, self.heads, self.kv_heads, self.head_dim, self.value_dim, cache.kv, cache.block_table, step.token_row,
                                          step.positions, cache.page_size, self.scale, self.softcap, self.window)
-        return ops.linear(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_mixer("capped_attention", CappedAttention)

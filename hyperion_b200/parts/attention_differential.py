@@ -116,7 +116,7 @@ class DifferentialAttention(Mixer):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("this attention writes a paged cache of its own; the schedule gave it none")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         k_off = self.q_width
         v_off = k_off + self.k_width
         q = torch.empty((x.shape[0], self.q_width), dtype=self.dtype, device=x.device)
@@ -130,7 +130,7 @@ class DifferentialAttention(Mixer):
             maps = ops.attention_general(q, self.heads, self.kv_heads, self.head_dim, self.value_dim, cache.kv, cache.block_table, step.token_row, step.positions,
                                          cache.page_size, self.scale, 0.0, self.window, keep_first=self.keep_first, maps=2, wide_out=True)
             fast_attention.differential_combine(maps, None, None, x.shape[0], self.heads, 1, self.value_dim, self.map_weight, self.eps, 1.0 - self.diff, gate, out)
-        return ops.linear(out, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(out, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_mixer("differential_attention", DifferentialAttention)

@@ -139,11 +139,12 @@ class LatentAttention(Mixer):
         key = self._expanded_key()
         pages, n_tiles = step.host[key]
         tokens = cq.shape[0]
-        q = ops.linear(cq, self.w_uq, None, self.dtype)
-        kv = ops.linear(latent, self.w_kv, None, self.dtype)
+        q = ops.project(cq, self.w_uq, None, self.dtype)
+        kv = ops.project(latent, self.w_kv, None, self.dtype)
         storage = torch.empty((pages, 2, self.heads, EXPANDED_PAGE, self.q_head), dtype=self.dtype, device=cq.device)
         table = step.extra[f"{key}_table"]
-        ops.latent_expand_(q, kv, part, self.heads, self.head_dim, self.value_dim, inv_freq, self.rot_dims, step.positions, step.token_row, table, storage)
+        ops.latent_expand_(q, kv, part, self.heads, self.head_dim, self.value_dim, inv_freq, self.rot_dims, step.positions, step.token_row, table, storage,
+                           settled=True)
         out = torch.empty((tokens, self.heads * self.value_dim), dtype=self.dtype, device=cq.device)
         fast_attention.attention_wide_keys(q, self.heads, storage, table, step.token_row, step.positions, step.extra[f"{key}_tiles"], n_tiles, self.scale, out, sinks=self.sink)
         return out
@@ -159,15 +160,15 @@ class LatentAttention(Mixer):
             raise ValueError("this attention writes a paged cache of its own; the schedule gave it none")
         tokens = x.shape[0]
         inv_freq = self.position.inv_freq if self.position is not None else None
-        proj = ops.linear(x, self.w_down, None, torch.float32)
+        proj = ops.project(x, self.w_down, None, torch.float32)
         expands = self.expands_fresh_prompts and self._expanded_key() in step.host
         latent = torch.empty((tokens, self.kv_rank), dtype=self.dtype, device=x.device) if expands else None
         part = torch.empty((tokens, self.rot_dim), dtype=self.dtype, device=x.device) if expands else None
         cq = ops.latent_prepare(proj, 0, self.q_rank, self.q_rank, self.kv_rank, self.rot_dim, self.q_norm, self.kv_norm, self.eps, inv_freq, self.rot_dims,
                                 step.positions, self.dtype, cache.kv, cache.block_table, step.token_row, cache.page_size, latent, part)
         if expands:
-            return ops.linear(self._attend_expanded(cq, latent, part, step, inv_freq), self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
-        q = ops.linear(cq, self.w_uq, None, self.dtype)
+            return ops.project(self._attend_expanded(cq, latent, part, step, inv_freq), self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        q = ops.project(cq, self.w_uq, None, self.dtype)
         plain = q.view(tokens, self.heads, self.q_head)[:, :, : self.head_dim].transpose(0, 1)
         q_lat = self._batched(plain, self.k_heads.to(q.dtype) if self.k_heads.dtype != q.dtype else self.k_heads, torch.float32)
         query = ops.latent_query(q, q_lat, self.heads, self.head_dim, self.rot_dim, inv_freq, self.rot_dims, step.positions)
@@ -182,7 +183,7 @@ class LatentAttention(Mixer):
         core = torch.empty((tokens, self.heads, self.value_dim), dtype=self.dtype, device=x.device)
         v_heads = self.v_heads.to(attn.dtype) if self.v_heads.dtype != attn.dtype else self.v_heads
         torch.bmm(attn.view(tokens, self.heads, self.kv_rank).transpose(0, 1), v_heads, out=core.transpose(0, 1))
-        return ops.linear(core.view(tokens, self.heads * self.value_dim), self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(core.view(tokens, self.heads * self.value_dim), self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_mixer("latent_attention", LatentAttention)

@@ -110,7 +110,7 @@ class RotatedValueAttention(GroupedQueryAttention):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("this attention writes a paged cache of its own; the schedule gave it none")
-        proj = ops.linear(x, self.w_qkv, self.b_qkv, torch.float32)
+        proj = ops.project(x, self.w_qkv, self.b_qkv, torch.float32)
         k_off, v_off = self.q_width, self.q_width + self.k_width
         q = torch.empty((x.shape[0], self.q_width), dtype=self.dtype, device=x.device)
         part, turned = self.position, self.value_position
@@ -118,7 +118,7 @@ class RotatedValueAttention(GroupedQueryAttention):
                                inv_freq=part.inv_freq if part is not None else None, rot_dims=part.dims if part is not None else 0,
                                rot_half=bool(getattr(part, "half", False)), cache=cache.kv, block_table=cache.block_table, token_row=step.token_row,
                                page_size=cache.page_size, v_inv_freq=turned.inv_freq if turned is not None else None,  # a value is cached turned by its own position
-                               v_rot_dims=turned.dims if turned is not None else 0, v_rot_half=bool(getattr(turned, "half", False)))
+                               v_rot_dims=turned.dims if turned is not None else 0, v_rot_half=bool(getattr(turned, "half", False)), settled=True)
         if self.fast:
             attn = self._attend_fast(q, step, cache)
         else:
@@ -126,7 +126,7 @@ class RotatedValueAttention(GroupedQueryAttention):
                                          step.positions, cache.page_size, self.scale, 0.0, self.window)
         if self.value_position is not None:  # the sum of a head's values is turned back by the query's position
             self._turn_values(attn, 0, self.heads, step.positions, -1.0)
-        return ops.linear(attn, self.w_o, self.b_o, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(attn, self.w_o, self.b_o, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_mixer("rotated_value_attention", RotatedValueAttention)

@@ -111,7 +111,7 @@ class SinkAttention(GroupedQueryAttention):
     def forward(self, x, step, cache, own_cache):
         if cache is None or own_cache == self.shares_kv:
             raise ValueError("this attention writes a cache of its own or reads the one its schedule entry names; the schedule gave it another")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         k_off = self.q_width
         v_off = k_off + self.k_width
         q = torch.empty((x.shape[0], self.q_width), dtype=self.dtype, device=x.device)
@@ -123,7 +123,7 @@ class SinkAttention(GroupedQueryAttention):
         else:
             attn = ops.attention_general(q, self.heads, self.kv_heads, self.head_dim, self.value_dim, cache.kv, cache.block_table, step.token_row, step.positions,
                                          cache.page_size, self.scale, 0.0, self.window, sinks=self.sink, gate=gate, gate_per_head=True)
-        return ops.linear(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_mixer("sink_attention", SinkAttention)

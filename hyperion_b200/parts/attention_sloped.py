@@ -111,18 +111,18 @@ class SlopedAttention(Mixer):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("this attention writes a paged cache of its own; the schedule gave it none")
-        proj = ops.linear(x, self.w_qkv, None, torch.float32)
+        proj = ops.project(x, self.w_qkv, None, torch.float32)
         q = torch.empty((x.shape[0], self.q_width), dtype=self.dtype, device=x.device)
         fast = self.fast and fast_attention.takes_distance_bias(self.head_dim, cache.page_size)
         ops.heads_prepare_wide(proj, 0, self.q_width, self.q_width + self.k_width, self.heads, self.kv_heads, self.head_dim, self.value_dim, step.positions,
                                q_out=q, cache=cache.kv, block_table=cache.block_table, token_row=step.token_row, page_size=cache.page_size,
-                               v_unit_eps=self.eps if self.value_unit_rms else None, q_head_scale=self.temp if fast else None)
+                               v_unit_eps=self.eps if self.value_unit_rms else None, q_head_scale=self.temp if fast else None, settled=True)
         if fast:
             attn = self._attend_fast(q, step, cache, bias=self.by_distance_log2, bias_per_position=self.per_position_log2)
-            return ops.linear(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+            return ops.project(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
         attn = ops.attention_general(q, self.heads, self.kv_heads, self.head_dim, self.value_dim, cache.kv, cache.block_table, step.token_row, step.positions,
                                      cache.page_size, self.scale, head_scale=self.temp, slopes=self.slopes, chunk=self.chunk)
-        return ops.linear(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(attn, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_mixer("sloped_attention", SlopedAttention)

@@ -44,7 +44,7 @@ class Branch(Mixer):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError(f"{type(self).__name__} keeps something per request; the schedule gave it none")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         out = torch.empty((x.shape[0], self.core_width), dtype=self.dtype, device=x.device)
         self.core(proj, 0, step, cache, out, 1.0)
-        return ops.linear(out, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(out, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta

@@ -90,7 +90,7 @@ class LinearHead(Head):
         return [("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})] + ([("elementwise", {})] if self.scale != 1.0 or self.softcap else [])
 
     def forward(self, x):
-        logits = ops.linear(x, self.weight, None, torch.float32)
+        logits = ops.project(x, self.weight, None, torch.float32)
         if self.scale != 1.0:
             ops.scale_(logits, self.scale)
         return ops.soft_cap_(logits, self.softcap) if self.softcap else logits

@@ -154,7 +154,7 @@ class ScoredExperts(FeedForward):
         if self.shared is not None:
             base = self.shared.forward(x, step)
             base = base.tensor() if hasattr(base, "tensor") else base
-            gate = ops.linear(x, self.w_shared_gate, None, torch.float32).reshape(-1)
+            gate = ops.project(x, self.w_shared_gate, None, torch.float32).reshape(-1)
         return moe.combine_weighted(y, where, weights, x, base, gate)
 
 

@@ -54,8 +54,8 @@ class SwiGLU(FeedForward):
         return [("elementwise", {}), ("gemm_tcgen05", {}), ("gemm_pair_tcgen05", {})]
 
     def forward(self, x, step):
-        act = ops.gated_linear(x, self.w_gate_up, self.block, self.dtype)
-        return ops.linear(act, self.w_down, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        act = ops.gated_linear(x, self.w_gate_up, self.block, self.dtype, settled=True)
+        return ops.project(act, self.w_down, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_feed_forward("swiglu", SwiGLU)
@@ -92,10 +92,10 @@ class ActivatedMLP(FeedForward):
     def forward(self, x, step):
         operation = getattr(ops, self.ACTIVATIONS[self.activation])
         if self.activation == "relu_squared":
-            act = operation(x, self.w_up, self.dtype)
+            act = operation(x, self.w_up, self.dtype, settled=True)
         else:
-            act = operation(ops.linear(x, self.w_up, None, self.dtype))
-        return ops.linear(act, self.w_down, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+            act = operation(ops.project(x, self.w_up, None, self.dtype))
+        return ops.project(act, self.w_down, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_feed_forward("activated_mlp", ActivatedMLP)
@@ -130,8 +130,8 @@ class ClampedGLU(FeedForward):
         return [("elementwise", {}), ("sgemm_f32", {}) if self.dtype == torch.float32 else ("gemm_tcgen05", {})]
 
     def forward(self, x, step):
-        act = ops.clamped_glu(ops.linear(x, self.w_gate_up, None, self.dtype), self.limit, self.slope)
-        return ops.linear(act, self.w_down, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        act = ops.clamped_glu(ops.project(x, self.w_gate_up, None, self.dtype), self.limit, self.slope)
+        return ops.project(act, self.w_down, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_feed_forward("clamped_glu", ClampedGLU)

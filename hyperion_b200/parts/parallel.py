@@ -126,7 +126,7 @@ class BiasedAttention(Branch):
         v_off = k_off + self.k_width
         ops.heads_prepare_wide(proj, col0, k_off, v_off, self.heads, self.kv_heads, self.head_dim, self.value_dim, step.positions, q_out=q,
                                q_norm=self.q_norm, k_norm=self.k_norm, norm_whole=True, eps=self.eps, cache=cache.kv, block_table=cache.block_table,
-                               token_row=step.token_row, page_size=cache.page_size)
+                               token_row=step.token_row, page_size=cache.page_size, settled=True)
         if self.fast and fast_attention.takes_distance_bias(self.head_dim, cache.page_size):
             # the tensor-core kernels store rows in 16-byte pieces: columns of a wider buffer whose rows do not start on such a piece
             # are filled through a buffer of their own
@@ -184,7 +184,8 @@ class Retention(Branch, ConstantDecay):
         k_off, v_off = col0 + self.qk_width, col0 + 2 * self.qk_width
         ops.heads_prepare_wide(proj, col0, k_off, v_off, self.heads, self.heads, self.n, self.e, step.positions, q_out=proj[:, col0:k_off],
                                k_out=proj[:, k_off:v_off], inv_freq=self.position.inv_freq if self.position is not None else None,
-                               rot_dims=self.position.dims if self.position is not None else 0, rot_half=True, k_scale=self.n ** -0.5)
+                               rot_dims=self.position.dims if self.position is not None else 0, rot_half=True, k_scale=self.n ** -0.5,
+                               settled=True)
         o = self._retain(proj, k_off, col0, v_off, cache, step)
         recurrent.gated_group_norm(o, proj, v_off + self.core_width, None, self.e, False, self.eps, self.dtype, scale=scale, out=out)
 
@@ -238,14 +239,14 @@ class ParallelMixers(Mixer):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache or len(cache) != len(self.branches):
             raise ValueError("parallel mixers keep what their branches keep; the schedule gave them something else")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         out = torch.empty((x.shape[0], self.core_width), dtype=self.dtype, device=x.device)
         col = at = 0
         for branch, scale, view in zip(self.branches, self.scales, cache):
             branch.core(proj, col, step, view, out[:, at : at + branch.core_width], scale)
             col += branch.in_width
             at += branch.core_width
-        return ops.linear(out, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(out, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 class ParallelNormedMixers(Mixer):
@@ -312,7 +313,7 @@ class ParallelNormedMixers(Mixer):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache or len(cache) != len(self.branches):
             raise ValueError("parallel mixers keep what their branches keep; the schedule gave them something else")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         # The second branch runs on a stream of its own, from the input product to its own output product, beside the first: a decode step is a chain of small kernels
         # that leave most of the GPU idle (7 % of a step at batch 8), and a prompt's recurrence has phases that do.  Results do not depend on it.
         beside = self._side_stream() if len(self.branches) == 2 else None
@@ -331,7 +332,7 @@ class ParallelNormedMixers(Mixer):
         branch = self.branches[index]
         out = torch.empty((x.shape[0], branch.core_width), dtype=self.dtype, device=x.device)
         branch.core(proj, self.columns[index], step, view, out, 1.0)
-        return ops.linear(out, self.w_out[index], None, self.dtype, may_leave_partials=True)
+        return ops.project(out, self.w_out[index], None, self.dtype, may_leave_partials=True)
 
     def _side_stream(self) -> torch.cuda.Stream:
         key = ("side_stream", str(self.device))

@@ -200,7 +200,7 @@ class GatedDeltaRule(_ScanMixer, ChunkedRule):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("the delta rule keeps a state per request; the schedule gave it none")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         state, slots, rows = cache.state, cache.slots, step.n_rows
         conv = recurrent.causal_conv_silu(proj, 0, self.w_conv, None, state, self.conv_off, slots, step.token_row, step.row_start)
         recurrent.conv_state_update(proj, 0, self.conv_channels, self.taps, state, self.conv_off, slots, step.row_start, rows)
@@ -210,7 +210,7 @@ class GatedDeltaRule(_ScanMixer, ChunkedRule):
                                                                None, state, 0, slots, step.row_start, rows, self.heads, self.groups, self.n, self.n_padded, self.e,
                                                                q_scale=self.n ** -0.5, below=below, out=out))
         y = recurrent.gated_group_norm(o, proj, self.gate_off, self.norm, self.e, False, self.eps, self.dtype)
-        return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 class StateSpaceMixer(_ScanMixer, Branch):
@@ -365,12 +365,12 @@ class SelectiveScanMixer(Mixer):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("the selective scan keeps a state per request; the schedule gave it none")
-        proj = ops.linear(x, self.w_in, None, torch.float32)  # [x | z]
+        proj = ops.project(x, self.w_in, None, torch.float32)  # [x | z]
         state, slots, rows = cache.state, cache.slots, step.n_rows
         conv = recurrent.causal_conv_silu(proj, 0, self.w_conv, self.b_conv, state, self.conv_off, slots, step.token_row, step.row_start)
         recurrent.conv_state_update(proj, 0, self.inner, self.taps, state, self.conv_off, slots, step.row_start, rows)
-        dbc = ops.linear(conv, self.w_x, None, torch.float32)  # [d | B | C]
-        dt = ops.linear(dbc[:, : self.rank], self.w_dt, self.b_dt, torch.float32)
+        dbc = ops.project(conv, self.w_x, None, torch.float32)  # [d | B | C]
+        dt = ops.project(dbc[:, : self.rank], self.w_dt, self.b_dt, torch.float32)
         # segments pay while one pass leaves the GPU mostly idle (measured on a B200 with a state of 16: 128 blocks 474 -> 298 us for
         # 2,048 tokens, 256 blocks 524 -> 538 us)
         segments = step.host.get("scan_segments", 0) if self.dtype == torch.bfloat16 and -(-self.inner // 32) <= 200 else 0
@@ -380,7 +380,7 @@ class SelectiveScanMixer(Mixer):
         else:
             y = recurrent.selective_scan(conv, dt, dbc, self.rank, self.rank + self.n, self.a, self.skip, proj, self.inner, state, 0, slots,
                                          step.row_start, rows, self.n, self.n_padded, self.dtype, precise=self.dtype == torch.float32)
-        return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 class WkvMixer(Mixer, ChunkedRule):
@@ -431,14 +431,14 @@ class WkvMixer(Mixer, ChunkedRule):
         state, slots, rows = cache.state, cache.slots, step.n_rows
         mixed = recurrent.token_shift_mix(x, self.mu, state, self.shift_off, slots, step.token_row, step.row_start)
         recurrent.token_shift_keep(x, state, self.shift_off, slots, step.row_start, rows)
-        r, k, v, gate = (ops.linear(mixed[i], w, None, torch.float32) for i, w in enumerate(self.w_in))
-        inner = recurrent.tanh_rows(ops.linear(mixed[4], self.w_1, None, torch.float32), self.dtype)
-        decay_in = ops.linear(inner, self.w_2, None, torch.float32)
+        r, k, v, gate = (ops.project(mixed[i], w, None, torch.float32) for i, w in enumerate(self.w_in))
+        inner = recurrent.tanh_rows(ops.project(mixed[4], self.w_1, None, torch.float32), self.dtype)
+        decay_in = ops.project(inner, self.w_2, None, torch.float32)
         o = self._walk(recurrent.RULE_WKV, k, r, v, decay_in, 0, None, 0, self.w0, self.bonus, cache, step, self.heads, 1.0,
                        lambda below, out: recurrent.wkv_scan(k, r, v, decay_in, 0, self.w0, self.bonus, state, 0, slots, step.row_start, rows, self.heads, self.n, self.n_padded,
                                                              self.n, below=below, out=out))
         y = recurrent.gated_group_norm(o, gate, 0, self.norm, self.n, False, self.eps, self.dtype)
-        return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 class ChannelDeltaRule(_ScanMixer, ChunkedRule):
@@ -488,19 +488,19 @@ class ChannelDeltaRule(_ScanMixer, ChunkedRule):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("the delta rule keeps a state per request; the schedule gave it none")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         state, slots, rows = cache.state, cache.slots, step.n_rows
         conv = recurrent.causal_conv_silu(proj, 0, self.w_conv, None, state, self.conv_off, slots, step.token_row, step.row_start)
         recurrent.conv_state_update(proj, 0, self.conv_channels, self.taps, state, self.conv_off, slots, step.row_start, rows)
-        decay = ops.linear(proj[:, self.a1_off : self.a1_off + self.decay_rank], self.w_a2, None, torch.float32)
-        gate = ops.linear(proj[:, self.g1_off : self.g1_off + self.gate_rank], self.w_g2, None, torch.float32)
+        decay = ops.project(proj[:, self.a1_off : self.a1_off + self.decay_rank], self.w_a2, None, torch.float32)
+        gate = ops.project(proj[:, self.g1_off : self.g1_off + self.gate_rank], self.w_g2, None, torch.float32)
         o = self._walk(recurrent.RULE_CHANNEL_DELTA, conv[:, self.qk_width :], conv, conv[:, 2 * self.qk_width :], decay, 0, proj, self.beta_off, self.a_log, self.dt_bias, cache,
                        step, self.groups, self.n ** -0.5,
                        lambda below, out: recurrent.channel_delta_scan(conv, self.qk_width, 0, 2 * self.qk_width, decay, proj, self.beta_off, self.a_log, self.dt_bias, state, 0, slots,
                                                                        step.row_start, rows, self.heads, self.groups, self.n, self.n_padded, self.e, q_scale=self.n ** -0.5,
                                                                        below=below, out=out))
         y = recurrent.gated_group_norm(o, gate, 0, self.norm, self.e, False, self.eps, self.dtype, sigmoid_gate=True)
-        return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 class LightningAttention(Mixer, ConstantDecay):
@@ -543,12 +543,12 @@ class LightningAttention(Mixer, ConstantDecay):
     def forward(self, x, step, cache, own_cache):
         if cache is None or not own_cache:
             raise ValueError("lightning attention keeps a state per request; the schedule gave it none")
-        proj = ops.linear(x, self.w_in, None, torch.float32)
+        proj = ops.project(x, self.w_in, None, torch.float32)
         k_off, v_off = self.qk_width, 2 * self.qk_width
         recurrent.silu_columns_(proj, 0, v_off + self.v_width)
         o = self._retain(proj, k_off, 0, v_off, cache, step)
         y = recurrent.gated_group_norm(o, proj, v_off + self.v_width, self.norm, self.v_width, False, self.eps, self.dtype, sigmoid_gate=True)
-        return ops.linear(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
+        return ops.project(y, self.w_o, None, self.dtype, may_leave_partials=True)  # the result is a residual delta
 
 
 register_mixer("channel_delta", ChannelDeltaRule)

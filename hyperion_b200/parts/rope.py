@@ -83,7 +83,7 @@ class InterleavedRotaryEncoding(PositionEncoding):
     def apply_(self, x, heads, head_dim, positions):
         if head_dim < self.dims:
             raise ValueError(f"rotary encoding of {self.dims} dimensions, used with heads of {head_dim}")
-        ops.heads_prepare_(x, heads, 0, head_dim, head_dim, positions, inv_freq=self.inv_freq, rot_dims=self.dims)
+        ops.heads_prepare_(x, heads, 0, head_dim, head_dim, positions, inv_freq=self.inv_freq, rot_dims=self.dims, settled=True)  # positions come with the step's copy from the host
 
 
 register_position("rope_interleaved", InterleavedRotaryEncoding)
@@ -103,7 +103,7 @@ class PartialHalfRotaryEncoding(InterleavedRotaryEncoding):
             raise ValueError("this rotation works on float rows")
         width = heads * head_dim
         ops.heads_prepare_wide(x, 0, 0, 0, heads, 0, head_dim, head_dim, positions, q_out=x[:, :width], k_out=x[:, :width], inv_freq=self.inv_freq,
-                               rot_dims=self.dims, rot_half=True)
+                               rot_dims=self.dims, rot_half=True, settled=True)
 
 
 register_position("rope_half_partial", PartialHalfRotaryEncoding)

@@ -93,7 +93,7 @@ def _gate_weights(part) -> dict[str, WeightSpec]:
 def _gated(part, x: torch.Tensor, y) -> GatedResult:
     """The inner part's result with the gate's pre-activations beside it: the norm that reads the result applies the gate in its own
     launch; any other reader multiplies when it asks for the tensor."""
-    return GatedResult(y, ops.linear(x, part.w_gate, None, torch.float32, may_leave_partials=True), part.b_gate)
+    return GatedResult(y, ops.project(x, part.w_gate, None, torch.float32, may_leave_partials=True), part.b_gate)
 
 
 class GatedMixer(_Wrapper, Mixer):
