@@ -27,37 +27,46 @@
 
 namespace {
 constexpr int ROUTE_MOST_SHARED = 200 * 1024;  // always allowed in full: another thread's call may come between a call's allowance and its launch
-// a block has a warp for every AT_ONCE experts, as far as that goes; eight tokens' sums leave two blocks of nine warps to an SM
-__host__ __device__ constexpr int route_most_threads(int tokens_of_block) { return tokens_of_block == 8 ? 288 : 512; }
-__host__ __device__ constexpr int route_at_once(int tokens_of_block) { return tokens_of_block == 1 ? 1 : 2; }
+
+// How a router's work is cut: tokens of a block, experts that a warp takes at a time, steps of its loop over the columns that are under way together, and the block's threads at
+// the most (a warp for every AT_ONCE experts, as far as that goes) and blocks on an SM that its registers leave room for.
+template <int TOKENS_, int AT_ONCE_, int UNROLL_, int THREADS_, int BLOCKS_>
+struct RouteCut {
+    static constexpr int TOKENS = TOKENS_, AT_ONCE = AT_ONCE_, UNROLL = UNROLL_, THREADS = THREADS_, BLOCKS = BLOCKS_;
+};
+typedef RouteCut<1, 1, 8, 512, 1> RouteEach;      // one token's latency: a warp per expert, all of a row's pieces asked for at once
+typedef RouteCut<1, 2, 4, 256, 1> RouteEachPair;  // several such blocks on an SM
+typedef RouteCut<4, 2, 4, 256, 1> RouteFour;
+typedef RouteCut<4, 2, 2, 512, 1> RouteFourWide;  // one block on an SM
+typedef RouteCut<8, 2, 2, 288, 2> RouteEight;
 
 // A block serves TOKENS tokens, their rows in shared memory as floats; a warp takes several experts at a time, so that what it reads of the rows serves
 // them all and what it reads of the router's matrix serves all the block's tokens.  A lane adds up every 32nd group of four columns in four chains of its
 // own (columns beyond a multiple of four go to the first chain), the chains are added in a fixed order and the lanes meet in a butterfly: a logit depends
-// on nothing but the row and the expert's weights, whatever TOKENS is.
-// With a token a block, a prompt is bound by the matrix coming from L2 once per token; with eight, two experts a warp, by what it reads of the rows in
-// shared memory and by too few warps (2,048 tokens of 2,048 columns, 18 outputs: 43.0 -> 20.8 us).  Steps of few tokens, which are one block's latency, take a token a
-// block and a warp per expert, all of a row's pieces asked for at once.
-template <typename T, int TOKENS>
+// on nothing but the row and the expert's weights, however the work is cut.
+// With a token a block, a prompt is bound by the matrix coming from L2 once per token; with several, by what it reads of the rows in shared memory and by too few warps
+// (which cut serves which step: route_cut below).
+template <typename T, typename Cut>
 __device__ __forceinline__ void router_logits(const T* __restrict__ x, int x_stride, const float* __restrict__ router, const float* __restrict__ bias, int first, int count,
                                               int hidden, int experts, float* rows, float* logits) {
-    constexpr int AT_ONCE = route_at_once(TOKENS), UNROLL = TOKENS == 1 ? 8 : 2;
+    constexpr int TOKENS = Cut::TOKENS, AT_ONCE = Cut::AT_ONCE, UNROLL = Cut::UNROLL;
     const int threads = blockDim.x;
     const int padded = (hidden + 3) & ~3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool rows_by_four = (hidden & 3) == 0 && (x_stride & 3) == 0 && (((uintptr_t)x) & (4 * sizeof(T) - 1)) == 0;
     if (rows_by_four) {
-        const int quads = hidden >> 2, all = TOKENS * quads;
-        for (int base = threadIdx.x; base < all; base += 4 * threads) {  // four pieces are asked for before the first is used
-            float v[4][4];
+        constexpr int ASKED = TOKENS == 1 ? 4 : TOKENS;  // pieces asked for before the first is used: four of a row, or the same piece of every row
+        const int quads = hidden >> 2;
+        for (int base = threadIdx.x; base < quads; base += (TOKENS == 1 ? ASKED : 1) * threads) {
+            float v[ASKED][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int piece = base + u * threads;
-                if (piece < all) load4(x + (size_t)(first + min(TOKENS == 1 ? 0 : piece / quads, count - 1)) * x_stride + (TOKENS == 1 ? piece : piece % quads) * 4, v[u]);
+            for (int u = 0; u < ASKED; ++u) {
+                const int piece = TOKENS == 1 ? base + u * threads : base;
+                if (piece < quads) load4(x + (size_t)(first + (TOKENS == 1 ? 0 : min(u, count - 1))) * x_stride + piece * 4, v[u]);
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int piece = base + u * threads;
-                if (piece < all) store4(rows + (size_t)piece * 4, v[u]);  // padded is hidden here
+            for (int u = 0; u < ASKED; ++u) {
+                const int piece = TOKENS == 1 ? base + u * threads : base;
+                if (piece < quads) store4(rows + (TOKENS == 1 ? 0 : (size_t)u * padded) + (size_t)piece * 4, v[u]);
             }
         }
     } else {
@@ -126,15 +135,16 @@ __device__ __forceinline__ void warp_best(float& value, int& index) {
 }
 
 // After the logits, warp j searches and weighs token j.
-template <typename T, int TOKENS>
-__global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 1) moe_route_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router, int tokens, int hidden,
+template <typename T, typename Cut>
+__global__ void __launch_bounds__(Cut::THREADS, Cut::BLOCKS) moe_route_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router, int tokens, int hidden,
                                                                           int experts, int top, int weighted, int* __restrict__ chosen, float* __restrict__ weights) {
+    constexpr int TOKENS = Cut::TOKENS;
     extern __shared__ __align__(16) float shared[];  // TOKENS rows (padded to a multiple of four), then a logit per token and expert
     float* logits = shared + (size_t)TOKENS * ((hidden + 3) & ~3);
     const int first = blockIdx.x * TOKENS, count = min(TOKENS, tokens - first), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     let_next_kernel_start();
     wait_for_previous_kernels();
-    router_logits<T, TOKENS>(x, x_stride, router, nullptr, first, count, hidden, experts, shared, logits);
+    router_logits<T, Cut>(x, x_stride, router, nullptr, first, count, hidden, experts, shared, logits);
     if (warp >= count) return;
     float* z = logits + warp * experts;
     const size_t t = first + warp;
@@ -161,17 +171,18 @@ __global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 
 // Softmax scores over all `outputs` of the router, choice by score + correction inside the best `group_keep` of `group_count` groups of
 // neighbours (a group's rank is its largest choice score; group_count <= 1: no groups), weights = plain score * scale.  The logits are
 // taken as in the kernel above; everything after them is warp j's work for token j, sums and searches in a fixed order.
-template <typename T, int TOKENS>
-__global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 1) moe_route_scored_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
+template <typename T, typename Cut>
+__global__ void __launch_bounds__(Cut::THREADS, Cut::BLOCKS) moe_route_scored_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
                                                                          const float* __restrict__ correction, int tokens, int hidden, int outputs, int top,
                                                                          int group_count, int group_keep, float scale, int* __restrict__ chosen,
                                                                          float* __restrict__ weights) {
+    constexpr int TOKENS = Cut::TOKENS;
     extern __shared__ __align__(16) float shared[];  // TOKENS rows; a logit per token and output; then per token: score, choice score and a flag per output, best and a flag per group
     const int groups = group_count > 0 ? group_count : 1, first = blockIdx.x * TOKENS, count = min(TOKENS, tokens - first), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* logits = shared + (size_t)TOKENS * ((hidden + 3) & ~3);
     let_next_kernel_start();
     wait_for_previous_kernels();
-    router_logits<T, TOKENS>(x, x_stride, router, nullptr, first, count, hidden, outputs, shared, logits);
+    router_logits<T, Cut>(x, x_stride, router, nullptr, first, count, hidden, outputs, shared, logits);
     if (warp >= count) return;
     const float* logit = logits + warp * outputs;
     float* score = logits + TOKENS * outputs + warp * (3 * outputs + 2 * groups);
@@ -235,10 +246,11 @@ __global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 
 }
 
 // Softmax over the chosen logits alone.
-template <typename T, int TOKENS>
-__global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 1) moe_route_softmax_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
+template <typename T, typename Cut>
+__global__ void __launch_bounds__(Cut::THREADS, Cut::BLOCKS) moe_route_softmax_kernel(const T* __restrict__ x, int x_stride, const float* __restrict__ router,
                                                                           const float* __restrict__ bias, int tokens, int hidden, int experts, int top,
                                                                           int* __restrict__ chosen, float* __restrict__ weights) {
+    constexpr int TOKENS = Cut::TOKENS;
     extern __shared__ __align__(16) float shared[];  // TOKENS rows, then per token: a logit per expert, the chosen logits
     const int padded = (hidden + 3) & ~3;
     float* logits = shared + (size_t)TOKENS * padded;
@@ -246,7 +258,7 @@ __global__ void __launch_bounds__(route_most_threads(TOKENS), TOKENS == 8 ? 2 : 
     const int first = blockIdx.x * TOKENS, count = min(TOKENS, tokens - first), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     let_next_kernel_start();
     wait_for_previous_kernels();
-    router_logits<T, TOKENS>(x, x_stride, router, bias, first, count, hidden, experts, shared, logits);
+    router_logits<T, Cut>(x, x_stride, router, bias, first, count, hidden, experts, shared, logits);
     if (warp >= count) return;
     float* z = logits + warp * experts;
     float* mine = picked + warp * top;
@@ -532,48 +544,69 @@ __global__ void moe_combine_weighted_bf16x8_kernel(const __nv_bfloat16* __restri
     }
 }
 
-// How many tokens a router's block takes: eight where that leaves about a block to an SM, fewer where the step or the shared memory of two blocks on an SM is
-// smaller, one where few tokens would leave the device empty (16 tokens, 16 experts: a token a block 5.6 us, as before).
+enum : int { ROUTE_EACH, ROUTE_EACH_PAIR, ROUTE_FOUR, ROUTE_FOUR_WIDE, ROUTE_EIGHT };
+
+// Which cut serves a step; bytes(n): the shared memory of n tokens.  Measured over 64 to 8,192 tokens of 1,024 to 7,168 columns and 4 to 256 outputs; below in us at 2,048 columns,
+// Each / EachPair / Four / FourWide / Eight:
+//   a block per SM at the most: Each (148 tokens, 64 outputs 8.1 / 8.4 / 11.7 / 10.9 / 28);
+//   outputs that eight warps take in one pass: Each and EachPair while all the tokens' blocks are on the device together (256 tokens, 8 outputs 4.1 / 4.6 / 5.0 / 5.4 / 8.3; 384 tokens, 12 outputs
+//   10.0 / 5.1 / 5.7 / 5.9 / 9.0), then Four (1,023 tokens, 8 outputs 13.5 / 9.3 / 7.3 / 7.4 / 9.2; with eight tokens a block and a token a block in turn before: 10.9 and 10.7);
+//   more outputs: EachPair up to two tokens an SM (256 tokens, 64 outputs 15.4 / 10.4 / 12.4 / 11.0 / 28), FourWide up to four, a block of up to 16 warps an SM (511 tokens 29 / 19.8 / 17.5 / 11.2 / 30),
+//   then Four (1,023 tokens 51 / 38 / 19.3 / 21.2 / 36), FourWide where four rows leave an SM one block all the same (7,168 columns, 64 outputs, 2,048 tokens 248 / 180 / 119 / 112 / -);
+//   Eight from eight tokens an SM on where its nine warps take the outputs in as few passes (2,048 tokens, 18 outputs 53 / 33 / 16.1 / 20.0 / 12.9; 64 outputs 101 / 67 / 36.9 / 41 / 37.6) and two of
+//   its blocks share an SM (4,096 columns 79 / 54 / 26.4 / 33 / 31).
 template <typename Bytes>
-int tokens_of_block(int tokens, Bytes bytes) {
-    if (tokens >= 1024 && bytes(8) <= 100 * 1024) return 8;
-    return tokens >= 512 && bytes(4) <= 100 * 1024 ? 4 : 1;
+int route_cut(int tokens, int outputs, int sms, Bytes bytes) {
+    const bool four_fit = bytes(4) <= ROUTE_MOST_SHARED, one_pass = outputs <= 16;
+    const long long pairs = (long long)tokens * outputs;
+    if (tokens <= sms) return ROUTE_EACH;
+    if (one_pass && pairs <= 14LL * sms && 2LL * tokens <= 7LL * sms) return ROUTE_EACH;
+    if (one_pass ? pairs <= 32LL * sms && 4LL * tokens <= 17LL * sms : tokens <= 2 * sms) return ROUTE_EACH_PAIR;
+    if (!four_fit) return ROUTE_EACH_PAIR;
+    if (!one_pass && tokens <= 4 * sms) return ROUTE_FOUR_WIDE;
+    if (tokens > 8 * sms && outputs > 8 && outputs <= 36 && bytes(8) <= 100 * 1024) return ROUTE_EIGHT;
+    return bytes(4) <= 100 * 1024 || outputs <= 32 ? ROUTE_FOUR : ROUTE_FOUR_WIDE;
 }
 
-template <typename... Params, typename... Args>
-int launch_router(void (*kernel)(Params...), int at_once, int tokens, int outputs, size_t shared, cudaStream_t stream, Args... args) {
+constexpr int ROUTE_TOKENS[] = {1, 1, 4, 4, 8};
+
+template <typename Cut, typename... Params, typename... Args>
+int launch_router(void (*kernel)(Params...), int tokens, int outputs, size_t shared, cudaStream_t stream, Args... args) {
     if (shared > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROUTE_MOST_SHARED);
-    const int each = route_at_once(at_once), wanted = (outputs + each - 1) / each, least = at_once > 4 ? at_once : 4;  // at least a warp per token
-    const int warps = wanted < least ? least : (wanted > route_most_threads(at_once) / 32 ? route_most_threads(at_once) / 32 : wanted);
-    return launch_after_previous(kernel, dim3((tokens + at_once - 1) / at_once), dim3(32 * warps), shared, stream, args...);
+    const int wanted = (outputs + Cut::AT_ONCE - 1) / Cut::AT_ONCE, least = Cut::TOKENS > 4 ? Cut::TOKENS : 4;  // at least a warp per token
+    const int warps = wanted < least ? least : (wanted > Cut::THREADS / 32 ? Cut::THREADS / 32 : wanted);
+    return launch_after_previous(kernel, dim3((tokens + Cut::TOKENS - 1) / Cut::TOKENS), dim3(32 * warps), shared, stream, args...);
 }
 }  // namespace
 
-#define HB_ROUTE_TOKENS()                        \
-    if (is_bf16) {                               \
-        if (at_once == 8) HB_ROUTE(__nv_bfloat16, 8); \
-        if (at_once == 4) HB_ROUTE(__nv_bfloat16, 4); \
-        HB_ROUTE(__nv_bfloat16, 1);              \
-    }                                            \
-    if (at_once == 8) HB_ROUTE(float, 8);        \
-    if (at_once == 4) HB_ROUTE(float, 4);        \
-    HB_ROUTE(float, 1)
+#define HB_ROUTE_CUTS(T)                                  \
+    switch (cut) {                                        \
+        case ROUTE_EACH: HB_ROUTE(T, RouteEach);          \
+        case ROUTE_EACH_PAIR: HB_ROUTE(T, RouteEachPair); \
+        case ROUTE_FOUR: HB_ROUTE(T, RouteFour);          \
+        case ROUTE_FOUR_WIDE: HB_ROUTE(T, RouteFourWide); \
+        default: HB_ROUTE(T, RouteEight);                 \
+    }
+#define HB_ROUTE_BY_TYPE()                    \
+    if (is_bf16) HB_ROUTE_CUTS(__nv_bfloat16) \
+    HB_ROUTE_CUTS(float)
 
+// sms (here and below): the device's multiprocessors.
 HB_EXPORT int hb_moe_route_scored(const void* x, int is_bf16, int x_stride, const float* router, const float* correction, int tokens, int hidden,
-                                  int outputs, int top, int group_count, int group_keep, float scale, int* chosen, float* weights, cudaStream_t stream) {
+                                  int outputs, int top, int group_count, int group_keep, float scale, int sms, int* chosen, float* weights, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (outputs <= 0 || outputs > 1024 || top <= 0 || top > outputs || hidden <= 0) return HB_UNSUPPORTED_SIZE;
     if (group_count > 1 && (outputs % group_count || group_keep <= 0 || group_keep > group_count || top > group_keep * (outputs / group_count)))
         return HB_BAD_ARGUMENT;
     const int groups = group_count > 0 ? group_count : 1;
     auto bytes = [&](int at_once) { return (size_t)at_once * (((hidden + 3) & ~3) + 4 * outputs + 2 * groups) * sizeof(float); };
-    const int at_once = tokens_of_block(tokens, bytes);
-    const size_t shared = bytes(at_once);
+    const int cut = route_cut(tokens, outputs, sms, bytes);
+    const size_t shared = bytes(ROUTE_TOKENS[cut]);
     if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
-#define HB_ROUTE(T, N)                                                                                                                                         \
-    return launch_router(moe_route_scored_kernel<T, N>, N, tokens, outputs, shared, stream, (const T*)x, x_stride, router, correction, tokens, hidden, outputs, top, group_count, \
+#define HB_ROUTE(T, C)                                                                                                                                         \
+    return launch_router<C>(moe_route_scored_kernel<T, C>, tokens, outputs, shared, stream, (const T*)x, x_stride, router, correction, tokens, hidden, outputs, top, group_count, \
                          group_keep, scale, chosen, weights)
-    HB_ROUTE_TOKENS();
+    HB_ROUTE_BY_TYPE();
 #undef HB_ROUTE
 }
 
@@ -598,31 +631,32 @@ HB_EXPORT int hb_moe_combine_weighted(const void* y, const int* slot_of, const f
     return launch_status();
 }
 
-HB_EXPORT int hb_moe_route(const void* x, int is_bf16, int x_stride, const float* router, int tokens, int hidden, int experts, int top, int weighted,
+HB_EXPORT int hb_moe_route(const void* x, int is_bf16, int x_stride, const float* router, int tokens, int hidden, int experts, int top, int weighted, int sms,
                            int* chosen, float* weights, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (experts <= 0 || experts > 1024 || top <= 0 || top > experts || hidden <= 0) return HB_UNSUPPORTED_SIZE;
     auto bytes = [&](int at_once) { return (size_t)at_once * (((hidden + 3) & ~3) + experts) * sizeof(float); };
-    const int at_once = tokens_of_block(tokens, bytes);
-    const size_t shared = bytes(at_once);
+    const int cut = route_cut(tokens, experts, sms, bytes);
+    const size_t shared = bytes(ROUTE_TOKENS[cut]);
     if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
-#define HB_ROUTE(T, N) return launch_router(moe_route_kernel<T, N>, N, tokens, experts, shared, stream, (const T*)x, x_stride, router, tokens, hidden, experts, top, weighted, chosen, weights)
-    HB_ROUTE_TOKENS();
+#define HB_ROUTE(T, C) return launch_router<C>(moe_route_kernel<T, C>, tokens, experts, shared, stream, (const T*)x, x_stride, router, tokens, hidden, experts, top, weighted, chosen, weights)
+    HB_ROUTE_BY_TYPE();
 #undef HB_ROUTE
 }
 
 HB_EXPORT int hb_moe_route_softmax(const void* x, int is_bf16, int x_stride, const float* router, const float* bias, int tokens, int hidden, int experts,
-                                   int top, int* chosen, float* weights, cudaStream_t stream) {
+                                   int top, int sms, int* chosen, float* weights, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (experts <= 0 || experts > 1024 || top <= 0 || top > experts || hidden <= 0) return HB_UNSUPPORTED_SIZE;
     auto bytes = [&](int at_once) { return (size_t)at_once * (((hidden + 3) & ~3) + experts + top) * sizeof(float); };
-    const int at_once = tokens_of_block(tokens, bytes);
-    const size_t shared = bytes(at_once);
+    const int cut = route_cut(tokens, experts, sms, bytes);
+    const size_t shared = bytes(ROUTE_TOKENS[cut]);
     if (shared > ROUTE_MOST_SHARED) return HB_UNSUPPORTED_SIZE;
-#define HB_ROUTE(T, N) return launch_router(moe_route_softmax_kernel<T, N>, N, tokens, experts, shared, stream, (const T*)x, x_stride, router, bias, tokens, hidden, experts, top, chosen, weights)
-    HB_ROUTE_TOKENS();
+#define HB_ROUTE(T, C) return launch_router<C>(moe_route_softmax_kernel<T, C>, tokens, experts, shared, stream, (const T*)x, x_stride, router, bias, tokens, hidden, experts, top, chosen, weights)
+    HB_ROUTE_BY_TYPE();
 #undef HB_ROUTE
-#undef HB_ROUTE_TOKENS
+#undef HB_ROUTE_BY_TYPE
+#undef HB_ROUTE_CUTS
 }
 
 // capacity: a multiple of pad, at least pairs + experts * (pad - 1) rounded up to it.  tile_expert and tile_rows (the real rows at the start

@@ -10,7 +10,7 @@ import torch
 
 from . import gemm
 from .basic import status_word, swiglu
-from .native import KernelError, check, f32, i32, is_bf16, library, ptr, require_cuda, stream_ptr
+from .native import KernelError, check, f32, i32, is_bf16, library, ptr, require_cuda, sm_count, stream_ptr
 
 PAD = 128  # an expert's rows are padded to whole tiles of this many rows
 STREAM_ROWS = 8  # rows the streaming kernel takes at once
@@ -46,7 +46,7 @@ def route(x: torch.Tensor, router: torch.Tensor, top: int, weighted: bool = True
     chosen = torch.empty((tokens, top), dtype=torch.int32, device=x.device)
     weights = torch.empty((tokens, top), dtype=torch.float32, device=x.device)
     check(library("moe").hb_moe_route(ptr(x), i32(is_bf16(x)), i32(x.stride(0)), ptr(router), i32(tokens), i32(hidden), i32(experts), i32(top),
-                                      i32(1 if weighted else 0), ptr(chosen), ptr(weights), stream_ptr()), "moe_route")
+                                      i32(1 if weighted else 0), i32(sm_count(x.device)), ptr(chosen), ptr(weights), stream_ptr()), "moe_route")
     return chosen, weights
 
 
@@ -65,7 +65,7 @@ def route_scored(x: torch.Tensor, router: torch.Tensor, correction: torch.Tensor
     chosen = torch.empty((tokens, top), dtype=torch.int32, device=x.device)
     weights = torch.empty((tokens, top), dtype=torch.float32, device=x.device)
     check(library("moe").hb_moe_route_scored(ptr(x), i32(is_bf16(x)), i32(x.stride(0)), ptr(router), ptr(correction), i32(tokens), i32(hidden),
-                                             i32(router.shape[0]), i32(top), i32(group_count), i32(group_keep), f32(scale), ptr(chosen), ptr(weights),
+                                             i32(router.shape[0]), i32(top), i32(group_count), i32(group_keep), f32(scale), i32(sm_count(x.device)), ptr(chosen), ptr(weights),
                                              stream_ptr()), "moe_route_scored")
     return chosen, weights
 
@@ -82,7 +82,7 @@ def route_softmax(x: torch.Tensor, router: torch.Tensor, bias: torch.Tensor | No
     chosen = torch.empty((tokens, top), dtype=torch.int32, device=x.device)
     weights = torch.empty((tokens, top), dtype=torch.float32, device=x.device)
     check(library("moe").hb_moe_route_softmax(ptr(x), i32(is_bf16(x)), i32(x.stride(0)), ptr(router), ptr(bias), i32(tokens), i32(hidden), i32(router.shape[0]), i32(top),
-                                              ptr(chosen), ptr(weights), stream_ptr()), "moe_route_softmax")
+                                              i32(sm_count(x.device)), ptr(chosen), ptr(weights), stream_ptr()), "moe_route_softmax")
     return chosen, weights
 
 
