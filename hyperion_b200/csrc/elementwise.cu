@@ -483,80 +483,63 @@ __global__ void rope_kv_store_kernel(T* __restrict__ x, int stride, int q_heads,
 }
 
 // bfloat16 with head sizes that are multiples of 16: every thread rotates 8 consecutive pairs (two 16-byte loads, two
-// 16-byte stores) or copies 8 values; same arithmetic per element as the scalar kernel.  A thread takes its piece of a head through TOKENS
-// tokens, whose pieces are all asked for before the first is used: with one token a block, a prompt's step was bound by its
-// blocks coming and going (2,048 tokens of 28 + 4 + 4 heads of 128: 15.5 -> 14.1 us).
-template <int TOKENS>
-__global__ void __launch_bounds__(256) rope_kv_store_bf16x8_kernel(__nv_bfloat16* __restrict__ x, int tokens, int stride, int q_heads, int kv_heads, int head_dim,
+// 16-byte stores) or copies 8 values; same arithmetic per element as the scalar kernel.  A thread that takes its piece through four tokens, all asked for
+// at once, is faster only where the rows come from memory (2,048 tokens of 28 + 4 + 4 heads of 128: 15.5 -> 14.1 us); behind the product that made them they lie
+// in L2: 8.5 us here and 9.5 so (16 + 4 + 4 heads: 5.9 and 8.2).
+__global__ void rope_kv_store_bf16x8_kernel(__nv_bfloat16* __restrict__ x, int stride, int q_heads, int kv_heads, int head_dim,
                                             const int* __restrict__ positions, const float2* __restrict__ table, int max_positions,
                                             __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, int table_width,
                                             const int* __restrict__ token_row, int page_size, int pages, int* status) {
-    const int t0 = blockIdx.x * TOKENS;
+    const int t = blockIdx.x;
     const int half = head_dim >> 1, chunks = half >> 3;  // 8-pair chunks per head
+    let_next_kernel_start();
+    const int pos = positions[t];  // positions and tables come with the step's one copy from the host, not from a kernel
+    const bool pos_ok = pos >= 0 && pos < max_positions;
+    const int block = pos_ok ? pos / page_size : 0;
+    const int page = pos_ok && block < table_width ? block_table[(size_t)token_row[t] * table_width + block] : -1;
+    wait_for_previous_kernels();
+    if (!pos_ok) {
+        if (threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_POSITION);
+        return;
+    }
+    const bool page_ok = page >= 0 && page < pages;
+    if (!page_ok && threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_PAGE);
+    const int slot = pos - block * page_size;
+    __nv_bfloat16* row = x + (size_t)t * stride;
+    const float2* cs = table + (size_t)pos * half;
+    const size_t page_base = (size_t)(page_ok ? page : 0) * 2 * kv_heads * page_size * head_dim;
     const int rotated = (q_heads + kv_heads) * chunks;
     const int total = rotated + kv_heads * 2 * chunks;  // values: head_dim / 8 chunks per head
-    const int e = blockIdx.y * blockDim.x + threadIdx.x;
-    const bool turns = e < rotated;
-    const int head = turns ? e / chunks : (e - rotated) / (2 * chunks);
-    const int i = (turns ? e - head * chunks : e - rotated - head * 2 * chunks) * 8;
-    const int at = (turns ? head : q_heads + kv_heads + head) * head_dim + i;
-    const bool stored = !turns || head >= q_heads;  // goes to the token's page
-    // where the page has this piece's place: keys first, then values
-    const size_t in_page = (size_t)(turns ? head - q_heads : kv_heads + head) * page_size * head_dim + i;
-    let_next_kernel_start();
-    int pos[TOKENS], page[TOKENS];
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < total; e += gridDim.y * blockDim.x) {
+        if (e < rotated) {
+            const int head = e / chunks, i = (e - head * chunks) * 8;
+            __nv_bfloat16* p = row + head * head_dim + i;
+            const uint4 lo4 = *reinterpret_cast<const uint4*>(p), hi4 = *reinterpret_cast<const uint4*>(p + half);
+            const __nv_bfloat16* lo = reinterpret_cast<const __nv_bfloat16*>(&lo4);
+            const __nv_bfloat16* hi = reinterpret_cast<const __nv_bfloat16*>(&hi4);
+            uint4 out_lo, out_hi;
+            __nv_bfloat16* y1 = reinterpret_cast<__nv_bfloat16*>(&out_lo);
+            __nv_bfloat16* y2 = reinterpret_cast<__nv_bfloat16*>(&out_hi);
 #pragma unroll
-    for (int u = 0; u < TOKENS; ++u) {  // positions and tables come with the step's one copy from the host, not from a kernel
-        pos[u] = t0 + u < tokens ? positions[t0 + u] : 0;
-        const bool pos_ok = pos[u] >= 0 && pos[u] < max_positions;
-        const int block = pos_ok ? pos[u] / page_size : 0;
-        page[u] = t0 + u < tokens && pos_ok && block < table_width ? block_table[(size_t)token_row[t0 + u] * table_width + block] : -1;
-    }
-    wait_for_previous_kernels();
-    uint4 lo4[TOKENS], hi4[TOKENS];
-#pragma unroll
-    for (int u = 0; u < TOKENS; ++u) {
-        if (e < total && t0 + u < tokens) {
-            const __nv_bfloat16* p = x + (size_t)(t0 + u) * stride + at;
-            lo4[u] = *reinterpret_cast<const uint4*>(p);
-            if (turns) hi4[u] = *reinterpret_cast<const uint4*>(p + half);
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < TOKENS; ++u) {
-        const int t = t0 + u;
-        if (t >= tokens) break;
-        if (pos[u] < 0 || pos[u] >= max_positions) {
-            if (threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_POSITION);
-            continue;
-        }
-        const bool page_ok = page[u] >= 0 && page[u] < pages;
-        if (!page_ok && threadIdx.x == 0 && blockIdx.y == 0) atomicOr(status, HB_STATUS_BAD_PAGE);
-        if (e >= total || (stored && !page_ok)) continue;
-        __nv_bfloat16* dst = stored ? cache + (size_t)page[u] * 2 * kv_heads * page_size * head_dim + in_page + (size_t)(pos[u] % page_size) * head_dim : x + (size_t)t * stride + at;
-        if (!turns) {
-            *reinterpret_cast<uint4*>(dst) = lo4[u];
-            continue;
-        }
-        const __nv_bfloat16* lo = reinterpret_cast<const __nv_bfloat16*>(&lo4[u]);
-        const __nv_bfloat16* hi = reinterpret_cast<const __nv_bfloat16*>(&hi4[u]);
-        uint4 out_lo, out_hi;
-        __nv_bfloat16* y1 = reinterpret_cast<__nv_bfloat16*>(&out_lo);
-        __nv_bfloat16* y2 = reinterpret_cast<__nv_bfloat16*>(&out_hi);
-        const float* cs = reinterpret_cast<const float*>(table + (size_t)pos[u] * half + i);  // cosine and sine in turn
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-            float c[4];
-            load4(cs + 2 * j, c);
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const float x1 = __bfloat162float(lo[j + k]), x2 = __bfloat162float(hi[j + k]);
-                y1[j + k] = __float2bfloat16_rn(x1 * c[2 * k] - x2 * c[2 * k + 1]);
-                y2[j + k] = __float2bfloat16_rn(x2 * c[2 * k] + x1 * c[2 * k + 1]);
+            for (int j = 0; j < 8; ++j) {
+                const float2 c = cs[i + j];
+                const float x1 = __bfloat162float(lo[j]), x2 = __bfloat162float(hi[j]);
+                y1[j] = __float2bfloat16_rn(x1 * c.x - x2 * c.y);
+                y2[j] = __float2bfloat16_rn(x2 * c.x + x1 * c.y);
             }
+            if (head < q_heads) {
+                *reinterpret_cast<uint4*>(p) = out_lo;
+                *reinterpret_cast<uint4*>(p + half) = out_hi;
+            } else if (page_ok) {
+                __nv_bfloat16* dst = cache + page_base + (((size_t)(head - q_heads)) * page_size + slot) * head_dim + i;
+                *reinterpret_cast<uint4*>(dst) = out_lo;
+                *reinterpret_cast<uint4*>(dst + half) = out_hi;
+            }
+        } else if (page_ok) {
+            const int f = e - rotated, head = f / (2 * chunks), i = (f - head * 2 * chunks) * 8;
+            const uint4 v = *reinterpret_cast<const uint4*>(row + (q_heads + kv_heads + head) * head_dim + i);
+            *reinterpret_cast<uint4*>(cache + page_base + (((size_t)(kv_heads + head)) * page_size + slot) * head_dim + i) = v;
         }
-        *reinterpret_cast<uint4*>(dst) = out_lo;
-        *reinterpret_cast<uint4*>(dst + half) = out_hi;
     }
 }
 
@@ -565,17 +548,16 @@ HB_EXPORT int hb_rope_kv_store(void* x, int is_bf16, int tokens, int stride, int
                                int table_width, const int* token_row, int page_size, int pages, int* status, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (head_dim & 1) return HB_UNSUPPORTED_SIZE;
-    if (is_bf16 && head_dim % 16 == 0 && stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)cache | (uintptr_t)table) & 15) == 0) {
+    if (is_bf16 && head_dim % 16 == 0 && stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)cache) & 15) == 0) {
+        // Up to 1,023 tokens a thread for every piece, in as many even blocks a token as that takes (28 + 4 + 4 heads of 128, in us: 8 tokens 1.53, 512 tokens 3.4; a loop over the pieces in up to eight
+        // blocks of 128 or 256 threads a token 1.66 and 3.9).  From there on one block a token that loops: blocks come and go half as often (32 + 32 + 32 heads, 1,531 tokens 13.1 and 15.5).
         const int items = (q_heads + 3 * kv_heads) * (head_dim / 16);  // pairs of eight entries, and the values' eights
-        const int across = (items + 255) / 256, threads = ((items + across - 1) / across + 31) / 32 * 32;
-        if (across > 65535) return HB_UNSUPPORTED_SIZE;
-#define HB_ROPE8(TOKENS)                                                                                                                                                 \
-    return launch_after_previous(rope_kv_store_bf16x8_kernel<TOKENS>, dim3((tokens + TOKENS - 1) / TOKENS, across), threads, 0, stream, (__nv_bfloat16*)x, tokens, stride, \
-                                 q_heads, kv_heads, head_dim, positions, (const float2*)table, max_positions, (__nv_bfloat16*)cache, block_table, table_width, token_row,  \
-                                 page_size, pages, status)
-        if (tokens >= 1024) HB_ROPE8(4);  // enough tokens for two blocks an SM all the same
-        HB_ROPE8(1);
-#undef HB_ROPE8
+        const int across = tokens < 1024 ? (items + 255) / 256 : 1;
+        const int threads = tokens < 1024 ? ((items + across - 1) / across + 31) / 32 * 32 : ((q_heads + 2 * kv_heads) * (head_dim / 16) >= 256 ? 256 : 128);
+        const dim3 grid8(tokens, across < 65535 ? across : 65535);
+        return launch_after_previous(rope_kv_store_bf16x8_kernel, grid8, threads, 0, stream, (__nv_bfloat16*)x, stride, q_heads, kv_heads, head_dim,
+                                     positions, (const float2*)table, max_positions, (__nv_bfloat16*)cache, block_table, table_width, token_row,
+                                     page_size, pages, status);
     }
     const int pairs = (q_heads + 2 * kv_heads) * (head_dim / 2);
     const int slices = tokens >= 512 ? 1 : min(16, (pairs + 255) / 256);
