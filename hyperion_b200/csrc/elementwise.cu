@@ -158,9 +158,9 @@ __global__ void add_rmsnorm_cached_kernel(float* __restrict__ h, const TD* __res
 // their sum in split order plus the bias, rounded to bfloat16 as the product's own reduction would store it.  Pieces are a
 // matter of their own instance (PIECES): with the room for them a thread holds 128 registers and an SM one block, and a prompt's
 // rows, which are bound by the bytes in flight, then take 2.4 times as long (2,048 rows of 3,584: 33.7 -> 14.9 us).
-// split-K pieces a thread asks for at once (products of a decode step are split 5 to 10 times); fewer where a thread holds
-// several groups of a wide row
-__host__ __device__ constexpr int pieces_ahead(int groups_per_thread) { return groups_per_thread == 1 ? 12 : (groups_per_thread == 2 ? 8 : 4); }
+// split-K pieces a thread asks for at once (products of a decode step are split 5 to 10 times): what its 128 registers hold; fewer where a thread has
+// several groups of a wide row.  (Twelve and eight spilled four registers in the instance with pieces: eight rows of 3,584 in five pieces 2.92 us, 2.76 so.)
+__host__ __device__ constexpr int pieces_ahead(int groups_per_thread) { return groups_per_thread == 1 ? 11 : (groups_per_thread == 2 ? 7 : 4); }
 struct SplitDelta {
     const float* partials;
     size_t split_stride;  // tokens * hidden
@@ -610,7 +610,9 @@ __global__ void rmsnorm_add_kernel(float* __restrict__ h, const TY* __restrict__
 }
 
 // bfloat16 sublayer outputs in rows of up to 8,192 values, a multiple of 8: a thread keeps its 8 values in registers between the
-// sum of squares and the add (one trip to memory), with 16-byte accesses.
+// sum of squares and the add (one trip to memory), with 16-byte accesses.  EARLY: the stream's row is asked for with the sublayer's, before the sum, which is what a few rows wait
+// for; many wide rows, which are bound by the memory, read it behind the sum, where they write it (2,048 rows of 8,192: 52.0 us early, 36.6 late; 64 rows of 896 1.6 early, 1.8 late).
+template <bool EARLY>
 __global__ void __launch_bounds__(1024) rmsnorm_add_bf16x8_kernel(float* __restrict__ h, const __nv_bfloat16* __restrict__ y, const float* __restrict__ weight,
                                           __nv_bfloat16* __restrict__ copy, int hidden, float eps) {
     __shared__ __align__(16) float scratch[32];
@@ -620,16 +622,22 @@ __global__ void __launch_bounds__(1024) rmsnorm_add_bf16x8_kernel(float* __restr
     float* hrow = h + (size_t)t * hidden + i;
     let_next_kernel_start();
     wait_for_previous_kernels();
-    if (active) {  // both rows and the weights are asked for before the sum
-        load8(weight + i, w);
+    if (active) {
         load8(y + (size_t)t * hidden + i, v);
-        load8(hrow, x);
+        if (EARLY) {
+            load8(weight + i, w);
+            load8(hrow, x);
+        }
     }
     float sum = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) sum = fmaf(v[k], v[k], sum);
     const float inv = 1.0f / sqrtf(block_sum(sum, scratch) / (float)hidden + eps);
     if (!active) return;
+    if (!EARLY) {
+        load8(hrow, x);
+        load8(weight + i, w);
+    }
 #pragma unroll
     for (int k = 0; k < 8; ++k) x[k] += v[k] * inv * w[k];
     store8(hrow, x);
@@ -641,7 +649,9 @@ HB_EXPORT int hb_rmsnorm_add(float* h, const void* y, int y_is_bf16, const float
     if (tokens <= 0) return 0;
     if (y_is_bf16 && hidden % 8 == 0 && hidden <= 8192 && (((uintptr_t)h | (uintptr_t)y | (uintptr_t)weight | (uintptr_t)copy) & 15) == 0) {
         const int lanes = ((hidden / 8 + 31) / 32) * 32;  // which kernel runs follows from the width alone
-        return launch_after_previous(rmsnorm_add_bf16x8_kernel, tokens, lanes, 0, stream, h, (const __nv_bfloat16*)y, weight, (__nv_bfloat16*)copy, hidden, eps);
+        if (tokens >= 512 && hidden >= 3072)  // the same bits either way
+            return launch_after_previous(rmsnorm_add_bf16x8_kernel<false>, tokens, lanes, 0, stream, h, (const __nv_bfloat16*)y, weight, (__nv_bfloat16*)copy, hidden, eps);
+        return launch_after_previous(rmsnorm_add_bf16x8_kernel<true>, tokens, lanes, 0, stream, h, (const __nv_bfloat16*)y, weight, (__nv_bfloat16*)copy, hidden, eps);
     }
     const int threads = hidden >= 2048 ? 512 : (hidden >= 512 ? 256 : 128);
     if (y_is_bf16)
