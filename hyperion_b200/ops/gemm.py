@@ -59,13 +59,13 @@ FEW_BF16, FEW_F32, FEW_SWIGLU, FEW_PIECES = 0, 1, 2, 3
 
 
 def takes_few_rows(x: torch.Tensor, w: torch.Tensor, gated_block: Optional[int] = None) -> bool:
-    """Whether a product of a few rows goes to ``csrc/few_rows.cu``: whole tiles of 16 rows of the matrix and of 64 of k, and a matrix small enough that the step is its waits, not
-    its bytes.  Measured in chains of such products, one to eight rows: [896, 896] 4.1 -> 2.2 us, [2,048, 2,048] 3.7 -> 2.8, [4,096, 2,048] 5.9 -> 4.8, [9,728, 896] with SwiGLU
+    """Whether ``csrc/few_rows.cu`` takes a product of a few rows (with SwiGLU; without it :func:`pays_few_rows` also asks what else could): whole tiles of 16 rows of the matrix and of 64 of k, and a
+    matrix small enough that the step is its waits, not its bytes.  Measured in chains of such products, one to eight rows: [896, 896] 4.1 -> 2.2 us, [2,048, 2,048] 3.7 -> 2.8, [4,096, 2,048] 5.9 -> 4.8, [9,728, 896] with SwiGLU
     8.1 -> 5.0, [16,384, 2,048] with SwiGLU 15.7 -> 14.3; beyond 20 MB only where k is short (a tile's sum over long k keeps few blocks busy: [4,096, 4,096] 6.9 -> 8.0),
     and not from some 70 MB on ([32,000, 2,048] 21.5 -> 24.6).  Nine to sixteen rows ask for twice the rows per unit: [2,048, 2,048] 3.9 -> 3.4, [4,096, 2,048] 6.1 -> 6.4,
     [9,728, 896] 8.9 -> 7.0.  ``gated_block``: with SwiGLU in the epilogue, over runs of that many gate rows."""
     m, (n, k) = x.shape[0], w.shape
-    if m > FEW_ROWS or not supported(x, w) or not w.is_contiguous() or k % 64 or n % 16:
+    if m > FEW_ROWS or k % 64 or n % 16 or n * k > 68 << 19 or not supported(x, w) or not w.is_contiguous():
         return False
     if gated_block is not None and (n % 32 or gated_block < 8 or (n // 2) % gated_block or (gated_block != n // 2 and gated_block & (gated_block - 1))):
         return False
@@ -73,6 +73,40 @@ def takes_few_rows(x: torch.Tensor, w: torch.Tensor, gated_block: Optional[int] 
     if m <= 8:
         return megabytes <= 20 or (k <= 2048 and megabytes <= 68)
     return megabytes <= 13 or (k < 2048 and megabytes <= 20)
+
+
+def pays_few_rows(m: int, n: int, k: int, pieces: bool, sms: int) -> bool:
+    """Whether a product without SwiGLU that ``csrc/few_rows.cu`` takes is also faster there than where else it would go: the split product of this file from k = 2,048 on, else
+    the library.  ``pieces``: the caller adds up parts of k.  Measured at n = 16 to 32,768 by k = 64 to 16,384, 1 to 16 rows, this kernel over the other:
+
+    * a block sums whole k for its tiles of 16 columns, so long k is a chain that splits do not have (8 rows, n 256: k 4,096 0.9, 8,192 1.28, 16,384 1.66), and tiles beyond two blocks to an SM are
+      a second turn (8 rows, k 2,048: n 4,096 0.82, 5,120 1.06, 8,192 0.93), which only short k bears (n 10,240: k 256 0.9, 1,024 1.06);
+    * where the split product's own blocks leave a second turn nearly empty it loses at any k (8 rows: [2,560, 2,048] 0.47, [1,536, 4,096] 0.69);
+    * left in pieces, up to four parts of k fill the device from few tiles (8 rows: [896, 4,864] 0.78, [256, 16,384] 0.73; with more tiles than SMs they are whole sums: [2,560, 3,072] 1.26);
+    * nine to sixteen rows ask for twice the rows per unit (16 rows: [1,024, 1,024] 0.70, [896, 4,864] 1.48 whole and 0.83 in pieces, [5,120, 1,024] 1.30)."""
+    if n * k > (20 << 19 if k > 2048 else 68 << 19):  # bound by its bytes (takes_few_rows has the line); most products of a large model end here
+        return False
+    tiles, slots = n // 16, 2 * sms
+    second_turn = k >= 2048 and sms < -(-n // 128) * choose_splits(n, k, m, sms) <= 1.5 * sms  # of the split product
+    if pieces and k >= 2048:
+        if second_turn:
+            return True
+        if m <= 8:
+            return tiles <= sms and (k <= 6144 or 3 * tiles <= 2 * sms)
+        return 8 * tiles < sms or (2 * tiles < sms and k <= 6144) or (tiles <= sms and k <= 2560)
+    if m <= 8:
+        if second_turn:
+            return True
+        if tiles <= slots:
+            return k <= 3072 or (k <= 4096 and (2 * tiles < sms or 1.56 * tiles >= slots))
+        if tiles <= 2 * slots:
+            return k <= 1024 or (k <= 2560 and tiles >= 1.6 * slots)
+        return k <= 256 and tiles <= 4 * slots
+    if second_turn:
+        return k <= 4096
+    if 2 * tiles < sms:
+        return k <= 2560
+    return 128 <= k <= 1536 if tiles <= sms else 768 <= k <= 1536 and tiles <= slots
 
 
 def few_rows(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, epilogue: int = FEW_BF16, block: int = 0, settled: bool = False):

@@ -18,7 +18,7 @@ import torch
 
 from . import gemm
 from .basic import sgemm_f32
-from .native import KernelError, require_cuda
+from .native import KernelError, require_cuda, sm_count
 
 
 SMALL_PRODUCT_BYTES = 64 << 20  # weights of at most this many bytes go to the library at more than 32 rows
@@ -63,13 +63,15 @@ def _takes_own_kernel(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) ->
     return k >= 2048 and m <= 64
 
 
-def _takes_few_rows(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype) -> bool:
+def _takes_few_rows(x: torch.Tensor, weight: torch.Tensor, bias, out_dtype, pieces: bool) -> bool:
     """Whether a bfloat16 product goes to the kernel for a few rows and a small matrix (``HYPERION_B200_GEMM`` = ``auto`` only).  The library keeps what the kernel has no form
     for: a bias that is not one dense number per column, a matrix of one row without its dimension, nothing to add up, and operands that ask for a gradient."""
     if x.dim() != 2 or weight.dim() != 2 or not 0 < x.shape[0] <= gemm.FEW_ROWS or 0 in weight.shape or gemm_policy() != "auto" or out_dtype not in (torch.bfloat16, torch.float32):
         return False
+    if not gemm.pays_few_rows(x.shape[0], *weight.shape, pieces, sm_count(x.device)) or not _is_one_per_column(bias, weight):
+        return False
     asks_for_gradient = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (x, weight, bias))
-    return _is_one_per_column(bias, weight) and not asks_for_gradient and gemm.takes_few_rows(x, weight)
+    return not asks_for_gradient and gemm.takes_few_rows(x, weight)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -89,7 +91,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     if weight.dtype != torch.bfloat16:
         raise KernelError(f"linear: weights are float32 or bfloat16, got {weight.dtype}")
     xin = x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16)
-    if _takes_few_rows(xin, weight, bias, out_dtype):
+    if _takes_few_rows(xin, weight, bias, out_dtype, may_leave_partials and out_dtype == torch.bfloat16):
         return gemm.few_rows(xin, weight, bias, gemm.FEW_F32 if out_dtype == torch.float32 else gemm.FEW_PIECES if may_leave_partials else gemm.FEW_BF16, settled=settled)
     if _takes_own_kernel(xin, weight, bias, out_dtype):
         epilogue = gemm.EPI_F32 if out_dtype == torch.float32 else gemm.EPI_BF16
