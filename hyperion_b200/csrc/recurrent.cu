@@ -1142,6 +1142,10 @@ HB_EXPORT int hb_residual_conv(const void* x, int is_bf16, int x_stride, int cha
     if (taps < 1) return HB_BAD_ARGUMENT;
     const bool by_eight = is_bf16 && taps <= 8 && channels % 8 == 0 && x_stride % 8 == 0 && out_stride % 8 == 0 &&
                           (((uintptr_t)x | (uintptr_t)out | (uintptr_t)weight) & 15) == 0;
+    // Runs of eight tokens where they still leave the device threads enough: a run is a chain of some 4 us, a step of single tokens reads its weights once per token.  The line lies where both took
+    // as long, in tokens times channels: two and three taps 1.6 million (2,048 channels, 3 taps: 512 tokens 3.5 and 4.4 us, 1,024 tokens 5.5 and 4.8), four taps 450,000 (256 tokens 4.6 and 4.6; 896
+    // channels 512 tokens 4.5 and 4.4), more taps 250,000 (2,048 channels, 8 taps: 128 tokens 5.3 and 6.5, 256 tokens 10.1 and 6.5; 512 channels, 512 tokens 6.4 and 5.5).  The same bits either way.
+    const bool long_runs = (long long)tokens * channels >= (taps <= 3 ? 1600000 : (taps == 4 ? 450000 : 250000));
     for (int first = 0; first < tokens; first += 65535) {
         const int count = tokens - first < 65535 ? tokens - first : 65535;
         if (by_eight) {
@@ -1150,9 +1154,9 @@ HB_EXPORT int hb_residual_conv(const void* x, int is_bf16, int x_stride, int cha
     residual_conv_bf16x8_kernel<T, RUN><<<dim3((channels / 8 + 127) / 128, (count + RUN - 1) / RUN), 128, 0, stream>>>(                                               \
         (const __nv_bfloat16*)x, x_stride, channels, weight, taps, state, (size_t)slot_stride, state_off, slots, token_row, row_start, (__nv_bfloat16*)out, out_stride, \
         first, end)
-#define HB_CONV8(T)                                                   \
-    case T:                                                           \
-        if (tokens >= 256) HB_CONV8_RUN(T, 8); else HB_CONV8_RUN(T, 1); \
+#define HB_CONV8(T)                                             \
+    case T:                                                     \
+        if (long_runs) HB_CONV8_RUN(T, 8); else HB_CONV8_RUN(T, 1); \
         break
             switch (taps) { HB_CONV8(1); HB_CONV8(2); HB_CONV8(3); HB_CONV8(4); HB_CONV8(5); HB_CONV8(6); HB_CONV8(7); HB_CONV8(8); }
 #undef HB_CONV8
