@@ -94,6 +94,16 @@ def plan(rows, tokens_per_tile: int) -> tuple[np.ndarray, np.ndarray]:
     return tiles[: 3 * n_tiles.value], items[: n_items.value]
 
 
+def tile_blocks(heads: int, kv_heads: int, tile_rows: int) -> int:
+    """Blocks that work on a tile of the tcgen05 kernel, whose planner may cut a step's tiles by their number (:func:`plan_prompts`); 0 for the other kernels' tiles."""
+    return kv_heads * -(-(heads // kv_heads) // tile_rows) if tile_rows == TC_TILE_ROWS else 0
+
+
+def tiles_key(tokens_per_tile: int, blocks: int) -> str:
+    """Under what name a step's tiles stand.  Tiles that may have been cut by the number of their ``blocks`` are not shared with layers of another number, nor with kernels that take them whole."""
+    return f"attn_tiles_{tokens_per_tile}" + (f"_{blocks}" if blocks else "")
+
+
 def plan_prompts(rows, tokens_per_tile: int, blocks: int, most: float = 0.5) -> tuple[np.ndarray, np.ndarray]:
     """:func:`plan` for the tcgen05 kernel: tiles of half the rows where tiles times the ``blocks`` (key/value heads and head chunks) of a tile are at most ``most`` of the SMs.
 

@@ -117,19 +117,17 @@ class GroupedQueryAttention(Mixer):
     @staticmethod
     def plans_for(heads: int, kv_heads: int, head_dim: int, rows_of=None) -> dict:
         """``rows_of(page_size)``: the virtual rows per tile, where another kernel than the usual one for this head size will run."""
-        halves = rows_of is None
+        own_blocks = rows_of is None
         rows_of = rows_of or (lambda page_size: fast_attention.tile_rows(head_dim, page_size))
 
         def plan(rows, packer, host):
             size = rows_of(host.get("page_size"))
             tokens_per_tile = fast_attention.tile_tokens(heads, kv_heads, size)
-            key = f"attn_tiles_{tokens_per_tile}"
+            blocks = fast_attention.tile_blocks(heads, kv_heads, size) if own_blocks else 0
+            key = fast_attention.tiles_key(tokens_per_tile, blocks)
             if key in host:
                 return
-            if halves and size == fast_attention.TC_TILE_ROWS:
-                tiles, items = fast_attention.plan_prompts(rows, tokens_per_tile, kv_heads * -(-heads // kv_heads // size))
-            else:
-                tiles, items = fast_attention.plan(rows, tokens_per_tile)
+            tiles, items = fast_attention.plan_prompts(rows, tokens_per_tile, blocks) if blocks else fast_attention.plan(rows, tokens_per_tile)
             host[key] = len(tiles) // 3
             host["attn_items"] = len(items)
             if len(tiles):
@@ -137,7 +135,7 @@ class GroupedQueryAttention(Mixer):
             if len(items) and "attn_items" not in [name for name, *_ in packer._items]:
                 packer.add("attn_items", items)
 
-        return {("attention_plan", heads // kv_heads, head_dim, rows_of(None), rows_of(16)): plan}
+        return {("attention_plan", heads // kv_heads, head_dim, rows_of(None), rows_of(16), kv_heads if own_blocks else None): plan}
 
     @staticmethod
     def _longest_short_row(rows) -> int:
@@ -153,7 +151,7 @@ class GroupedQueryAttention(Mixer):
         if out is None:
             out = torch.empty((step.n_tokens, self.heads * self.head_dim), dtype=self.dtype, device=qkv.device)
         size = fast_attention.tile_rows(self.head_dim, step.host.get("page_size"))
-        key = f"attn_tiles_{fast_attention.tile_tokens(self.heads, self.kv_heads, size)}"
+        key = fast_attention.tiles_key(fast_attention.tile_tokens(self.heads, self.kv_heads, size), fast_attention.tile_blocks(self.heads, self.kv_heads, size))
         n_tiles, n_items = step.host.get(key, 0), step.host.get("attn_items", 0)
         if n_tiles:
             fast_attention.attention_tiles(qkv, self.heads, cache.kv, cache.block_table, step.token_row, step.positions,

@@ -101,7 +101,7 @@ class DifferentialAttention(Mixer):
     def _attend_fast(self, q, gate, step, cache, out):
         heads, kv_heads = 2 * self.heads, self.kv_heads
         size = self._tile_rows(step.host.get("page_size"))
-        key = f"attn_tiles_{fast_attention.tile_tokens(heads, kv_heads, size)}"
+        key = fast_attention.tiles_key(fast_attention.tile_tokens(heads, kv_heads, size), 0)
         n_tiles, n_items = step.host.get(key, 0), step.host.get("attn_items", 0)
         after = (self.scale, self.window, self.keep_first, gate, self.map_weight, self.eps, 1.0 - self.diff, out)
         if n_tiles:
