@@ -47,7 +47,9 @@ def _common_dtype(tensors) -> torch.dtype:
 EXPANDED_TOKENS = 300  # of a step, per prompt.  What the other way saves grows with the square of a prompt, what it adds (one product more, its keys and values written out) with
 # the step's tokens.  A step of 8 layers, 4 of them over latents of 16 heads, expanded and through the latent, in us: one prompt of 200 tokens 872 and 844, two of 256 1,074 and
 # 1,060, five of 300 1,342 and 1,421, three of 400 1,355 and 1,475, one of 1,024 1,622 and 1,906, one of 1,531 2,238 and 2,919; four of 128 999 and 927.
-EXPANDED_BYTES = 256 << 20  # of a step's keys and values per layer; longer prompts keep to the latent
+# More heads meet earlier: a step of one layer, the host's planning among it, expanded over latent with 16, 32 and 64 heads: 512 tokens 1.04, 0.97, 0.83; four prompts of 300 1.02, 0.92, 0.78.
+EXPANDED_BYTES = 480 << 20  # of what a layer of such a step makes beside its queries: pages, the product that fills them, the dense latents (16 heads of 128 + 64: 21.6 KB a token, where the
+# queries carried into the latent and what comes back of it are 66 KB).  Longer prompts keep to the latent.
 EXPANDED_PAGE = 64
 
 
@@ -95,6 +97,8 @@ class LatentAttention(Mixer):
         self.v_heads = tensors["uv"].reshape(self.heads, self.value_dim, self.kv_rank).transpose(1, 2).contiguous()  # [H, R, e]
         self.sink = tensors["sink"].to(torch.float32).contiguous() if self.has_sink else None
         self.w_kv = torch.cat([tensors["uk"], tensors["uv"]], dim=0).contiguous() if self.expands_fresh_prompts else None  # every head's keys, then every head's values
+        if self.w_kv is not None and self.w_kv.dtype == self.k_heads.dtype:  # the keys' half is what stands above, once is enough (the values' lie the other way round)
+            self.k_heads = self.w_kv[: self.heads * self.head_dim].view(self.heads, self.head_dim, self.kv_rank)
 
     def cache_request(self):
         return PagedTokens((1,), (self.record,), 0)
@@ -117,7 +121,7 @@ class LatentAttention(Mixer):
             pages = -(-counts // EXPANDED_PAGE)
             total = int(pages.sum())
             if (rows.positions.any() or int(counts.min()) <= fast_attention.TOKEN_SHAPE_MAX or int(counts.sum()) < EXPANDED_TOKENS * len(counts)
-                    or total * EXPANDED_PAGE * 2 * self.heads * self.q_head * 2 > EXPANDED_BYTES):
+                    or self._expanded_bytes(total * EXPANDED_PAGE, int(counts.sum())) > EXPANDED_BYTES):
                 return
             table = np.full((len(counts), int(pages.max())), -1, dtype=np.int32)
             ends = np.cumsum(pages)
@@ -130,6 +134,9 @@ class LatentAttention(Mixer):
 
         plan.tells_fresh_prompts = True  # the runner keeps graphs of such steps apart
         return {("latent_plan", self._expanded_key()): plan}
+
+    def _expanded_bytes(self, slots: int, tokens: int) -> int:
+        return 2 * (slots * 2 * self.heads * self.q_head + tokens * (self.heads * (self.head_dim + self.value_dim) + self.record))
 
     def _expanded_key(self) -> str:
         return f"latent_{self.heads}_{self.q_head}"
