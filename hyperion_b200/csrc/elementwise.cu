@@ -486,13 +486,26 @@ __global__ void rope_kv_store_kernel(T* __restrict__ x, int stride, int q_heads,
 // 16-byte stores) or copies 8 values; same arithmetic per element as the scalar kernel.  A thread that takes its piece through four tokens, all asked for
 // at once, is faster only where the rows come from memory (2,048 tokens of 28 + 4 + 4 heads of 128: 15.5 -> 14.1 us); behind the product that made them they lie
 // in L2: 8.5 us here and 9.5 so (16 + 4 + 4 heads: 5.9 and 8.2).
+// AHEAD: a step of few tokens, one round trip to memory long, takes its cosines and sines in 16-byte pieces beside the entries (a token of the smallest model 664.7 -> 661.8 us, with the divisions
+// before the wait); prompts lose by the registers that takes (1,531 tokens of 28 + 4 + 4 heads of 128: 6.8 and 7.9 us).  The same arithmetic.
+template <bool AHEAD>
 __global__ void rope_kv_store_bf16x8_kernel(__nv_bfloat16* __restrict__ x, int stride, int q_heads, int kv_heads, int head_dim,
                                             const int* __restrict__ positions, const float2* __restrict__ table, int max_positions,
                                             __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, int table_width,
                                             const int* __restrict__ token_row, int page_size, int pages, int* status) {
     const int t = blockIdx.x;
     const int half = head_dim >> 1, chunks = half >> 3;  // 8-pair chunks per head
+    const int rotated = (q_heads + kv_heads) * chunks;
+    const int total = rotated + kv_heads * 2 * chunks;  // values: head_dim / 8 chunks per head
     let_next_kernel_start();
+    // the divisions that find a thread's first piece are done while the kernel before still runs
+    int e = blockIdx.y * blockDim.x + threadIdx.x, head, i;
+    auto find_piece = [&]() {
+        const bool turns = e < rotated;
+        head = turns ? e / chunks : (e - rotated) / (2 * chunks);
+        i = (turns ? e - head * chunks : e - rotated - head * 2 * chunks) * 8;
+    };
+    find_piece();
     const int pos = positions[t];  // positions and tables come with the step's one copy from the host, not from a kernel
     const bool pos_ok = pos >= 0 && pos < max_positions;
     const int block = pos_ok ? pos / page_size : 0;
@@ -508,21 +521,25 @@ __global__ void rope_kv_store_bf16x8_kernel(__nv_bfloat16* __restrict__ x, int s
     __nv_bfloat16* row = x + (size_t)t * stride;
     const float2* cs = table + (size_t)pos * half;
     const size_t page_base = (size_t)(page_ok ? page : 0) * 2 * kv_heads * page_size * head_dim;
-    const int rotated = (q_heads + kv_heads) * chunks;
-    const int total = rotated + kv_heads * 2 * chunks;  // values: head_dim / 8 chunks per head
-    for (int e = blockIdx.y * blockDim.x + threadIdx.x; e < total; e += gridDim.y * blockDim.x) {
+    while (e < total) {
         if (e < rotated) {
-            const int head = e / chunks, i = (e - head * chunks) * 8;
             __nv_bfloat16* p = row + head * head_dim + i;
             const uint4 lo4 = *reinterpret_cast<const uint4*>(p), hi4 = *reinterpret_cast<const uint4*>(p + half);
             const __nv_bfloat16* lo = reinterpret_cast<const __nv_bfloat16*>(&lo4);
             const __nv_bfloat16* hi = reinterpret_cast<const __nv_bfloat16*>(&hi4);
+            float2 turn[8];
+#pragma unroll
+            for (int j = 0; j < (AHEAD ? 8 : 0); j += 2) {
+                const float4 two = *reinterpret_cast<const float4*>(cs + i + j);
+                turn[j] = make_float2(two.x, two.y);
+                turn[j + 1] = make_float2(two.z, two.w);
+            }
             uint4 out_lo, out_hi;
             __nv_bfloat16* y1 = reinterpret_cast<__nv_bfloat16*>(&out_lo);
             __nv_bfloat16* y2 = reinterpret_cast<__nv_bfloat16*>(&out_hi);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const float2 c = cs[i + j];
+                const float2 c = AHEAD ? turn[j] : cs[i + j];
                 const float x1 = __bfloat162float(lo[j]), x2 = __bfloat162float(hi[j]);
                 y1[j] = __float2bfloat16_rn(x1 * c.x - x2 * c.y);
                 y2[j] = __float2bfloat16_rn(x2 * c.x + x1 * c.y);
@@ -536,10 +553,11 @@ __global__ void rope_kv_store_bf16x8_kernel(__nv_bfloat16* __restrict__ x, int s
                 *reinterpret_cast<uint4*>(dst + half) = out_hi;
             }
         } else if (page_ok) {
-            const int f = e - rotated, head = f / (2 * chunks), i = (f - head * 2 * chunks) * 8;
             const uint4 v = *reinterpret_cast<const uint4*>(row + (q_heads + kv_heads + head) * head_dim + i);
             *reinterpret_cast<uint4*>(cache + page_base + (((size_t)(kv_heads + head)) * page_size + slot) * head_dim + i) = v;
         }
+        e += gridDim.y * blockDim.x;
+        if (e < total) find_piece();
     }
 }
 
@@ -548,14 +566,18 @@ HB_EXPORT int hb_rope_kv_store(void* x, int is_bf16, int tokens, int stride, int
                                int table_width, const int* token_row, int page_size, int pages, int* status, cudaStream_t stream) {
     if (tokens <= 0) return 0;
     if (head_dim & 1) return HB_UNSUPPORTED_SIZE;
-    if (is_bf16 && head_dim % 16 == 0 && stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)cache) & 15) == 0) {
+    if (is_bf16 && head_dim % 16 == 0 && stride % 8 == 0 && (((uintptr_t)x | (uintptr_t)cache | (uintptr_t)table) & 15) == 0) {
         // Up to 1,023 tokens a thread for every piece, in as many even blocks a token as that takes (28 + 4 + 4 heads of 128, in us: 8 tokens 1.53, 512 tokens 3.4; a loop over the pieces in up to eight
         // blocks of 128 or 256 threads a token 1.66 and 3.9).  From there on one block a token that loops: blocks come and go half as often (32 + 32 + 32 heads, 1,531 tokens 13.1 and 15.5).
         const int items = (q_heads + 3 * kv_heads) * (head_dim / 16);  // pairs of eight entries, and the values' eights
         const int across = tokens < 1024 ? (items + 255) / 256 : 1;
         const int threads = tokens < 1024 ? ((items + across - 1) / across + 31) / 32 * 32 : ((q_heads + 2 * kv_heads) * (head_dim / 16) >= 256 ? 256 : 128);
         const dim3 grid8(tokens, across < 65535 ? across : 65535);
-        return launch_after_previous(rope_kv_store_bf16x8_kernel, grid8, threads, 0, stream, (__nv_bfloat16*)x, stride, q_heads, kv_heads, head_dim,
+        if (tokens < 256)
+            return launch_after_previous(rope_kv_store_bf16x8_kernel<true>, grid8, threads, 0, stream, (__nv_bfloat16*)x, stride, q_heads, kv_heads, head_dim,
+                                         positions, (const float2*)table, max_positions, (__nv_bfloat16*)cache, block_table, table_width, token_row,
+                                         page_size, pages, status);
+        return launch_after_previous(rope_kv_store_bf16x8_kernel<false>, grid8, threads, 0, stream, (__nv_bfloat16*)x, stride, q_heads, kv_heads, head_dim,
                                      positions, (const float2*)table, max_positions, (__nv_bfloat16*)cache, block_table, table_width, token_row,
                                      page_size, pages, status);
     }
