@@ -18,8 +18,9 @@
 // share the key tiles and meet only where a tile changes hands: 222 us; 471 -> 353 us at 2,048 tokens, 963 -> 705 us with 32 heads; 1,000 tokens beside seven decoded ones
 // behind 1,500: 144 -> 107 us (a decoded token leaves the block's second set without rows: it only copies).
 // With splits > 1 a block walks only its share of the key tiles and leaves an unnormalised result with its maximum and sum in a
-// workspace; a second kernel merges the shares.  A row's result depends on the positions of the key tiles only, never on how the
-// request was cut into steps or on the rest of the batch.
+// workspace; a second kernel merges the shares.  In this kernel a row's result depends on the positions of the key tiles only, never on how the
+// request was cut into steps or on the rest of the batch.  (Which steps come here does: one of nothing but long enough prompts from position 0 takes keys and values made per
+// head, with roundings of their own: parts/attention_latent.py.)
 #include "common.cuh"
 #include <type_traits>
 

@@ -27,7 +27,7 @@
 // half of the row's columns each:  o = a1 - lambda a2, o / sqrt(mean(o^2) + eps) * post * sigmoid(gate), exchanging what they need of one
 // another (1 / sum, the sum of squares) through shared memory.
 // Queries and keys may be wider than values (HB_KEY_DIM 192 over values of 128: attention over latents whose prompts' keys and values have been made per head); the
-// cache's rows are then as wide as a key and a value is its row's first entries.  1,531 tokens of 16 such heads: 51 us, 165 on mma.sync (attention_tma.cu), 225 over
+// cache's rows are then as wide as a key and a value is its row's first entries.  1,531 tokens of 16 such heads: 40 us in tiles of 128 rows, 51 of 256, 165 on mma.sync (attention_tma.cu), 225 over
 // the latents themselves (attention_latent.cu), which takes 3.4 times the operations.
 // Every mbarrier wait is bounded; a wait that runs out sets HB_STATUS_WAIT_EXPIRED, all roles leave their loops, the block
 // takes no further item, tensor memory is freed and the block returns.

@@ -514,10 +514,9 @@ __global__ void __launch_bounds__(512) gated_group_norm4_kernel(const float* __r
     }
 }
 
-// The same for groups of up to 1,024 columns: a warp per (token, group), four of them in a block; the lanes' partial sums
-// meet in a butterfly of fixed shape.
-// Groups of whole 16-byte pieces: a lane keeps its CHUNKS fours in registers, so that a row is read once and in 16-byte accesses, all of them asked for
-// before the sum (2,048 tokens of 16 groups of 128: 19.3 us column by column, 11.1 so).
+// Groups of up to 1,024 columns in whole 16-byte pieces: a warp per (token, group), four of them in a block; a lane keeps its CHUNKS fours in registers, so that a row is read
+// once and in 16-byte accesses, all of them asked for before the sum (2,048 tokens of 16 groups of 128: 19.3 us column by column, 11.1 so).  A lane adds up fours of neighbouring
+// columns where the kernel below adds up every 32nd: another order of the same float sum, in both element types.
 template <typename TO, int CHUNKS>
 __global__ void __launch_bounds__(128) gated_group_norm_warp4_kernel(const float* __restrict__ y, int y_stride, const float* __restrict__ gate, int gate_stride, int gate_off,
                                               const float* __restrict__ weight, int weight_len, int group, int groups, int gate_first, float eps, float scale,
@@ -564,6 +563,7 @@ __global__ void __launch_bounds__(128) gated_group_norm_warp4_kernel(const float
     }
 }
 
+// The same for any group of up to 1,024 columns: the lanes' partial sums meet in a butterfly of fixed shape.
 template <typename TO>
 __global__ void gated_group_norm_warp_kernel(const float* __restrict__ y, int y_stride, const float* __restrict__ gate, int gate_stride,
                                              int gate_off, const float* __restrict__ weight, int weight_len, int group, int groups, int gate_first,

@@ -109,7 +109,7 @@ def plan_prompts(rows, tokens_per_tile: int, blocks: int, most: float = 0.5) -> 
 
     A block that works on one half's 128 rows alone takes about 0.77 of the time per key tile.  With twice as many blocks and an SM for each that is the step's gain (1,000 tokens of 4
     key/value heads, 64 blocks: 49 -> 38 us, with a window 29 -> 25); where the tiles come back in a second turn it is lost, unless they differ in length as a whole prompt's do
-    (96 blocks of a 1,531-token prompt: 53 -> 40 us; 128 blocks of a 2,048-token one: 52 -> 60).  How far a tile's keys reach is not among what the captured steps are told apart by,
+    (96 blocks of a 1,531-token prompt: 51 -> 40 us; 128 blocks of a 2,048-token one: 52 -> 60).  How far a tile's keys reach is not among what the captured steps are told apart by,
     so the general rule asks for one turn."""
     tiles, items = plan(rows, tokens_per_tile)
     if tokens_per_tile >= 2 and len(tiles) and len(tiles) // 3 * blocks <= most * sm_count():
